@@ -156,7 +156,7 @@ def run_b200(args):
     if args.edge_source_sums:
         from fairchem_b200 import backbone as _bb
 
-        _bb._GemmState.node_sums = False
+        _bb._GemmState.node_sums = _bb._GemmState.native = False
     if args.generic_kernels:
         from fairchem_b200 import ops as _ops
 

@@ -74,6 +74,10 @@ SIGNATURES = {
     "fcb200_rg_neighbor_counts_static": [P, P, I32, I64, I64, P, P, I64, F32, P, P],
     "fcb200_gemm_tf32": [P, I64, P, P, I64, P, P, I64, I64, I32, I32, I32, P, P],
     "fcb200_split_tf32": [P, P, P, I64, P],
+    "fcb200_model_sizes": [P, P, P],
+    "fcb200_model_forward": [P, P, P],
+    "fcb200_model_energy": [P, P, P],
+    "fcb200_model_backward": [P, P, P],
 }
 
 ERRORS = {-1: "invalid argument (null pointer, negative size or unsupported shape)",
@@ -102,6 +106,7 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
         fn = getattr(lib, name)  # AttributeError here means header and library disagree
         fn.argtypes = argtypes
         fn.restype = ctypes.c_int
+    lib.fcb200_set_launch_hook.restype = None
     _lib = lib
     return lib
 

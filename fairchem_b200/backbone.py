@@ -30,7 +30,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import ops
+from . import ops, step
 from .graph import generate_graph, get_pbc_shifts
 from .ops import EdgeGraph
 
@@ -338,7 +338,8 @@ class _GemmState:
     split16 = {}           # same key -> (weight ref, half high part, half low part, scale)
     a_scale = None         # precision 2: one-element device tensor, the power of two A operands are scaled by (None = 1)
     fused_conv = True      # precision 2: one launch per SO(2) convolution with the gate in the epilogue
-    node_sums = True       # gather backward: both halves summed per node in the kernels (else source half per edge + segmented sum)
+    native = True          # whole evaluation from native code (fairchem_b200.step) where it applies; False: the per-op path
+    node_sums = True       # per-op path, gather backward: both halves summed per node in the kernels (else source half per edge + segmented sum)
 
 
 def set_gemm_precision(p: int) -> None:
@@ -359,7 +360,8 @@ class HalfRangeError(RuntimeError):
 
 def read_gemm_status() -> int:
     """The contraction kernels' device status word, read and cleared: 0 = fine, 1 = a bounded wait expired inside a
-    kernel, 2 = an operand or output left the half-precision range (precision 2 only)."""
+    kernel, 2 = an operand or output left the half-precision range (precision 2 only), 3 = charge, spin or atomic number
+    outside the embedding tables."""
     if _GemmState.status is None:
         return 0
     code = int(_GemmState.status.item())
@@ -371,6 +373,8 @@ def read_gemm_status() -> int:
 def raise_gemm_status(code: int) -> None:
     if code == 0:
         return
+    if code == 3:
+        raise ValueError("charge outside [-100, 100], spin outside [0, 100] or atomic number outside the embedding table")
     if code == 2:
         raise HalfRangeError("tcgen05 GEMM: an operand left the half-precision range; results are invalid "
                              "(use set_gemm_precision(3), or energy_forces(), which falls back by itself)")
@@ -1343,6 +1347,36 @@ class eSCNMDBackboneB200(nn.Module):
         with torch.enable_grad():
             return self._forward(data, gamma)
 
+    def _forward_native(self, data, gamma):
+        """The whole evaluation from native code (fairchem_b200.step); None when it does not apply."""
+        plan = step.ModelPlan.of(self)
+        pos = data["pos"]
+        if plan is None or pos.dtype != torch.float32 or not pos.is_cuda or pos.device != plan.device or pos.shape[0] == 0:
+            return None
+        z, batch, nsys = data["atomic_numbers"], data["batch"], len(data["natoms"])
+        edge_index, cell_offsets = self._graph(data)
+        data["scatter_target"] = edge_index[1]
+        if edge_index.shape[1] == 0:  # isolated atoms: see _forward
+            edge_index = torch.zeros(2, 1, dtype=torch.long, device=pos.device)
+            cell_offsets = torch.zeros(1, 3, dtype=pos.dtype, device=pos.device)
+            shift = torch.tensor([[self.cutoff, 0.0, 0.0]], dtype=pos.dtype, device=pos.device)
+        else:
+            edge_sys = None if data["cell"].shape[0] == 1 else batch[edge_index[1]]
+            shift = get_pbc_shifts(data["cell"].to(pos.dtype), cell_offsets, edge_sys).contiguous()
+        self.last_graph = {"edge_index": edge_index, "cell_offsets": cell_offsets}
+        graph = step.StepGraph.from_edges(edge_index[0], edge_index[1], pos.shape[0], self.edge_chunk_size)
+        want_grad = torch.is_grad_enabled() and pos.requires_grad
+        run = step.BackboneStep(plan, pos.detach().contiguous(), graph, z.to(torch.int32), batch.to(torch.int32),
+                                plan.dataset_index(self, data["dataset"]), data["charge"].long().contiguous(),
+                                data["spin"].long().contiguous(), shift, None if gamma is None else gamma.contiguous(), nsys, want_grad,
+                                self.regress_stress, _status(pos.device))
+        if not run.plan_memory():
+            return None
+        run.virial = {"num_systems": nsys} if self.regress_stress else None
+        x = step.BackboneFn.apply(pos, run)
+        run.embedding = x
+        return {"node_embedding": x, "batch": batch, "virial": run.virial, "step": run}
+
     def _forward(self, data, gamma):
         from .parallel import halo_collect
 
@@ -1354,6 +1388,10 @@ class eSCNMDBackboneB200(nn.Module):
         if (self.regress_forces or self.regress_stress) and not self.direct_forces:
             pos.requires_grad_(True)
         c, nb = self.sphere_channels, self.num_distance_basis
+        if data.get("gp_plan", None) is None:
+            out = self._forward_native(data, gamma)
+            if out is not None:
+                return out
         csd = self.csd_embedding(data["charge"], data["spin"], data.get("dataset", None))
 
         # graph-parallel run: this rank owns plan.node_partition and reads plan.halo_ids from its peers
@@ -1421,9 +1459,36 @@ class MLP_EFS_HeadB200(nn.Module):
         self.energy_block = nn.Sequential(nn.Linear(c, h), nn.SiLU(), nn.Linear(h, h), nn.SiLU(), nn.Linear(h, 1))
         self.regress_forces, self.regress_stress = backbone.regress_forces, backbone.regress_stress
 
+    def _forward_native(self, data, emb):
+        """Energy and forces straight from the evaluation that made ``emb`` (no autograd graph in between)."""
+        run = emb.get("step", None)
+        if run is None or run.keep is None or emb["node_embedding"] is not run.embedding or run.embedding._version != 0:
+            return None
+        want = self.regress_forces or self.regress_stress
+        model = run.plan.with_head(self)
+        if model is None or (want and not run.ev.want_grad):
+            return None
+        out = {"energy": run.energy(model)}
+        if want:
+            out["forces"] = run.backward(model, None, -1.0)
+        if self.regress_stress:
+            out["stress"] = self._stress(data, run.virial["virial"])
+        return out
+
+    @staticmethod
+    def _stress(data, w):
+        # stress = sym(sum_e dE/dvec_e (x) vec_e) / volume, flattened [B,9] as the reference returns it
+        volume = torch.det(data["cell"].double()).abs().view(-1, 1, 1)
+        return ((w + w.transpose(1, 2)) / 2 / volume).reshape(-1, 9)
+
     def forward(self, data, emb, check_status: bool = True):
         """``check_status=False`` leaves the contraction status word unread: a graph-parallel caller must first agree
         on it with its peers (a rank that raised alone would leave the others waiting in the next collective)."""
+        out = self._forward_native(data, emb)
+        if out is not None:
+            if check_status:
+                check_gemm_status()
+            return out
         with torch.enable_grad():
             eb = self.energy_block
             h = emb["node_embedding"][:, 0]
@@ -1437,10 +1502,7 @@ class MLP_EFS_HeadB200(nn.Module):
                 (grad,) = torch.autograd.grad(energy.sum(), data["pos"], create_graph=False)
                 out["forces"] = -grad
             if self.regress_stress:
-                # stress = sym(sum_e dE/dvec_e (x) vec_e) / volume, flattened [B,9] as the reference returns it
-                w = emb["virial"]["virial"]
-                volume = torch.det(data["cell"].double()).abs().view(-1, 1, 1)
-                out["stress"] = ((w + w.transpose(1, 2)) / 2 / volume).reshape(-1, 9)
+                out["stress"] = self._stress(data, emb["virial"]["virial"])
             if check_status:
                 check_gemm_status()
         return out

@@ -6,6 +6,13 @@
 
 namespace fcb200 {
 
+__host__ __device__ constexpr double csqrt(double x) {
+    if (x <= 0.0) return 0.0;
+    double g = x > 1.0 ? x : 1.0;
+    for (int i = 0; i < 64; ++i) g = 0.5 * (g + x / g);
+    return g;
+}
+
 template <int LMAX> struct Shape {
     static constexpr int kL = (LMAX + 1) * (LMAX + 1);
     __host__ __device__ static constexpr int mm(int l) { return l < 2 ? l : 2; }

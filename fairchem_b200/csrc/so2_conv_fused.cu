@@ -36,7 +36,8 @@ enum Mode : int32_t {
     kSiluBwd = 4,   // planes[:, out_col ...] = split(v * d/dy silu(y[:, y_col ...]))
     kGatedBwd = 5,  // planes[:, out_col ...] = split(v * sigmoid(gate)); gate gradient summed over consecutive tiles
 };
-enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4 };
+// kGateSilu: the gate is sigmoid(silu(g)), the scalar MLP of the node-wise feed-forward, instead of sigmoid(g)
+enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8 };
 
 struct Tile {
     int32_t a_col;     // first input column of this tile's K range
@@ -245,6 +246,7 @@ __device__ __forceinline__ void epilogue(const CUtensorMap& map_y, const CUtenso
             const uint32_t acc_t = tmem_base + (uint32_t)(buf * kAccCols) + ((uint32_t)(q * 32) << 16);
             const int mode = t.mode;
             const bool keep = (t.flags & kKeep) != 0 && (mode == kSilu || mode == kGated);
+            const bool gate_silu = (t.flags & kGateSilu) != 0;
             const bool fin = mode == kGatedBwd && (t.flags & kLast) != 0;
             const int n_in = mode == kGatedBwd ? 2 : ((mode == kGated || mode == kSiluBwd) ? 1 : 0);
 #pragma unroll
@@ -328,7 +330,7 @@ __device__ __forceinline__ void epilogue(const CUtensorMap& map_y, const CUtenso
                             float g[8];
                             ld_row8(b0, lane, u, g);
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) o[i] = v[8 * u + i] * sigmoid_f(g[i]) * o_scale;
+                            for (int i = 0; i < 8; ++i) o[i] = v[8 * u + i] * sigmoid_f(gate_silu ? g[i] * sigmoid_f(g[i]) : g[i]) * o_scale;
                         } else if (mode == kSiluBwd) {
                             float y0[8];
                             ld_row8(b0, lane, u, y0);
@@ -343,11 +345,17 @@ __device__ __forceinline__ void epilogue(const CUtensorMap& map_y, const CUtenso
                             ld_row8(b1, lane, u, yr);
 #pragma unroll
                             for (int i = 0; i < 8; ++i) {
+                                float slope = 1.f;
+                                if (gate_silu) {
+                                    const float sg = sigmoid_f(g[i]);
+                                    slope = sg * (1.f + g[i] * (1.f - sg));
+                                    g[i] *= sg;
+                                }
                                 g[i] = sigmoid_f(g[i]);
                                 o[i] = v[8 * u + i] * g[i] * o_scale;
                                 const float prev = (t.flags & kFirst) ? 0.f : acc[c2][8 * u + i];
                                 acc[c2][8 * u + i] = fmaf(v[8 * u + i], yr[i], prev);
-                                if (fin) acc[c2][8 * u + i] *= g[i] * (1.f - g[i]) * o_scale;
+                                if (fin) acc[c2][8 * u + i] *= slope * g[i] * (1.f - g[i]) * o_scale;
                             }
                         }
                         stage_split8(st_out, st_out + 2048u, lane, u, o, amax);

@@ -10,7 +10,7 @@ library; there is no CPU implementation.
 from __future__ import annotations
 
 import math
-from ctypes import c_float, c_int32, c_int64, c_void_p
+from ctypes import CFUNCTYPE, c_char_p, c_float, c_int32, c_int64, c_void_p
 from typing import List, Optional
 
 import torch
@@ -100,6 +100,20 @@ class LaunchProfiler:
         end.record()
         self.records.append((name, start, end, nbytes, flops, launches))
 
+    def native(self, name, begin, nbytes, flops, launches):
+        """Launch hook of the whole-model evaluation (fcb200_set_launch_hook): called before and after each launch."""
+        if begin:
+            self._start = None
+            if self.timed:
+                self._start = torch.cuda.Event(enable_timing=True)
+                self._start.record()
+            return
+        end = None
+        if self.timed:
+            end = torch.cuda.Event(enable_timing=True)
+            end.record()
+        self.records.append((name.decode(), self._start, end, nbytes, flops, launches))
+
     def summary(self) -> dict:
         torch.cuda.synchronize()
         out = {}
@@ -118,11 +132,15 @@ class LaunchProfiler:
 
 
 _PROFILER: Optional[LaunchProfiler] = None
+_NATIVE_HOOK = None  # keeps the callback the library holds alive
 
 
 def set_profiler(p: Optional[LaunchProfiler]) -> None:
-    global _PROFILER
+    global _PROFILER, _NATIVE_HOOK
     _PROFILER = p
+    hook = CFUNCTYPE(None, c_char_p, c_int32, c_int64, c_int64, c_int32)
+    _NATIVE_HOOK = hook() if p is None else hook(p.native)
+    _lib.load().fcb200_set_launch_hook(_NATIVE_HOOK)
 
 
 def _launch(name: str, cname: str, args, nbytes: int = 0, flops: int = 0, launches: int = 1) -> None:

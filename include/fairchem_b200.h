@@ -552,6 +552,84 @@ int fcb200_lx_edge_geometry_bwd(const float* pos, const int32_t* src, const int3
                                 int32_t num_basis, float basis_start, float basis_stop, float basis_width,
                                 int64_t num_edges, int64_t num_nodes, int32_t lmax, void* stream);
 
+/* ---------------------------------------------------------------- whole-model evaluation */
+
+/*
+ * One energy(+forces) evaluation of the eSCN-MD backbone (src/fairchem/core/models/uma/escn_md.py:700-905) and its
+ * energy head (escn_md.py:1062-1168) issued from native code: every launch of both passes, no host work between them.
+ * Channels (sphere, hidden, edge) are 128, lmax is 2 or 4, mmax 2; contractions run with half-split operands.
+ * The structs hold DEVICE pointers unless a comment says otherwise.
+ */
+typedef struct { /* half-split matrix [rows, cols] = (hi + lo 2^-11) / scale, see fcb200_split_f16 */
+    const void *hi, *lo;
+    float scale;
+    int32_t rows, cols;
+} fcb200_weight;
+
+typedef struct {
+    fcb200_weight conv1[3], conv1_t[3], conv2[3], conv2_t[3]; /* m-blocks in block form, and their transposes */
+    fcb200_weight radial_out, radial_out_t;                   /* [3 lmax 256, 128] */
+    fcb200_weight ffn_in;    /* [gates lmax*128 | degree 0 | degree 1 | ...] x 128 */
+    fcb200_weight ffn_in_t0; /* 128 x [gates | degree 0] */
+    fcb200_weight ffn_in_t;  /* degrees 1.. transposed, stacked: [lmax*128, 128] */
+    fcb200_weight ffn_out, ffn_out_t; /* degrees stacked: [(lmax+1)*128, 128] */
+    const float *conv1_bias, *conv2_bias, *radial_out_bias, *ffn_in_bias, *ffn_out_bias;
+    const float *norm1_w, *norm1_b, *norm2_w, *norm2_b;
+    float eps1, eps2;
+} fcb200_layer;
+
+typedef struct {
+    int32_t lmax, num_layers, num_basis, num_elements;
+    float cutoff, basis_start, basis_stop, basis_width, rescale, radial_eps, norm_eps;
+    const fcb200_layer* layers; /* HOST array */
+    /* the hidden layers of the num_layers + 1 radial MLPs (the edge-degree embedding's last) side by side */
+    fcb200_weight rad_w0, rad_w1, rad_w1_t, rad_w0_t; /* [nets*128, num_basis], [nets*128, 128] x 2, [num_basis, nets*128] */
+    const float *rad_b0, *rad_b1, *ln1_w, *ln1_b, *ln2_w, *ln2_b;
+    const float *table_src, *table_tgt; /* [num_elements, nets*128] */
+    fcb200_weight degree_out, degree_out_t;
+    const float* degree_out_bias;
+    const float *element_emb, *norm_w, *norm_b;
+    const float *charge_emb, *spin_emb, *dataset_emb, *csd_w_t, *csd_b; /* csd_w_t [384, 128] */
+    /* energy head; absent when head_w3 is null */
+    fcb200_weight head_w1, head_w1_t, head_w2, head_w2_t;
+    const float *head_b1, *head_b2, *head_w3, *head_b3, *head_scale;
+} fcb200_model;
+
+typedef struct {
+    int64_t num_nodes, num_edges;
+    int32_t num_systems, num_chunks;
+    int32_t want_grad;   /* keep what the backward pass needs */
+    int32_t keep_radial; /* also keep the radial weights (else recomputed per chunk) */
+    const float *pos, *shift, *gamma; /* [N,3]; [E,3] or null; [E] or null */
+    const int32_t *src, *tgt, *row_ptr, *src_ptr, *src_perm;
+    const int32_t* chunk_src; /* [(num_chunks+1), N]: per node, first position of src_perm with an edge id >= the chunk's first
+                                 edge; null with one chunk */
+    const int32_t *z, *batch, *dataset; /* [N], [N], [num_systems] */
+    const int64_t *charge, *spin;       /* [num_systems] */
+    const int64_t *chunk_node, *chunk_edge; /* HOST arrays [num_chunks+1] */
+    void *keep, *scratch; /* 1024-byte aligned, sizes from fcb200_model_sizes */
+    float* x_out;         /* [N, (lmax+1)^2, 128] */
+    double* energy;       /* [num_systems], zeroed by the caller */
+    const float* grad_x;  /* backward without the head: gradient of x_out */
+    float* grad_pos;      /* [N,3], times grad_sign */
+    float grad_sign;      /* +1: gradient, -1: forces */
+    double* virial;       /* [num_systems, 9], zeroed by the caller, or null */
+    int32_t* status;      /* raised to 1 / 2 as by the contractions, 3: charge or spin outside the embedding tables */
+} fcb200_eval;
+
+/* bytes of keep, and of scratch in the forward and in the backward pass */
+int fcb200_model_sizes(const fcb200_model* model_host, const fcb200_eval* eval_host, int64_t* sizes_host);
+int fcb200_model_forward(const fcb200_model* model_host, const fcb200_eval* eval_host, void* stream);
+/* energy of the evaluation that filled keep (after fcb200_model_forward) */
+int fcb200_model_energy(const fcb200_model* model_host, const fcb200_eval* eval_host, void* stream);
+/* grad_pos (and virial): from the sum of the energies (grad_x null) or from a gradient of x_out */
+int fcb200_model_backward(const fcb200_model* model_host, const fcb200_eval* eval_host, void* stream);
+
+/* Called around every kernel (or group of kernels) of the functions above, on the host: begin = 1 before, 0 after.
+ * For accounting; null removes it. */
+typedef void (*fcb200_launch_hook)(const char* name, int32_t begin, int64_t bytes, int64_t flops, int32_t launches);
+void fcb200_set_launch_hook(fcb200_launch_hook hook);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,101 @@
+"""Whole-model native evaluation (csrc/model_step.cu) against the per-op path, at the sizes where its dispatch changes:
+one atom without neighbours, ragged row tiles, node counts on both sides of the shared-node kernels, several chunks."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "one_atom": (lambda s: s.molecule_batch(1, 1, 1, seed=1), {}),
+    "molecule_9": (lambda s: s.molecule_batch(1, 9, 9, seed=2), {}),
+    "molecules_7": (lambda s: s.molecule_batch(7, 3, 31, seed=3), {}),
+    "fcc_32_chunks": (lambda s: s.fcc_cu((2, 2, 2), seed=4), {"edge_chunk_size": 257}),
+    "alloy_stress": (lambda s: s.bcc_alloy((3, 4, 5), seed=5), {"regress_stress": True}),
+    "water_2200": (lambda s: s.water_box(2200, seed=6), {"edge_chunk_size": 30000}),
+    "batch_stress": (lambda s: s.merge([s.fcc_cu((2, 2, 2), seed=1), s.bcc_alloy((2, 3, 2), seed=2)]), {"regress_stress": True}),
+}
+
+
+def _model(B, cfg_name, **kw):
+    from fairchem_b200 import weights
+
+    cfg = getattr(weights, cfg_name)
+    if cfg_name == "ESCN_MD_L4":
+        cfg = dict(cfg, num_layers=2)
+    return B.build_model(cfg, weights.random_init_state_dict(cfg, 0), device="cuda", **kw)
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-12))
+
+
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+@pytest.mark.parametrize("name", list(CASES))
+def test_native_evaluation_matches_per_op_path(cfg, name):
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    make, kw = CASES[name]
+    bb, head = _model(B, cfg, **kw)
+    data = make(synthetic).to("cuda")
+    out = {}
+    for native in (True, False):
+        B._GemmState.native = native
+        try:
+            d = data.clone()
+            emb = bb(d)
+            assert ("step" in emb) == native
+            out[native] = head(d, emb)
+        finally:
+            B._GemmState.native = True
+    assert set(out[True]) == set(out[False])
+    # energies are sums of per-atom terms of order 0.1 that may cancel
+    e, ref = out[True]["energy"], out[False]["energy"]
+    assert bool(((e - ref).abs() < 5e-6 * ref.abs().clamp_min(0.1 * len(data.pos))).all())
+    f = out[False]["forces"]
+    if float(f.abs().max()) > 1e-6:
+        assert _rel(out[True]["forces"], f) < 2e-5
+    if "stress" in out[True]:
+        assert _rel(out[True]["stress"], out[False]["stress"]) < 5e-5
+
+
+def test_gradient_of_the_node_embedding_and_repeated_use():
+    """The embedding is differentiable on its own, an energy-only model keeps nothing, and a released evaluation says so."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S")
+    data = synthetic.molecule_batch(3, 5, 12, seed=9).to("cuda")
+    grads = []
+    weight = None
+    for native in (True, False):
+        B._GemmState.native = native
+        try:
+            d = data.clone()
+            x = bb(d)["node_embedding"]
+            weight = torch.randn(x.shape, generator=torch.Generator("cuda").manual_seed(1), device="cuda") if weight is None else weight
+            grads.append(torch.autograd.grad((x * weight).sum(), d["pos"])[0])
+        finally:
+            B._GemmState.native = True
+    assert _rel(grads[0], grads[1]) < 2e-5
+    d = data.clone()
+    emb = bb(d)
+    first = head(d, emb)
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(emb["node_embedding"].sum(), d["pos"])
+    bb2, head2 = _model(B, "UMA_S", regress_forces=False)
+    d = data.clone()
+    out = head2(d, bb2(d))
+    assert set(out) == {"energy"} and _rel(out["energy"], first["energy"]) < 1e-6
+
+
+def test_out_of_table_charge_is_an_error():
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S")
+    d = synthetic.molecule_batch(2, 5, 5, seed=1).to("cuda")
+    d["charge"] = torch.tensor([0, 400], device="cuda")
+    with pytest.raises(ValueError):
+        head(d, bb(d))
