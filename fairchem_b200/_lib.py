@@ -74,6 +74,9 @@ SIGNATURES = {
     "fcb200_rg_neighbor_counts_static": [P, P, I32, I64, I64, P, P, I64, F32, P, P],
     "fcb200_gemm_tf32": [P, I64, P, P, I64, P, P, I64, I64, I32, I32, I32, P, P],
     "fcb200_split_tf32": [P, P, P, I64, P],
+    "fcb200_graph_systems": [P, P],
+    "fcb200_graph_select": [P, P],
+    "fcb200_graph_fill": [P, P],
     "fcb200_model_sizes": [P, P, P],
     "fcb200_model_forward": [P, P, P],
     "fcb200_model_energy": [P, P, P],

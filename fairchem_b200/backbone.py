@@ -1353,29 +1353,29 @@ class eSCNMDBackboneB200(nn.Module):
         pos = data["pos"]
         if plan is None or pos.dtype != torch.float32 or not pos.is_cuda or pos.device != plan.device or pos.shape[0] == 0:
             return None
-        z, batch, nsys = data["atomic_numbers"], data["batch"], len(data["natoms"])
-        edge_index, cell_offsets = self._graph(data)
-        data["scatter_target"] = edge_index[1]
-        if edge_index.shape[1] == 0:  # isolated atoms: see _forward
-            edge_index = torch.zeros(2, 1, dtype=torch.long, device=pos.device)
-            cell_offsets = torch.zeros(1, 3, dtype=pos.dtype, device=pos.device)
-            shift = torch.tensor([[self.cutoff, 0.0, 0.0]], dtype=pos.dtype, device=pos.device)
+        status = _status(pos.device)
+        graph = step.StepGraph(self, data, status, torch.is_grad_enabled() and pos.requires_grad)
+        if self.otf_graph and not self.always_use_pbc and graph.build():
+            edge_index, cell_offsets = graph.edge_index, graph.cell_offsets
         else:
-            edge_sys = None if data["cell"].shape[0] == 1 else batch[edge_index[1]]
-            shift = get_pbc_shifts(data["cell"].to(pos.dtype), cell_offsets, edge_sys).contiguous()
+            edge_index, cell_offsets = self._graph(data)
+            if edge_index.shape[1] == 0:  # isolated atoms: see _forward
+                edge_index = torch.zeros(2, 1, dtype=torch.long, device=pos.device)
+                cell_offsets = torch.zeros(1, 3, dtype=pos.dtype, device=pos.device)
+                graph.from_edges(edge_index[0], edge_index[1], torch.tensor([[self.cutoff, 0.0, 0.0]], dtype=pos.dtype, device=pos.device))
+            else:
+                edge_sys = None if data["cell"].shape[0] == 1 else data["batch"][edge_index[1]]
+                graph.from_edges(edge_index[0], edge_index[1], get_pbc_shifts(data["cell"].to(pos.dtype), cell_offsets, edge_sys).contiguous())
+        data["scatter_target"] = edge_index[1]
         self.last_graph = {"edge_index": edge_index, "cell_offsets": cell_offsets}
-        graph = step.StepGraph.from_edges(edge_index[0], edge_index[1], pos.shape[0], self.edge_chunk_size)
-        want_grad = torch.is_grad_enabled() and pos.requires_grad
-        run = step.BackboneStep(plan, pos.detach().contiguous(), graph, z.to(torch.int32), batch.to(torch.int32),
-                                plan.dataset_index(self, data["dataset"]), data["charge"].long().contiguous(),
-                                data["spin"].long().contiguous(), shift, None if gamma is None else gamma.contiguous(), nsys, want_grad,
-                                self.regress_stress, _status(pos.device))
+        run = step.BackboneStep(plan, graph, plan.dataset_index(self, data["dataset"]), data["charge"], data["spin"], gamma,
+                                self.regress_stress, status)
         if not run.plan_memory():
             return None
-        run.virial = {"num_systems": nsys} if self.regress_stress else None
+        run.virial = {"num_systems": graph.systems} if self.regress_stress else None
         x = step.BackboneFn.apply(pos, run)
         run.embedding = x
-        return {"node_embedding": x, "batch": batch, "virial": run.virial, "step": run}
+        return {"node_embedding": x, "batch": data["batch"], "virial": run.virial, "step": run}
 
     def _forward(self, data, gamma):
         from .parallel import halo_collect

@@ -92,7 +92,9 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
     const bool keep = ev.want_grad != 0;
     // per-edge tensors that only the backward pass reads shrink to one chunk when there is none; row counts of the large
     // ones are rounded up so that a slowly changing edge count (molecular dynamics) asks for the same block every step
-    const int64_t unit = e > (1 << 20) ? 65536 : 4096, er = (e + unit - 1) / unit * unit, ek = keep ? er : ec;
+    int64_t unit = 1024;  // 1/64 to 1/32 of the edges
+    while (unit * 64 < e) unit *= 2;
+    const int64_t er = (e + unit - 1) / unit * unit, ek = keep ? er : ec;
     Arena k{static_cast<char*>(ev.keep)};
     L.vec = k.take<float4>(er);
     L.wig = k.take<float>(er * d.nw);
@@ -686,6 +688,8 @@ static int check(const fcb200_model* m, const fcb200_eval* e) {
     if (m->num_layers + 1 > 40 || e->num_nodes < 1 || e->num_edges < 1 || e->num_systems < 1 || e->num_chunks < 1 || !e->chunk_node || !e->chunk_edge)
         return FCB200_EINVAL;
     if (e->chunk_edge[0] != 0 || e->chunk_edge[e->num_chunks] != e->num_edges || e->chunk_node[e->num_chunks] != e->num_nodes) return FCB200_EINVAL;
+    for (int c = 0; c < e->num_chunks; ++c)
+        if (e->chunk_edge[c + 1] <= e->chunk_edge[c] || e->chunk_node[c + 1] <= e->chunk_node[c]) return FCB200_EINVAL;
     return FCB200_OK;
 }
 static int check_call(const fcb200_model* m, const fcb200_eval* e) {

@@ -222,6 +222,7 @@ class SkinNeighborList:
         self.cutoff, self.max_neighbors, self.skin = float(cutoff), int(max_neighbors), float(skin)
         self._cand = self._pos0 = self._cell0 = self._natoms0 = self._pbc0 = None
         self._key = None
+        self.origin = None  # device copies of what the list was built for, for the native evaluation's own check
         self.searches = self.refreshes = 0
 
     @staticmethod
@@ -245,17 +246,23 @@ class SkinNeighborList:
         return float(moved) <= (0.5 * self.skin) ** 2
 
     @torch.no_grad()
+    def search(self, data, pbc=None) -> None:
+        """New candidate list at the current positions."""
+        self._cand = _search(data, self.cutoff + self.skin, pbc)
+        self._pos0 = data.pos.detach().float().clone()
+        self._cell0 = data.cell.detach().clone()
+        self._natoms0 = data.natoms.tolist()
+        self._pbc0 = self._pbc_of(data, pbc)
+        self._key = (int(data.pos.shape[0]), tuple(int(v) for v in data.natoms.shape), data.pos.device,
+                     None if getattr(data, "node_partition", None) is None else int(data.node_partition.shape[0]))
+        self.origin = None
+        self.searches += 1
+
+    @torch.no_grad()
     def update(self, data, pbc=None):
         """(edge_index, cell_offsets, neighbors) at the current positions of ``data``."""
         if not self._reusable(data, pbc):
-            self._cand = _search(data, self.cutoff + self.skin, pbc)
-            self._pos0 = data.pos.detach().float().clone()
-            self._cell0 = data.cell.detach().clone()
-            self._natoms0 = data.natoms.tolist()
-            self._pbc0 = self._pbc_of(data, pbc)
-            self._key = (int(data.pos.shape[0]), tuple(int(v) for v in data.natoms.shape), data.pos.device,
-                         None if getattr(data, "node_partition", None) is None else int(data.node_partition.shape[0]))
-            self.searches += 1
+            self.search(data, pbc)
             if self.skin == 0.0:
                 return _select(self._cand, self.max_neighbors)
         else:

@@ -199,26 +199,24 @@ def _stream():
 class BackboneStep:
     """One evaluation: graph arrays, outputs and the memory that the backward pass reads."""
 
-    def __init__(self, plan: ModelPlan, pos, graph, z, batch, dataset, charge, spin, shift, gamma, num_systems: int, want_grad: bool,
-                 want_virial: bool, status):
+    def __init__(self, plan: ModelPlan, graph: "StepGraph", dataset, charge, spin, gamma, want_virial: bool, status):
         self.plan, self.model = plan, plan.model
-        dev = pos.device
-        self.nodes, self.systems = pos.shape[0], num_systems
-        e = self.ev = EvalStruct()
-        e.num_nodes, e.num_edges, e.num_systems = self.nodes, graph.num_edges, num_systems
-        e.num_chunks, e.want_grad = graph.num_chunks, int(want_grad)
-        self.refs = [pos, graph, z, batch, dataset, charge, spin, shift, gamma, status]
-        e.pos, e.z, e.batch, e.dataset = pos.data_ptr(), z.data_ptr(), batch.data_ptr(), dataset.data_ptr()
-        e.charge, e.spin, e.status = charge.data_ptr(), spin.data_ptr(), status.data_ptr()
-        e.shift = None if shift is None else shift.data_ptr()
+        self.nodes, self.systems, self.device = graph.nodes, graph.systems, graph.device
+        e, g = EvalStruct(), graph.g
+        self.ev = e
+        e.num_nodes, e.num_edges, e.num_systems = self.nodes, graph.num_edges, self.systems
+        e.num_chunks, e.want_grad = graph.num_chunks, int(graph.want_grad)
+        charge, spin = charge.to(self.device, torch.int64).contiguous(), spin.to(self.device, torch.int64).contiguous()
+        gamma = None if gamma is None else gamma.contiguous()
+        self.refs = [graph, dataset, charge, spin, gamma, status]
+        for name in ("pos", "z", "batch", "src", "tgt", "row_ptr", "src_ptr", "src_perm"):
+            setattr(e, name, getattr(g, name))
+        e.shift, e.dataset, e.charge, e.spin = graph.shift, dataset.data_ptr(), charge.data_ptr(), spin.data_ptr()
         e.gamma = None if gamma is None else gamma.data_ptr()
-        e.src, e.tgt, e.row_ptr = graph.src.data_ptr(), graph.tgt.data_ptr(), graph.row_ptr.data_ptr()
-        e.src_ptr, e.src_perm = graph.src_ptr.data_ptr(), graph.src_perm.data_ptr()
-        e.chunk_src = None if graph.chunk_src is None else graph.chunk_src.data_ptr()
+        e.status = status.data_ptr()
+        e.chunk_src = g.chunk_src if graph.num_chunks > 1 else None
         e.chunk_node, e.chunk_edge = ctypes.cast(graph.chunk_node, c_void_p), ctypes.cast(graph.chunk_edge, c_void_p)
-        self.want_virial = want_virial
-        self.virial = None
-        self.device = dev
+        self.want_virial, self.virial = want_virial, None
         self.sizes = (c_int64 * 3)()
         self.keep = self.scratch = None
 
@@ -289,25 +287,172 @@ class BackboneFn(torch.autograd.Function):
         return ctx.step.backward(ctx.step.model, grad_x.contiguous(), 1.0), None
 
 
-class StepGraph:
-    """Index arrays of one edge list (sorted by target) for the native evaluation."""
+class GraphStruct(Structure):
+    _fields_ = ([("num_nodes", c_int64)]
+                + [(n, c_int32) for n in ("num_systems", "num_elements", "max_neighbors", "stride", "chunk_edges", "want_totals")]
+                + [("radius", c_float), ("radius_sq", c_float)]
+                + [(n, c_void_p) for n in ("pos", "cell", "pbc", "natoms", "batch64", "z64", "sys", "bbox", "z", "batch", "rows", "count",
+                                           "row_ptr", "info", "status")]
+                + [("num_sources", c_int64), ("num_cells", c_int64)]
+                + [(n, c_void_p) for n in ("cell_count", "source_cell", "cell_ptr", "cell_fill", "bucket", "cand_ptr", "cand_id",
+                                           "cand_sys", "pos0", "cell0", "pbc0", "natoms0")]
+                + [("limit_sq", c_float), ("num_chunks", c_int32), ("num_edges", c_int64)]
+                + [(n, c_void_p) for n in ("src", "tgt", "shift", "edge_index", "cell_offsets", "src_count", "src_ptr", "src_tmp",
+                                           "src_perm", "chunk_src")])
 
-    @classmethod
-    def from_edges(cls, src, tgt, num_nodes: int, chunk_edges: int):
-        g = ops.EdgeGraph(src, tgt, num_nodes)
-        self = cls()
-        self.src, self.tgt, self.row_ptr, self.src_ptr, self.src_perm = g.src, g.tgt, g.row_ptr, g.src_ptr, g.src_perm
-        e = self.num_edges = g.num_edges
-        n = self.num_chunks = max(1, (e + chunk_edges // 2) // chunk_edges)
-        cut = torch.searchsorted(g.row_ptr, torch.arange(1, n, device=src.device, dtype=torch.int32) * (e // n)) if n > 1 else None
-        nodes = [0] + ([] if cut is None else cut.tolist()) + [num_nodes]
-        nodes = sorted(set(nodes))
-        n = self.num_chunks = len(nodes) - 1
-        edges = [0] + ([] if n == 1 else g.row_ptr[torch.tensor(nodes[1:-1], device=src.device)].tolist()) + [e]
+
+INFO_WORDS, INFO_NODES, INFO_EDGES = 1040, 8, 8 + 513
+STRIDE_MAX = 512     # kept neighbours of one target that graph_select_kernel can hold
+BRUTE_NODES = 8192   # below: every periodic image in reach is tried, no grid and no host read to size one
+BRUTE_PAIRS = 4e9    # above that, still the faster way while the systems of a batch are small
+
+
+class _Carve:
+    """Sub-arrays of one int32 allocation, 256-byte aligned."""
+
+    def __init__(self, device, **sizes):
+        offsets, total = {}, 0
+        for name, n in sizes.items():
+            offsets[name] = total
+            total += (n + 63) // 64 * 64
+        self.block = torch.empty(total, dtype=torch.int32, device=device)
+        base = self.block.data_ptr()
+        self.ptr = {name: base + 4 * o for name, o in offsets.items()}
+        self.offsets = offsets
+
+    def view(self, name: str, n: int) -> torch.Tensor:
+        return self.block[self.offsets[name]:self.offsets[name] + n]
+
+
+class StepGraph:
+    """Index arrays of one evaluation for csrc/model_step.cu (edges sorted by target; ``None`` from ``build`` when the
+    general path has to decide: too many neighbours, a degenerate cell)."""
+
+    def __init__(self, bb, data, status, want_grad: bool):
+        self.bb, self.data, self.want_grad = bb, data, want_grad
+        pos = self.pos = data["pos"].detach().contiguous()
+        self.device, self.nodes, self.systems = pos.device, pos.shape[0], len(data["natoms"])
+        n, b = self.nodes, self.systems
+        self.a = _Carve(self.device, sys=b * 24, bbox=b * 6, z=n, batch=n, count=n, row_ptr=n + 1, info=INFO_WORDS)
+        g = self.g = GraphStruct()
+        g.num_nodes, g.num_systems, g.num_elements = n, b, bb.max_num_elements
+        g.max_neighbors, g.chunk_edges = int(bb.max_neighbors), bb.edge_chunk_size
+        g.radius, g.radius_sq = bb.cutoff, bb.cutoff * bb.cutoff
+        pbc = data["pbc"] if data["pbc"].dtype == torch.bool else data["pbc"].bool()
+        cell = data["cell"].detach().to(torch.float32)
+        self.alive = [cell.contiguous(), pbc.contiguous(), *(data[k].long().contiguous() for k in ("natoms", "batch", "atomic_numbers")), status]
+        if any(t.device != self.device for t in self.alive):  # small host tensors next to device positions
+            self.alive = [t.to(self.device) for t in self.alive]
+        if self.alive[1].numel() != 3 * b:
+            self.alive[1] = self.alive[1].reshape(-1, 3).expand(b, 3).contiguous()
+        g.pos = pos.data_ptr()
+        g.cell, g.pbc, g.natoms, g.batch64, g.z64, g.status = (t.data_ptr() for t in self.alive)
+        for name, p in self.a.ptr.items():
+            setattr(g, name, p)
+        self.chunk_src = self.edge_index = self.cell_offsets = self.shift = None
+
+    def _call(self, name):
+        _lib.call(name, byref(self.g), _stream())
+
+    def _info(self):
+        return self.a.view("info", INFO_WORDS).cpu()
+
+    def _finish_info(self, info) -> bool:
+        self.num_edges, n = int(info[0]), int(info[2])
+        nodes, edges = info[INFO_NODES:INFO_NODES + n + 1].tolist(), info[INFO_EDGES:INFO_EDGES + n + 1].tolist()
+        if any(b <= a for a, b in zip(edges, edges[1:])):  # a target with more edges than a chunk: do not cut
+            n, nodes, edges = 1, [0, self.nodes], [0, self.num_edges]
+        self.num_chunks = n
         self.chunk_node, self.chunk_edge = (c_int64 * (n + 1))(*nodes), (c_int64 * (n + 1))(*edges)
-        self.chunk_src = None
-        if n > 1:
-            key = g.src.long()[g.src_perm.long()] * e + g.src_perm.long()
-            want = torch.arange(num_nodes, device=src.device)[None] * e + torch.tensor(edges, device=src.device)[:, None]
-            self.chunk_src = torch.searchsorted(key, want).to(torch.int32).contiguous()
+
+    def build(self) -> bool:
+        """Search, selection and tables from the positions.  False: not for this path."""
+        g, bb = self.g, self.bb
+        nl = bb.neighbor_list
+        k = g.max_neighbors
+        g.stride = min(STRIDE_MAX, 2 * k + 8) if k > 0 else STRIDE_MAX
+        g.want_totals = int(self.nodes > BRUTE_NODES and nl is None)
+        self._call("fcb200_graph_systems")
+        rows = torch.empty(self.nodes * g.stride * 2, dtype=torch.int32, device=self.device)
+        g.rows = rows.data_ptr()
+        if nl is not None:
+            info = self._select_kept(nl)
+        else:
+            if g.want_totals:
+                head = self.a.view("info", 8).cpu()
+                if int(head[1]):
+                    return False
+                g.num_sources, g.num_cells = int(head[4]), int(head[5])
+                if float(head.view(torch.float32)[6]) > BRUTE_PAIRS:
+                    c = _Carve(self.device, cell_count=g.num_cells + 1, cell_ptr=g.num_cells + 1, cell_fill=g.num_cells + 1,
+                               source_cell=g.num_sources, bucket=4 * g.num_sources)
+                    for name, p in c.ptr.items():
+                        setattr(g, name, p)
+            self._call("fcb200_graph_select")
+            info = self._info()
+        if info is None or int(info[1]) or int(info[0]) == 0:
+            return False
+        self._finish_info(info)
+        self._edges()
+        e = self.num_edges
+        edge_index = torch.empty(2, e, dtype=torch.int64, device=self.device)
+        offsets = torch.empty(e, 3, dtype=torch.float32, device=self.device)
+        self.edge_index, self.cell_offsets = edge_index, offsets
+        g.edge_index, g.cell_offsets = edge_index.data_ptr(), offsets.data_ptr()
+        self._call("fcb200_graph_fill")
+        return True
+
+    def _select_kept(self, nl):
+        """Selection from a SkinNeighborList's candidates, refreshed by a new search when they have expired."""
+        g, data = self.g, self.data
+        key = (self.nodes, tuple(data["natoms"].shape), self.device, None)
+        if nl.skin > 0.0 and nl._cand is not None and nl._key == key and nl.origin is not None:
+            pos0, cell0, pbc0, natoms0 = nl.origin
+            g.pos0, g.cell0, g.pbc0, g.natoms0 = pos0.data_ptr(), cell0.data_ptr(), pbc0.data_ptr(), natoms0.data_ptr()
+            g.limit_sq = (0.5 * nl.skin) ** 2
+            self._candidates(nl)
+            self._call("fcb200_graph_select")
+            info = self._info()
+            if not int(info[3]):
+                nl.refreshes += 1
+                return info
+        nl.search(data, data["pbc"])
+        nl.origin = (nl._pos0, self.alive[0].clone(), self.alive[1].clone(), self.alive[2].clone())
+        g.pos0 = None
+        self._candidates(nl)
+        self._call("fcb200_graph_select")
+        return self._info()
+
+    def _candidates(self, nl):
+        c = nl._cand
+        self.g.cand_ptr, self.g.cand_id, self.g.cand_sys = c.cand_ptr.data_ptr(), c.cand_id.data_ptr(), c.sys_t.data_ptr()
+        self.candidates = c
+
+    def _edges(self):
+        e, n = self.num_edges, self.nodes
+        sizes = dict(src=e, tgt=e, shift=3 * e)
+        if self.want_grad:
+            sizes.update(src_count=n, src_ptr=n + 1, src_tmp=e, src_perm=e)
+            if self.num_chunks > 1:
+                sizes["chunk_src"] = (self.num_chunks + 1) * n
+        self.b = _Carve(self.device, **sizes)
+        for name, p in self.b.ptr.items():
+            setattr(self.g, name, p)
+        self.g.num_edges, self.g.num_chunks = e, self.num_chunks
+        self.shift = self.g.shift
+
+    def from_edges(self, src, tgt, shift):
+        """Tables for a given edge list (int64, sorted by target) and its shift vectors."""
+        g = self.g
+        self._call("fcb200_graph_systems")
+        g.rows, g.cand_sys = None, None
+        e = self.num_edges = src.shape[0]
+        self.num_chunks = max(1, min(512, (e + g.chunk_edges // 2) // g.chunk_edges))
+        self._edges()
+        self.b.view("src", e).copy_(src)
+        self.b.view("tgt", e).copy_(tgt)
+        self.alive.append(shift)
+        self.shift = shift.data_ptr()
+        self._call("fcb200_graph_fill")
+        self._finish_info(self._info())
         return self

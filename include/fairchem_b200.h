@@ -625,6 +625,46 @@ int fcb200_model_energy(const fcb200_model* model_host, const fcb200_eval* eval_
 /* grad_pos (and virial): from the sum of the energies (grad_x null) or from a gradient of x_out */
 int fcb200_model_backward(const fcb200_model* model_host, const fcb200_eval* eval_host, void* stream);
 
+/* Graph of an evaluation (csrc/graph_step.cu): fcb200_graph_systems, then fcb200_graph_select, one host read of `info`,
+ * then fcb200_graph_fill.  `info` words: 0 edges, 1 nonzero = left to the general path, 2 chunks, 3 nonzero = kept
+ * candidates expired, 4 / 5 source and cell totals, 6 candidate pairs (float), 8.. chunk nodes, 8 + 513.. chunk edges. */
+#define FCB200_GRAPH_INFO_WORDS 1040
+typedef struct {
+    int64_t num_nodes;
+    int32_t num_systems, num_elements, max_neighbors, stride, chunk_edges, want_totals;
+    float radius, radius_sq;
+    const float *pos, *cell;
+    const uint8_t* pbc;
+    const int64_t *natoms, *batch64, *z64;
+    int32_t* sys;            /* [num_systems, FCB200_SYS_WORDS] out */
+    float* bbox;             /* [num_systems, 6] out */
+    int32_t *z, *batch;      /* [N] out */
+    int32_t *rows, *count, *row_ptr, *info; /* [N, stride, 2], [N], [N+1], [FCB200_GRAPH_INFO_WORDS] out */
+    int32_t* status;
+    /* cell-list search (cell_ptr set) */
+    int64_t num_sources, num_cells;
+    int32_t *cell_count, *source_cell, *cell_ptr, *cell_fill;
+    float* bucket;
+    /* kept candidates (cand_ptr set); pos0.. set: also check whether they still apply */
+    const int32_t *cand_ptr, *cand_id, *cand_sys;
+    const float *pos0, *cell0;
+    const uint8_t* pbc0;
+    const int64_t* natoms0;
+    float limit_sq;
+    /* fill; rows null: src / tgt are given, sorted by target */
+    int32_t num_chunks;
+    int64_t num_edges;
+    int32_t *src, *tgt;
+    float* shift;
+    int64_t* edge_index;
+    float* cell_offsets;
+    int32_t *src_count, *src_ptr, *src_tmp, *src_perm; /* src_ptr null: no by-source order */
+    int32_t* chunk_src;                                /* [(num_chunks+1), N] or null */
+} fcb200_graph;
+int fcb200_graph_systems(const fcb200_graph* graph_host, void* stream);
+int fcb200_graph_select(const fcb200_graph* graph_host, void* stream);
+int fcb200_graph_fill(const fcb200_graph* graph_host, void* stream);
+
 /* Called around every kernel (or group of kernels) of the functions above, on the host: begin = 1 before, 0 after.
  * For accounting; null removes it. */
 typedef void (*fcb200_launch_hook)(const char* name, int32_t begin, int64_t bytes, int64_t flops, int32_t launches);
