@@ -138,7 +138,7 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         L.radial = b.take<float>(ec * d.nrad * 2 * C);
         L.m = planes(b, ec, d.nm * 2 * C);
         L.a = planes(b, ec, d.nm * C);
-        L.y_c = keep ? nullptr : b.take<float>(ec * (d.lmax == 2 ? d.gates : d.yw));
+        L.y_c = keep ? nullptr : b.take<float>(ec * d.gates);
         L.msg_c = keep ? nullptr : b.take<float>(ec * d.nm * C);
         L.xn2 = planes(b, n, d.nl * C);
         L.a2 = planes(b, n, d.nl * C);
@@ -183,14 +183,10 @@ struct Conv {
     std::vector<int32_t> t;
     const fcb200_weight* w[3] = {};
     const float* bias[3] = {};
-    int kmax = 0;
     int64_t macs = 0;
-    bool k64 = true;
     void tile(int a_col, int k, int wi, int w_row, int out_col, int mode = kPlain, int y_col = 0, int gate_col = 0, int flags = 0) {
         const int v[9] = {a_col, k, wi, w_row, out_col, mode, y_col, gate_col, flags};
         t.insert(t.end(), v, v + 9);
-        kmax = std::max(kmax, k);
-        k64 = k64 && k % 64 == 0;
         macs += 128LL * k;
     }
     int count() const { return (int)t.size() / 9; }
@@ -219,8 +215,7 @@ struct Run {
         return rc;
     }
 
-    // One launch of tile list c on rows [m] of half planes.  64-deep operand stages win 2-10 % while no K exceeds 512,
-    // 32-deep ones beyond.
+    // one launch of tile list c on rows [m] of half planes
     int conv(const char* name, const Conv& c, const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, int rot_begin, float* y,
              int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m) const {
         const void *hi[3] = {}, *lo[3] = {};
@@ -232,19 +227,13 @@ struct Run {
         hook(name, 1, bytes, flops);
         const int rc = fcb200_so2_conv_fused(a_hi, a_lo, lda, a_cols, hi, lo, rows, cols, sc, c.bias, c.t.data(), c.count(), rot_begin, y,
                                              ldy, y_cols, o ? o->hi : nullptr, o ? o->lo : nullptr, o ? o->ld : 0, o_cols, a_scale,
-                                             o_scale, m, c.kmax <= 512 && c.k64 ? 2 : 0, ev.status, stream);
+                                             o_scale, m, 0, ev.status, stream);
         hook(name, 0, bytes, flops);
         return rc;
     }
-    // c [m, n] = planes x w^T through the tile-parallel GEMM
-    int gemm(const char* name, const __half* a_hi, const __half* a_lo, int64_t lda, const fcb200_weight& w, const float* scale,
-             const float* bias, float* c, int64_t ldc, int64_t m) const {
-        const int64_t bytes = 4 * m * (w.rows + w.cols), flops = 2 * m * w.rows * w.cols;
-        hook(name, 1, bytes, flops);
-        const int rc = fcb200_gemm_f16x2_presplit(a_hi, a_lo, lda, w.hi, w.lo, w.cols, w.scale, scale, bias, c, ldc, m, w.rows, w.cols,
-                                                  ev.status, stream);
-        hook(name, 0, bytes, flops);
-        return rc;
+    // c [m, w.rows] = planes x w^T
+    int gemm(const char* name, const Planes& a, const fcb200_weight& w, const float* scale, float* c, int64_t ldc, int64_t m) const {
+        return conv(name, linear(w, nullptr), a.hi, a.lo, a.ld, w.cols, 0, c, ldc, w.rows, nullptr, 0, scale, nullptr, m);
     }
 
     // plain tiles of the m-blocks w[0..2] side by side (transposed = the given matrices are already the transposes)
@@ -270,10 +259,6 @@ struct Run {
         if (r < 2 * d.lmax) return r % d.lmax + 1;
         return (r - 2 * d.lmax) % (d.lmax - 1) + 2;
     }
-    // the separate launches of the wide first convolution of lmax 4 (K up to 2048): the row-tile-major fused launch counts
-    // on L2 for its A re-reads, and the tiles of all CTAs together do not fit there
-    bool wide() const { return d.lmax == 4; }
-
     int forward();
     int energy();
     int backward();
@@ -389,20 +374,16 @@ int Run::layer_forward(int l, const float* ffn_prev) {
         });
     }));
     const bool keep = ev.want_grad != 0;
-    Conv c1, c2 = blocks(w.conv2);
-    c2.bias[0] = w.conv2_bias;
-    if (!wide()) {
-        c1 = blocks(w.conv1);  // gate tiles first, then the rows
-        c1.bias[0] = w.conv1_bias;
-        for (int i = d.lmax; i < c1.count(); ++i) {
-            int32_t* t = &c1.t[9 * i];
-            const int r = i - d.lmax;
-            t[4] = r * C;
-            t[5] = r == 0 ? kSilu : kGated;
-            t[6] = (d.lmax + r) * C;
-            t[7] = r == 0 ? 0 : (degree_of_row(r) - 1) * C;
-            t[8] = keep ? kKeep : 0;
-        }
+    Conv c1 = blocks(w.conv1), c2 = blocks(w.conv2);  // conv 1: gate tiles first, then the rows
+    c1.bias[0] = w.conv1_bias, c2.bias[0] = w.conv2_bias;
+    for (int i = d.lmax; i < c1.count(); ++i) {
+        int32_t* t = &c1.t[9 * i];
+        const int r = i - d.lmax;
+        t[4] = r * C;
+        t[5] = r == 0 ? kSilu : kGated;
+        t[6] = (d.lmax + r) * C;
+        t[7] = r == 0 ? 0 : (degree_of_row(r) - 1) * C;
+        t[8] = keep ? kKeep : 0;
     }
     return chunks([&](int, int64_t e0, int64_t ec, int64_t n0, int64_t n1) {
         FCB_TRY(radial_out(l, e0, ec));
@@ -413,17 +394,8 @@ int Run::layer_forward(int l, const float* ffn_prev) {
             return fcb200_lx_gather_rotate_fwd_h(q.xn1, ev.src + e0, ev.tgt + e0, L.wig + e0 * d.nw, radial_of(l, e0), L.m.hi, L.m.lo, nullptr, ec, n, C, d.lmax, stream);
         }));
         float* y = keep ? q.y + e0 * d.yw : L.y_c;
-        if (wide()) {
-            int a = 0, o = 0;
-            for (int i = 0; i < 3; ++i) {
-                FCB_TRY(gemm("gemm_f16x2_presplit", L.m.hi + a, L.m.lo + a, L.m.ld, w.conv1[i], nullptr, i == 0 ? w.conv1_bias : nullptr, y + o, d.yw, ec));
-                a += w.conv1[i].cols, o += w.conv1[i].rows;
-            }
-            FCB_TRY(op("so2_gate_fwd", ec * 4 * C * (d.lmax + 2 * d.nm), [&] { return fcb200_lx_so2_gate_fwd_h(y, L.a.hi, L.a.lo, nullptr, ec, C, d.lmax, stream); }));
-        } else {
-            const int64_t yw = keep ? d.yw : d.gates;
-            FCB_TRY(conv("so2_conv_fused_conv1_gate", c1, L.m.hi, L.m.lo, L.m.ld, L.m.ld, d.lmax, y, yw, yw, &L.a, L.a.ld, nullptr, nullptr, ec));
-        }
+        const int64_t yw = keep ? d.yw : d.gates;
+        FCB_TRY(conv("so2_conv_fused_conv1_gate", c1, L.m.hi, L.m.lo, L.m.ld, L.m.ld, d.lmax, y, yw, yw, &L.a, L.a.ld, nullptr, nullptr, ec));
         float* msg = keep ? q.msg + e0 * d.nm * C : L.msg_c;
         FCB_TRY(conv("so2_conv_fused_conv2", c2, L.a.hi, L.a.lo, L.a.ld, L.a.ld, 0, msg, d.nm * C, d.nm * C, nullptr, 0, nullptr, nullptr, ec));
         return op("rotate_back_reduce_fwd", ec * 4 * (d.nm * C + d.nw) + (n1 - n0) * row * 8,
@@ -540,7 +512,7 @@ int Run::layer_backward(int l) {
     // edge block
     const float* scale = &s[1].scale;
     if (cudaMemsetAsync(L.gxn, 0, n * row * 4, st) != cudaSuccess) return launch_status();
-    Conv c2, c1;
+    Conv c2, c1 = blocks(w.conv1_t);
     {
         const Conv p = blocks(w.conv2_t);  // rows of one degree back to back: their gate gradient stays in registers
         c2.w[0] = p.w[0], c2.w[1] = p.w[1], c2.w[2] = p.w[2];
@@ -561,7 +533,6 @@ int Run::layer_backward(int l) {
                 }
         }
     }
-    if (!wide()) c1 = blocks(w.conv1_t);
     const bool first_layer = l == md.num_layers - 1;
     FCB_TRY(chunks([&](int c, int64_t e0, int64_t ec, int64_t n0, int64_t n1) {
         if (!q.rad) FCB_TRY(radial_out(l, e0, ec));
@@ -575,15 +546,7 @@ int Run::layer_backward(int l) {
             });
         }));
         FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, d.yw, d.yw, &L.gy, L.gy.ld, scale, scale, ec));
-        if (wide()) {
-            int a = 0, o = 0;
-            for (int i = 0; i < 3; ++i) {
-                FCB_TRY(gemm("gemm_f16x2_presplit", L.gy.hi + a, L.gy.lo + a, L.gy.ld, w.conv1_t[i], scale, nullptr, L.gm + o, d.nm * 2 * C, ec));
-                a += w.conv1_t[i].cols, o += w.conv1_t[i].rows;
-            }
-        } else {
-            FCB_TRY(conv("so2_conv_fused_conv1_bwd", c1, L.gy.hi, L.gy.lo, L.gy.ld, L.gy.ld, 0, L.gm, d.nm * 2 * C, d.nm * 2 * C, nullptr, 0, scale, nullptr, ec));
-        }
+        FCB_TRY(conv("so2_conv_fused_conv1_bwd", c1, L.gy.hi, L.gy.lo, L.gy.ld, L.gy.ld, 0, L.gm, d.nm * 2 * C, d.nm * 2 * C, nullptr, 0, scale, nullptr, ec));
         const int64_t gb = ec * 4LL * (2 * d.nm * C + 2 * 2 * d.nrad * C + d.nw + 12) + (n1 - n0) * row * 4 * 4;
         FCB_TRY(op("gather_rotate_bwd", gb, [&] {
             return by_lmax([&](auto lm) {
@@ -592,7 +555,7 @@ int Run::layer_backward(int l) {
                 return launch_gather_bwd<LM, 1>(*this, q.xn1, ev.row_ptr, ev.row_ptr + 1, rad, L.gxn, false, scale, e0, n0, n1);
             });
         }, 0, 2));
-        return gemm("gemm_f16x2_presplit", L.grad.hi, L.grad.lo, L.grad.ld, w.radial_out_t, scale, nullptr,
+        return gemm("so2_conv_fused_radial_out_bwd", L.grad, w.radial_out_t, scale,
                     reinterpret_cast<float*>(L.h2) + e0 * L.rw + (int64_t)l * C, L.rw, ec);
     }));
     return op("rms_norm_sh_bwd", n * row * 16, [&] {
@@ -647,7 +610,7 @@ int Run::backward() {
             });
         }));
         float* gh = reinterpret_cast<float*>(L.h2) + e0 * L.rw;
-        FCB_TRY(gemm("gemm_f16x2_presplit", L.gr3.hi, L.gr3.lo, L.gr3.ld, md.degree_out_t, scale, nullptr, gh + (int64_t)md.num_layers * C, L.rw, ec));
+        FCB_TRY(gemm("so2_conv_fused_radial_out_bwd", L.gr3, md.degree_out_t, scale, gh + (int64_t)md.num_layers * C, L.rw, ec));
         const int grid = warp_grid(ec * nets, 8);
         FCB_TRY(op("radial_act_bwd", ec * nets * 1544, [&] {
             radial_bwd_kernel<<<grid, 256, 0, st>>>(gh, L.pre2 + e0 * L.rw, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b,
@@ -660,7 +623,7 @@ int Run::backward() {
                                                     L.rst1 + e0 * nets * 2, L.rp.out(), L.rw, C, L.scales, nscale, L.rad_scale, e0, ec, nets);
             return 0;
         }));
-        FCB_TRY(gemm("gemm_f16x2_presplit", L.rp.hi, L.rp.lo, L.rw, md.rad_w0_t, L.rad_scale, nullptr, L.ggauss, md.num_basis, ec));
+        FCB_TRY(gemm("so2_conv_fused_radial_in", L.rp, md.rad_w0_t, L.rad_scale, L.ggauss, md.num_basis, ec));
         return op("edge_geometry_bwd", ec * 4 * (md.num_basis + 9 + 4 + 8 + 3), [&] {
             return by_lmax([&](auto lm) {
                 geometry_bwd_kernel<decltype(lm)::value><<<(unsigned)((ec + 127) / 128), 128, 0, st>>>(

@@ -1,10 +1,11 @@
-// One launch per SO(2) convolution: a persistent CTA owns a 128-edge row tile and walks the output column
-// tiles of all m-blocks of the convolution in turn (each with its own slice of the input columns, weight
-// matrix and K extent), with the gate activation -- or its derivative -- applied in the epilogue, so that
-// the convolution output never makes a round trip through memory as float32 just to be gated:
+// One launch per SO(2) convolution: a persistent CTA takes 128-edge row tiles and walks the output column tiles of the
+// convolution's m-blocks (each with its own slice of the input columns, weight matrix and K extent), with the gate
+// activation -- or its derivative -- applied in the epilogue, so that the convolution output never makes a round trip
+// through memory as float32 just to be gated:
 //
 //   conv 1 forward : A = rotated+radial-scaled rows (hi, lo planes)  ->  tiles [gate scalars | rows]
-//                    gate tiles  : raw float32 into y (later tiles of the same warp read them back through TMA)
+//                    gate tiles  : raw float32 into y; their sigmoid stays in the epilogue's registers for the rows of that
+//                                  degree, which follow
 //                    row tiles   : row 0 -> v * sigmoid(v); row (l, m) -> v * sigmoid(gate[l-1]); written as the
 //                                  (hi, lo) half planes conv 2 reads; raw y rows are stored only when the backward
 //                                  pass will want them
@@ -17,10 +18,20 @@
 //
 // Replaces SO2_Convolution.forward + GateActivation.forward of the reference
 // (src/fairchem/core/models/uma/nn/so2_layers.py:600-647, src/fairchem/core/models/uma/nn/activation.py:146-165)
-// and their autograd twins.  Arithmetic, tile shape, operand format, accumulators and the bounded waits are those
-// of gemm_f16x2_presplit_kernel; what differs is the tile schedule (row tile outermost, so the gate scalars and
-// all rows of an edge pass through one thread), eight epilogue warps (two per TMEM lane quarter, each taking
-// half of the tile's columns) and the epilogue modes.
+// and their autograd twins.  Arithmetic and accumulators are those of gemm_f16x2_presplit_kernel.
+//
+// What bounds it, and the layout that follows.  Per 64-deep k-step a 128 x 128 tile takes 768 cycles of MMA and 64 KiB of
+// operands.  Main loop alone (no epilogue), M = 131 072, N = 512, K = 512 / 1024, issued TFLOP/s: two 64 KiB stages
+// 1250 / 1150, three 1527 / 1544, CTA pairs on 256 x 256 tiles with three stages 1555 / 1510; the MMAs alone reach 1516
+// on operands in the 64-byte swizzle and 1736 in the 128-byte one.  So: 128-byte swizzle, 64-deep stages, three of them
+// (192 KiB) -- which leaves 32 KiB for the epilogue, one 4 KiB tile for each of its eight warps.  A warp turns its 32 x 32
+// accumulator block in that tile from a row per lane to whole lines per instruction and does everything else on registers
+// and global memory directly (the forms with TMA-fed input and output tiles needed 64-96 KiB and two or five operand
+// stages of half the depth).
+// us per launch at M = 131 072, lmax 2, four 32-deep or two 64-deep stages with TMA epilogues -> this: conv 1 + gate
+// 1219 -> 985, conv 2 499 -> 377, its backward + gate 780 -> 655, conv 1 backward 1050 -> 890, radial output layer
+// 263 -> 243.  Still above the main loop's own time: the epilogues' instruction stream (the gate's backward: 1500 per
+// 32 x 32 chunk) and 64-byte plane stores share the SM with it.
 #include "gemm_f16_common.cuh"
 
 namespace fcb200 {
@@ -29,61 +40,52 @@ namespace fused {
 using namespace f16;
 
 enum Mode : int32_t {
-    kPlain = 0,     // float32 tile -> y[:, out_col ...] through TMA
-    kGateRaw = 1,   // (unused: gate scalars are kPlain tiles listed before Plan::rot_begin)
+    kPlain = 0,     // float32 tile -> y[:, out_col ...]
+    kGateRaw = 1,   // (unused: gate scalars are kPlain tiles with kGateSrc)
     kSilu = 2,      // planes[:, out_col ...] = split(v * sigmoid(v));                       keep: y[:, y_col ...] = v
-    kGated = 3,     // planes[:, out_col ...] = split(v * sigmoid(y[:, gate_col ...]));      keep: y[:, y_col ...] = v
+    kGated = 3,     // planes[:, out_col ...] = split(v * sigmoid(gate));                    keep: y[:, y_col ...] = v
     kSiluBwd = 4,   // planes[:, out_col ...] = split(v * d/dy silu(y[:, y_col ...]))
     kGatedBwd = 5,  // planes[:, out_col ...] = split(v * sigmoid(gate)); gate gradient summed over consecutive tiles
 };
-// kGateSilu: the gate is sigmoid(silu(g)), the scalar MLP of the node-wise feed-forward, instead of sigmoid(g)
-enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8 };
+// kGateSilu: the gate is sigmoid(silu(g)), the scalar MLP of the node-wise feed-forward, instead of sigmoid(g).
+// kGateSrc (set on the host): a gate tile of the rows that follow
+enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8, kGateSrc = 16 };
 
 struct Tile {
-    int32_t a_col;     // first input column of this tile's K range
-    int32_t k;         // K extent (multiple of 32)
-    int32_t w;         // weight matrix 0..2
-    int32_t w_row;     // first output row of the weight matrix (multiple of 128)
-    int32_t out_col;   // where the result goes (column of y for float32 modes, of the planes for split modes)
-    int32_t mode;
-    int32_t y_col;     // column of y holding this row's raw value (kSilu/kGated keep, kSiluBwd/kGatedBwd read)
-    int32_t gate_col;  // column of y (and of the gradient planes / scratch) of the gate scalars of this row's degree
-    int32_t flags;
-    int32_t pad;
+    int16_t a_col;     // first input column of this tile's K range
+    int16_t k;         // K extent (multiple of 32)
+    int16_t w;         // weight matrix 0..2
+    int16_t w_row;     // first output row of the weight matrix (multiple of 128)
+    int16_t out_col;   // where the result goes (column of y for float32 modes, of the planes for split modes)
+    int16_t mode;
+    int16_t y_col;     // column of y holding this row's raw value (kSilu/kGated keep, kSiluBwd/kGatedBwd read)
+    int16_t gate_col;  // column of y (and of the gradient planes) of the gate scalars of this row's degree
+    int16_t flags;
+    int16_t pad;
 };
-constexpr int kMaxTiles = 40;  // lmax 4: 19 rows x 2C = 38 column tiles in the conv-1 backward
+constexpr int kMaxTiles = 40;   // tiles a caller may list; lmax 4: 19 rows x 2C = 38 column tiles in the conv-1 backward
+constexpr int kMaxPlan = 80;    // tiles of a plan: a gate tile may be repeated for each of its rows
+// A work item is one row tile times one group of consecutive tiles [begin[g], begin[g + 1]): what has to pass through one
+// CTA in order.  See group_tiles() on the host.
 struct Plan {
-    int32_t ntiles;
-    int32_t rot_begin;  // tiles [rot_begin, ntiles) may run in any order: every CTA starts at a different one of them
-    int32_t pad[2];
-    Tile t[kMaxTiles];
+    int32_t groups;
+    int16_t begin[kMaxPlan + 1];
+    Tile t[kMaxPlan];
 };
 
-// Loop position -> tile.  All CTAs walk the same weight tiles; started together they would ask L2 for the same lines
-// at the same moment, so each CTA (or pair) begins the freely ordered part of the list at its own offset.
-__device__ __forceinline__ int tile_at(const Plan& plan, int pos, int rot) {
-    const int free = plan.ntiles - plan.rot_begin;
-    return (pos < plan.rot_begin || free <= 1) ? pos : plan.rot_begin + (pos - plan.rot_begin + rot) % free;
-}
-
-// NBUF staging tiles per epilogue warp: 3 for plans with gated modes, 2 for plans of plain tiles only, which leaves
-// room for one more stage of the operand ring (the ring's depth is what covers the latency of the operand loads)
-template <int NBUF> struct Cfg {
-    static constexpr int kStages = NBUF == 3 ? 4 : 5;
-    static constexpr int kPairStages = NBUF == 3 ? 5 : 6;
-    static constexpr int kEpiWarpBytes = NBUF * 4096;
-};
-constexpr int kStageBytes = 4 * BM * BK * 2;           // A_hi | A_lo | W_hi | W_lo, 8 KiB each
-constexpr int kHalfTile = BM * BK * 2;
+constexpr int KB = 64;                               // k extent of a ring stage: 128-byte rows, 128-byte swizzle
+constexpr int kStages = 3;
+constexpr int kPart = BM * KB * 2;                   // A_hi | A_lo | W_hi | W_lo, 16 KiB each
+constexpr int kStageBytes = 4 * kPart;
 constexpr int kEpiWarps = 8;
-constexpr int kThreads = 64 + 32 * kEpiWarps;          // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
+constexpr int kThreads = 128 + 32 * kEpiWarps;       // warp 0 TMA, warp 1 MMA, 2-3 idle, warps 4-11 epilogue
+// Registers: launched with 168 a thread (12 warps on 4 schedulers); the first warpgroup gives up what the two epilogue
+// warpgroups take, 128 * 40 + 256 * 232 = 384 * 168.
+constexpr int kIdleRegs = 40, kEpiRegs = 232;
+static_assert(128 * kIdleRegs + 32 * kEpiWarps * kEpiRegs <= kThreads * 168, "register split");
 constexpr int kAccCols = 2 * BN, kTmemCols = 2 * kAccCols;
-// KB = k extent of one ring stage: 32 (64-byte rows, 64-byte swizzle) or 64 (128-byte rows, 128-byte swizzle, two
-// stages of 64 KiB)
-template <int NBUF, int KB> constexpr int ring_stages() { return KB == 64 ? 2 : Cfg<NBUF>::kStages; }
-template <int NBUF, int KB = BK> constexpr int smem_bytes() {
-    return ring_stages<NBUF, KB>() * 4 * BM * KB * 2 + kEpiWarps * Cfg<NBUF>::kEpiWarpBytes + 1024 + 256;
-}
+constexpr int kSmemBytes = kStages * kStageBytes + kEpiWarps * 4096 + 1024 + 256;
+
 // K-major, 128-byte swizzle: rows at a 128 B pitch, 8-row groups 1024 B apart
 __device__ __forceinline__ uint64_t smem_desc128(uint32_t addr) {
     uint64_t d = 0;
@@ -99,7 +101,9 @@ struct Params {
     const float* bias[3];
     float w_scale[3];
     float* y;          // raw conv-1 output / float32 output
-    int64_t ldy;
+    int32_t ldy, y_cols;
+    __half *o_hi, *o_lo;
+    int32_t ldo;
     const float* a_scale;  // power of two the A planes were written with (null = 1)
     const float* o_scale;  // power of two the output planes are written with (null = 1)
     int64_t m_total;
@@ -110,334 +114,289 @@ struct Params {
 // instead of the ~20 of expf and an IEEE division -- the epilogue evaluates it for every output element
 __device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
 
-// pack (a, b) * already-applied scale into hi and lo half pairs; track the largest magnitude
-__device__ __forceinline__ void pack2(float a, float b, uint32_t& hi, uint32_t& lo, float& amax) {
-    amax = fmaxf(amax, fmaxf(fabsf(a), fabsf(b)));
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 hf = __half22float2(h);
-    const __half2 l = __floats2half2_rn((a - hf.x) * kLoScale, (b - hf.y) * kLoScale);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// 8 consecutive values -> one 16-byte unit of the hi staging tile and one of the lo staging tile.
-// Row `lane` of a 32-row x 64-byte tile with the 64-byte swizzle: unit index XOR ((row >> 1) & 3).
-__device__ __forceinline__ void stage_split8(uint32_t hi_base, uint32_t lo_base, int lane, int unit, const float (&v)[8], float& amax) {
-    uint32_t h[4], l[4];
+// Largest |hi| so far, NaN-propagating: an overflowed or invalid value becomes inf or NaN as a half, so this one packed
+// maximum per pair replaces range checks on the float32 values.
+__device__ __forceinline__ void store_split(__half* hi, __half* lo, int off, const float (&o)[4], __half2& top) {
+    uint2 h, l;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) pack2(v[2 * i], v[2 * i + 1], h[i], l[i], amax);
-    const uint32_t off = (uint32_t)(lane * 64 + ((unit ^ ((lane >> 1) & 3)) * 16));
-    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(hi_base + off), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
-    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(lo_base + off), "r"(l[0]), "r"(l[1]), "r"(l[2]), "r"(l[3]) : "memory");
-}
-
-// 4 consecutive float32 -> 16-byte chunk `v4` of row `lane` of a 32-row x 128-byte tile with the 128-byte swizzle
-__device__ __forceinline__ void stage_f32x4(uint32_t base, int lane, int v4, float a, float b, float c, float d) {
-    const uint32_t dst = base + (uint32_t)(lane * 128 + ((v4 ^ (lane & 7)) * 16));
-    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
-
-
-// ---- CTA pairs (cta_group::2): two CTAs of a cluster share a 256-row tile and each holds half of the B operand ----
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// TMA load whose completion is signalled on a barrier that may live in the peer CTA (no multicast: the data lands in
-// this CTA's own shared memory only)
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-// arrive on the barrier at this offset in both CTAs of the pair once the MMAs issued so far have completed
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-                 "h"((uint16_t)3)
-                 : "memory");
-}
-// instruction descriptor of the pair MMA: M = 256 (128 rows in each CTA), N columns
-constexpr uint32_t instr_desc_pair(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24); }
-template <int N>
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8, %9, %10, %11, %12}, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(instr_desc_pair(N)), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u),
-          "r"(0u), "r"(0u), "r"(0u)
-        : "memory");
-}
-
-// own row (`lane`) of a 32 x 32 float32 tile that TMA landed with the 128-byte swizzle: values [8u, 8u + 8)
-__device__ __forceinline__ void ld_row8(uint32_t base, int lane, int u, float (&o)[8]) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t src = base + (uint32_t)(lane * 128 + (((2 * u + h) ^ (lane & 7)) * 16));
-        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(o[4 * h]), "=f"(o[4 * h + 1]), "=f"(o[4 * h + 2]), "=f"(o[4 * h + 3]) : "r"(src));
+    for (int j = 0; j < 2; ++j) {
+        const float a = o[2 * j], b = o[2 * j + 1];
+        const __half2 hh = __floats2half2_rn(a, b);
+        const float2 hf = __half22float2(hh);
+        const __half2 ll = __floats2half2_rn((a - hf.x) * kLoScale, (b - hf.y) * kLoScale);
+        top = __hmax2_nan(top, __habs2(hh));
+        (j ? h.y : h.x) = *reinterpret_cast<const uint32_t*>(&hh);
+        (j ? l.y : l.x) = *reinterpret_cast<const uint32_t*>(&ll);
     }
+    __stcs(reinterpret_cast<uint2*>(hi + off), h);  // streamed: not read again by this kernel
+    __stcs(reinterpret_cast<uint2*>(lo + off), l);
 }
 
-// Epilogue warps 2..9: warp w reads TMEM lanes [32 (w % 4), +32) -- one accumulator row per thread -- and takes the
-// 64 columns [64 h, 64 h + 64) of every tile, h = (w - 2) / 4, in two chunks of 32.  Per warp three 4 KiB
-// shared-memory tiles: B0 and B1 receive the 32 x 32 float32 tiles of y a gated mode reads (TMA loads, so the
-// global reads are whole lines and each thread then takes its own row from shared memory), B2 stages the output;
-// B1 doubles as the staging tile of a kept y row or of a finished gate gradient.  Launches of plain tiles rotate
-// the output over all three.
-// PAIR: the CTA is one of a pair that shares 256-row tiles; `unit` is the tile stride owner (CTA or pair index),
-// `units` their number, `row_off` this CTA's first row inside a tile, and `tempty0` a shared::cluster address of the
-// leader's accumulator-free barriers.
-template <bool PAIR, int NBUF>
-__device__ __forceinline__ void epilogue(const CUtensorMap& map_y, const CUtensorMap& map_ohi, const CUtensorMap& map_olo,
-                                         const Plan& plan, const Params& prm, int64_t tiles_m, uint32_t tmem_base,
-                                         uint32_t epi_base, uint32_t tfull0, uint32_t tempty0, uint32_t ld_bar0,
-                                         volatile int* abort_flag, volatile int* range_flag, int64_t unit, int64_t units,
-                                         int row_off) {
-    constexpr int kTileRows = PAIR ? 2 * BM : BM;
+#define FCB_TMEM_LD16(r, taddr)                                                                                           \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "                                                                \
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"                         \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),        \
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])   \
+                 : "r"(taddr)                                                                                             \
+                 : "memory")
+
+// What the epilogue of a launch has to be able to do; fixes how many registers it keeps between tiles.
+enum Kind { kPlainKind = 0, kForwardKind = 1, kBackwardKind = 2 };
+
+// Epilogue warps 4..11: warp w reads TMEM lanes [32 (w % 4), +32) -- one accumulator row per lane -- and takes the columns
+// [64 h, 64 h + 64) of every tile, h = (w - 4) / 4, in two chunks of 32.  A chunk is turned in the warp's shared tile to
+// "lane = row 4 i + lane / 8, columns 4 (lane % 8)": 128-byte lines per row for every global access, and the same
+// (row, column) in the same thread for every tile, so gates and gate-gradient sums stay in registers.
+template <int KIND>
+__device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, int64_t items, uint32_t tmem_base, uint32_t tile,
+                                         uint32_t tfull0, uint32_t tempty0, volatile int* abort_flag, volatile int* range_flag) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = warp & 3;
-    const int ew = warp - 2;
-    const int half = ew >> 2;
-    const uint32_t b0 = epi_base + (uint32_t)(ew * Cfg<NBUF>::kEpiWarpBytes), b1 = b0 + 4096u, b2 = b0 + 8192u;  // b2 only if NBUF == 3
-    const uint32_t ld_bar = ld_bar0 + 8u * ew;
-    uint32_t ld_phase = 0;
-    int rot = 0;             // plain chunks staged so far (output buffer = rot % 3)
-    int last_kind = -1;      // 0 plain, 1 anything else
-    bool b1_stored = false;  // the previous chunk issued a store that reads B1
+    const int q = warp & 3, half = (warp - 4) >> 2;
+    const int rr = lane >> 3, c4 = (lane & 7) * 4;
     const float a_scale = prm.a_scale ? *prm.a_scale : 1.0f;
     const float o_scale = prm.o_scale ? *prm.o_scale : 1.0f;
-    const int ntiles = plan.ntiles;
-    const uint64_t stream_out = l2_policy_evict_first();  // outputs are not read again by this kernel (the gate scalars are: default policy)
-    float amax = 0.f;
-    float acc[2][32];  // gate-gradient sums over the rows of a degree (kGatedBwd), per chunk
+    __half2 top = __floats2half2_rn(0.f, 0.f);
+    float keepv[KIND == kPlainKind ? 1 : 2][32];  // forward: sigmoid of the gate; backward: gate-gradient sums
+    // Loads run one chunk ahead where the registers allow it: the second chunk's accumulator columns without a backward
+    // input, else the y rows of the next chunk.
+    constexpr bool kAhead = KIND != kBackwardKind;
+    float yv[KIND == kBackwardKind ? 32 : 1];
+    float sg[KIND == kBackwardKind ? 2 : 1][32];  // backward: sigmoid of the degree's gate, read once at its first row
+    // y lines of a backward tile on their way to L2 one tile early (lane = row; a warp's 64 columns are two lines)
+    auto prefetch = [&](int64_t item2, int ti2) {
+        if constexpr (KIND == kBackwardKind) {
+            const int64_t row = item2 / plan.groups * BM + q * 32 + lane;
+            if (row < prm.m_total) {
+                const float* p = prm.y + row * prm.ldy + plan.t[ti2].y_col + half * 64;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
+            }
+        }
+    };
+    uint32_t r[kAhead ? 32 : 1], c[kAhead ? 32 : 1];
     int64_t tcount = 0;
-    bool ok = true;
-    for (int64_t mt = unit; mt < tiles_m && ok; mt += units) {
-        const int64_t row0 = mt * kTileRows + row_off + q * 32;
-        const bool live = row0 < prm.m_total;  // else this warp's 32 rows lie entirely below the matrix
-        for (int ti = 0; ti < ntiles; ++ti, ++tcount) {
-            const Tile& t = plan.t[tile_at(plan, ti, (int)(unit % 64))];
+    for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const int64_t mt = item / plan.groups;
+        const int g = (int)(item - mt * plan.groups);
+        const int64_t row0 = mt * BM + q * 32;
+        const int live = (int)(prm.m_total - row0 < 32 ? prm.m_total - row0 : 32);  // rows of this warp inside the matrix
+        // 32 rows of at most 32 767 columns: offsets inside a warp's block fit 32 bits
+        float* const yrow = prm.y + (row0 + rr) * prm.ldy + c4;
+        __half* const ohi = prm.o_hi + (row0 + rr) * prm.ldo + c4;
+        __half* const olo = prm.o_lo + (row0 + rr) * prm.ldo + c4;
+        auto fetch = [&](int y_col, int c2) {
+            if constexpr (KIND == kBackwardKind) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 a = rr + 4 * i < live ? __ldcs(reinterpret_cast<const float4*>(yrow + 4 * i * prm.ldy + y_col + (half * 2 + c2) * 32)) : f4zero();
+                    yv[4 * i] = a.x, yv[4 * i + 1] = a.y, yv[4 * i + 2] = a.z, yv[4 * i + 3] = a.w;
+                }
+            }
+        };
+        fetch(plan.t[plan.begin[g]].y_col, 0);
+        for (int ti = plan.begin[g]; ti < plan.begin[g + 1]; ++ti, ++tcount) {
+            const Tile& t = plan.t[ti];
+            const int mode = t.mode;
             const int buf = (int)(tcount & 1);
             const uint32_t use = (uint32_t)((tcount >> 1) & 1);
-            ok = mbar_wait(tfull0 + 8u * buf, use, abort_flag);
+            if constexpr (KIND == kBackwardKind) {
+                if (ti + 1 < plan.begin[g + 1]) prefetch(item, ti + 1);
+                else if (item + gridDim.x < items) prefetch(item + gridDim.x, plan.begin[(int)((item + gridDim.x) % plan.groups)]);
+            }
+            bool ok = mbar_wait(tfull0 + 8u * buf, use, abort_flag);
             ok = __all_sync(kFull, ok);
-            if (!ok) break;
+            if (!ok) return;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float out_scale = 1.0f / (a_scale * prm.w_scale[t.w]);
             const float corr_scale = out_scale / kLoScale;
             const float* bias = prm.bias[t.w];
-            const uint32_t acc_t = tmem_base + (uint32_t)(buf * kAccCols) + ((uint32_t)(q * 32) << 16);
-            const int mode = t.mode;
-            const bool keep = (t.flags & kKeep) != 0 && (mode == kSilu || mode == kGated);
+            const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols) + ((uint32_t)(q * 32) << 16);  // main columns [0, 128), corrections [128, 256)
             const bool gate_silu = (t.flags & kGateSilu) != 0;
-            const bool fin = mode == kGatedBwd && (t.flags & kLast) != 0;
-            const int n_in = mode == kGatedBwd ? 2 : ((mode == kGated || mode == kSiluBwd) ? 1 : 0);
+            if constexpr (kAhead) {
+                FCB_TMEM_LD32(r, acc + (uint32_t)(half * 64));
+                FCB_TMEM_LD32(c, acc + (uint32_t)(BN + half * 64));
+            }
 #pragma unroll
             for (int c2 = 0; c2 < 2; ++c2) {
                 const int col = (half * 2 + c2) * 32;  // within the tile
-                // 1. inputs of the gated modes, fetched while the accumulator is read
-                if (live && n_in > 0) {
-                    if (lane == 0) {
-                        if (last_kind == 0 || (n_in == 2 && b1_stored)) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                        // first tile after the gate scalars: this thread's stores of them have landed before they are read back
-                        if (ti == plan.rot_begin && plan.rot_begin > 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-                        mbar_expect_tx(ld_bar, (uint32_t)(n_in * 4096));
-                        tma_load_2d(b0, &map_y, (mode == kSiluBwd ? t.y_col : t.gate_col) + col, (int)row0, ld_bar);
-                        if (n_in == 2) tma_load_2d(b1, &map_y, t.y_col + col, (int)row0, ld_bar);
-                    }
-                }
-                // 2. accumulator -> registers
-                float v[32];
-                {
-                    uint32_t r[32], c[32];
-                    // single CTA: main sums in columns [0, 128), corrections in [128, 256).  Pair: 64-column blocks
-                    // hh(0:32, 64:96) | corr(0:64) | hh(32:64, 96:128) | corr(64:128)
-                    const int chunk = half * 2 + c2;
-                    const uint32_t main_col = PAIR ? (uint32_t)((chunk & 1) * 128 + (chunk >> 1) * 32) : (uint32_t)col;
-                    const uint32_t corr_col = PAIR ? (uint32_t)(64 + (chunk >> 1) * 128 + (chunk & 1) * 32) : (uint32_t)(BN + col);
-                    FCB_TMEM_LD32(r, acc_t + main_col);
-                    FCB_TMEM_LD32(c, acc_t + corr_col);
+                // 1. accumulator -> shared tile, row `lane`
+                float poison = 0.f;  // becomes NaN if any value is inf or NaN (an overflowed half upstream)
+                auto stage4 = [&](int v4, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, uint32_t c0, uint32_t c1, uint32_t c2_, uint32_t c3) {
+                    const float v0 = fmaf(__uint_as_float(c0), corr_scale, __uint_as_float(r0) * out_scale);
+                    const float v1 = fmaf(__uint_as_float(c1), corr_scale, __uint_as_float(r1) * out_scale);
+                    const float v2 = fmaf(__uint_as_float(c2_), corr_scale, __uint_as_float(r2) * out_scale);
+                    const float v3 = fmaf(__uint_as_float(c3), corr_scale, __uint_as_float(r3) * out_scale);
+                    if (KIND == kPlainKind || mode == kPlain) poison = fmaf(v0, 0.f, fmaf(v1, 0.f, fmaf(v2, 0.f, fmaf(v3, 0.f, poison))));
+                    const uint32_t dst = tile + (uint32_t)(lane * 128 + ((v4 ^ (lane & 7)) * 16));
+                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "f"(v0), "f"(v1), "f"(v2), "f"(v3) : "memory");
+                };
+                if constexpr (kAhead) {
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    float poison = 0.f;  // becomes NaN if any value is inf or NaN (an overflowed half upstream)
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        v[i] = fmaf(__uint_as_float(c[i]), corr_scale, __uint_as_float(r[i]) * out_scale);
-                        poison = fmaf(v[i], 0.f, poison);
+                    for (int v = 0; v < 8; ++v)
+                        stage4(v, r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3], c[4 * v], c[4 * v + 1], c[4 * v + 2], c[4 * v + 3]);
+                    if (c2 == 0) {
+                        FCB_TMEM_LD32(r, acc + (uint32_t)(col + 32));
+                        FCB_TMEM_LD32(c, acc + (uint32_t)(BN + col + 32));
                     }
-                    if (poison != poison && row0 + lane < prm.m_total) *range_flag = 1;
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t rh[16], ch[16];
+                        FCB_TMEM_LD16(rh, acc + (uint32_t)(col + 16 * h));
+                        FCB_TMEM_LD16(ch, acc + (uint32_t)(BN + col + 16 * h));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int v = 0; v < 4; ++v)
+                            stage4(4 * h + v, rh[4 * v], rh[4 * v + 1], rh[4 * v + 2], rh[4 * v + 3], ch[4 * v], ch[4 * v + 1], ch[4 * v + 2], ch[4 * v + 3]);
+                    }
                 }
-                if (!live) continue;
-                if (bias) {
+                if (c2 == 1) {  // hand the accumulator back to the MMA thread
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive(tempty0 + 8u * buf);
+                }
+                if (poison != poison && lane < live) *range_flag = 1;
+                __syncwarp();
+                // 2. whole lines: the mode's arithmetic and its stores
+                float4 b = f4zero();
+                if (bias) b = ld4(bias + t.w_row + col + c4);
+                // body(i, x, in): row rr + 4 i of the chunk, four columns
+                auto rows = [&](auto&& body) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        const float4 b = ld4(bias + t.w_row + col + 4 * i);
-                        v[4 * i] += b.x, v[4 * i + 1] += b.y, v[4 * i + 2] += b.z, v[4 * i + 3] += b.w;
+                        const int row = rr + 4 * i;
+                        float x[4];
+                        const uint32_t src = tile + (uint32_t)(row * 128 + (((lane & 7) ^ (row & 7)) * 16));
+                        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(src) : "memory");
+                        if constexpr (KIND != kBackwardKind) x[0] += b.x, x[1] += b.y, x[2] += b.z, x[3] += b.w;
+                        body(i, x, row < live);
                     }
-                }
-                // 3. staging tiles free, inputs landed
-                uint32_t st_out;
-                if (mode == kPlain) {
-                    if (lane == 0) {
-                        if (last_kind != 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                        else if (NBUF == 3) asm volatile("cp.async.bulk.wait_group.read 2;" ::: "memory");
-                        else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    }
-                    st_out = b0 + (uint32_t)((rot % NBUF) * 4096);
-                    ++rot;
-                    last_kind = 0;
+                };
+                float* const yo = yrow + col;
+                __half *const ph = ohi + t.out_col + col, *const pl = olo + t.out_col + col;
+                auto store_y = [&](int i, int at, const float (&x)[4]) {
+                    __stcs(reinterpret_cast<float4*>(yo + 4 * i * prm.ldy + at), make_float4(x[0], x[1], x[2], x[3]));
+                };
+                if (KIND == kPlainKind || mode == kPlain) {
+                    const bool inside = t.out_col + col + c4 < prm.y_cols;
+                    rows([&](int i, const float (&x)[4], bool in) {
+                        if (in && inside) store_y(i, t.out_col, x);
+                        if constexpr (KIND == kForwardKind) {
+                            if (t.flags & kGateSrc) {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) keepv[c2][4 * i + j] = sigmoid_f(gate_silu ? x[j] * sigmoid_f(x[j]) : x[j]);
+                            }
+                        }
+                    });
+                } else if constexpr (KIND == kForwardKind) {
+                    const bool keep = (t.flags & kKeep) != 0;
+                    if (mode == kSilu)
+                        rows([&](int i, const float (&x)[4], bool in) {
+                            if (!in) return;
+                            if (keep) store_y(i, t.y_col, x);
+                            float o[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) o[j] = x[j] * sigmoid_f(x[j]) * o_scale;
+                            store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                        });
+                    else
+                        rows([&](int i, const float (&x)[4], bool in) {
+                            if (!in) return;
+                            if (keep) store_y(i, t.y_col, x);
+                            float o[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) o[j] = x[j] * keepv[c2][4 * i + j] * o_scale;
+                            store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                        });
+                } else if (mode == kSiluBwd) {
+                    rows([&](int i, const float (&x)[4], bool in) {
+                        float o[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float y0 = yv[4 * i + j], s = sigmoid_f(y0);
+                            o[j] = x[j] * s * (1.f + y0 * (1.f - s)) * o_scale;
+                        }
+                        if (in) store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                    });
                 } else {
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    st_out = b2;
-                    last_kind = 1;
-                }
-                if (n_in > 0) {
-                    ok = mbar_wait(ld_bar, ld_phase, abort_flag);
-                    ld_phase ^= 1u;
-                }
-                ok = __all_sync(kFull, ok);  // also orders lane 0's wait before everybody's staging writes
-                if (!ok) break;
-                // 4. the mode's arithmetic, staged for the stores
-                if (mode == kPlain || keep) {
-                    const uint32_t st_f32 = mode == kPlain ? st_out : b1;
+                    if (t.flags & kFirst) {
+                        float4 ga[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) stage_f32x4(st_f32, lane, i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                }
-                if (mode != kPlain) {
+                        for (int i = 0; i < 8; ++i) ga[i] = rr + 4 * i < live ? ld4(yo + 4 * i * prm.ldy + t.gate_col) : f4zero();
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        float o[8];
-                        if (mode == kSilu) {
+                        for (int i = 0; i < 8; ++i) {
+                            const float v[4] = {ga[i].x, ga[i].y, ga[i].z, ga[i].w};
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) o[i] = v[8 * u + i] * sigmoid_f(v[8 * u + i]) * o_scale;
-                        } else if (mode == kGated) {
-                            float g[8];
-                            ld_row8(b0, lane, u, g);
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) o[i] = v[8 * u + i] * sigmoid_f(gate_silu ? g[i] * sigmoid_f(g[i]) : g[i]) * o_scale;
-                        } else if (mode == kSiluBwd) {
-                            float y0[8];
-                            ld_row8(b0, lane, u, y0);
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                const float sg = sigmoid_f(y0[i]);
-                                o[i] = v[8 * u + i] * sg * (1.f + y0[i] * (1.f - sg)) * o_scale;
+                            for (int j = 0; j < 4; ++j) {
+                                sg[c2][4 * i + j] = sigmoid_f(gate_silu ? v[j] * sigmoid_f(v[j]) : v[j]);
+                                keepv[c2][4 * i + j] = 0.f;
                             }
-                        } else {  // kGatedBwd
-                            float g[8], yr[8];
-                            ld_row8(b0, lane, u, g);
-                            ld_row8(b1, lane, u, yr);
+                        }
+                    }
+                    rows([&](int i, const float (&x)[4], bool in) {
+                        float o[4];
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                float slope = 1.f;
-                                if (gate_silu) {
-                                    const float sg = sigmoid_f(g[i]);
-                                    slope = sg * (1.f + g[i] * (1.f - sg));
-                                    g[i] *= sg;
+                        for (int j = 0; j < 4; ++j) {
+                            o[j] = x[j] * sg[c2][4 * i + j] * o_scale;
+                            keepv[c2][4 * i + j] = fmaf(x[j], yv[4 * i + j], keepv[c2][4 * i + j]);
+                        }
+                        if (in) store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                    });
+                    if (t.flags & kLast) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            if (rr + 4 * i >= live) continue;
+                            float d[4], slope[4] = {1.f, 1.f, 1.f, 1.f};
+                            if (gate_silu) {
+                                const float4 gr = ld4(yo + 4 * i * prm.ldy + t.gate_col);
+                                const float gv[4] = {gr.x, gr.y, gr.z, gr.w};
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const float s = sigmoid_f(gv[j]);
+                                    slope[j] = s * (1.f + gv[j] * (1.f - s));
                                 }
-                                g[i] = sigmoid_f(g[i]);
-                                o[i] = v[8 * u + i] * g[i] * o_scale;
-                                const float prev = (t.flags & kFirst) ? 0.f : acc[c2][8 * u + i];
-                                acc[c2][8 * u + i] = fmaf(v[8 * u + i], yr[i], prev);
-                                if (fin) acc[c2][8 * u + i] *= slope * g[i] * (1.f - g[i]) * o_scale;
                             }
-                        }
-                        stage_split8(st_out, st_out + 2048u, lane, u, o, amax);
-                    }
-                    if (fin) {  // every thread has read its y row out of B1: stage the finished gate gradient there
-                        __syncwarp();
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            float a[8];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) a[i] = acc[c2][8 * u + i];
-                            stage_split8(b1, b1 + 2048u, lane, u, a, amax);
+                            for (int j = 0; j < 4; ++j) d[j] = keepv[c2][4 * i + j] * slope[j] * sg[c2][4 * i + j] * (1.f - sg[c2][4 * i + j]) * o_scale;
+                            store_split(ohi + t.gate_col + col, olo + t.gate_col + col, 4 * i * prm.ldo, d, top);
                         }
                     }
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) {
-                    if (mode == kPlain) {
-                        if (ti < plan.rot_begin) tma_store_2d(&map_y, st_out, t.out_col + col, (int)row0);  // gate scalars: read back
-                        else tma_store_2d_hint(&map_y, st_out, t.out_col + col, (int)row0, stream_out);
-                    } else {
-                        if (keep) tma_store_2d_hint(&map_y, b1, t.y_col + col, (int)row0, stream_out);
-                        tma_store_2d_hint(&map_ohi, st_out, t.out_col + col, (int)row0, stream_out);
-                        tma_store_2d_hint(&map_olo, st_out + 2048u, t.out_col + col, (int)row0, stream_out);
-                        if (fin) {
-                            tma_store_2d_hint(&map_ohi, b1, t.gate_col + col, (int)row0, stream_out);
-                            tma_store_2d_hint(&map_olo, b1 + 2048u, t.gate_col + col, (int)row0, stream_out);
-                        }
-                    }
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                }
-                b1_stored = keep || fin;
-            }
-            if (!ok) break;
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            // hand the accumulator back to the MMA thread: every thread in the single-CTA kernel, one lane per warp in
-            // the pair kernel (there the barrier may sit in the other SM and an arrive is a round trip)
-            if (PAIR) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * buf);
-            } else {
-                mbar_arrive(tempty0 + 8u * buf);
+                if (c2 == 0) fetch(t.y_col, 1);
+                else if (ti + 1 < plan.begin[g + 1]) fetch(plan.t[ti + 1].y_col, 0);
+                __syncwarp();  // the shared tile is free again
             }
         }
     }
-    if (!(amax <= kHalfMax)) *range_flag = 1;  // also catches NaN
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // all stores of this warp have landed
+    if (!(__half2float(__hmax_nan(__low2half(top), __high2half(top))) <= kHalfMax)) *range_flag = 1;  // inf or NaN
 }
 
-template <int NBUF, int KB = BK>
+template <int KIND>
 __global__ void __launch_bounds__(kThreads, 1)
     so2_conv_fused_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
                           const __grid_constant__ CUtensorMap map_whi0, const __grid_constant__ CUtensorMap map_wlo0,
                           const __grid_constant__ CUtensorMap map_whi1, const __grid_constant__ CUtensorMap map_wlo1,
                           const __grid_constant__ CUtensorMap map_whi2, const __grid_constant__ CUtensorMap map_wlo2,
-                          const __grid_constant__ CUtensorMap map_y, const __grid_constant__ CUtensorMap map_ohi,
-                          const __grid_constant__ CUtensorMap map_olo, const __grid_constant__ Plan plan,
-                          const __grid_constant__ Params prm, int64_t tiles_m) {
-    constexpr int S = ring_stages<NBUF, KB>();
-    constexpr int kStage = 4 * BM * KB * 2, kPart = BM * KB * 2;  // A_hi | A_lo | W_hi | W_lo
+                          const __grid_constant__ Plan plan, const __grid_constant__ Params prm, int64_t items) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t epi_base = base + S * kStage;
-    const uint32_t bar_base = epi_base + kEpiWarps * Cfg<NBUF>::kEpiWarpBytes;
-    // barrier block: full[S] | empty[S] | tmem_full[2] | tmem_empty[2] | tmem slot, abort flag, range flag, pad | ld[8]
+    const uint32_t epi_base = base + kStages * kStageBytes;
+    const uint32_t bar_base = epi_base + kEpiWarps * 4096;
+    // barrier block: full[S] | empty[S] | tmem_full[2] | tmem_empty[2] | tmem slot, abort flag, range flag
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (S + s); };
-    auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * S + b); };
-    auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * S + 2 + b); };
-    auto ld_bar = [&](int w) { return bar_base + 8u * (2 * S + 6 + w); };  // one per epilogue warp, after the flag words
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
+    auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * kStages + b); };
+    auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * kStages + 2 + b); };
     uint8_t* const bar_generic = smem_raw + (bar_base - smem_u32(smem_raw));
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_generic + 8 * (2 * S + 4));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * S + 4) + 4);
-    volatile int* range_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * S + 4) + 8);
-    auto half_addr = [&](int s, int which) { return base + s * kStage + which * kPart; };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_generic + 8 * (2 * kStages + 4));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kStages + 4) + 4);
+    volatile int* range_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kStages + 4) + 8);
+    auto part_addr = [&](int s, int which) { return base + s * kStageBytes + which * kPart; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ntiles = plan.ntiles;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -445,7 +404,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(tfull_bar(b), 1);
             mbar_init(tempty_bar(b), 32 * kEpiWarps);
         }
-        for (int w = 0; w < kEpiWarps; ++w) mbar_init(ld_bar(w), 1);
         *abort_flag = 0;
         *range_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -463,40 +421,46 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
-        if (lane == 0) {
+    if (warp >= 4) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+        epilogue<KIND>(plan, prm, items, tmem_base, epi_base + (uint32_t)((warp - 4) * 4096), tfull_bar(0), tempty_bar(0), abort_flag, range_flag);
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIdleRegs));
+        if (warp == 0 && lane == 0) {
             int64_t it = 0;
             bool ok = true;
             // an A tile is fetched again for each of the output tiles of its m-block, the weights by every CTA: keep
             // both in L2 ahead of the streamed outputs
             const uint64_t keep = l2_policy_evict_last();
-            for (int64_t mt = blockIdx.x; mt < tiles_m && ok; mt += gridDim.x) {
-                for (int ti = 0; ti < ntiles && ok; ++ti) {
-                    const Tile& t = plan.t[tile_at(plan, ti, (int)(blockIdx.x % 64))];
+            for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                const int64_t mt = item / plan.groups;
+                const int g = (int)(item - mt * plan.groups);
+                for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti) {
+                    const Tile& t = plan.t[ti];
                     const CUtensorMap* whi = t.w == 0 ? &map_whi0 : (t.w == 1 ? &map_whi1 : &map_whi2);
                     const CUtensorMap* wlo = t.w == 0 ? &map_wlo0 : (t.w == 1 ? &map_wlo1 : &map_wlo2);
-                    const int num_kb = t.k / KB;
+                    const int num_kb = (t.k + KB - 1) / KB;
                     for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                        const int s = (int)(it % S);
-                        const uint32_t ph = (uint32_t)((it / S) & 1);
+                        const int s = (int)(it % kStages);
+                        const uint32_t ph = (uint32_t)((it / kStages) & 1);
                         ok = mbar_wait(empty_bar(s), ph ^ 1u, abort_flag);
                         if (!ok) break;
-                        mbar_expect_tx(full_bar(s), kStage);
-                        tma_load_2d_hint(half_addr(s, 0), &map_ahi, t.a_col + kb * KB, (int)(mt * BM), full_bar(s), keep);
-                        tma_load_2d_hint(half_addr(s, 1), &map_alo, t.a_col + kb * KB, (int)(mt * BM), full_bar(s), keep);
-                        tma_load_2d_hint(half_addr(s, 2), whi, kb * KB, t.w_row, full_bar(s), keep);
-                        tma_load_2d_hint(half_addr(s, 3), wlo, kb * KB, t.w_row, full_bar(s), keep);
+                        mbar_expect_tx(full_bar(s), kStageBytes);
+                        tma_load_2d_hint(part_addr(s, 0), &map_ahi, t.a_col + kb * KB, (int)(mt * BM), full_bar(s), keep);
+                        tma_load_2d_hint(part_addr(s, 1), &map_alo, t.a_col + kb * KB, (int)(mt * BM), full_bar(s), keep);
+                        tma_load_2d_hint(part_addr(s, 2), whi, kb * KB, t.w_row, full_bar(s), keep);
+                        tma_load_2d_hint(part_addr(s, 3), wlo, kb * KB, t.w_row, full_bar(s), keep);
                     }
                 }
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
+        if (warp == 1 && lane == 0) {
             int64_t it = 0, tcount = 0;
             bool ok = true;
-            for (int64_t mt = blockIdx.x; mt < tiles_m && ok; mt += gridDim.x) {
-                for (int ti = 0; ti < ntiles && ok; ++ti, ++tcount) {
-                    const int num_kb = plan.t[tile_at(plan, ti, (int)(blockIdx.x % 64))].k / KB;
+            for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                const int g = (int)(item % plan.groups);
+                for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti, ++tcount) {
+                    const int k = plan.t[ti].k, num_kb = (k + KB - 1) / KB;
                     const int buf = (int)(tcount & 1);
                     const uint32_t use = (uint32_t)((tcount >> 1) & 1);
                     ok = mbar_wait(tempty_bar(buf), use ^ 1u, abort_flag);  // epilogue has drained this accumulator
@@ -504,18 +468,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols);
                     for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                        const int s = (int)(it % S);
-                        const uint32_t ph = (uint32_t)((it / S) & 1);
+                        const int s = (int)(it % kStages);
+                        const uint32_t ph = (uint32_t)((it / kStages) & 1);
                         ok = mbar_wait(full_bar(s), ph, abort_flag);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         // W_hi | W_lo are adjacent: one 256-wide MMA on a_hi gives a_hi*w_hi (main accumulator) and
                         // a_hi*w_lo (correction accumulator); a 128-wide MMA adds a_lo*w_hi to the correction
-                        auto desc = [](uint32_t addr) { return KB == 64 ? smem_desc128(addr) : smem_desc64(addr); };
-                        const uint64_t da_hi = desc(half_addr(s, 0)), da_lo = desc(half_addr(s, 1));
-                        const uint64_t dw = desc(half_addr(s, 2));
+                        const uint64_t da_hi = smem_desc128(part_addr(s, 0)), da_lo = smem_desc128(part_addr(s, 1));
+                        const uint64_t dw = smem_desc128(part_addr(s, 2));
+                        const int steps = (k - kb * KB + 15) / 16;  // columns past k belong to a neighbour: not multiplied
 #pragma unroll
                         for (int j = 0; j < KB / 16; ++j) {
+                            if (j >= steps) break;
                             const uint64_t adv = (uint64_t)(j * 2);
                             const uint32_t first = (kb > 0 || j > 0) ? 1u : 0u;
                             umma_f16<2 * BN>(acc, da_hi + adv, dw + adv, first);
@@ -527,9 +492,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
         }
-    } else {
-        epilogue<false, NBUF>(map_y, map_ohi, map_olo, plan, prm, tiles_m, tmem_base, epi_base, tfull_bar(0), tempty_bar(0), ld_bar(0),
-                        abort_flag, range_flag, blockIdx.x, gridDim.x, 0);
     }
 
     __syncwarp();
@@ -545,234 +507,108 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-
-// ---------------------------------------------------------------------------------------------------------------
-// The same schedule on CTA pairs.  Two CTAs of a cluster own a 256-edge row tile (128 rows each); one thread of
-// the leader CTA issues tcgen05.mma.cta_group::2 (M = 256), which reads each CTA's A rows from that CTA's shared
-// memory and half of the B rows from each.  What bounds these contractions is the stream of operand bytes from L2
-// into shared memory (a 128 x 128 tile re-reads 32 KiB per 32-deep k-step); in a pair each CTA fetches only half of
-// the weight tile, 24 KiB per k-step, and the ring is one stage deeper.  Per stage a CTA holds
-//     A_hi | A_lo (its 128 rows) | X (128 weight rows, see below)
-//     X leader: W_hi[0:32) ; W_hi[64:96) ; W_lo[0:64)        X peer: W_hi[32:64) ; W_hi[96:128) ; W_lo[64:128)
-// (row ranges relative to the tile's first output column).  Then
-//     a_hi x [X_leader ; X_peer]                 (N = 256)  fills 64-column blocks  hh(0:32,64:96) | hl(0:64) | hh(32:64,96:128) | hl(64:128)
-//     a_lo x [X_leader[0:32)  ; X_peer[0:32)]    (N = 64)   adds  lh(0:64)   to the second block
-//     a_lo x [X_leader[32:64) ; X_peer[32:64)]   (N = 64)   adds  lh(64:128) to the fourth block
-// so every weight row is fetched once per pair and the main and correction sums of a 32-column chunk are still two
-// contiguous TMEM ranges.  TMA loads carry no multicast: every CTA fetches what lands in its own shared memory;
-// their completion is counted on the leader's barrier.  tcgen05.commit with the pair mask frees a stage / publishes
-// an accumulator in both CTAs.
-// ---------------------------------------------------------------------------------------------------------------
-constexpr int kPairStageBytes = 3 * kHalfTile;  // 24 KiB
-template <int NBUF> constexpr int pair_smem_bytes() {
-    return Cfg<NBUF>::kPairStages * kPairStageBytes + kEpiWarps * Cfg<NBUF>::kEpiWarpBytes + 1024 + 256;
-}
-
-template <int NBUF>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-    so2_conv_pair_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
-                         const __grid_constant__ CUtensorMap map_whi0, const __grid_constant__ CUtensorMap map_wlo0,
-                         const __grid_constant__ CUtensorMap map_whi1, const __grid_constant__ CUtensorMap map_wlo1,
-                         const __grid_constant__ CUtensorMap map_whi2, const __grid_constant__ CUtensorMap map_wlo2,
-                         const __grid_constant__ CUtensorMap map_y,
-                         const __grid_constant__ CUtensorMap map_ohi, const __grid_constant__ CUtensorMap map_olo,
-                         const __grid_constant__ Plan plan, const __grid_constant__ Params prm, int64_t tiles_m) {
-    constexpr int S = Cfg<NBUF>::kPairStages;
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t epi_base = base + S * kPairStageBytes;
-    const uint32_t bar_base = epi_base + kEpiWarps * Cfg<NBUF>::kEpiWarpBytes;
-    // barrier block as in the single-CTA kernel; full[] and tmem_empty[] are used in the leader only
-    auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (S + s); };
-    auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * S + b); };
-    auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * S + 2 + b); };
-    auto ld_bar = [&](int w) { return bar_base + 8u * (2 * S + 6 + w); };
-    uint8_t* const bar_generic = smem_raw + (bar_base - smem_u32(smem_raw));
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_generic + 8 * (2 * S + 4));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * S + 4) + 4);
-    volatile int* range_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * S + 4) + 8);
-    // a stage: A_hi | A_lo | X   (the weight maps here have 32-row (W_hi) and 64-row (W_lo) boxes)
-    auto part_addr = [&](int s, int which) { return base + s * kPairStageBytes + which * kHalfTile; };
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ntiles = plan.ntiles;
-    const uint32_t rank = cluster_ctarank();
-    const bool leader = rank == 0;
-    const int64_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S; ++s) {
-            mbar_init(full_bar(s), 1);   // the leader's producer expects both CTAs' bytes; the peer only issues its loads
-            mbar_init(empty_bar(s), 1);  // the leader's commit, delivered to both CTAs
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(tfull_bar(b), 1);
-            mbar_init(tempty_bar(b), 2 * kEpiWarps);  // one lane of every epilogue warp of both CTAs
-        }
-        for (int w = 0; w < kEpiWarps; ++w) mbar_init(ld_bar(w), 1);
-        *abort_flag = 0;
-        *range_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
-                     "r"((uint32_t)kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    cluster_sync_all();  // both CTAs' barriers are initialised before either signals the other
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_slot;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            int64_t it = 0;
-            bool ok = true;
-            for (int64_t mt = pair; mt < tiles_m && ok; mt += pairs) {
-                const int row = (int)(mt * 2 * BM + rank * BM);
-                for (int ti = 0; ti < ntiles && ok; ++ti) {
-                    const Tile& t = plan.t[tile_at(plan, ti, (int)(pair % 64))];
-                    const CUtensorMap* whi = t.w == 0 ? &map_whi0 : (t.w == 1 ? &map_whi1 : &map_whi2);
-                    const CUtensorMap* wlo = t.w == 0 ? &map_wlo0 : (t.w == 1 ? &map_wlo1 : &map_wlo2);
-                    const int r_hi = t.w_row + (int)rank * 32, r_lo = t.w_row + (int)rank * 64;
-                    const int num_kb = t.k / BK;
-                    for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                        const int s = (int)(it % S);
-                        const uint32_t ph = (uint32_t)((it / S) & 1);
-                        ok = mbar_wait(empty_bar(s), ph ^ 1u, abort_flag);
-                        if (!ok) break;
-                        const uint32_t lead_full = map_to_cta(full_bar(s), 0);
-                        // a remote arrive costs the issuing thread a round trip to the other SM: the leader alone announces
-                        // the bytes of both CTAs, the peer's loads just complete on the leader's barrier
-                        if (leader) mbar_expect_tx(full_bar(s), 2 * kPairStageBytes);
-                        tma_load_2d_pair(part_addr(s, 0), &map_ahi, t.a_col + kb * BK, row, lead_full);
-                        tma_load_2d_pair(part_addr(s, 1), &map_alo, t.a_col + kb * BK, row, lead_full);
-                        tma_load_2d_pair(part_addr(s, 2), whi, kb * BK, r_hi, lead_full);
-                        tma_load_2d_pair(part_addr(s, 2) + 2048u, whi, kb * BK, r_hi + 64, lead_full);
-                        tma_load_2d_pair(part_addr(s, 2) + 4096u, wlo, kb * BK, r_lo, lead_full);
-                    }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0 && leader) {
-            int64_t it = 0, tcount = 0;
-            bool ok = true;
-            for (int64_t mt = pair; mt < tiles_m && ok; mt += pairs) {
-                for (int ti = 0; ti < ntiles && ok; ++ti, ++tcount) {
-                    const int num_kb = plan.t[tile_at(plan, ti, (int)(pair % 64))].k / BK;
-                    const int buf = (int)(tcount & 1);
-                    const uint32_t use = (uint32_t)((tcount >> 1) & 1);
-                    ok = mbar_wait(tempty_bar(buf), use ^ 1u, abort_flag);  // both epilogues have drained this accumulator
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols);
-                    for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                        const int s = (int)(it % S);
-                        const uint32_t ph = (uint32_t)((it / S) & 1);
-                        ok = mbar_wait(full_bar(s), ph, abort_flag);  // both CTAs' tiles have landed
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint64_t da_hi = smem_desc64(part_addr(s, 0)), da_lo = smem_desc64(part_addr(s, 1));
-                        const uint64_t dx = smem_desc64(part_addr(s, 2)), dx32 = smem_desc64(part_addr(s, 2) + 2048u);
-#pragma unroll
-                        for (int j = 0; j < BK / 16; ++j) {
-                            const uint64_t adv = (uint64_t)(j * 2);
-                            const uint32_t first = (kb > 0 || j > 0) ? 1u : 0u;
-                            umma_f16_pair<2 * BN>(acc, da_hi + adv, dx + adv, first);
-                            umma_f16_pair<BN / 2>(acc + 64, da_lo + adv, dx + adv, 1u);
-                            umma_f16_pair<BN / 2>(acc + 192, da_lo + adv, dx32 + adv, 1u);
-                        }
-                        umma_commit_pair(empty_bar(s));
-                    }
-                    if (ok) umma_commit_pair(tfull_bar(buf));
-                }
-            }
-        }
-    } else {
-        epilogue<true, NBUF>(map_y, map_ohi, map_olo, plan, prm, tiles_m, tmem_base, epi_base, tfull_bar(0), map_to_cta(tempty_bar(0), 0),
-                       ld_bar(0), abort_flag, range_flag, pair, pairs, (int)rank * BM);
-    }
-
-    __syncwarp();
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    cluster_sync_all();  // neither CTA leaves, nor frees tensor memory, while its peer can still reach it
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols) : "memory");
-    }
-    if (threadIdx.x == 0 && prm.status) {
-        if (*abort_flag) atomicExch(prm.status, 1);
-        else if (*range_flag) atomicCAS(prm.status, 0, 2);
-    }
-}
-
-// 2-D row-major half matrix [rows, cols], row stride ld elements; box = 32 columns x box_rows rows, 64-byte swizzle
-static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, int box_cols = 32) {
+// 2-D row-major half matrix [rows, cols], row stride ld elements; box = 64 columns x 128 rows, 128-byte swizzle
+static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return FCB200_EINVAL;
     cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t gstride[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {(cuuint32_t)KB, (cuuint32_t)BM};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? FCB200_OK : FCB200_EINVAL;
-}
-
-// float32 [rows, cols] with row stride ld; box = 32 x 32, 128-byte swizzle
-static int map_f32(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int64_t ld) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return FCB200_EINVAL;
-    cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t gstride[1] = {(cuuint64_t)ld * 4};
-    cuuint32_t box[2] = {32u, 32u};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), gdim, gstride, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? FCB200_OK : FCB200_EINVAL;
 }
 
-// How many CTA pairs the device runs at once with this kernel's resources (cached per device); 0 on failure.
-static int pair_capacity() {
-    static int cap[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    const bool cached = dev >= 0 && dev < 64;
-    if (cached && cap[dev] > 0) return cap[dev];
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * 74, 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = pair_smem_bytes<3>();
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, so2_conv_pair_kernel<3>, &cfg) != cudaSuccess || n <= 0) {
-        cudaGetLastError();
-        n = sm_count() / 2;
+// ---- work items ----------------------------------------------------------------------------------------------------
+// How a tile list is cut into groups (Plan::groups); a CTA takes (row tile, group) items in turn.
+//   natural  what shares nothing is apart: every plain tile, row 0, and the rows of a degree with their gate tile (forward)
+//            or their gate-gradient sum (backward)
+//   fine     forward gated rows one by one, each after its own copy of the gate tile (the gate is computed again)
+enum Grouping { kAuto = 0, kNatural = 1, kFine = 2 };
+
+struct Groups {
+    int n = 0;           // tiles
+    int groups = 0;
+    int16_t begin[kMaxPlan + 1] = {};
+    int16_t tile[kMaxPlan] = {};  // index into the caller's list
+    int cost[kMaxPlan] = {};      // of a group, in units of K
+    bool ok = true;
+};
+
+// a tile's fixed share (epilogue, ring start-up) in units of its K extent, from launches of one row tile
+constexpr int kTileCost = 192;
+
+static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
+    Groups g;
+    auto put = [&](int i) {
+        if (g.n >= kMaxPlan) {
+            g.ok = false;
+            return;
+        }
+        g.tile[g.n++] = (int16_t)i;
+        g.cost[g.groups] += t[i].k + kTileCost;
+    };
+    auto close = [&] { g.begin[++g.groups] = (int16_t)g.n; };
+    auto gate_of = [&](int col) {
+        for (int i = 0; i < rot_begin; ++i)
+            if (t[i].mode == kPlain && t[i].out_col == col) return i;
+        return -1;
+    };
+    bool done[kMaxTiles] = {};
+    for (int i = 0; i < n && g.ok; ++i) {
+        if (done[i] || (t[i].flags & kGateSrc)) continue;
+        if (t[i].mode == kGated) {
+            const int gate = gate_of(t[i].gate_col);
+            if (gate < 0) {
+                g.ok = false;
+                break;
+            }
+            bool opened = false;
+            for (int j = i; j < n; ++j) {
+                if (t[j].mode != kGated || t[j].gate_col != t[i].gate_col) continue;
+                if (!opened || how == kFine) {
+                    if (opened) close();
+                    put(gate);
+                    opened = true;
+                }
+                put(j);
+                done[j] = true;
+            }
+        } else if (t[i].mode == kGatedBwd) {
+            for (int j = i; j < n; ++j) {
+                put(j);
+                done[j] = true;
+                if (t[j].flags & kLast) break;
+            }
+        } else {
+            put(i);
+        }
+        close();
     }
-    if (cached) cap[dev] = n;
-    return n;
+    return g;
+}
+
+// longest CTA of a static round-robin over rows x groups items, in units of K
+static int64_t makespan(const Groups& g, int64_t rows, int ctas) {
+    const int64_t items = rows * g.groups;
+    int64_t total = 0, most = 0;
+    for (int i = 0; i < g.groups; ++i) total += g.cost[i], most = g.cost[i] > most ? g.cost[i] : most;
+    if (items > 16LL * ctas * g.groups) return rows * total / ctas + most;
+    int64_t worst = 0;
+    for (int c = 0; c < ctas && c < items; ++c) {
+        int64_t sum = 0;
+        for (int64_t i = c; i < items; i += ctas) sum += g.cost[i % g.groups];
+        worst = sum > worst ? sum : worst;
+    }
+    return worst;
 }
 
 }  // namespace fused
 }  // namespace fcb200
 
 using namespace fcb200;
-
-extern "C" int fcb200_conv_pair_capacity(void) { return fused::pair_capacity(); }
 
 extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, const void* const* w_hi,
                                      const void* const* w_lo, const int64_t* w_rows, const int64_t* w_cols,
@@ -784,57 +620,79 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
     if (!a_hi || !a_lo || !w_hi || !w_lo || !w_rows || !w_cols || !w_scale || !tiles || !y || m < 0) return FCB200_EINVAL;
     Plan plan{};
     Params prm{};
+    Tile list[kMaxTiles] = {};
+    const int grouping = variant >> 4;
+    if ((variant & 15) > 2 || grouping < kAuto || grouping > kFine) return FCB200_EINVAL;
     if (num_tiles <= 0 || num_tiles > kMaxTiles) return FCB200_ERANGE;
-    if (variant < 0 || variant > 2) return FCB200_EINVAL;
-    if (variant == 2)  // 64-deep stages need every K extent to be a multiple of 64; otherwise the 32-deep form runs
-        for (int i = 0; i < num_tiles; ++i)
-            if (tiles[9 * i + 1] % 64) variant = 0;
-    const int kb_cols = variant == 2 ? 64 : 32;  // k extent of a ring stage
-    if (lda % 8 || lda < a_cols || ldy % 4 || ldy < y_cols) return FCB200_EINVAL;
+    if (lda % 8 || lda < a_cols || ldy % 4 || ldy < y_cols || y_cols % 4) return FCB200_EINVAL;
     if (!aligned16(a_hi) || !aligned16(a_lo) || !aligned16(y)) return FCB200_EALIGN;
     if (o_hi || o_lo) {
         if (!o_hi || !o_lo || ldo % 8 || ldo < o_cols) return FCB200_EINVAL;
         if (!aligned16(o_hi) || !aligned16(o_lo)) return FCB200_EALIGN;
     }
     if (rot_begin < 0 || rot_begin > num_tiles) return FCB200_EINVAL;
-    plan.ntiles = num_tiles;
-    plan.rot_begin = rot_begin;
     bool used[3] = {false, false, false};
-    bool plain_only = true;
+    bool gated = false, forward = false, backward = false;
     for (int i = 0; i < num_tiles; ++i) {
-        Tile& t = plan.t[i];
+        Tile& t = list[i];
         const int32_t* d = tiles + 9 * i;
+        for (int j = 0; j < 9; ++j)
+            if (d[j] < 0 || d[j] > 32767) return FCB200_ERANGE;
         t.a_col = d[0], t.k = d[1], t.w = d[2], t.w_row = d[3], t.out_col = d[4], t.mode = d[5], t.y_col = d[6], t.gate_col = d[7];
-        t.flags = d[8];
+        t.flags = d[8] & 15;
         if (t.w < 0 || t.w > 2 || !w_hi[t.w] || !w_lo[t.w]) return FCB200_EINVAL;
-        if (t.k <= 0 || t.k % kb_cols || t.k > w_cols[t.w] || t.a_col < 0 || t.a_col % 8 || t.a_col + t.k > a_cols) return FCB200_EINVAL;
-        if (t.w_row < 0 || t.w_row % BN || t.w_row + BN > w_rows[t.w]) return FCB200_EINVAL;
-        if (t.mode < kPlain || t.mode > kGatedBwd || t.mode == kGateRaw || t.out_col < 0 || t.out_col % 8) return FCB200_EINVAL;
+        if (t.k <= 0 || t.k % 32 || t.k > w_cols[t.w] || t.a_col < 0 || t.a_col % 8 || t.a_col + t.k > a_cols) return FCB200_EINVAL;
+        if (t.w_row % BN || t.w_row >= w_rows[t.w]) return FCB200_EINVAL;
+        if (t.mode > kGatedBwd || t.mode == kGateRaw || t.out_col % 8) return FCB200_EINVAL;
         const bool split = t.mode >= kSilu;
+        if (w_rows[t.w] - t.w_row < BN && (split || w_rows[t.w] % 4 || t.out_col + (w_rows[t.w] - t.w_row) != y_cols)) return FCB200_EINVAL;
         if (split && (!o_hi || t.out_col + BN > o_cols)) return FCB200_EINVAL;
-        if (!split && t.out_col + BN > y_cols) return FCB200_EINVAL;
+        if (!split && t.out_col + (w_rows[t.w] - t.w_row < BN ? w_rows[t.w] - t.w_row : BN) > y_cols) return FCB200_EINVAL;
         const bool reads_gate = t.mode == kGated || t.mode == kGatedBwd;
-        if (reads_gate && (t.gate_col < 0 || t.gate_col % 4 || t.gate_col + BN > y_cols)) return FCB200_EINVAL;
+        if (reads_gate && (t.gate_col % 4 || t.gate_col + BN > y_cols)) return FCB200_EINVAL;
         const bool uses_y = t.mode == kSiluBwd || t.mode == kGatedBwd || ((t.mode == kSilu || t.mode == kGated) && (t.flags & kKeep));
-        if (uses_y && (t.y_col < 0 || t.y_col % 4 || t.y_col + BN > y_cols)) return FCB200_EINVAL;
+        if (uses_y && (t.y_col % 4 || t.y_col + BN > y_cols)) return FCB200_EINVAL;
         if (t.mode == kGatedBwd && t.gate_col + BN > o_cols) return FCB200_EINVAL;
         used[t.w] = true;
-        plain_only = plain_only && t.mode == kPlain;
+        gated = gated || t.mode == kGated;
+        forward = forward || t.mode == kSilu || t.mode == kGated;
+        backward = backward || t.mode == kSiluBwd || t.mode == kGatedBwd;
     }
+    if (forward && backward) return FCB200_EINVAL;
     if (m == 0) return FCB200_OK;
-    CUtensorMap mah, mal, mw[6], my, moh, mol;
-    int rc = map_half(&mah, a_hi, m, a_cols, lda, BM, kb_cols);
-    if (!rc) rc = map_half(&mal, a_lo, m, a_cols, lda, BM, kb_cols);
+    for (int i = 0; i < rot_begin && gated; ++i)
+        if (list[i].mode == kPlain) {
+            list[i].flags |= kGateSrc;
+            for (int j = rot_begin; j < num_tiles; ++j)  // what the gate is follows from the rows that use it
+                if (list[j].mode == kGated && list[j].gate_col == list[i].out_col) list[i].flags |= list[j].flags & kGateSilu;
+        }
+    // Row tiles times natural groups are the items: CTAs that run together share an A tile in L2 and the last wave is one
+    // group deep, not one list (M = 131 072, second convolution: 417 us row tile by row tile, 377 so; M = 60 000, first
+    // convolution: 528 / 446).  Few row tiles still leave SMs without work; then the gated rows go one by one where that
+    // shortens the longest CTA by more than the estimate's error (M = 7 680: 104 -> 87 us, M = 640: 59 -> 36 us).
+    const int64_t rows_m = (m + BM - 1) / BM;
+    Groups grp = group_tiles(list, num_tiles, rot_begin, grouping == kFine ? kFine : kNatural);
+    if (!grp.ok) return FCB200_EINVAL;
+    if (grouping == kAuto && gated) {
+        const Groups fine = group_tiles(list, num_tiles, rot_begin, kFine);
+        if (fine.ok && 10 * makespan(fine, rows_m, sm_count()) < 9 * makespan(grp, rows_m, sm_count())) grp = fine;
+    }
+    plan.groups = grp.groups;
+    for (int i = 0; i <= grp.groups; ++i) plan.begin[i] = grp.begin[i];
+    for (int i = 0; i < grp.n; ++i) plan.t[i] = list[grp.tile[i]];
+    CUtensorMap mah, mal, mw[6];
+    int rc = map_half(&mah, a_hi, m, a_cols, lda);
+    if (!rc) rc = map_half(&mal, a_lo, m, a_cols, lda);
     int first = -1;
     for (int i = 0; i < 3 && !rc; ++i) {
         if (!used[i]) continue;
         if (first < 0) first = i;
         if (w_cols[i] % 8 || !aligned16(w_hi[i]) || !aligned16(w_lo[i]) || !(w_scale[i] > 0.f)) return FCB200_EINVAL;
-        rc = map_half(&mw[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i], BN, kb_cols);
-        if (!rc) rc = map_half(&mw[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i], BN, kb_cols);
+        rc = map_half(&mw[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i]);
+        if (!rc) rc = map_half(&mw[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i]);
         prm.w_scale[i] = w_scale[i];
         prm.bias[i] = bias ? bias[i] : nullptr;
-        if (prm.bias[i] && !aligned16(prm.bias[i])) return FCB200_EALIGN;
+        if (prm.bias[i] && (!aligned16(prm.bias[i]) || w_rows[i] % BN)) return FCB200_EALIGN;
     }
     if (rc) return rc;
     for (int i = 0; i < 3; ++i)
@@ -842,69 +700,20 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
             mw[2 * i] = mw[2 * first], mw[2 * i + 1] = mw[2 * first + 1];
             prm.w_scale[i] = 1.f;
         }
-    rc = map_f32(&my, y, m, y_cols, ldy);
-    if (rc) return rc;
-    if (o_hi) {
-        rc = map_half(&moh, o_hi, m, o_cols, ldo, 32);
-        if (!rc) rc = map_half(&mol, o_lo, m, o_cols, ldo, 32);
-        if (rc) return rc;
-    } else {
-        moh = mah, mol = mal;  // no split-output tile exists (checked above)
-    }
-    prm.y = y, prm.ldy = ldy, prm.a_scale = a_scale, prm.o_scale = o_scale;
+    if (ldy > 32767 || ldo > 32767) return FCB200_ERANGE;
+    prm.y = y, prm.ldy = (int32_t)ldy, prm.y_cols = (int32_t)y_cols, prm.a_scale = a_scale, prm.o_scale = o_scale;
+    prm.o_hi = static_cast<__half*>(o_hi), prm.o_lo = static_cast<__half*>(o_lo), prm.ldo = (int32_t)ldo;
     prm.m_total = m, prm.status = status;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (variant == 1) {
-        CUtensorMap mp[6];  // W_hi with 32-row boxes, W_lo with 64-row boxes
-        for (int i = 0; i < 3; ++i) {
-            const int j = used[i] ? i : first;
-            rc = map_half(&mp[2 * i], w_hi[j], w_rows[j], w_cols[j], w_cols[j], 32);
-            if (!rc) rc = map_half(&mp[2 * i + 1], w_lo[j], w_rows[j], w_cols[j], w_cols[j], 64);
-            if (rc) return rc;
-        }
-        const int64_t tiles_m = (m + 2 * BM - 1) / (2 * BM);
-        const int max_pairs = pair_capacity();
-        if (max_pairs <= 0) return FCB200_EINVAL;
-        const int pairs = (int)(tiles_m < max_pairs ? tiles_m : max_pairs);
-        if (plain_only) {
-            static bool attr_done[64] = {};
-            if (const int arc = ensure_dynamic_smem(so2_conv_pair_kernel<2>, pair_smem_bytes<2>(), attr_done)) return arc;
-            so2_conv_pair_kernel<2><<<2 * pairs, kThreads, pair_smem_bytes<2>(), st>>>(mah, mal, mp[0], mp[1], mp[2], mp[3], mp[4],
-                                                                                      mp[5], my, moh, mol, plan, prm, tiles_m);
-        } else {
-            static bool attr_done[64] = {};
-            if (const int arc = ensure_dynamic_smem(so2_conv_pair_kernel<3>, pair_smem_bytes<3>(), attr_done)) return arc;
-            so2_conv_pair_kernel<3><<<2 * pairs, kThreads, pair_smem_bytes<3>(), st>>>(mah, mal, mp[0], mp[1], mp[2], mp[3], mp[4],
-                                                                                      mp[5], my, moh, mol, plan, prm, tiles_m);
-        }
+    const int64_t items = rows_m * plan.groups;
+    const int grid = (int)(items < sm_count() ? items : sm_count());
+    auto launch = [&](auto kernel, bool (&done)[64]) {
+        if (const int arc = ensure_dynamic_smem(kernel, kSmemBytes, done)) return arc;
+        kernel<<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm, items);
         return launch_status();
-    }
-    const int64_t tiles_m = (m + BM - 1) / BM;
-    const int grid = (int)(tiles_m < sm_count() ? tiles_m : sm_count());
-    if (variant == 2) {
-        if (plain_only) {
-            static bool attr_done[64] = {};
-            if (const int arc = ensure_dynamic_smem(so2_conv_fused_kernel<2, 64>, smem_bytes<2, 64>(), attr_done)) return arc;
-            so2_conv_fused_kernel<2, 64><<<grid, kThreads, smem_bytes<2, 64>(), st>>>(mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4],
-                                                                                     mw[5], my, moh, mol, plan, prm, tiles_m);
-        } else {
-            static bool attr_done[64] = {};
-            if (const int arc = ensure_dynamic_smem(so2_conv_fused_kernel<3, 64>, smem_bytes<3, 64>(), attr_done)) return arc;
-            so2_conv_fused_kernel<3, 64><<<grid, kThreads, smem_bytes<3, 64>(), st>>>(mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4],
-                                                                                     mw[5], my, moh, mol, plan, prm, tiles_m);
-        }
-        return launch_status();
-    }
-    if (plain_only) {
-        static bool attr_done[64] = {};
-        if (const int arc = ensure_dynamic_smem(so2_conv_fused_kernel<2>, smem_bytes<2>(), attr_done)) return arc;
-        so2_conv_fused_kernel<2><<<grid, kThreads, smem_bytes<2>(), st>>>(mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], my, moh,
-                                                                         mol, plan, prm, tiles_m);
-    } else {
-        static bool attr_done[64] = {};
-        if (const int arc = ensure_dynamic_smem(so2_conv_fused_kernel<3>, smem_bytes<3>(), attr_done)) return arc;
-        so2_conv_fused_kernel<3><<<grid, kThreads, smem_bytes<3>(), st>>>(mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], my, moh,
-                                                                         mol, plan, prm, tiles_m);
-    }
-    return launch_status();
+    };
+    static bool done[3][64] = {};
+    if (forward) return launch(so2_conv_fused_kernel<kForwardKind>, done[0]);
+    if (backward) return launch(so2_conv_fused_kernel<kBackwardKind>, done[1]);
+    return launch(so2_conv_fused_kernel<kPlainKind>, done[2]);
 }

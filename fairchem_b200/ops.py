@@ -658,12 +658,10 @@ def gemm_f16x2_presplit_(a_hi: Tensor, a_lo: Tensor, w_hi: Tensor, w_lo: Tensor,
 CONV_PLAIN, CONV_GATE_RAW, CONV_SILU, CONV_GATED, CONV_SILU_BWD, CONV_GATED_BWD = range(6)
 CONV_FIRST, CONV_LAST, CONV_KEEP = 1, 2, 4
 CONV_MAX_TILES = 40
-# Launch form of so2_conv_fused_: 0 one CTA per 128-edge tile with 32-deep ring stages, 1 CTA pairs on 256-edge tiles,
-# 2 one CTA per tile with 64-deep stages (128-byte swizzle), -1 the measured choice per launch: 64-deep stages when no
-# tile's K exceeds CONV_K64_MAX (the second convolution, its backward and the radial output layer gain 1-10 %), else
-# 32-deep ones (the first convolution's wide plans lose 1-4 % with 64-deep stages)
+# Accepted for earlier launch forms (0, 1, 2; -1 = none); there is one form now.
 CONV_VARIANT = -1
-CONV_K64_MAX = 512
+# How a launch's tile list is cut into work items: 0 the choice of the library, 1 natural groups, 2 fine (csrc/so2_conv_fused.cu)
+CONV_GROUPING = 0
 
 
 @_op("so2_conv_fused", ("y", "o_hi", "o_lo", "status"))
@@ -674,10 +672,10 @@ def so2_conv_fused_(a_hi: Tensor, a_lo: Tensor, w_hi: List[Tensor], w_lo: List[T
     """One launch for all m-blocks of an SO(2) convolution with the gate (or its derivative) in the epilogue.
 
     ``a_hi/a_lo`` [E, Ka] are the input planes, ``w_*`` the (up to three) half-split weight matrices, ``tiles`` a flat
-    list of 9 integers per 128-column output tile (a_col, k, w, w_row, out_col, mode, y_col, gate_col, flags); tiles from
-    position ``rot_begin`` on may run in any order (every CTA starts at a different one).  ``y``
+    list of 9 integers per 128-column output tile (a_col, k, w, w_row, out_col, mode, y_col, gate_col, flags); with gated
+    tiles, the plain tiles before position ``rot_begin`` are their gate scalars.  ``y``
     [E, >=gates] float32 receives the float32 modes and the raw gate scalars and is read by the gated modes; ``o_hi/o_lo``
-    receive the split modes.  ``variant`` selects the launch form (see ``CONV_VARIANT``, the default)."""
+    receive the split modes.  ``variant`` is accepted for earlier launch forms."""
     for t in (a_hi, a_lo):
         if not t.is_cuda or t.dtype != torch.float16 or t.dim() != 2 or t.stride(1) != 1 or t.shape != a_hi.shape \
                 or t.stride(0) != a_hi.stride(0):
@@ -707,10 +705,8 @@ def so2_conv_fused_(a_hi: Tensor, a_lo: Tensor, w_hi: List[Tensor], w_lo: List[T
     biases = (c_void_p * 3)(None if bias0 is None else bias0.data_ptr(), None, None)
     tl = (c_int32 * len(tiles))(*tiles)
     if variant < 0:
-        variant = CONV_VARIANT
-    if variant < 0:
-        ks = [tiles[9 * i + 1] for i in range(nt)]
-        variant = 2 if max(ks) <= CONV_K64_MAX and all(k % 64 == 0 for k in ks) else 0
+        variant = max(CONV_VARIANT, 0)
+    variant += 16 * CONV_GROUPING
     flops = 2 * m * 128 * sum(tiles[9 * i + 1] for i in range(nt))
     nbytes = 4 * m * (a_hi.shape[1] + 128 * nt)
     _launch("so2_conv_fused" + label, "fcb200_so2_conv_fused",

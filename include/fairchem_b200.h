@@ -413,20 +413,14 @@ int fcb200_gemm_f16x2_presplit(const void* a_hi, const void* a_lo, int64_t lda, 
  *                mode 5  planes[:, out_col..] = split(v * sigmoid(y[:, gate_col..])) and the gate gradient
  *                        sum_rows v * y[:, y_col..] summed over CONSECUTIVE tiles (flag 1: first row of the
  *                        degree, flag 2: last row -> planes[:, gate_col..] = split(sum * s * (1 - s)))
- *   rot_begin    tiles [rot_begin, num_tiles) may run in any order (each CTA starts at a different one, so that the
- *                CTAs do not all ask L2 for the same weight lines at once); mode-0 tiles that write gate scalars
- *                read by mode-3 tiles come before rot_begin; num_tiles for a mode-5 plan (its order matters)
  *   y            [M, y_cols] float32, row stride ldy; o_hi/o_lo [M, o_cols] half planes, row stride ldo, written
  *                times *o_scale (device pointers to powers of two, NULL = 1)
  *   status       as in fcb200_gemm_f16x2_presplit
- *   variant      0: one CTA per 128-edge tile, operand ring of 32-deep k stages; 1: CTA pairs (tcgen05
- *                cta_group::2) on 256-edge tiles, each CTA streaming half of the weight operand; 2: as 0 with
- *                64-deep k stages (128-byte swizzle; runs as 0 when some k is not a multiple of 64).  Same results.
+ *   variant      bits 4..: how the list is cut into work items: 0 the library's choice, 1 natural groups, 2 fine;
+ *                bits 0..3 (0, 1 or 2) are accepted for callers of earlier launch forms and ignored.  Same results.
+ *   rot_begin    with gated tiles: the plain tiles before this position are their gate scalars
  * At most 40 tiles; every k a multiple of 32, w_row a multiple of 128.
  */
-/* Number of CTA pairs variant 1 of fcb200_so2_conv_fused runs at once on the current device (0 if it cannot be told). */
-int fcb200_conv_pair_capacity(void);
-
 int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, const void* const* w_hi,
                           const void* const* w_lo, const int64_t* w_rows, const int64_t* w_cols, const float* w_scale,
                           const float* const* bias, const int32_t* tiles, int32_t num_tiles, int32_t rot_begin, float* y,
