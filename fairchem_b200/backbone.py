@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import contextlib
 import math
+import weakref
 from dataclasses import dataclass
 from typing import Optional
 
@@ -1364,7 +1365,7 @@ class eSCNMDBackboneB200(nn.Module):
             return None
         run.virial = {"num_systems": graph.systems} if self.regress_stress else None
         x = step.BackboneFn.apply(pos, run)
-        run.embedding = x
+        run.embedding = weakref.ref(x)  # x's autograd node holds the run: a strong reference would be a cycle
         return {"node_embedding": x, "batch": data["batch"], "virial": run.virial, "step": run}
 
     def _forward(self, data, gamma):
@@ -1452,7 +1453,7 @@ class MLP_EFS_HeadB200(nn.Module):
     def _forward_native(self, data, emb):
         """Energy and forces straight from the evaluation that made ``emb`` (no autograd graph in between)."""
         run = emb.get("step", None)
-        if run is None or run.keep is None or emb["node_embedding"] is not run.embedding or run.embedding._version != 0:
+        if run is None or run.keep is None or emb["node_embedding"] is not run.embedding() or emb["node_embedding"]._version != 0:
             return None
         want = self.regress_forces or self.regress_stress
         model = run.plan.with_head(self)

@@ -227,15 +227,21 @@ class BackboneStep:
             e.keep_radial = keep_radial
             _lib.call("fcb200_model_sizes", byref(self.model), byref(e), sizes)
             need = sizes[0] + max(sizes[1], sizes[2] if e.want_grad else 0)
-            if need < (1 << 30):  # what any free GPU has; spares the memory query of small systems
+            if need < (1 << 28) or need < self._cached():  # what any GPU in use has, or what the allocator already holds
                 return True
             if not hasattr(self, "avail"):
                 free, self.total = torch.cuda.mem_get_info(self.device)
-                self.avail = free + torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+                self.avail = free + self._cached()
             # the largest kept set only with room to spare
             if need * (1.15 if keep_radial else 1.0) + 0.03 * self.total < self.avail:
                 return True
         return False
+
+    def _cached(self) -> int:
+        """Bytes the caching allocator holds and does not use.  Asking the driver for free memory instead takes
+        10-40 ms now and then, so that is left to evaluations that need more than this."""
+        stats = torch._C._cuda_memoryStats(self.device.index)
+        return stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
 
     def _block(self, nbytes: int) -> torch.Tensor:
         return torch.empty(nbytes, dtype=torch.uint8, device=self.device)
