@@ -103,6 +103,8 @@ def complete_cell(cell: np.ndarray) -> np.ndarray:
 def wrap_positions(pos: np.ndarray, cell: np.ndarray, pbc: np.ndarray) -> np.ndarray:
     """Positions moved into the cell along the periodic directions (fractional coordinate modulo 1, no tolerance:
     ``ase.geometry.wrap_positions(..., eps=0)`` as called by ``AtomicData.from_ase``)."""
+    if not any(pbc):
+        return np.asarray(pos, dtype=np.float64)
     frac = np.linalg.solve(cell.T, np.asarray(pos, dtype=np.float64).T).T
     for i in range(3):
         if pbc[i]:

@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(128)
                         const float* __restrict__ shift, const float* __restrict__ gamma, float4* __restrict__ vec,
                         float* __restrict__ env, float* __restrict__ wig, __half* __restrict__ g_hi, __half* __restrict__ g_lo,
                         BasisParams bp, int64_t num_edges) {
+    pdl_sync();
     constexpr int W = Shape<LMAX>::kW;
     extern __shared__ float sm[];  // [128][W]
     __shared__ float sd[128];
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(128)
     geometry_bwd_kernel(const float4* __restrict__ vec, const float* __restrict__ wig, const float4* __restrict__ tau_n,
                         const float4* __restrict__ tau_e, const float* __restrict__ g_gauss, float* __restrict__ grad_vec,
                         BasisParams bp, int64_t num_edges) {
+    pdl_sync();
     constexpr int W = Shape<LMAX>::kW;
     __shared__ float sgd[128];
     const int tid = threadIdx.x;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(128)
 __global__ void __launch_bounds__(256)
     grad_pos_kernel(const float* __restrict__ grad_vec, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ src_ptr,
                     const int32_t* __restrict__ src_perm, float* __restrict__ grad_pos, float sign, int64_t num_nodes) {
+    pdl_sync();
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (n >= num_nodes) return;
@@ -199,6 +202,7 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN)
                        const int32_t* __restrict__ row_ptr, int64_t e_base, const float* __restrict__ residual,
                        const float* __restrict__ emb, const int32_t* __restrict__ z, const float* __restrict__ sys,
                        const int32_t* __restrict__ batch, float* __restrict__ out, float inv_rescale, int64_t n0, int64_t n1) {
+    pdl_sync();
     using S = Shape<LMAX>;
     constexpr int kWarps = WPN == 1 ? 4 : WPN;
     constexpr int rows_in = MODE == 0 ? S::kM : LMAX + 1;
@@ -319,6 +323,7 @@ __global__ void __launch_bounds__(128, LMAX == 2 ? 4 : 3)
                            const float* __restrict__ env, const int32_t* __restrict__ tgt, Out grad_msg,
                            const float* __restrict__ scale_ptr, float* __restrict__ tau_e, int accumulate, float inv_rescale,
                            int64_t e_base, int64_t num_edges) {
+    pdl_sync();
     using S = Shape<LMAX>;
     grad_msg.load_scale(scale_ptr);
     constexpr int rows_in = MODE == 0 ? S::kM : LMAX + 1;
@@ -434,6 +439,7 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
                       const int32_t* __restrict__ hi, const int32_t* __restrict__ perm, const float* __restrict__ wig,
                       const float* __restrict__ radial, float* __restrict__ gx, float* __restrict__ tau, int store_tau,
                       RadOut grad_radial, const float* __restrict__ scale_ptr, int64_t e_base, int64_t n0, int64_t n1) {
+    pdl_sync();
     using S = Shape<LMAX>;
     grad_radial.load_scale(scale_ptr);
     constexpr int kWarps = WPN == 1 ? 4 : WPN;

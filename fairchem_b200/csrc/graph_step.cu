@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(1024)
     graph_systems_kernel(int64_t num_nodes, const float* __restrict__ pos, const float* __restrict__ cell, const uint8_t* __restrict__ pbc,
                          const int64_t* __restrict__ natoms, int nsys, float radius, int32_t* __restrict__ sys, float* __restrict__ bbox,
                          int32_t* __restrict__ info) {
+    pdl_sync();
     __shared__ long long s_begin[32];
     __shared__ float s_lo[32][3], s_hi[32][3];
     const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, threads = blockDim.x, warps = threads >> 5;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(1024)
 
 // first source and first grid cell of every system, and their totals; one block
 __global__ void __launch_bounds__(32) graph_offsets_kernel(int32_t* __restrict__ sys, int nsys, int32_t* __restrict__ info) {
+    pdl_sync();
     if (threadIdx.x != 0) return;
     long long src = 0, cells = 0;
     double pairs = 0.0;
@@ -126,6 +128,7 @@ __global__ void __launch_bounds__(32) graph_offsets_kernel(int32_t* __restrict__
 __global__ void graph_convert_kernel(const int64_t* __restrict__ z64, const int64_t* __restrict__ batch64, int32_t* __restrict__ z,
                                      int32_t* __restrict__ batch, int64_t n, int num_elements, int nsys, int32_t* __restrict__ info,
                                      int32_t* __restrict__ status) {
+    pdl_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 8) info[i] = 0;  // the kernels that raise words of it run after this one
     if (i >= n) return;
@@ -141,6 +144,7 @@ __global__ void graph_moved_kernel(const float* __restrict__ pos, const float* _
                                    const float* __restrict__ cell, const float* __restrict__ cell0, const uint8_t* __restrict__ pbc,
                                    const uint8_t* __restrict__ pbc0, const int64_t* __restrict__ natoms, const int64_t* __restrict__ natoms0,
                                    int nsys, int32_t* __restrict__ info) {
+    pdl_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool moved = false;
     if (i < n) {
@@ -163,6 +167,7 @@ __global__ void __launch_bounds__(256)
                         const int32_t* __restrict__ cand_ptr, const int32_t* __restrict__ cand_id, float radius, float radius_sq,
                         int max_neighbors, int2* __restrict__ rows, int stride, int32_t* __restrict__ count, int32_t* __restrict__ info,
                         int64_t num_nodes) {
+    pdl_sync();
     __shared__ float s_d2[8][kCap];
     __shared__ int2 s_id[8][kCap];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -288,6 +293,7 @@ __global__ void __launch_bounds__(256)
 // exclusive scan by one block; with info: the total and the chunk boundaries (node whose first edge reaches c * E / chunks)
 __global__ void __launch_bounds__(1024)
     graph_scan_kernel(const int32_t* __restrict__ counts, int32_t* __restrict__ ptr, int64_t n, int chunk_edges, int32_t* __restrict__ info) {
+    pdl_sync();
     __shared__ int warp_tot[32];
     __shared__ int carry;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -359,6 +365,7 @@ __global__ void __launch_bounds__(256)
                       const int32_t* __restrict__ row_ptr, int32_t* __restrict__ src, int32_t* __restrict__ tgt, float* __restrict__ shift,
                       int64_t* __restrict__ edge_index, float* __restrict__ offsets, int32_t* __restrict__ src_count, int64_t num_edges,
                       int64_t num_nodes) {
+    pdl_sync();
     const int lane = threadIdx.x & 31;
     const int64_t t = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (t >= num_nodes) return;
@@ -380,6 +387,7 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void graph_count_kernel(const int32_t* __restrict__ node, int32_t* __restrict__ count, int64_t num_edges) {
+    pdl_sync();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e < num_edges) atomicAdd(count + node[e], 1);
 }
@@ -387,6 +395,7 @@ __global__ void graph_count_kernel(const int32_t* __restrict__ node, int32_t* __
 // edges into their source's segment, in any order ...
 __global__ void graph_bucket_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ src_ptr, int32_t* __restrict__ left,
                                     int32_t* __restrict__ unsorted, int64_t num_edges) {
+    pdl_sync();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= num_edges) return;
     const int s = src[e];
@@ -397,6 +406,7 @@ __global__ void graph_bucket_kernel(const int32_t* __restrict__ src, const int32
 __global__ void __launch_bounds__(256)
     graph_order_kernel(const int32_t* __restrict__ unsorted, const int32_t* __restrict__ src_ptr, int32_t* __restrict__ perm,
                        int32_t* __restrict__ chunk_src, const int32_t* __restrict__ edge_cut, int chunks, int64_t num_nodes) {
+    pdl_sync();
     const int lane = threadIdx.x & 31;
     const int64_t n = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (n >= num_nodes) return;
@@ -416,6 +426,12 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// short kernels of a small graph: see launch_pdl
+struct PdlScope {
+    explicit PdlScope(int64_t nodes) { pdl_launches = nodes * 30 <= kPdlEdges; }
+    ~PdlScope() { pdl_launches = false; }
+};
+
 }  // namespace step
 }  // namespace fcb200
 
@@ -427,18 +443,20 @@ int fcb200_graph_systems(const fcb200_graph* g, void* stream) {
     if (!g || g->num_nodes < 1 || g->num_systems < 1 || !(g->radius > 0.f)) return FCB200_EINVAL;
     if (!g->pos || !g->cell || !g->pbc || !g->natoms || !g->batch64 || !g->z64 || !g->sys || !g->bbox || !g->z || !g->batch || !g->info || !g->status)
         return FCB200_EINVAL;
+    const step::PdlScope scope(g->num_nodes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    step::graph_convert_kernel<<<(unsigned)((g->num_nodes + 255) / 256), 256, 0, st>>>(g->z64, g->batch64, g->z, g->batch, g->num_nodes,
+    launch_pdl(step::graph_convert_kernel, dim3((unsigned)((g->num_nodes + 255) / 256)), dim3(256), 0, st, g->z64, g->batch64, g->z, g->batch, g->num_nodes,
                                                                                       g->num_elements, g->num_systems, g->info, g->status);
     // few systems: a block each has to sweep many atoms
-    step::graph_systems_kernel<<<g->num_systems, g->num_systems < 148 ? 1024 : 128, 0, st>>>(g->num_nodes, g->pos, g->cell, g->pbc, g->natoms, g->num_systems, g->radius, g->sys, g->bbox,
+    launch_pdl(step::graph_systems_kernel, dim3(g->num_systems), dim3(g->num_systems < 148 ? 1024 : 128), 0, st, g->num_nodes, g->pos, g->cell, g->pbc, g->natoms, g->num_systems, g->radius, g->sys, g->bbox,
                                                                g->info);
-    if (g->want_totals) step::graph_offsets_kernel<<<1, 32, 0, st>>>(g->sys, g->num_systems, g->info);
+    if (g->want_totals) launch_pdl(step::graph_offsets_kernel, dim3(1), dim3(32), 0, st, g->sys, g->num_systems, g->info);
     return launch_status();
 }
 
 int fcb200_graph_select(const fcb200_graph* g, void* stream) {
     if (!g || g->num_nodes < 1 || !g->rows || !g->count || !g->row_ptr || g->stride < 1 || g->chunk_edges < 1) return FCB200_EINVAL;
+    const step::PdlScope scope(g->num_nodes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)((g->num_nodes + 7) / 8);
     const float r2 = g->radius_sq;
@@ -447,10 +465,10 @@ int fcb200_graph_select(const fcb200_graph* g, void* stream) {
         if (g->pos0) {
             if (!g->cell0 || !g->pbc0 || !g->natoms0) return FCB200_EINVAL;
             const int64_t n = g->num_nodes > 9LL * g->num_systems ? g->num_nodes : 9LL * g->num_systems;
-            step::graph_moved_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g->pos, g->pos0, g->limit_sq, g->num_nodes, g->cell, g->cell0,
+            launch_pdl(step::graph_moved_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, g->pos, g->pos0, g->limit_sq, g->num_nodes, g->cell, g->cell0,
                                                                                   g->pbc, g->pbc0, g->natoms, g->natoms0, g->num_systems, g->info);
         }
-        step::graph_select_kernel<2><<<grid, 256, 0, st>>>(g->pos, g->cand_sys, g->num_systems, g->batch, nullptr, nullptr, nullptr, g->cand_ptr,
+        launch_pdl(step::graph_select_kernel<2>, dim3(grid), dim3(256), 0, st, g->pos, g->cand_sys, g->num_systems, g->batch, nullptr, nullptr, nullptr, g->cand_ptr,
                                                            g->cand_id, g->radius, r2, g->max_neighbors, reinterpret_cast<int2*>(g->rows),
                                                            g->stride, g->count, g->info, g->num_nodes);
     } else if (g->cell_ptr) {
@@ -459,25 +477,26 @@ int fcb200_graph_select(const fcb200_graph* g, void* stream) {
         if (cudaMemsetAsync(g->cell_fill, 0, (size_t)(g->num_cells + 1) * 4, st) != cudaSuccess) return launch_status();
         int rc = fcb200_rg_count_sources(g->pos, g->sys, g->num_systems, g->num_sources, g->cell_count, g->source_cell, stream);
         if (rc) return rc;
-        step::graph_scan_kernel<<<1, 1024, 0, st>>>(g->cell_count, g->cell_ptr, g->num_cells, 1, nullptr);
+        launch_pdl(step::graph_scan_kernel, dim3(1), dim3(1024), 0, st, g->cell_count, g->cell_ptr, g->num_cells, 1, nullptr);
         rc = fcb200_rg_fill_buckets(g->pos, g->sys, g->num_systems, g->num_sources, g->source_cell, g->cell_ptr, g->cell_fill, g->bucket,
                                     g->num_cells, stream);
         if (rc) return rc;
-        step::graph_select_kernel<1><<<grid, 256, 0, st>>>(g->pos, g->sys, g->num_systems, g->batch, nullptr, g->cell_ptr,
+        launch_pdl(step::graph_select_kernel<1>, dim3(grid), dim3(256), 0, st, g->pos, g->sys, g->num_systems, g->batch, nullptr, g->cell_ptr,
                                                            reinterpret_cast<const float4*>(g->bucket), nullptr, nullptr, g->radius, r2,
                                                            g->max_neighbors, reinterpret_cast<int2*>(g->rows), g->stride, g->count, g->info,
                                                            g->num_nodes);
     } else {
-        step::graph_select_kernel<0><<<grid, 256, 0, st>>>(g->pos, g->sys, g->num_systems, g->batch, g->bbox, nullptr, nullptr, nullptr, nullptr,
+        launch_pdl(step::graph_select_kernel<0>, dim3(grid), dim3(256), 0, st, g->pos, g->sys, g->num_systems, g->batch, g->bbox, nullptr, nullptr, nullptr, nullptr,
                                                            g->radius, r2, g->max_neighbors, reinterpret_cast<int2*>(g->rows), g->stride, g->count,
                                                            g->info, g->num_nodes);
     }
-    step::graph_scan_kernel<<<1, 1024, 0, st>>>(g->count, g->row_ptr, g->num_nodes, g->chunk_edges, g->info);
+    launch_pdl(step::graph_scan_kernel, dim3(1), dim3(1024), 0, st, g->count, g->row_ptr, g->num_nodes, g->chunk_edges, g->info);
     return launch_status();
 }
 
 int fcb200_graph_fill(const fcb200_graph* g, void* stream) {
     if (!g || g->num_edges < 1 || !g->src || !g->tgt || !g->row_ptr) return FCB200_EINVAL;
+    const step::PdlScope scope(g->num_nodes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t n = g->num_nodes, e = g->num_edges;
     const unsigned gn = (unsigned)((n + 7) / 8), ge = (unsigned)((e + 255) / 256);
@@ -487,20 +506,20 @@ int fcb200_graph_fill(const fcb200_graph* g, void* stream) {
     }
     if (g->rows) {
         if (!g->shift || !g->edge_index || !g->cell_offsets || !g->batch) return FCB200_EINVAL;
-        step::graph_fill_kernel<<<gn, 256, 0, st>>>(g->cand_sys ? g->cand_sys : g->sys, g->batch, reinterpret_cast<const int2*>(g->rows), g->stride,
+        launch_pdl(step::graph_fill_kernel, dim3(gn), dim3(256), 0, st, g->cand_sys ? g->cand_sys : g->sys, g->batch, reinterpret_cast<const int2*>(g->rows), g->stride,
                                                     g->row_ptr, g->src, g->tgt, g->shift, g->edge_index, g->cell_offsets,
                                                     g->src_ptr ? g->src_count : nullptr, e, n);
     } else {  // edges given by the caller, sorted by target: row_ptr and the by-source counts from them
         if (!g->count) return FCB200_EINVAL;
         if (cudaMemsetAsync(g->count, 0, (size_t)n * 4, st) != cudaSuccess) return launch_status();
-        step::graph_count_kernel<<<ge, 256, 0, st>>>(g->tgt, g->count, e);
-        step::graph_scan_kernel<<<1, 1024, 0, st>>>(g->count, g->row_ptr, n, g->chunk_edges, g->info);
-        if (g->src_ptr) step::graph_count_kernel<<<ge, 256, 0, st>>>(g->src, g->src_count, e);
+        launch_pdl(step::graph_count_kernel, dim3(ge), dim3(256), 0, st, g->tgt, g->count, e);
+        launch_pdl(step::graph_scan_kernel, dim3(1), dim3(1024), 0, st, g->count, g->row_ptr, n, g->chunk_edges, g->info);
+        if (g->src_ptr) launch_pdl(step::graph_count_kernel, dim3(ge), dim3(256), 0, st, g->src, g->src_count, e);
     }
     if (g->src_ptr) {
-        step::graph_scan_kernel<<<1, 1024, 0, st>>>(g->src_count, g->src_ptr, n, 1, nullptr);
-        step::graph_bucket_kernel<<<ge, 256, 0, st>>>(g->src, g->src_ptr, g->src_count, g->src_tmp, e);
-        step::graph_order_kernel<<<gn, 256, 0, st>>>(g->src_tmp, g->src_ptr, g->src_perm, g->chunk_src, g->info + step::kInfoEdgeCut,
+        launch_pdl(step::graph_scan_kernel, dim3(1), dim3(1024), 0, st, g->src_count, g->src_ptr, n, 1, nullptr);
+        launch_pdl(step::graph_bucket_kernel, dim3(ge), dim3(256), 0, st, g->src, g->src_ptr, g->src_count, g->src_tmp, e);
+        launch_pdl(step::graph_order_kernel, dim3(gn), dim3(256), 0, st, g->src_tmp, g->src_ptr, g->src_perm, g->chunk_src, g->info + step::kInfoEdgeCut,
                                                      g->num_chunks, n);
     }
     return launch_status();

@@ -201,7 +201,10 @@ struct Run {
     void* stream;
     Run(const fcb200_model& m, const fcb200_eval& e, void* s, bool backward) : md(m), ev(e), d(m.lmax), st(static_cast<cudaStream_t>(s)), stream(s) {
         lay_out(m, e, backward, L);
+        pdl_launches = e.num_edges <= kPdlEdges;
     }
+    ~Run() { pdl_launches = false; }
+    Run(const Run&) = delete;
 
     void hook(const char* name, int begin, int64_t bytes, int64_t flops = 0, int launches = 1) const {
         if (g_hook) g_hook(name, begin, bytes, flops, launches);
@@ -307,11 +310,9 @@ static int launch_rotate_back(const Run& r, const float* msg, int64_t e_base, co
         constexpr int bytes = WPN * Shape<LMAX>::kL * C * 4;
         static bool done[64] = {};
         FCB_TRY(raise_smem(rotate_back_kernel<LMAX, MODE, WPN>, bytes, done));
-        rotate_back_kernel<LMAX, MODE, WPN><<<(int)(n1 - n0), WPN * 32, bytes, r.st>>>(
-            msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
+        launch_pdl((rotate_back_kernel<LMAX, MODE, WPN>), dim3((int)(n1 - n0)), dim3(WPN * 32), bytes, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
     } else {
-        rotate_back_kernel<LMAX, MODE, 1><<<warp_grid(n1 - n0, 4), 128, 0, r.st>>>(
-            msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
+        launch_pdl((rotate_back_kernel<LMAX, MODE, 1>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
     }
     return FCB200_OK;
 }
@@ -322,11 +323,9 @@ static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, co
     constexpr int WPN = 8;
     const Layout& L = r.L;
     if (share_node(n1 - n0)) {
-        gather_bwd_kernel<LMAX, HALF, WPN><<<(int)(n1 - n0), WPN * 32, WPN * 9 * C * 4, r.st>>>(
-            L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, L.tau_n, store_tau, L.grad.out(), scale, e0, n0, n1);
+        launch_pdl((gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>), dim3((int)(n1 - n0)), dim3(WPN * 32), WPN * 9 * C * 4, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, L.tau_n, store_tau, L.grad.out(), scale, e0, n0, n1);
     } else {
-        gather_bwd_kernel<LMAX, HALF, 1><<<warp_grid(n1 - n0, 4), 128, 0, r.st>>>(
-            L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, L.tau_n, store_tau, L.grad.out(), scale, e0, n0, n1);
+        launch_pdl((gather_bwd_kernel<LMAX, HALF, 1, OutSplit>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, L.tau_n, store_tau, L.grad.out(), scale, e0, n0, n1);
     }
     return FCB200_OK;
 }
@@ -347,14 +346,14 @@ int Run::radial_hidden_forward() {
                      0, pre1, L.rw, L.rw, nullptr, 0, nullptr, nullptr, ec));
         const int grid = warp_grid(ec * nets, 8);
         FCB_TRY(op("radial_act_fwd", ec * nets * 1040, [&] {
-            radial_fwd_kernel<<<grid, 256, 0, st>>>(pre1, md.table_src, md.table_tgt, ev.z, ev.src, ev.tgt, md.ln1_w, md.ln1_b, md.radial_eps,
+            launch_pdl(radial_fwd_kernel, dim3(grid), dim3(256), 0, st, pre1, md.table_src, md.table_tgt, ev.z, ev.src, ev.tgt, md.ln1_w, md.ln1_b, md.radial_eps,
                                                     L.h1.out(), L.rw, C, L.rst1 + k0 * nets * 2, e0, ec, nets);
             return 0;
         }));
         FCB_TRY(conv("so2_conv_fused_radial_in", c1, L.h1.hi, L.h1.lo, L.rw, L.rw, 0, pre2, L.rw, L.rw, nullptr, 0, nullptr, nullptr, ec));
         __half* h = L.h2 + e0 * L.rw * 2;
         return op("radial_act_fwd", ec * nets * 1032, [&] {
-            radial_fwd_kernel<<<grid, 256, 0, st>>>(pre2, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b, md.radial_eps,
+            launch_pdl(radial_fwd_kernel, dim3(grid), dim3(256), 0, st, pre2, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b, md.radial_eps,
                                                     OutSplit{h, h + C, 1.0f}, L.rw * 2, 2 * C, L.rst2 + k0 * nets * 2, e0, ec, nets);
             return 0;
         });
@@ -368,7 +367,7 @@ int Run::layer_forward(int l, const float* ffn_prev) {
     const float* x_prev = l == 0 ? q.x0 : L.layer[l - 1].x1;
     FCB_TRY(op("rms_norm_sh_fwd", n * row * 4 * (ffn_prev ? 4 : 2), [&] {
         return by_lmax([&](auto lm) {
-            norm_fwd_kernel<decltype(lm)::value><<<warp_grid(n, 4), 128, 0, st>>>(x_prev, ffn_prev, q.x0, w.norm1_w, w.norm1_b, L.sys, ev.batch,
+            launch_pdl(norm_fwd_kernel<decltype(lm)::value>, dim3(warp_grid(n, 4)), dim3(128), 0, st, x_prev, ffn_prev, q.x0, w.norm1_w, w.norm1_b, L.sys, ev.batch,
                                                                                 q.xn1, OutSplit{}, OutSplit{}, q.st1, w.eps1, n);
             return 0;
         });
@@ -409,7 +408,7 @@ int Run::ffn_forward(int l) {
     const int64_t n = L.n, row = d.nl * C;
     FCB_TRY(op("rms_norm_sh_fwd", n * row * 8, [&] {
         return by_lmax([&](auto lm) {
-            norm_fwd_kernel<decltype(lm)::value><<<warp_grid(n, 4), 128, 0, st>>>(q.x1, nullptr, nullptr, w.norm2_w, w.norm2_b, nullptr, nullptr,
+            launch_pdl(norm_fwd_kernel<decltype(lm)::value>, dim3(warp_grid(n, 4)), dim3(128), 0, st, q.x1, nullptr, nullptr, w.norm2_w, w.norm2_b, nullptr, nullptr,
                                                                                 nullptr, L.xn2.out(), OutSplit{}, q.st2, w.eps2, n);
             return 0;
         });
@@ -431,7 +430,7 @@ int Run::ffn_forward(int l) {
 int Run::forward() {
     const int64_t n = L.n, e = L.e;
     FCB_TRY(op("system_embedding", 0, [&] {
-        system_kernel<<<ev.num_systems, C, 0, st>>>(ev.charge, ev.spin, ev.dataset, md.charge_emb, md.spin_emb, md.dataset_emb, md.csd_w_t, md.csd_b,
+        launch_pdl(system_kernel, dim3(ev.num_systems), dim3(8 * C), 0, st, ev.charge, ev.spin, ev.dataset, md.charge_emb, md.spin_emb, md.dataset_emb, md.csd_w_t, md.csd_b,
                                                     L.sys, ev.status);
         return 0;
     }));
@@ -441,7 +440,7 @@ int Run::forward() {
             constexpr int bytes = 128 * Shape<LM>::kW * 4;
             static bool done[64] = {};
             FCB_TRY(raise_smem(geometry_fwd_kernel<LM>, bytes, done));
-            geometry_fwd_kernel<LM><<<(unsigned)((e + 127) / 128), 128, bytes, st>>>(ev.pos, ev.src, ev.tgt, ev.shift, ev.gamma, L.vec, L.env, L.wig,
+            launch_pdl(geometry_fwd_kernel<LM>, dim3((unsigned)((e + 127) / 128)), dim3(128), bytes, st, ev.pos, ev.src, ev.tgt, ev.shift, ev.gamma, L.vec, L.env, L.wig,
                                                                                     L.gauss.hi, L.gauss.lo, basis(), e);
             return 0;
         });
@@ -459,7 +458,7 @@ int Run::forward() {
     }
     return op("rms_norm_sh_fwd", n * d.nl * C * 16, [&] {
         return by_lmax([&](auto lm) {
-            norm_fwd_kernel<decltype(lm)::value><<<warp_grid(n, 4), 128, 0, st>>>(L.layer.back().x1, L.ffn_out, L.xl, md.norm_w, md.norm_b, nullptr,
+            launch_pdl(norm_fwd_kernel<decltype(lm)::value>, dim3(warp_grid(n, 4)), dim3(128), 0, st, L.layer.back().x1, L.ffn_out, L.xl, md.norm_w, md.norm_b, nullptr,
                                                                                 nullptr, ev.x_out, OutSplit{}, L.row0.out(), L.stl, md.norm_eps, n);
             return 0;
         });
@@ -477,7 +476,7 @@ int Run::energy() {
     FCB_TRY(conv("head", c2, L.hh.hi, L.hh.lo, C, C, 0, L.hy2, C, C, nullptr, 0, nullptr, nullptr, n));
     const int per = n < 148 * 64 ? 1 : 16;
     return op("energy_sum", n * C * 4, [&] {
-        energy_kernel<<<(unsigned)((n + 8 * per - 1) / (8 * per)), 256, 0, st>>>(L.hy2, md.head_w3, md.head_b3, ev.batch, ev.energy, n, per);
+        launch_pdl(energy_kernel, dim3((unsigned)((n + 8 * per - 1) / (8 * per))), dim3(256), 0, st, L.hy2, md.head_w3, md.head_b3, ev.batch, ev.energy, n, per);
         return 0;
     });
 }
@@ -489,7 +488,7 @@ int Run::layer_backward(int l) {
     const int k = 2 * (md.num_layers - 1 - l);
     Scale* s = L.scales + k;
     // node feed-forward
-    FCB_TRY(op("split_planes", n * row * 8, [&] { split_kernel<<<warp_grid(n * row / 4, 256), 256, 0, st>>>(L.g, L.gp.out(), &s->scale, n * row / 4); return 0; }));
+    FCB_TRY(op("split_planes", n * row * 8, [&] { launch_pdl(split_kernel, dim3(warp_grid(n * row / 4, 256)), dim3(256), 0, st, L.g, L.gp.out(), &s->scale, n * row / 4); return 0; }));
     Conv b2, b1;
     b2.w[0] = &w.ffn_out_t;
     b1.w[0] = &w.ffn_in_t0, b1.w[1] = &w.ffn_in_t;
@@ -505,7 +504,7 @@ int Run::layer_backward(int l) {
     FCB_TRY(conv("ffn_in_bwd", b1, L.gy2.hi, L.gy2.lo, fw, fw, 0, L.gxn, row, row, nullptr, 0, &s->scale, nullptr, n));
     FCB_TRY(op("rms_norm_sh_bwd", n * row * 16, [&] {
         return by_lmax([&](auto lm) {
-            norm_bwd_kernel<decltype(lm)::value, false><<<warp_grid(n, 4), 128, 0, st>>>(L.gxn, q.x1, w.norm2_w, q.st2, L.g, L.g1, s + 1, n);
+            launch_pdl((norm_bwd_kernel<decltype(lm)::value, false>), dim3(warp_grid(n, 4)), dim3(128), 0, st, L.gxn, q.x1, w.norm2_w, q.st2, L.g, L.g1, s + 1, n);
             return 0;
         });
     }));
@@ -540,8 +539,7 @@ int Run::layer_backward(int l) {
         float* y = q.y + e0 * d.yw;
         FCB_TRY(op("rotate_back_bwd", ec * 4 * (d.nl * C + 2 * d.nm * C + d.nw + 9), [&] {
             return by_lmax([&](auto lm) {
-                rotate_back_bwd_kernel<decltype(lm)::value, 0, OutSplit><<<warp_grid(ec, 4), 128, 0, st>>>(
-                    L.g1, q.msg + e0 * d.nm * C, L.wig, L.env, ev.tgt, L.gmsg.out(), scale, L.tau_e, !first_layer, 1.0f, e0, ec);
+                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 0, OutSplit>), dim3(warp_grid(ec, 4)), dim3(128), 0, st, L.g1, q.msg + e0 * d.nm * C, L.wig, L.env, ev.tgt, L.gmsg.out(), scale, L.tau_e, !first_layer, 1.0f, e0, ec);
                 return 0;
             });
         }));
@@ -560,7 +558,7 @@ int Run::layer_backward(int l) {
     }));
     return op("rms_norm_sh_bwd", n * row * 16, [&] {
         return by_lmax([&](auto lm) {
-            norm_bwd_kernel<decltype(lm)::value, false><<<warp_grid(n, 4), 128, 0, st>>>(L.gxn, q.x0, w.norm1_w, q.st1, L.g1, L.g, s + 2, n);
+            launch_pdl((norm_bwd_kernel<decltype(lm)::value, false>), dim3(warp_grid(n, 4)), dim3(128), 0, st, L.gxn, q.x0, w.norm1_w, q.st1, L.g1, L.g, s + 2, n);
             return 0;
         });
     });
@@ -572,7 +570,7 @@ int Run::backward() {
     if (cudaMemsetAsync(L.scales, 0, nscale * sizeof(Scale), st) != cudaSuccess) return launch_status();
     if (!ev.grad_x) {
         FCB_TRY(op("energy_bwd", n * C * 8, [&] {
-            energy_bwd_kernel<<<warp_grid(n * C / 4, 256), 256, 0, st>>>(L.hy2, md.head_w3, L.hg.out(), md.head_scale, n);
+            launch_pdl(energy_bwd_kernel, dim3(warp_grid(n * C / 4, 256)), dim3(256), 0, st, L.hy2, md.head_w3, L.hg.out(), md.head_scale, n);
             return 0;
         }));
         Conv b2, b1;
@@ -588,9 +586,9 @@ int Run::backward() {
         return by_lmax([&](auto lm) {
             constexpr int LM = decltype(lm)::value;
             if (ev.grad_x)
-                norm_bwd_kernel<LM, false><<<warp_grid(n, 4), 128, 0, st>>>(ev.grad_x, L.xl, md.norm_w, L.stl, nullptr, L.g, L.scales, n);
+                launch_pdl((norm_bwd_kernel<LM, false>), dim3(warp_grid(n, 4)), dim3(128), 0, st, ev.grad_x, L.xl, md.norm_w, L.stl, nullptr, L.g, L.scales, n);
             else
-                norm_bwd_kernel<LM, true><<<warp_grid(n, 4), 128, 0, st>>>(L.g0, L.xl, md.norm_w, L.stl, nullptr, L.g, L.scales, n);
+                launch_pdl((norm_bwd_kernel<LM, true>), dim3(warp_grid(n, 4)), dim3(128), 0, st, L.g0, L.xl, md.norm_w, L.stl, nullptr, L.g, L.scales, n);
             return 0;
         });
     }));
@@ -604,8 +602,7 @@ int Run::backward() {
         FCB_TRY(degree_out(e0, ec));
         FCB_TRY(op("edge_degree_bwd", ec * 4 * (d.nl * C + 2 * (d.lmax + 1) * C + d.nw + 9), [&] {
             return by_lmax([&](auto lm) {
-                rotate_back_bwd_kernel<decltype(lm)::value, 1, OutSplit><<<warp_grid(ec, 4), 128, 0, st>>>(
-                    L.g, L.r3, L.wig, L.env, ev.tgt, L.gr3.out(), scale, L.tau_e, 1, 1.0f / md.rescale, e0, ec);
+                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 1, OutSplit>), dim3(warp_grid(ec, 4)), dim3(128), 0, st, L.g, L.r3, L.wig, L.env, ev.tgt, L.gr3.out(), scale, L.tau_e, 1, 1.0f / md.rescale, e0, ec);
                 return 0;
             });
         }));
@@ -613,21 +610,20 @@ int Run::backward() {
         FCB_TRY(gemm("so2_conv_fused_radial_out_bwd", L.gr3, md.degree_out_t, scale, gh + (int64_t)md.num_layers * C, L.rw, ec));
         const int grid = warp_grid(ec * nets, 8);
         FCB_TRY(op("radial_act_bwd", ec * nets * 1544, [&] {
-            radial_bwd_kernel<<<grid, 256, 0, st>>>(gh, L.pre2 + e0 * L.rw, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b,
+            launch_pdl(radial_bwd_kernel, dim3(grid), dim3(256), 0, st, gh, L.pre2 + e0 * L.rw, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b,
                                                     L.rst2 + e0 * nets * 2, L.rp.out(), L.rw, C, L.scales, nscale, L.rad_scale, e0, ec, nets);
             return 0;
         }));
         FCB_TRY(conv("so2_conv_fused_radial_in", c1, L.rp.hi, L.rp.lo, L.rw, L.rw, 0, L.rh, L.rw, L.rw, nullptr, 0, L.rad_scale, nullptr, ec));
         FCB_TRY(op("radial_act_bwd", ec * nets * 1544, [&] {
-            radial_bwd_kernel<<<grid, 256, 0, st>>>(L.rh, L.pre1 + e0 * L.rw, md.table_src, md.table_tgt, ev.z, ev.src, ev.tgt, md.ln1_w, md.ln1_b,
+            launch_pdl(radial_bwd_kernel, dim3(grid), dim3(256), 0, st, L.rh, L.pre1 + e0 * L.rw, md.table_src, md.table_tgt, ev.z, ev.src, ev.tgt, md.ln1_w, md.ln1_b,
                                                     L.rst1 + e0 * nets * 2, L.rp.out(), L.rw, C, L.scales, nscale, L.rad_scale, e0, ec, nets);
             return 0;
         }));
         FCB_TRY(gemm("so2_conv_fused_radial_in", L.rp, md.rad_w0_t, L.rad_scale, L.ggauss, md.num_basis, ec));
         return op("edge_geometry_bwd", ec * 4 * (md.num_basis + 9 + 4 + 8 + 3), [&] {
             return by_lmax([&](auto lm) {
-                geometry_bwd_kernel<decltype(lm)::value><<<(unsigned)((ec + 127) / 128), 128, 0, st>>>(
-                    L.vec + e0, L.wig + e0 * d.nw, reinterpret_cast<float4*>(L.tau_n) + e0, reinterpret_cast<float4*>(L.tau_e) + e0, L.ggauss,
+                launch_pdl(geometry_bwd_kernel<decltype(lm)::value>, dim3((unsigned)((ec + 127) / 128)), dim3(128), 0, st, L.vec + e0, L.wig + e0 * d.nw, reinterpret_cast<float4*>(L.tau_n) + e0, reinterpret_cast<float4*>(L.tau_e) + e0, L.ggauss,
                     L.grad_vec + e0 * 3, basis(), ec);
                 return 0;
             });
@@ -636,12 +632,12 @@ int Run::backward() {
     if (ev.virial) {
         const int per = e < 148 * 64 * 8 ? 8 : 128;
         FCB_TRY(op("virial", e * 28, [&] {
-            virial_kernel<<<(unsigned)((e + 8 * per - 1) / (8 * per)), 256, 0, st>>>(L.grad_vec, L.vec, ev.tgt, ev.batch, ev.virial, e, per);
+            launch_pdl(virial_kernel, dim3((unsigned)((e + 8 * per - 1) / (8 * per))), dim3(256), 0, st, L.grad_vec, L.vec, ev.tgt, ev.batch, ev.virial, e, per);
             return 0;
         }));
     }
     return op("grad_pos", e * 24 + n * 12, [&] {
-        grad_pos_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(L.grad_vec, ev.row_ptr, ev.src_ptr, ev.src_perm, ev.grad_pos, ev.grad_sign, n);
+        launch_pdl(grad_pos_kernel, dim3((unsigned)((n + 7) / 8)), dim3(256), 0, st, L.grad_vec, ev.row_ptr, ev.src_ptr, ev.src_perm, ev.grad_pos, ev.grad_sign, n);
         return 0;
     });
 }

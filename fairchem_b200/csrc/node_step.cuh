@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(128)
                     const float* __restrict__ weight, const float* __restrict__ bias, const float* __restrict__ sys,
                     const int32_t* __restrict__ batch, float* __restrict__ out_f32, OutSplit planes, OutSplit row0,
                     float* __restrict__ stats, float eps, int64_t num_nodes) {
+    pdl_sync();
     constexpr int kL = (LMAX + 1) * (LMAX + 1);
     planes.s = row0.s = 1.0f;
     const int lane = threadIdx.x & 31, c = lane * 4;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(128)
     norm_bwd_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ weight,
                     const float* __restrict__ stats, const float* __restrict__ residual, float* __restrict__ grad_x,
                     Scale* __restrict__ scale_out, int64_t num_nodes) {
+    pdl_sync();
     constexpr int kL = (LMAX + 1) * (LMAX + 1);
     const int lane = threadIdx.x & 31, c = lane * 4;
     float amax = 0.f;
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(128)
 // half planes of a float32 tensor times a device scale
 __global__ void __launch_bounds__(256)
     split_kernel(const float* __restrict__ in, OutSplit out, const float* __restrict__ scale_ptr, int64_t quads) {
+    pdl_sync();
     out.load_scale(scale_ptr);
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < quads; i += (int64_t)gridDim.x * 256) out.st(i * 4, ld4(in + i * 4));
 }
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(256)
                       const int32_t* __restrict__ z, const int32_t* __restrict__ src, const int32_t* __restrict__ tgt,
                       const float* __restrict__ gamma, const float* __restrict__ beta, float eps, OutSplit out, int64_t out_ld,
                       int out_net, float* __restrict__ stats, int64_t e_base, int64_t num_edges, int nets) {
+    pdl_sync();
     out.s = 1.0f;
     const int lane = threadIdx.x & 31, c = lane * 4;
     const int64_t items = num_edges * nets, width = (int64_t)nets * C;
@@ -178,6 +182,7 @@ __global__ void __launch_bounds__(256)
                       const int32_t* __restrict__ tgt, const float* __restrict__ gamma, const float* __restrict__ beta,
                       const float* __restrict__ stats, OutSplit out, int64_t out_ld, int out_net, const Scale* __restrict__ scales,
                       int num_scales, float* __restrict__ scale_out, int64_t e_base, int64_t num_edges, int nets) {
+    pdl_sync();
     float s = scales[0].scale;
     for (int i = 1; i < num_scales; ++i) s = fminf(s, scales[i].scale);
     out.s = s;
@@ -211,25 +216,34 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// ---- system embedding: silu(W [charge | spin | dataset] + b), one block per system, thread = output channel ---------
-__global__ void __launch_bounds__(C)
+// ---- system embedding: silu(W [charge | spin | dataset] + b), one block per system ----------------------------------
+// Eight threads share an output channel, 48 of the 384 products each: one system is a latency chain (384 dependent
+// multiply-adds behind their weight loads took 25 us).
+__global__ void __launch_bounds__(8 * C)
     system_kernel(const int64_t* __restrict__ charge, const int64_t* __restrict__ spin, const int32_t* __restrict__ dataset,
                   const float* __restrict__ charge_emb, const float* __restrict__ spin_emb, const float* __restrict__ dataset_emb,
                   const float* __restrict__ w_t, const float* __restrict__ bias, float* __restrict__ out, int32_t* __restrict__ status) {
-    __shared__ float in[3 * C];
-    const int s = blockIdx.x, c = threadIdx.x;
+    pdl_sync();
+    __shared__ float part[8][C];
+    const int s = blockIdx.x, c = threadIdx.x & (C - 1), p = threadIdx.x / C;
     int64_t q = charge[s] + 100, m = spin[s];
     if (q < 0 || q > 200 || m < 0 || m > 100) {  // outside the embedding tables: report, do not read
-        if (c == 0) atomicExch(status, 3);
+        if (threadIdx.x == 0) atomicExch(status, 3);
         q = m = 0;
     }
-    in[c] = charge_emb[q * C + c];
-    in[C + c] = spin_emb[m * C + c];
-    in[2 * C + c] = dataset_emb[dataset[s] * C + c];
+    const float* rows[3] = {charge_emb + q * C, spin_emb + m * C, dataset_emb + (int64_t)dataset[s] * C};
+    float acc = 0.f;
+#pragma unroll 16
+    for (int j = 0; j < 48; ++j) {
+        const int k = p * 48 + j;
+        acc = fmaf(__ldg(rows[k / C] + k % C), __ldg(w_t + k * C + c), acc);
+    }
+    part[p][c] = acc;
     __syncthreads();
-    float acc = bias[c];
-#pragma unroll 8
-    for (int k = 0; k < 3 * C; ++k) acc = fmaf(in[k], w_t[k * C + c], acc);
+    if (p) return;
+    acc = bias[c];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc += part[i][c];
     out[s * C + c] = acc * sigm(acc);
 }
 
@@ -239,6 +253,7 @@ __global__ void __launch_bounds__(C)
 __global__ void __launch_bounds__(256)
     energy_kernel(const float* __restrict__ y, const float* __restrict__ w, const float* __restrict__ b, const int32_t* __restrict__ batch,
                   double* __restrict__ energy, int64_t num_nodes, int per_warp) {
+    pdl_sync();
     const int lane = threadIdx.x & 31, c = lane * 4;
     const int64_t n0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * per_warp;
     const float4 wv = ld4(w + c);
@@ -262,6 +277,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     energy_bwd_kernel(const float* __restrict__ y, const float* __restrict__ w, OutSplit out, const float* __restrict__ scale_ptr,
                       int64_t num_nodes) {
+    pdl_sync();
     out.load_scale(scale_ptr);
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < num_nodes * (C / 4); i += (int64_t)gridDim.x * 256) {
         const float4 v = ld4(y + i * 4), wv = ld4(w + (i % (C / 4)) * 4);
@@ -273,6 +289,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     virial_kernel(const float* __restrict__ grad_vec, const float4* __restrict__ vec, const int32_t* __restrict__ tgt,
                   const int32_t* __restrict__ batch, double* __restrict__ virial, int64_t num_edges, int per_warp) {
+    pdl_sync();
     const int lane = threadIdx.x & 31;
     const int64_t w0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * per_warp;
     const int i = lane / 3, j = lane % 3;  // lanes 0..8 own one component each

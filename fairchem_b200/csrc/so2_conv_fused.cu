@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    pdl_sync();  // barriers and tensor memory are set up while the predecessor finishes
 
     if (warp >= 4) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
@@ -709,7 +710,7 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
     const int grid = (int)(items < sm_count() ? items : sm_count());
     auto launch = [&](auto kernel, bool (&done)[64]) {
         if (const int arc = ensure_dynamic_smem(kernel, kSmemBytes, done)) return arc;
-        kernel<<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm, items);
+        launch_pdl(kernel, dim3(grid), dim3(kThreads), kSmemBytes, st, mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm, items);
         return launch_status();
     };
     static bool done[3][64] = {};

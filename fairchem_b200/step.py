@@ -9,6 +9,7 @@ counts, another contraction mode, a partitioned system); those run the per-op pa
 from __future__ import annotations
 
 import ctypes
+import operator
 from ctypes import POINTER, Structure, byref, c_float, c_int32, c_int64, c_void_p
 
 import torch
@@ -52,8 +53,11 @@ class EvalStruct(Structure):
                 + [("grad_sign", c_float), ("virial", c_void_p), ("status", c_void_p)])
 
 
-def _versions(params) -> tuple:
-    return tuple([p._version for p in params] + [p.data_ptr() for p in params])
+_VERSION = operator.attrgetter("_version")
+
+
+def _versions(params) -> list:
+    return [*map(_VERSION, params), *map(torch.Tensor.data_ptr, params)]
 
 
 class _Weights:
@@ -137,24 +141,24 @@ class ModelPlan:
 
     @staticmethod
     def supported(bb) -> bool:
-        from .backbone import _GemmState
-
+        """Shapes that csrc/model_step.cu is written for."""
         nets = _radial_nets(bb)
-        return (_GemmState.precision == 2 and _GemmState.fused_conv and _GemmState.native and not ops.generic_kernels()
-                and ops.CONV_VARIANT == -1 and bb.keep_level is None and bb.sphere_channels == C and bb.hidden_channels == C
-                and bb.edge_channels == C and bb.num_distance_basis % 32 == 0 and 1 <= bb.num_layers < 40
+        return (bb.sphere_channels == C and bb.hidden_channels == C and bb.edge_channels == C and bb.num_distance_basis % 32 == 0
+                and 1 <= bb.num_layers < 40
                 and all(len(n.net) == 7 and n.net[1].eps == n.net[4].eps == nets[0].net[1].eps for n in nets))
 
     @classmethod
     def of(cls, bb):
         """The backbone's plan, or None when the native path does not apply."""
-        if not cls.supported(bb):
+        from .backbone import _GemmState as mode
+
+        if not (mode.precision == 2 and mode.fused_conv and mode.native and ops.CONV_VARIANT == -1 and bb.keep_level is None) or ops.generic_kernels():
             return None
         plan = getattr(bb, "_step_plan", None)
         if plan is not None and plan.versions == _versions(plan.params):
             return plan
         params = list(bb.parameters())
-        if not params[0].is_cuda or any(p.dtype != torch.float32 for p in params):
+        if not cls.supported(bb) or not params[0].is_cuda or any(p.dtype != torch.float32 for p in params):
             return None
         bb._step_plan = plan = cls(bb, params)
         return plan
@@ -163,7 +167,7 @@ class ModelPlan:
         """The model struct with the energy head's weights filled in (cached on the head), or None."""
         eb = head.energy_block
         params = list(eb.parameters())
-        key = (id(self), _versions(params))
+        key = (id(self), *_versions(params))
         hit = getattr(head, "_step_model", None)
         if hit is not None and hit[0] == key:
             return hit[1]
