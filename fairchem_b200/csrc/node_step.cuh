@@ -144,8 +144,37 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- hidden activations of the radial MLPs ------------------------------------------------------------------------
-// SiLU(LayerNorm(pre + element tables)) for `nets` MLPs side by side, one warp per (edge, net).  Rows: pre [E, nets*C],
-// stats [E, nets, 2]; output planes at out_off = i * out_ld + net * out_net.
+// SiLU(LayerNorm(pre + element tables)) for `nets` MLPs side by side.  Rows: pre [E, nets*C], stats [E, nets, 2]; output
+// planes at i * out_ld + net * out_net.  One warp per edge and kNetBatch nets: one row of 512 bytes per warp left the
+// loads and the two reductions of a row in series (3.1 M edges x 5 nets: 10.8 ms forward, 14.0 ms backward).
+constexpr int kNetBatch = 3;
+
+struct RadialItem {
+    int64_t i;
+    int net0, n;
+};
+__device__ __forceinline__ RadialItem radial_item(int64_t it, int nets) {
+    const int groups = (nets + kNetBatch - 1) / kNetBatch;
+    const int64_t i = it / groups;
+    const int net0 = (int)(it - i * groups) * kNetBatch;
+    return {i, net0, min(kNetBatch, nets - net0)};
+}
+__host__ __device__ inline int64_t radial_items(int64_t edges, int nets) { return edges * ((nets + kNetBatch - 1) / kNetBatch); }
+
+__device__ __forceinline__ void radial_rows(float4 (&y)[kNetBatch], const RadialItem& q, const float* __restrict__ pre, const float* __restrict__ ts,
+                                            const float* __restrict__ tt, const int32_t* __restrict__ z, const int32_t* __restrict__ src,
+                                            const int32_t* __restrict__ tgt, int64_t e_base, int64_t width, int c) {
+#pragma unroll
+    for (int b = 0; b < kNetBatch; ++b) y[b] = b < q.n ? ld4(pre + q.i * width + (q.net0 + b) * C + c) : f4zero();
+    if (ts) {
+        const float* s0 = ts + z[src[e_base + q.i]] * width + q.net0 * C + c;
+        const float* t0 = tt + z[tgt[e_base + q.i]] * width + q.net0 * C + c;
+#pragma unroll
+        for (int b = 0; b < kNetBatch; ++b)
+            if (b < q.n) y[b] = add4(y[b], add4(ld4(s0 + b * C), ld4(t0 + b * C)));
+    }
+}
+
 __global__ void __launch_bounds__(256)
     radial_fwd_kernel(const float* __restrict__ pre, const float* __restrict__ ts, const float* __restrict__ tt,
                       const int32_t* __restrict__ z, const int32_t* __restrict__ src, const int32_t* __restrict__ tgt,
@@ -154,23 +183,29 @@ __global__ void __launch_bounds__(256)
     pdl_sync();
     out.s = 1.0f;
     const int lane = threadIdx.x & 31, c = lane * 4;
-    const int64_t items = num_edges * nets, width = (int64_t)nets * C;
+    const int64_t items = radial_items(num_edges, nets), width = (int64_t)nets * C;
     for (int64_t it = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); it < items; it += (int64_t)gridDim.x * 8) {
-        const int64_t i = it / nets;
-        const int net = (int)(it - i * nets), col = net * C + c;
-        float4 y = ld4(pre + i * width + col);
-        if (ts) {
-            y = add4(y, ld4(ts + z[src[e_base + i]] * width + col));
-            y = add4(y, ld4(tt + z[tgt[e_base + i]] * width + col));
+        const RadialItem q = radial_item(it, nets);
+        float4 y[kNetBatch];
+        radial_rows(y, q, pre, ts, tt, z, src, tgt, e_base, width, c);
+        float mean[kNetBatch], rstd[kNetBatch];
+#pragma unroll
+        for (int b = 0; b < kNetBatch; ++b) mean[b] = warp_sum(hsum4(y[b])) * (1.0f / C);
+#pragma unroll
+        for (int b = 0; b < kNetBatch; ++b) {
+            y[b] = make_float4(y[b].x - mean[b], y[b].y - mean[b], y[b].z - mean[b], y[b].w - mean[b]);
+            rstd[b] = rsqrtf(warp_sum(dot4(y[b], y[b])) * (1.0f / C) + eps);
         }
-        const float mean = warp_sum(hsum4(y)) * (1.0f / C);
-        const float4 d = make_float4(y.x - mean, y.y - mean, y.z - mean, y.w - mean);
-        const float rstd = rsqrtf(warp_sum(dot4(d, d)) * (1.0f / C) + eps);
-        const float4 gm = ld4(gamma + col), b = ld4(beta + col);
-        const float4 v = make_float4(fmaf(d.x * rstd, gm.x, b.x), fmaf(d.y * rstd, gm.y, b.y), fmaf(d.z * rstd, gm.z, b.z),
-                                     fmaf(d.w * rstd, gm.w, b.w));
-        out.st(i * out_ld + net * out_net + c, make_float4(v.x * sigm(v.x), v.y * sigm(v.y), v.z * sigm(v.z), v.w * sigm(v.w)));
-        if (lane == 0) *reinterpret_cast<float2*>(stats + it * 2) = make_float2(mean, rstd);
+#pragma unroll
+        for (int b = 0; b < kNetBatch; ++b) {
+            if (b >= q.n) break;
+            const int col = (q.net0 + b) * C + c;
+            const float4 gm = ld4(gamma + col), bt = ld4(beta + col), d = y[b];
+            const float4 v = make_float4(fmaf(d.x * rstd[b], gm.x, bt.x), fmaf(d.y * rstd[b], gm.y, bt.y), fmaf(d.z * rstd[b], gm.z, bt.z),
+                                         fmaf(d.w * rstd[b], gm.w, bt.w));
+            out.st(q.i * out_ld + (q.net0 + b) * out_net + c, make_float4(v.x * sigm(v.x), v.y * sigm(v.y), v.z * sigm(v.z), v.w * sigm(v.w)));
+            if (lane == 0) *reinterpret_cast<float2*>(stats + (q.i * nets + q.net0 + b) * 2) = make_float2(mean[b], rstd[b]);
+        }
     }
 }
 
@@ -188,31 +223,36 @@ __global__ void __launch_bounds__(256)
     out.s = s;
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = s;
     const int lane = threadIdx.x & 31, c = lane * 4;
-    const int64_t items = num_edges * nets, width = (int64_t)nets * C;
+    const int64_t items = radial_items(num_edges, nets), width = (int64_t)nets * C;
     for (int64_t it = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); it < items; it += (int64_t)gridDim.x * 8) {
-        const int64_t i = it / nets;
-        const int net = (int)(it - i * nets), col = net * C + c;
-        float4 y = ld4(pre + i * width + col);
-        if (ts) {
-            y = add4(y, ld4(ts + z[src[e_base + i]] * width + col));
-            y = add4(y, ld4(tt + z[tgt[e_base + i]] * width + col));
-        }
-        const float2 st = *reinterpret_cast<const float2*>(stats + it * 2);
-        const float4 go = ld4(grad_out + i * width + col), gm = ld4(gamma + col), b = ld4(beta + col);
-        const float xh[4] = {(y.x - st.x) * st.y, (y.y - st.x) * st.y, (y.z - st.x) * st.y, (y.w - st.x) * st.y};
-        const float g[4] = {gm.x, gm.y, gm.z, gm.w}, bb[4] = {b.x, b.y, b.z, b.w}, gv[4] = {go.x, go.y, go.z, go.w};
-        float dx[4], s1 = 0.f, s2 = 0.f;
+        const RadialItem q = radial_item(it, nets);
+        float4 y[kNetBatch], go[kNetBatch];
+        float2 st[kNetBatch];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            dx[j] = gv[j] * dsilu(fmaf(xh[j], g[j], bb[j])) * g[j];
-            s1 += dx[j];
-            s2 = fmaf(dx[j], xh[j], s2);
+        for (int b = 0; b < kNetBatch; ++b) {
+            go[b] = b < q.n ? ld4(grad_out + q.i * width + (q.net0 + b) * C + c) : f4zero();
+            st[b] = b < q.n ? *reinterpret_cast<const float2*>(stats + (q.i * nets + q.net0 + b) * 2) : make_float2(0.f, 0.f);
         }
-        s1 = warp_sum(s1) * (1.0f / C);
-        s2 = warp_sum(s2) * (1.0f / C);
-        out.st(i * out_ld + net * out_net + c,
-               make_float4(st.y * (dx[0] - s1 - xh[0] * s2), st.y * (dx[1] - s1 - xh[1] * s2), st.y * (dx[2] - s1 - xh[2] * s2),
-                           st.y * (dx[3] - s1 - xh[3] * s2)));
+        radial_rows(y, q, pre, ts, tt, z, src, tgt, e_base, width, c);
+        float s1[kNetBatch], s2[kNetBatch];
+#pragma unroll
+        for (int b = 0; b < kNetBatch; ++b) {
+            const int col = (q.net0 + (b < q.n ? b : 0)) * C + c;
+            const float4 gm = ld4(gamma + col), bt = ld4(beta + col);
+            const float4 xh = make_float4((y[b].x - st[b].x) * st[b].y, (y[b].y - st[b].x) * st[b].y, (y[b].z - st[b].x) * st[b].y, (y[b].w - st[b].x) * st[b].y);
+            go[b] = make_float4(go[b].x * dsilu(fmaf(xh.x, gm.x, bt.x)) * gm.x, go[b].y * dsilu(fmaf(xh.y, gm.y, bt.y)) * gm.y,
+                                go[b].z * dsilu(fmaf(xh.z, gm.z, bt.z)) * gm.z, go[b].w * dsilu(fmaf(xh.w, gm.w, bt.w)) * gm.w);
+            y[b] = xh;
+            s1[b] = warp_sum(hsum4(go[b])) * (1.0f / C);
+            s2[b] = warp_sum(dot4(go[b], xh)) * (1.0f / C);
+        }
+#pragma unroll
+        for (int b = 0; b < kNetBatch; ++b) {
+            if (b >= q.n) break;
+            out.st(q.i * out_ld + (q.net0 + b) * out_net + c,
+                   make_float4(st[b].y * (go[b].x - s1[b] - y[b].x * s2[b]), st[b].y * (go[b].y - s1[b] - y[b].y * s2[b]),
+                               st[b].y * (go[b].z - s1[b] - y[b].z * s2[b]), st[b].y * (go[b].w - s1[b] - y[b].w * s2[b])));
+        }
     }
 }
 

@@ -114,22 +114,57 @@ struct Params {
 // instead of the ~20 of expf and an IEEE division -- the epilogue evaluates it for every output element
 __device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
 
-// Largest |hi| so far, NaN-propagating: an overflowed or invalid value becomes inf or NaN as a half, so this one packed
-// maximum per pair replaces range checks on the float32 values.
-__device__ __forceinline__ void store_split(__half* hi, __half* lo, int off, const float (&o)[4], __half2& top) {
+// Two float32 in a register pair; the packed instructions halve the epilogue's multiply and add count.
+typedef uint64_t f32x2;
+__device__ __forceinline__ f32x2 pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+template <class F> __device__ __forceinline__ f32x2 map2(f32x2 v, F f) {
+    float a, b;
+    unpack(v, a, b);
+    return pack(f(a), f(b));
+}
+
+// Two values -> packed halves hi and lo.  `top`: largest |hi| so far, NaN-propagating: an overflowed or invalid value
+// becomes inf or NaN as a half, so one packed maximum per pair replaces range checks on the float32 values.
+__device__ __forceinline__ void split2(f32x2 v, uint32_t& hi, uint32_t& lo, __half2& top) {
+    float a, b;
+    unpack(v, a, b);
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 hf = __half22float2(h);
+    unpack(mul2(fma2(pack(hf.x, hf.y), pack(-1.f, -1.f), v), pack(kLoScale, kLoScale)), a, b);
+    const __half2 l = __floats2half2_rn(a, b);
+    top = __hmax2_nan(top, __habs2(h));
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+__device__ __forceinline__ void store_split(__half* hi, __half* lo, int off, f32x2 o0, f32x2 o1, bool in, __half2& top) {
     uint2 h, l;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const float a = o[2 * j], b = o[2 * j + 1];
-        const __half2 hh = __floats2half2_rn(a, b);
-        const float2 hf = __half22float2(hh);
-        const __half2 ll = __floats2half2_rn((a - hf.x) * kLoScale, (b - hf.y) * kLoScale);
-        top = __hmax2_nan(top, __habs2(hh));
-        (j ? h.y : h.x) = *reinterpret_cast<const uint32_t*>(&hh);
-        (j ? l.y : l.x) = *reinterpret_cast<const uint32_t*>(&ll);
+    split2(o0, h.x, l.x, top);
+    split2(o1, h.y, l.y, top);
+    if (in) {
+        __stcs(reinterpret_cast<uint2*>(hi + off), h);  // streamed: not read again by this kernel
+        __stcs(reinterpret_cast<uint2*>(lo + off), l);
     }
-    __stcs(reinterpret_cast<uint2*>(hi + off), h);  // streamed: not read again by this kernel
-    __stcs(reinterpret_cast<uint2*>(lo + off), l);
+}
+__device__ __forceinline__ void store_pair(float* p, f32x2 a, f32x2 b) {
+    asm volatile("st.global.cs.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void load_pair(const float* p, f32x2& a, f32x2& b) {
+    asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
 }
 
 #define FCB_TMEM_LD16(r, taddr)                                                                                           \
@@ -156,12 +191,13 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
     const float a_scale = prm.a_scale ? *prm.a_scale : 1.0f;
     const float o_scale = prm.o_scale ? *prm.o_scale : 1.0f;
     __half2 top = __floats2half2_rn(0.f, 0.f);
-    float keepv[KIND == kPlainKind ? 1 : 2][32];  // forward: sigmoid of the gate; backward: gate-gradient sums
+    // per chunk and row: forward: o_scale * sigmoid of the gate; backward: gate-gradient sums
+    f32x2 keepv[KIND == kPlainKind ? 1 : 2][16];
     // Loads run one chunk ahead where the registers allow it: the second chunk's accumulator columns without a backward
     // input, else the y rows of the next chunk.
     constexpr bool kAhead = KIND != kBackwardKind;
-    float yv[KIND == kBackwardKind ? 32 : 1];
-    float sg[KIND == kBackwardKind ? 2 : 1][32];  // backward: sigmoid of the degree's gate, read once at its first row
+    f32x2 yv[KIND == kBackwardKind ? 16 : 1];
+    f32x2 sg[KIND == kBackwardKind ? 2 : 1][16];  // backward: o_scale * sigmoid of the degree's gate, read once at its first row
     // y lines of a backward tile on their way to L2 one tile early (lane = row; a warp's 64 columns are two lines)
     auto prefetch = [&](int64_t item2, int ti2) {
         if constexpr (KIND == kBackwardKind) {
@@ -188,8 +224,8 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
             if constexpr (KIND == kBackwardKind) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const float4 a = rr + 4 * i < live ? __ldcs(reinterpret_cast<const float4*>(yrow + 4 * i * prm.ldy + y_col + (half * 2 + c2) * 32)) : f4zero();
-                    yv[4 * i] = a.x, yv[4 * i + 1] = a.y, yv[4 * i + 2] = a.z, yv[4 * i + 3] = a.w;
+                    yv[2 * i] = yv[2 * i + 1] = 0;
+                    if (rr + 4 * i < live) load_pair(yrow + 4 * i * prm.ldy + y_col + (half * 2 + c2) * 32, yv[2 * i], yv[2 * i + 1]);
                 }
             }
         };
@@ -207,8 +243,8 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
             ok = __all_sync(kFull, ok);
             if (!ok) return;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float out_scale = 1.0f / (a_scale * prm.w_scale[t.w]);
-            const float corr_scale = out_scale / kLoScale;
+            const float out_scale = 1.0f / (a_scale * prm.w_scale[t.w]);  // a power of two: scaling after the sum is exact
+            const f32x2 os2 = pack(out_scale, out_scale);
             const float* bias = prm.bias[t.w];
             const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols) + ((uint32_t)(q * 32) << 16);  // main columns [0, 128), corrections [128, 256)
             const bool gate_silu = (t.flags & kGateSilu) != 0;
@@ -220,15 +256,14 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
             for (int c2 = 0; c2 < 2; ++c2) {
                 const int col = (half * 2 + c2) * 32;  // within the tile
                 // 1. accumulator -> shared tile, row `lane`
-                float poison = 0.f;  // becomes NaN if any value is inf or NaN (an overflowed half upstream)
+                f32x2 poison = 0;  // becomes NaN if any value is inf or NaN (an overflowed half upstream)
                 auto stage4 = [&](int v4, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, uint32_t c0, uint32_t c1, uint32_t c2_, uint32_t c3) {
-                    const float v0 = fmaf(__uint_as_float(c0), corr_scale, __uint_as_float(r0) * out_scale);
-                    const float v1 = fmaf(__uint_as_float(c1), corr_scale, __uint_as_float(r1) * out_scale);
-                    const float v2 = fmaf(__uint_as_float(c2_), corr_scale, __uint_as_float(r2) * out_scale);
-                    const float v3 = fmaf(__uint_as_float(c3), corr_scale, __uint_as_float(r3) * out_scale);
-                    if (KIND == kPlainKind || mode == kPlain) poison = fmaf(v0, 0.f, fmaf(v1, 0.f, fmaf(v2, 0.f, fmaf(v3, 0.f, poison))));
+                    const f32x2 lo = pack(1.0f / kLoScale, 1.0f / kLoScale);
+                    const f32x2 v01 = fma2(pack(__uint_as_float(c0), __uint_as_float(c1)), lo, pack(__uint_as_float(r0), __uint_as_float(r1)));
+                    const f32x2 v23 = fma2(pack(__uint_as_float(c2_), __uint_as_float(c3)), lo, pack(__uint_as_float(r2), __uint_as_float(r3)));
+                    if (KIND == kPlainKind || mode == kPlain) poison = fma2(v01, 0, fma2(v23, 0, poison));
                     const uint32_t dst = tile + (uint32_t)(lane * 128 + ((v4 ^ (lane & 7)) * 16));
-                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "f"(v0), "f"(v1), "f"(v2), "f"(v3) : "memory");
+                    asm volatile("st.shared.v2.b64 [%0], {%1,%2};" ::"r"(dst), "l"(v01), "l"(v23) : "memory");
                 };
                 if constexpr (kAhead) {
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -255,110 +290,99 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     mbar_arrive(tempty0 + 8u * buf);
                 }
-                if (poison != poison && lane < live) *range_flag = 1;
+                {
+                    float p0, p1;
+                    unpack(poison, p0, p1);
+                    if (!(p0 + p1 == 0.f) && lane < live) *range_flag = 1;
+                }
                 __syncwarp();
                 // 2. whole lines: the mode's arithmetic and its stores
                 float4 b = f4zero();
                 if (bias) b = ld4(bias + t.w_row + col + c4);
-                // body(i, x, in): row rr + 4 i of the chunk, four columns
+                const f32x2 b01 = pack(b.x, b.y), b23 = pack(b.z, b.w);
+                // body(i, x01, x23, in): row rr + 4 i of the chunk, four columns
                 auto rows = [&](auto&& body) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const int row = rr + 4 * i;
-                        float x[4];
+                        f32x2 x0, x1;
                         const uint32_t src = tile + (uint32_t)(row * 128 + (((lane & 7) ^ (row & 7)) * 16));
-                        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(src) : "memory");
-                        if constexpr (KIND != kBackwardKind) x[0] += b.x, x[1] += b.y, x[2] += b.z, x[3] += b.w;
-                        body(i, x, row < live);
+                        asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(x0), "=l"(x1) : "r"(src) : "memory");
+                        if constexpr (KIND == kBackwardKind) body(i, mul2(x0, os2), mul2(x1, os2), row < live);
+                        else body(i, fma2(x0, os2, b01), fma2(x1, os2, b23), row < live);
                     }
                 };
                 float* const yo = yrow + col;
                 __half *const ph = ohi + t.out_col + col, *const pl = olo + t.out_col + col;
-                auto store_y = [&](int i, int at, const float (&x)[4]) {
-                    __stcs(reinterpret_cast<float4*>(yo + 4 * i * prm.ldy + at), make_float4(x[0], x[1], x[2], x[3]));
-                };
+                auto gate_of = [&](float v) { return o_scale * sigmoid_f(gate_silu ? v * sigmoid_f(v) : v); };
                 if (KIND == kPlainKind || mode == kPlain) {
                     const bool inside = t.out_col + col + c4 < prm.y_cols;
-                    rows([&](int i, const float (&x)[4], bool in) {
-                        if (in && inside) store_y(i, t.out_col, x);
+                    rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                        if (in && inside) store_pair(yo + 4 * i * prm.ldy + t.out_col, x0, x1);
                         if constexpr (KIND == kForwardKind) {
                             if (t.flags & kGateSrc) {
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) keepv[c2][4 * i + j] = sigmoid_f(gate_silu ? x[j] * sigmoid_f(x[j]) : x[j]);
+                                keepv[c2][2 * i] = map2(x0, gate_of);
+                                keepv[c2][2 * i + 1] = map2(x1, gate_of);
                             }
                         }
                     });
                 } else if constexpr (KIND == kForwardKind) {
                     const bool keep = (t.flags & kKeep) != 0;
-                    if (mode == kSilu)
-                        rows([&](int i, const float (&x)[4], bool in) {
-                            if (!in) return;
-                            if (keep) store_y(i, t.y_col, x);
-                            float o[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) o[j] = x[j] * sigmoid_f(x[j]) * o_scale;
-                            store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                    if (mode == kSilu) {
+                        auto sig = [&](float v) { return o_scale * sigmoid_f(v); };
+                        rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                            if (in && keep) store_pair(yo + 4 * i * prm.ldy + t.y_col, x0, x1);
+                            store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, map2(x0, sig)), mul2(x1, map2(x1, sig)), in, top);
                         });
-                    else
-                        rows([&](int i, const float (&x)[4], bool in) {
-                            if (!in) return;
-                            if (keep) store_y(i, t.y_col, x);
-                            float o[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) o[j] = x[j] * keepv[c2][4 * i + j] * o_scale;
-                            store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                    } else {
+                        rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                            if (in && keep) store_pair(yo + 4 * i * prm.ldy + t.y_col, x0, x1);
+                            store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, keepv[c2][2 * i]), mul2(x1, keepv[c2][2 * i + 1]), in, top);
                         });
+                    }
                 } else if (mode == kSiluBwd) {
-                    rows([&](int i, const float (&x)[4], bool in) {
-                        float o[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float y0 = yv[4 * i + j], s = sigmoid_f(y0);
-                            o[j] = x[j] * s * (1.f + y0 * (1.f - s)) * o_scale;
-                        }
-                        if (in) store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                    auto slope = [&](float v) {
+                        const float q = sigmoid_f(v);
+                        return o_scale * q * (1.f + v * (1.f - q));
+                    };
+                    rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                        store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, map2(yv[2 * i], slope)), mul2(x1, map2(yv[2 * i + 1], slope)), in, top);
                     });
                 } else {
                     if (t.flags & kFirst) {
-                        float4 ga[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) ga[i] = rr + 4 * i < live ? ld4(yo + 4 * i * prm.ldy + t.gate_col) : f4zero();
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            const float v[4] = {ga[i].x, ga[i].y, ga[i].z, ga[i].w};
+                            sg[c2][2 * i] = sg[c2][2 * i + 1] = 0;
+                            if (rr + 4 * i < live) load_pair(yo + 4 * i * prm.ldy + t.gate_col, sg[c2][2 * i], sg[c2][2 * i + 1]);
+                        }
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                sg[c2][4 * i + j] = sigmoid_f(gate_silu ? v[j] * sigmoid_f(v[j]) : v[j]);
-                                keepv[c2][4 * i + j] = 0.f;
-                            }
+                        for (int i = 0; i < 16; ++i) {
+                            sg[c2][i] = map2(sg[c2][i], gate_of);
+                            keepv[c2][i] = 0;
                         }
                     }
-                    rows([&](int i, const float (&x)[4], bool in) {
-                        float o[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            o[j] = x[j] * sg[c2][4 * i + j] * o_scale;
-                            keepv[c2][4 * i + j] = fmaf(x[j], yv[4 * i + j], keepv[c2][4 * i + j]);
-                        }
-                        if (in) store_split(ph, pl, 4 * i * prm.ldo, o, top);
+                    rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                        keepv[c2][2 * i] = fma2(x0, yv[2 * i], keepv[c2][2 * i]);
+                        keepv[c2][2 * i + 1] = fma2(x1, yv[2 * i + 1], keepv[c2][2 * i + 1]);
+                        store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, sg[c2][2 * i]), mul2(x1, sg[c2][2 * i + 1]), in, top);
                     });
                     if (t.flags & kLast) {
+                        const float inv = 1.0f / o_scale;
+                        auto dsig = [&](float v) { return v * (1.f - v * inv); };  // o_scale * sigmoid'
+                        auto dsilu = [&](float v) {
+                            const float q = sigmoid_f(v);
+                            return q * (1.f + v * (1.f - q));
+                        };
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            if (rr + 4 * i >= live) continue;
-                            float d[4], slope[4] = {1.f, 1.f, 1.f, 1.f};
+                            f32x2 d0 = mul2(keepv[c2][2 * i], map2(sg[c2][2 * i], dsig)), d1 = mul2(keepv[c2][2 * i + 1], map2(sg[c2][2 * i + 1], dsig));
+                            const bool in = rr + 4 * i < live;
                             if (gate_silu) {
-                                const float4 gr = ld4(yo + 4 * i * prm.ldy + t.gate_col);
-                                const float gv[4] = {gr.x, gr.y, gr.z, gr.w};
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float s = sigmoid_f(gv[j]);
-                                    slope[j] = s * (1.f + gv[j] * (1.f - s));
-                                }
+                                f32x2 g0 = 0, g1 = 0;
+                                if (in) load_pair(yo + 4 * i * prm.ldy + t.gate_col, g0, g1);
+                                d0 = mul2(d0, map2(g0, dsilu)), d1 = mul2(d1, map2(g1, dsilu));
                             }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) d[j] = keepv[c2][4 * i + j] * slope[j] * sg[c2][4 * i + j] * (1.f - sg[c2][4 * i + j]) * o_scale;
-                            store_split(ohi + t.gate_col + col, olo + t.gate_col + col, 4 * i * prm.ldo, d, top);
+                            store_split(ohi + t.gate_col + col, olo + t.gate_col + col, 4 * i * prm.ldo, d0, d1, in, top);
                         }
                     }
                 }
