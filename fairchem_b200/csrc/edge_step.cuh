@@ -471,7 +471,7 @@ template <int LMAX, int HALF, int WPN, class RadOut>
 __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
     gather_bwd_kernel(const float* __restrict__ grad, const float* __restrict__ x, const int32_t* __restrict__ lo,
                       const int32_t* __restrict__ hi, const int32_t* __restrict__ perm, const float* __restrict__ wig,
-                      const float* __restrict__ radial, float* __restrict__ gx, float* __restrict__ tau, int store_tau,
+                      const float* __restrict__ radial, float* __restrict__ gx, int store_gx, float* __restrict__ tau, int store_tau,
                       RadOut grad_radial, const float* __restrict__ scale_ptr, int64_t e_base, int64_t n0, int64_t n1) {
     pdl_sync();
     using S = Shape<LMAX>;
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
     const int64_t stride = WPN == 1 ? (int64_t)gridDim.x * kWarps : gridDim.x;
     for (int64_t n = n0 + (WPN == 1 ? (int64_t)blockIdx.x * kWarps + wid : blockIdx.x); n < n1; n += stride) {
         const int eb = lo[n], ee = hi[n];
-        if (eb == ee) continue;
+        if (eb == ee && !store_gx) continue;  // store_gx: the first contribution to every node's gradient
         const float* x_base = x + n * (int64_t)S::kL * C;
         float* g_base = gx + n * (int64_t)S::kL * C;
         auto pass = [&](auto lo_tag, auto hi_tag, bool add_tau) {
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
 #pragma unroll
                 for (int r = 0; r < kRows; ++r) {
                     float* o = g_base + (LLO * LLO + r) * C + c0;
-                    st4(o, add4(ld4(o), acc[r]));
+                    st4(o, store_gx ? acc[r] : add4(ld4(o), acc[r]));
                 }
             } else {
 #pragma unroll
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
                 __syncthreads();
                 for (int r = wid; r < kRows; r += WPN) {
                     float* o = g_base + (LLO * LLO + r) * C + c0;
-                    float4 v = ld4(o);
+                    float4 v = store_gx ? f4zero() : ld4(o);
 #pragma unroll
                     for (int i = 0; i < WPN; ++i) v = add4(v, ld4(part + (i * kRows + r) * C + c0));
                     st4(o, v);

@@ -218,9 +218,9 @@ struct Run {
         return rc;
     }
 
-    // one launch of tile list c on rows [m] of half planes
+    // one launch of tile list c on rows [m] of half planes; raw: see so2_conv_fused
     int conv(const char* name, const Conv& c, const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, int rot_begin, float* y,
-             int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m) const {
+             int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m, float* raw = nullptr) const {
         const void *hi[3] = {}, *lo[3] = {};
         int64_t rows[3] = {}, cols[3] = {};
         float sc[3] = {1.f, 1.f, 1.f};
@@ -228,9 +228,9 @@ struct Run {
             if (c.w[i]) hi[i] = c.w[i]->hi, lo[i] = c.w[i]->lo, rows[i] = c.w[i]->rows, cols[i] = c.w[i]->cols, sc[i] = c.w[i]->scale;
         const int64_t bytes = 4 * m * (a_cols + 128LL * c.count()), flops = 2 * m * c.macs;
         hook(name, 1, bytes, flops);
-        const int rc = fcb200_so2_conv_fused(a_hi, a_lo, lda, a_cols, hi, lo, rows, cols, sc, c.bias, c.t.data(), c.count(), rot_begin, y,
+        const int rc = so2_conv_fused(a_hi, a_lo, lda, a_cols, hi, lo, rows, cols, sc, c.bias, c.t.data(), c.count(), rot_begin, y,
                                              ldy, y_cols, o ? o->hi : nullptr, o ? o->lo : nullptr, o ? o->ld : 0, o_cols, a_scale,
-                                             o_scale, m, 0, ev.status, stream);
+                                             o_scale, m, 0, ev.status, stream, raw);
         hook(name, 0, bytes, flops);
         return rc;
     }
@@ -318,14 +318,14 @@ static int launch_rotate_back(const Run& r, const float* msg, int64_t e_base, co
 }
 
 template <int LMAX, int HALF>
-static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, const int32_t* hi, const float* radial, float* gx, bool store_tau,
+static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, const int32_t* hi, const float* radial, float* gx, bool store_gx, bool store_tau,
                              const float* scale, int64_t e0, int64_t n0, int64_t n1) {
     constexpr int WPN = 8;
     const Layout& L = r.L;
     if (share_node(n1 - n0)) {
-        launch_pdl((gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>), dim3((int)(n1 - n0)), dim3(WPN * 32), WPN * 9 * C * 4, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, L.tau_n, store_tau, L.grad.out(), scale, e0, n0, n1);
+        launch_pdl((gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>), dim3((int)(n1 - n0)), dim3(WPN * 32), WPN * 9 * C * 4, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
     } else {
-        launch_pdl((gather_bwd_kernel<LMAX, HALF, 1, OutSplit>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, L.tau_n, store_tau, L.grad.out(), scale, e0, n0, n1);
+        launch_pdl((gather_bwd_kernel<LMAX, HALF, 1, OutSplit>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
     }
     return FCB200_OK;
 }
@@ -500,7 +500,7 @@ int Run::layer_backward(int l) {
         else b1.tile((d.lmax + r) * C, C, 1, (deg - 1) * C, r * C);
     }
     const int64_t fw = (d.lmax + d.nl) * C;
-    FCB_TRY(conv("ffn_out_gate_bwd", b2, L.gp.hi, L.gp.lo, row, row, b2.count(), q.ffn_y, fw, fw, &L.gy2, fw, &s->scale, &s->scale, n));
+    FCB_TRY(conv("ffn_out_gate_bwd", b2, L.gp.hi, L.gp.lo, row, row, b2.count(), q.ffn_y, fw, fw, &L.gy2, fw, &s->scale, &s->scale, n, L.gxn));
     FCB_TRY(conv("ffn_in_bwd", b1, L.gy2.hi, L.gy2.lo, fw, fw, 0, L.gxn, row, row, nullptr, 0, &s->scale, nullptr, n));
     FCB_TRY(op("rms_norm_sh_bwd", n * row * 16, [&] {
         return by_lmax([&](auto lm) {
@@ -510,7 +510,6 @@ int Run::layer_backward(int l) {
     }));
     // edge block
     const float* scale = &s[1].scale;
-    if (cudaMemsetAsync(L.gxn, 0, n * row * 4, st) != cudaSuccess) return launch_status();
     Conv c2, c1 = blocks(w.conv1_t);
     {
         const Conv p = blocks(w.conv2_t);  // rows of one degree back to back: their gate gradient stays in registers
@@ -543,14 +542,14 @@ int Run::layer_backward(int l) {
                 return 0;
             });
         }));
-        FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, d.yw, d.yw, &L.gy, L.gy.ld, scale, scale, ec));
+        FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, d.yw, d.yw, &L.gy, L.gy.ld, scale, scale, ec, L.gm));
         FCB_TRY(conv("so2_conv_fused_conv1_bwd", c1, L.gy.hi, L.gy.lo, L.gy.ld, L.gy.ld, 0, L.gm, d.nm * 2 * C, d.nm * 2 * C, nullptr, 0, scale, nullptr, ec));
         const int64_t gb = ec * 4LL * (2 * d.nm * C + 2 * 2 * d.nrad * C + d.nw + 12) + (n1 - n0) * row * 4 * 4;
         FCB_TRY(op("gather_rotate_bwd", gb, [&] {
             return by_lmax([&](auto lm) {
                 constexpr int LM = decltype(lm)::value;
-                FCB_TRY((launch_gather_bwd<LM, 0>(*this, q.xn1, src_lo(c), src_hi(c), rad, L.gxn, first_layer, scale, e0, 0, n)));
-                return launch_gather_bwd<LM, 1>(*this, q.xn1, ev.row_ptr, ev.row_ptr + 1, rad, L.gxn, false, scale, e0, n0, n1);
+                FCB_TRY((launch_gather_bwd<LM, 0>(*this, q.xn1, src_lo(c), src_hi(c), rad, L.gxn, c == 0, first_layer, scale, e0, 0, n)));
+                return launch_gather_bwd<LM, 1>(*this, q.xn1, ev.row_ptr, ev.row_ptr + 1, rad, L.gxn, false, false, scale, e0, n0, n1);
             });
         }, 0, 2));
         return gemm("so2_conv_fused_radial_out_bwd", L.grad, w.radial_out_t, scale,

@@ -48,8 +48,9 @@ enum Mode : int32_t {
     kGatedBwd = 5,  // planes[:, out_col ...] = split(v * sigmoid(gate)); gate gradient summed over consecutive tiles
 };
 // kGateSilu: the gate is sigmoid(silu(g)), the scalar MLP of the node-wise feed-forward, instead of sigmoid(g).
-// kGateSrc (set on the host): a gate tile of the rows that follow
-enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8, kGateSrc = 16 };
+// kGateSrc (set on the host): a gate tile of the rows that follow.  kSolo (host): a backward gated row on its own; its raw
+// value goes to Params::raw and gate_sum_kernel adds up the rows of a degree.
+enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8, kGateSrc = 16, kSolo = 32 };
 
 struct Tile {
     int16_t a_col;     // first input column of this tile's K range
@@ -61,7 +62,7 @@ struct Tile {
     int16_t y_col;     // column of y holding this row's raw value (kSilu/kGated keep, kSiluBwd/kGatedBwd read)
     int16_t gate_col;  // column of y (and of the gradient planes) of the gate scalars of this row's degree
     int16_t flags;
-    int16_t pad;
+    int16_t raw_col;   // kSolo: column of Params::raw
 };
 constexpr int kMaxTiles = 40;   // tiles a caller may list; lmax 4: 19 rows x 2C = 38 column tiles in the conv-1 backward
 constexpr int kMaxPlan = 80;    // tiles of a plan: a gate tile may be repeated for each of its rows
@@ -108,6 +109,8 @@ struct Params {
     const float* o_scale;  // power of two the output planes are written with (null = 1)
     int64_t m_total;
     int32_t* status;
+    float* raw;        // [m, raw_ld] values of the kSolo tiles
+    int32_t raw_ld;
 };
 
 // 1 / (1 + e^-v) on the special-function unit (ex2.approx, rcp.approx): relative error ~2^-22, a few instructions
@@ -349,7 +352,8 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
                         store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, map2(yv[2 * i], slope)), mul2(x1, map2(yv[2 * i + 1], slope)), in, top);
                     });
                 } else {
-                    if (t.flags & kFirst) {
+                    const bool solo = (t.flags & kSolo) != 0;
+                    if (t.flags & (kFirst | kSolo)) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             sg[c2][2 * i] = sg[c2][2 * i + 1] = 0;
@@ -362,11 +366,12 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
                         }
                     }
                     rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                        if (solo && in) store_pair(prm.raw + (row0 + rr + 4 * i) * prm.raw_ld + t.raw_col + col + c4, x0, x1);
                         keepv[c2][2 * i] = fma2(x0, yv[2 * i], keepv[c2][2 * i]);
                         keepv[c2][2 * i + 1] = fma2(x1, yv[2 * i + 1], keepv[c2][2 * i + 1]);
                         store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, sg[c2][2 * i]), mul2(x1, sg[c2][2 * i + 1]), in, top);
                     });
-                    if (t.flags & kLast) {
+                    if ((t.flags & kLast) && !solo) {
                         const float inv = 1.0f / o_scale;
                         auto dsig = [&](float v) { return v * (1.f - v * inv); };  // o_scale * sigmoid'
                         auto dsilu = [&](float v) {
@@ -532,6 +537,46 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
+// Gate gradients of a backward launch whose rows ran one by one: per degree sum_r raw_r y_r in row order (the fused
+// multiply-adds of the in-epilogue sum), times the gate's slope, as planes.  One warp per row of the matrix.
+struct GateSums {
+    int32_t degrees, hidden_silu;
+    int16_t gate_col[8], begin[9];
+    int16_t raw_col[kMaxTiles], y_col[kMaxTiles];
+};
+__global__ void __launch_bounds__(256) gate_sum_kernel(const __grid_constant__ GateSums g, const __grid_constant__ Params prm) {
+    pdl_sync();
+    const int lane = threadIdx.x & 31, c = lane * 4;
+    const float o_scale = prm.o_scale ? *prm.o_scale : 1.0f;
+    __half2 top = __floats2half2_rn(0.f, 0.f);
+    for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < prm.m_total; row += (int64_t)gridDim.x * 8) {
+        const float* y = prm.y + row * prm.ldy + c;
+        const float* raw = prm.raw + row * prm.raw_ld + c;
+        for (int d = 0; d < g.degrees; ++d) {
+            f32x2 s0 = 0, s1 = 0, g0, g1;
+            load_pair(y + g.gate_col[d], g0, g1);
+            for (int r = g.begin[d]; r < g.begin[d + 1]; ++r) {
+                f32x2 x0, x1, y0, y1;
+                load_pair(raw + g.raw_col[r], x0, x1);
+                load_pair(y + g.y_col[r], y0, y1);
+                s0 = fma2(x0, y0, s0), s1 = fma2(x1, y1, s1);
+            }
+            auto slope = [&](float v) {
+                float k = 1.f;
+                if (g.hidden_silu) {
+                    const float q = sigmoid_f(v);
+                    k = q * (1.f + v * (1.f - q));
+                    v *= q;
+                }
+                const float q = sigmoid_f(v);
+                return k * q * (1.f - q) * o_scale;
+            };
+            store_split(prm.o_hi + row * prm.ldo + c, prm.o_lo + row * prm.ldo + c, g.gate_col[d], mul2(s0, map2(g0, slope)), mul2(s1, map2(g1, slope)), true, top);
+        }
+    }
+    if (!(__half2float(__hmax_nan(__low2half(top), __high2half(top))) <= kHalfMax) && prm.status) atomicCAS(prm.status, 0, 2);
+}
+
 // 2-D row-major half matrix [rows, cols], row stride ld elements; box = 64 columns x 128 rows, 128-byte swizzle
 static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld) {
     EncodeTiledFn fn = encode_fn();
@@ -550,7 +595,8 @@ static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t col
 // How a tile list is cut into groups (Plan::groups); a CTA takes (row tile, group) items in turn.
 //   natural  what shares nothing is apart: every plain tile, row 0, and the rows of a degree with their gate tile (forward)
 //            or their gate-gradient sum (backward)
-//   fine     forward gated rows one by one, each after its own copy of the gate tile (the gate is computed again)
+//   fine     gated rows one by one: forward each after its own copy of the gate tile (the gate is computed again), backward
+//            with the gate-gradient sums left to a second kernel
 enum Grouping { kAuto = 0, kNatural = 1, kFine = 2 };
 
 struct Groups {
@@ -605,7 +651,7 @@ static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
             for (int j = i; j < n; ++j) {
                 put(j);
                 done[j] = true;
-                if (t[j].flags & kLast) break;
+                if ((t[j].flags & kLast) || how == kFine) break;
             }
         } else {
             put(i);
@@ -613,6 +659,24 @@ static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
         close();
     }
     return g;
+}
+
+// rows of every degree of a backward list and where their raw values go
+static bool split_sums(Tile* t, int n, GateSums& g) {
+    int rows = 0;
+    for (int i = 0; i < n; ++i) {
+        if (t[i].mode != kGatedBwd) continue;
+        if (t[i].flags & kFirst) {
+            if (g.degrees == 8) return false;
+            g.gate_col[g.degrees++] = t[i].gate_col;
+            g.hidden_silu = (t[i].flags & kGateSilu) != 0;
+        }
+        if (!g.degrees || t[i].gate_col != g.gate_col[g.degrees - 1]) return false;
+        t[i].raw_col = (int16_t)(rows * BN);
+        g.raw_col[rows] = t[i].raw_col, g.y_col[rows] = t[i].y_col;
+        g.begin[g.degrees] = (int16_t)++rows;
+    }
+    return g.degrees > 0;
 }
 
 // longest CTA of a static round-robin over rows x groups items, in units of K
@@ -635,12 +699,14 @@ static int64_t makespan(const Groups& g, int64_t rows, int ctas) {
 
 using namespace fcb200;
 
-extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, const void* const* w_hi,
+namespace fcb200 {
+
+int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, const void* const* w_hi,
                                      const void* const* w_lo, const int64_t* w_rows, const int64_t* w_cols,
                                      const float* w_scale, const float* const* bias, const int32_t* tiles, int32_t num_tiles,
                                      int32_t rot_begin, float* y, int64_t ldy, int64_t y_cols, void* o_hi, void* o_lo, int64_t ldo, int64_t o_cols,
                                      const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status,
-                                     void* stream) {
+                                     void* stream, float* raw) {
     using namespace fused;
     if (!a_hi || !a_lo || !w_hi || !w_lo || !w_rows || !w_cols || !w_scale || !tiles || !y || m < 0) return FCB200_EINVAL;
     Plan plan{};
@@ -696,11 +762,20 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
     // convolution: 528 / 446).  Few row tiles still leave SMs without work; then the gated rows go one by one where that
     // shortens the longest CTA by more than the estimate's error (M = 7 680: 104 -> 87 us, M = 640: 59 -> 36 us).
     const int64_t rows_m = (m + BM - 1) / BM;
-    Groups grp = group_tiles(list, num_tiles, rot_begin, grouping == kFine ? kFine : kNatural);
+    Groups grp = group_tiles(list, num_tiles, rot_begin, grouping == kFine && !backward ? kFine : kNatural);
     if (!grp.ok) return FCB200_EINVAL;
     if (grouping == kAuto && gated) {
         const Groups fine = group_tiles(list, num_tiles, rot_begin, kFine);
         if (fine.ok && 10 * makespan(fine, rows_m, sm_count()) < 9 * makespan(grp, rows_m, sm_count())) grp = fine;
+    }
+    // backward: the same, if there is room for the raw rows and the second kernel (about 5 us, 600 units of K) pays
+    GateSums sums{};
+    const bool solo = backward && raw && grouping != kNatural && split_sums(list, num_tiles, sums) &&
+                      (grouping == kFine || makespan(group_tiles(list, num_tiles, rot_begin, kFine), rows_m, sm_count()) + 600 < makespan(grp, rows_m, sm_count()));
+    if (solo) {
+        for (int i = 0; i < num_tiles; ++i)
+            if (list[i].mode == kGatedBwd) list[i].flags |= kSolo;
+        grp = group_tiles(list, num_tiles, rot_begin, kFine);
     }
     plan.groups = grp.groups;
     for (int i = 0; i <= grp.groups; ++i) plan.begin[i] = grp.begin[i];
@@ -729,6 +804,7 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
     prm.y = y, prm.ldy = (int32_t)ldy, prm.y_cols = (int32_t)y_cols, prm.a_scale = a_scale, prm.o_scale = o_scale;
     prm.o_hi = static_cast<__half*>(o_hi), prm.o_lo = static_cast<__half*>(o_lo), prm.ldo = (int32_t)ldo;
     prm.m_total = m, prm.status = status;
+    prm.raw = raw, prm.raw_ld = sums.begin[sums.degrees] * BN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int64_t items = rows_m * plan.groups;
     const int grid = (int)(items < sm_count() ? items : sm_count());
@@ -739,6 +815,23 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
     };
     static bool done[3][64] = {};
     if (forward) return launch(so2_conv_fused_kernel<kForwardKind>, done[0]);
-    if (backward) return launch(so2_conv_fused_kernel<kBackwardKind>, done[1]);
+    if (backward) {
+        const int brc = launch(so2_conv_fused_kernel<kBackwardKind>, done[1]);
+        if (brc || !solo) return brc;
+        launch_pdl(gate_sum_kernel, dim3(warp_grid(m, 8)), dim3(256), 0, st, sums, prm);
+        return launch_status();
+    }
     return launch(so2_conv_fused_kernel<kPlainKind>, done[2]);
+}
+
+}  // namespace fcb200
+
+extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, const void* const* w_hi,
+                                     const void* const* w_lo, const int64_t* w_rows, const int64_t* w_cols,
+                                     const float* w_scale, const float* const* bias, const int32_t* tiles, int32_t num_tiles,
+                                     int32_t rot_begin, float* y, int64_t ldy, int64_t y_cols, void* o_hi, void* o_lo, int64_t ldo, int64_t o_cols,
+                                     const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status,
+                                     void* stream) {
+    return so2_conv_fused(a_hi, a_lo, lda, a_cols, w_hi, w_lo, w_rows, w_cols, w_scale, bias, tiles, num_tiles, rot_begin, y, ldy, y_cols, o_hi, o_lo, ldo,
+                          o_cols, a_scale, o_scale, m, variant, status, stream, nullptr);
 }
