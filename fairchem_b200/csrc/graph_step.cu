@@ -394,10 +394,10 @@ __global__ void graph_count_kernel(const int32_t* __restrict__ node, int32_t* __
 
 // edges into their source's segment, in any order ...
 __global__ void graph_bucket_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ src_ptr, int32_t* __restrict__ left,
-                                    int32_t* __restrict__ unsorted, int64_t num_edges) {
+                                    int32_t* __restrict__ unsorted, const int32_t* __restrict__ num_edges) {
     pdl_sync();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= num_edges) return;
+    if (e >= *num_edges) return;  // the arrays may be larger than the edge list
     const int s = src[e];
     unsorted[src_ptr[s] + atomicSub(left + s, 1) - 1] = (int)e;
 }
@@ -518,7 +518,7 @@ int fcb200_graph_fill(const fcb200_graph* g, void* stream) {
     }
     if (g->src_ptr) {
         launch_pdl(step::graph_scan_kernel, dim3(1), dim3(1024), 0, st, g->src_count, g->src_ptr, n, 1, nullptr);
-        launch_pdl(step::graph_bucket_kernel, dim3(ge), dim3(256), 0, st, g->src, g->src_ptr, g->src_count, g->src_tmp, e);
+        launch_pdl(step::graph_bucket_kernel, dim3(ge), dim3(256), 0, st, g->src, g->src_ptr, g->src_count, g->src_tmp, g->row_ptr + n);
         launch_pdl(step::graph_order_kernel, dim3(gn), dim3(256), 0, st, g->src_tmp, g->src_ptr, g->src_perm, g->chunk_src, g->info + step::kInfoEdgeCut,
                                                      g->num_chunks, n);
     }

@@ -16,9 +16,11 @@ the reference rebuilds the graph on every call.
 
 from __future__ import annotations
 
+import threading
 from dataclasses import dataclass, field
 from typing import Mapping, Optional
 
+import numpy as np
 import torch
 
 from .synthetic import AtomicDataLike
@@ -32,6 +34,8 @@ class Normalizer:
     rmsd: float = 1.0
 
     def denorm(self, x: torch.Tensor) -> torch.Tensor:
+        if self.rmsd == 1.0 and self.mean == 0.0:
+            return x  # two launches less on the way out of a small system
         return x * self.rmsd + self.mean
 
 
@@ -68,22 +72,47 @@ def default_tasks(backbone) -> dict:
     return tasks
 
 
+class _Staging(threading.local):
+    """Pinned block a thread's host inputs are packed into, and the event after its last copy."""
+
+    def __init__(self):
+        self.block = self.bytes = self.copied = None
+
+    def get(self, nbytes: int) -> np.ndarray:
+        if self.block is None or self.block.numel() < nbytes:
+            self.block = torch.empty(max(2 * nbytes, 1 << 16), dtype=torch.uint8, pin_memory=True)
+            self.bytes = self.block.numpy()
+        elif self.copied is not None:
+            self.copied.synchronize()  # the previous call's copy has read the block
+        return self.bytes
+
+
+_staging = _Staging()
+_PACK_LIMIT = 1 << 24  # larger inputs are copied tensor by tensor: their launches do not matter
+
+
 def _packed_copy(data: AtomicDataLike, device) -> AtomicDataLike:
     """``data.to(device)`` with the host tensors in one pinned block and one copy: eight small copies cost ~15 us each."""
-    host = [(k, v.contiguous()) for k, v in data.items() if torch.is_tensor(v) and v.device.type == "cpu"]
-    offsets, total = [], 0
-    for _, v in host:
-        offsets.append(total)
-        total += (v.numel() * v.element_size() + 255) // 256 * 256
-    block = torch.empty(total, dtype=torch.uint8, pin_memory=True)
-    for (_, v), o in zip(host, offsets):
-        block[o:o + v.numel() * v.element_size()].view(v.dtype).copy_(v.view(-1))
-    moved = block.to(device, non_blocking=True)
-    out = AtomicDataLike()
+    host, total = [], 0
     for k, v in data.items():
-        out[k] = v.to(device) if torch.is_tensor(v) and v.device.type != "cpu" else v
-    for (k, v), o in zip(host, offsets):
-        out[k] = moved[o:o + v.numel() * v.element_size()].view(v.dtype).view(v.shape)
+        if torch.is_tensor(v) and v.device.type == "cpu":
+            n = v.numel() * v.element_size()
+            host.append((k, v, total, n))
+            total += (n + 255) // 256 * 256
+    if total > _PACK_LIMIT:
+        return data.to(device)
+    stage = _staging.get(total)
+    for _, v, o, n in host:
+        stage[o:o + n] = v.detach().reshape(-1).view(torch.uint8).numpy()
+    with torch.cuda.device(device):
+        moved = _staging.block[:total].to(device, non_blocking=True)
+        _staging.copied = torch.cuda.current_stream().record_event()
+    out = AtomicDataLike(data)
+    for k, v, o, n in host:
+        out[k] = moved[o:o + n].view(v.dtype).view(v.shape)
+    for k, v in data.items():
+        if torch.is_tensor(v) and v.device.type != "cpu" and v.device != device:
+            out[k] = v.to(device)
     return out
 
 

@@ -367,13 +367,17 @@ class StepGraph:
     def _info(self):
         return self.a.view("info", INFO_WORDS).cpu()
 
-    def _finish_info(self, info) -> bool:
-        self.num_edges, n = int(info[0]), int(info[2])
+    def _set_chunks(self, edges: int, node_cut: list, edge_cut: list):
+        self.num_edges, n = edges, len(node_cut) - 1
+        self.num_chunks = n
+        self.chunk_node, self.chunk_edge = (c_int64 * (n + 1))(*node_cut), (c_int64 * (n + 1))(*edge_cut)
+
+    def _finish_info(self, info):
+        n = int(info[2])
         nodes, edges = info[INFO_NODES:INFO_NODES + n + 1].tolist(), info[INFO_EDGES:INFO_EDGES + n + 1].tolist()
         if any(b <= a for a, b in zip(edges, edges[1:])):  # a target with more edges than a chunk: do not cut
-            n, nodes, edges = 1, [0, self.nodes], [0, self.num_edges]
-        self.num_chunks = n
-        self.chunk_node, self.chunk_edge = (c_int64 * (n + 1))(*nodes), (c_int64 * (n + 1))(*edges)
+            nodes, edges = [0, self.nodes], [0, int(info[0])]
+        self._set_chunks(int(info[0]), nodes, edges)
 
     def build(self) -> bool:
         """Search, selection and tables from the positions.  False: not for this path."""
@@ -383,8 +387,20 @@ class StepGraph:
         g.stride = min(STRIDE_MAX, 2 * k + 8) if k > 0 else STRIDE_MAX
         g.want_totals = int(self.nodes > BRUTE_NODES and nl is None)
         self._call("fcb200_graph_systems")
-        rows = torch.empty(self.nodes * g.stride * 2, dtype=torch.int32, device=self.device)
+        capacity = self.nodes * g.stride
+        rows = torch.empty(capacity * 2, dtype=torch.int32, device=self.device)
         g.rows = rows.data_ptr()
+        # Few nodes: the edge arrays are sized for every kept-neighbour slot, so that they are filled before the host learns
+        # the edge count instead of after it.
+        if nl is None and self.nodes <= BRUTE_NODES and 2 * capacity < 3 * g.chunk_edges:
+            self._call("fcb200_graph_select")
+            self._fill(capacity, 1)
+            info = self.a.view("info", 8).tolist()
+            if info[1] or info[0] == 0:
+                return False
+            self._set_chunks(info[0], [0, self.nodes], [0, info[0]])
+            self.edge_index, self.cell_offsets = self.edge_index[:, :info[0]], self.cell_offsets[:info[0]]
+            return True
         if nl is not None:
             info = self._select_kept(nl)
         else:
@@ -403,14 +419,15 @@ class StepGraph:
         if info is None or int(info[1]) or int(info[0]) == 0:
             return False
         self._finish_info(info)
-        self._edges()
-        e = self.num_edges
-        edge_index = torch.empty(2, e, dtype=torch.int64, device=self.device)
-        offsets = torch.empty(e, 3, dtype=torch.float32, device=self.device)
-        self.edge_index, self.cell_offsets = edge_index, offsets
-        g.edge_index, g.cell_offsets = edge_index.data_ptr(), offsets.data_ptr()
-        self._call("fcb200_graph_fill")
+        self._fill(self.num_edges, self.num_chunks)
         return True
+
+    def _fill(self, capacity: int, chunks: int):
+        self._edges(capacity, chunks)
+        self.edge_index = torch.empty(2, capacity, dtype=torch.int64, device=self.device)
+        self.cell_offsets = torch.empty(capacity, 3, dtype=torch.float32, device=self.device)
+        self.g.edge_index, self.g.cell_offsets = self.edge_index.data_ptr(), self.cell_offsets.data_ptr()
+        self._call("fcb200_graph_fill")
 
     def _select_kept(self, nl):
         """Selection from a SkinNeighborList's candidates, refreshed by a new search when they have expired."""
@@ -438,17 +455,17 @@ class StepGraph:
         self.g.cand_ptr, self.g.cand_id, self.g.cand_sys = c.cand_ptr.data_ptr(), c.cand_id.data_ptr(), c.sys_t.data_ptr()
         self.candidates = c
 
-    def _edges(self):
-        e, n = self.num_edges, self.nodes
+    def _edges(self, e: int, chunks: int):
+        n = self.nodes
         sizes = dict(src=e, tgt=e, shift=3 * e)
         if self.want_grad:
             sizes.update(src_count=n, src_ptr=n + 1, src_tmp=e, src_perm=e)
-            if self.num_chunks > 1:
-                sizes["chunk_src"] = (self.num_chunks + 1) * n
+            if chunks > 1:
+                sizes["chunk_src"] = (chunks + 1) * n
         self.b = _Carve(self.device, **sizes)
         for name, p in self.b.ptr.items():
             setattr(self.g, name, p)
-        self.g.num_edges, self.g.num_chunks = e, self.num_chunks
+        self.g.num_edges, self.g.num_chunks = e, chunks
         self.shift = self.g.shift
 
     def from_edges(self, src, tgt, shift):
@@ -456,9 +473,8 @@ class StepGraph:
         g = self.g
         self._call("fcb200_graph_systems")
         g.rows, g.cand_sys = None, None
-        e = self.num_edges = src.shape[0]
-        self.num_chunks = max(1, min(512, (e + g.chunk_edges // 2) // g.chunk_edges))
-        self._edges()
+        e = src.shape[0]
+        self._edges(e, max(1, min(512, (e + g.chunk_edges // 2) // g.chunk_edges)))
         self.b.view("src", e).copy_(src)
         self.b.view("tgt", e).copy_(tgt)
         self.alive.append(shift)

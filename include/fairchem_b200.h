@@ -647,10 +647,10 @@ typedef struct {
     float limit_sq;
     /* fill; rows null: src / tgt are given, sorted by target */
     int32_t num_chunks;
-    int64_t num_edges;
+    int64_t num_edges; /* with rows: the capacity of the edge arrays, at least the edge count (then unknown to the host) */
     int32_t *src, *tgt;
     float* shift;
-    int64_t* edge_index;
+    int64_t* edge_index; /* [2, num_edges] */
     float* cell_offsets;
     int32_t *src_count, *src_ptr, *src_tmp, *src_perm; /* src_ptr null: no by-source order */
     int32_t* chunk_src;                                /* [(num_chunks+1), N] or null */
