@@ -768,10 +768,15 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         const Groups fine = group_tiles(list, num_tiles, rot_begin, kFine);
         if (fine.ok && 10 * makespan(fine, rows_m, sm_count()) < 9 * makespan(grp, rows_m, sm_count())) grp = fine;
     }
-    // backward: the same, if there is room for the raw rows and the second kernel (about 5 us, 600 units of K) pays
+    // backward: the same, if there is room for the raw rows and the second kernel pays: about 5 us, 600 units of K, and its
+    // reads and the raw rows' writes at the memory's rate, 55 KB a unit (without that term 120 000 edges of lmax 4 took the second
+    // kernel: 1.79 + 0.39 ms for 1.46)
     GateSums sums{};
-    const bool solo = backward && raw && grouping != kNatural && split_sums(list, num_tiles, sums) &&
-                      (grouping == kFine || makespan(group_tiles(list, num_tiles, rot_begin, kFine), rows_m, sm_count()) + 600 < makespan(grp, rows_m, sm_count()));
+    bool solo = backward && raw && grouping != kNatural && split_sums(list, num_tiles, sums);
+    if (solo && grouping != kFine) {
+        const int64_t extra = 600 + m * (sums.begin[sums.degrees] + sums.degrees) * (BN * 8) / 55000;
+        solo = makespan(group_tiles(list, num_tiles, rot_begin, kFine), rows_m, sm_count()) + extra < makespan(grp, rows_m, sm_count());
+    }
     if (solo) {
         for (int i = 0; i < num_tiles; ++i)
             if (list[i].mode == kGatedBwd) list[i].flags |= kSolo;
