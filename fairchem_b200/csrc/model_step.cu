@@ -388,9 +388,11 @@ int Run::layer_forward(int l, const float* ffn_prev) {
         FCB_TRY(radial_out(l, e0, ec));
         const int64_t gb = ec * (4LL * (2 * d.nl * C + 2 * d.nm * C + d.nw + d.nrad * 2 * C) + 8);
         FCB_TRY(op("gather_rotate_fwd", gb, [&] {
-            if (d.lmax == 2)
-                return fcb200_gather_rotate_fwd_h(q.xn1, ev.src + e0, ev.tgt + e0, L.wig + e0 * d.nw, radial_of(l, e0), L.m.hi, L.m.lo, nullptr, ec, n, C, stream);
-            return fcb200_lx_gather_rotate_fwd_h(q.xn1, ev.src + e0, ev.tgt + e0, L.wig + e0 * d.nw, radial_of(l, e0), L.m.hi, L.m.lo, nullptr, ec, n, C, d.lmax, stream);
+            return by_lmax([&](auto lm) {
+                constexpr int LM = decltype(lm)::value;
+                launch_pdl(gather_fwd_kernel<LM>, dim3(warp_grid(2 * ec, 4, 148 * (LM == 2 ? 5 : 3) * 4)), dim3(128), 0, st, q.xn1, ev.src + e0, ev.tgt + e0, L.wig + e0 * d.nw, radial_of(l, e0), L.m.out(), ec);
+                return 0;
+            });
         }));
         float* y = keep ? q.y + e0 * d.yw : L.y_c;
         const int64_t yw = keep ? d.yw : d.gates;
@@ -538,7 +540,7 @@ int Run::layer_backward(int l) {
         float* y = q.y + e0 * d.yw;
         FCB_TRY(op("rotate_back_bwd", ec * 4 * (d.nl * C + 2 * d.nm * C + d.nw + 9), [&] {
             return by_lmax([&](auto lm) {
-                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 0, OutSplit>), dim3(warp_grid(ec, 4)), dim3(128), 0, st, L.g1, q.msg + e0 * d.nm * C, L.wig, L.env, ev.tgt, L.gmsg.out(), scale, L.tau_e, !first_layer, 1.0f, e0, ec);
+                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 0, OutSplit>), dim3(warp_grid(ec, 4, 148 * 12)), dim3(128), 0, st, L.g1, q.msg + e0 * d.nm * C, L.wig, L.env, ev.tgt, L.gmsg.out(), scale, L.tau_e, !first_layer, 1.0f, e0, ec);
                 return 0;
             });
         }));
@@ -601,7 +603,7 @@ int Run::backward() {
         FCB_TRY(degree_out(e0, ec));
         FCB_TRY(op("edge_degree_bwd", ec * 4 * (d.nl * C + 2 * (d.lmax + 1) * C + d.nw + 9), [&] {
             return by_lmax([&](auto lm) {
-                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 1, OutSplit>), dim3(warp_grid(ec, 4)), dim3(128), 0, st, L.g, L.r3, L.wig, L.env, ev.tgt, L.gr3.out(), scale, L.tau_e, 1, 1.0f / md.rescale, e0, ec);
+                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 1, OutSplit>), dim3(warp_grid(ec, 4, 148 * 12)), dim3(128), 0, st, L.g, L.r3, L.wig, L.env, ev.tgt, L.gr3.out(), scale, L.tau_e, 1, 1.0f / md.rescale, e0, ec);
                 return 0;
             });
         }));
