@@ -453,22 +453,32 @@ template <int LMAX> __host__ __device__ constexpr int slots_of(int lo, int hi) {
     return s;
 }
 
+__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// lmax 4, by source: a chunk holds few edges of a source, and its three passes would each begin with an empty stage
+template <int LMAX, int HALF> constexpr bool ahead = LMAX == 2 || HALF == 1;
+constexpr int kGatherRows = 15;  // rows and radial weights of an edge in the widest pass (degrees 0-2)
+
 // HALF 0: source columns, the node's edges through perm (by-source order); HALF 1: target columns, consecutive edges.
-// Degrees LLO..LHI in one pass over the node's edges.  What bounds it is latency: a warp walks its edges in turn, and with
-// each degree's rows requested when their turn came an edge cost four round trips to memory (100 000 atoms, per layer:
-// 10.7 + 7.2 ms).  All rows and radial weights of an edge are requested at once, and the next edge's Wigner entries with
-// them.
+// Degrees LLO..LHI in one pass over the node's edges.  Bound by memory once enough of it is asked for at a time: a warp
+// walks its edges in turn.  The gradient rows and radial weights of the next edge are copied to shared memory (two stages
+// of 7.5 KB a warp, every lane the 16 bytes of a row that it reads itself, so nothing has to synchronise) while this one
+// is worked on.  us per launch, all rows of an edge requested when its turn came -> this: 129 000 edges of lmax 2, by source
+// 344 -> 307, by target 299 -> 250; 120 000 edges of lmax 4, by target 834 -> 660, by source 805 -> 890, hence ahead<>.
 template <int LMAX, int LLO, int LHI, int HALF, int STEP, class RadOut>
 __device__ __forceinline__ void gather_bwd_pass(const float* __restrict__ grad, const float* __restrict__ x_base,
                                                 const float* __restrict__ wig, const float* __restrict__ radial,
                                                 const RadOut& grad_radial, const int32_t* __restrict__ perm,
                                                 float* __restrict__ tau, bool add_tau, int64_t e_base, int eb, int ee, int lane,
-                                                float* w, float4 (&acc)[(LHI + 1) * (LHI + 1) - LLO * LLO]) {
+                                                float* w, float* stages, float4 (&acc)[(LHI + 1) * (LHI + 1) - LLO * LLO]) {
     using S = Shape<LMAX>;
     constexpr int kRows = (LHI + 1) * (LHI + 1) - LLO * LLO, R0 = LLO * LLO;
     constexpr int W0 = S::woff(LLO), WN = S::woff(LHI + 1) - W0;
     constexpr int NR = rows_of<LMAX>(LLO, LHI), NS = slots_of<LMAX>(LLO, LHI);
     static_assert(WN <= 64, "two Wigner entries a lane");
+    static_assert(NR + NS <= kGatherRows, "a stage");
+    constexpr bool kAhead = ahead<LMAX, HALF>;
     const int c0 = lane * 4;
     float4 xv[kRows];
 #pragma unroll
@@ -477,35 +487,65 @@ __device__ __forceinline__ void gather_bwd_pass(const float* __restrict__ grad, 
         acc[r] = f4zero();
     }
     if (eb >= ee) return;
-    int64_t e = HALF == 0 ? (int64_t)__ldg(perm + eb) : (int64_t)eb;  // global edge
-    float w0 = lane < WN ? __ldg(wig + e * S::kW + W0 + lane) : 0.f, w1 = lane + 32 < WN ? __ldg(wig + e * S::kW + W0 + 32 + lane) : 0.f;
-    for (int k = eb; k < ee; k += STEP) {
-        const int64_t i = e - e_base;  // row of the chunk's buffers
-        const int64_t ecur = e;
-        const float* go_base = grad + i * (int64_t)S::kM * 2 * C + HALF * C + c0;
-        const int64_t rad_base = i * (int64_t)S::kRad * 2 * C + HALF * C + c0;
-        float4 go[NR], rd[NS];
-        {
-            int r = 0, q = 0;
+    auto edge = [&](int k) -> int64_t { return HALF == 0 ? (int64_t)__ldg(perm + k) : (int64_t)k; };
+    // every gradient row (l, m) and radial weight (l, |m|) of edge row i of the chunk's buffers, in the order of the pass
+    auto rows = [&](int64_t i, auto&& use) {
+        const float* go = grad + i * (int64_t)S::kM * 2 * C + HALF * C + c0;
+        const float* rd = radial + i * (int64_t)S::kRad * 2 * C + HALF * C + c0;
+        int r = 0;
 #pragma unroll
-            for (int l = LLO; l <= LHI; ++l) {
+        for (int l = LLO; l <= LHI; ++l) {
 #pragma unroll
-                for (int m = -S::mm(l); m <= S::mm(l); ++m) go[r++] = __ldcs(reinterpret_cast<const float4*>(go_base + S::mrow(l, m) * 2 * C));
-#pragma unroll
-                for (int am = 0; am <= S::mm(l); ++am) rd[q++] = __ldcs(reinterpret_cast<const float4*>(radial + rad_base + S::radslot(l, am) * 2 * C));
-            }
+            for (int m = -S::mm(l); m <= S::mm(l); ++m) use(r++, go + S::mrow(l, m) * 2 * C);
         }
+#pragma unroll
+        for (int l = LLO; l <= LHI; ++l) {
+#pragma unroll
+            for (int am = 0; am <= S::mm(l); ++am) use(r++, rd + S::radslot(l, am) * 2 * C);
+        }
+    };
+    auto request = [&](int64_t i, int stage) {
+        float* dst = stages + stage * kGatherRows * C + c0;
+        if constexpr (kAhead) rows(i, [&](int r, const float* p) { copy_async16(dst + r * C, p); });
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    int64_t e = edge(eb), next = eb + STEP < ee ? edge(eb + STEP) : 0;  // global edges
+    request(e - e_base, 0);
+    commit();
+    float w0 = lane < WN ? __ldg(wig + e * S::kW + W0 + lane) : 0.f, w1 = lane + 32 < WN ? __ldg(wig + e * S::kW + W0 + 32 + lane) : 0.f;
+    int stage = 0;
+    for (int k = eb; k < ee; k += STEP, stage ^= 1) {
+        const int64_t ecur = e;
+        float4 v[NR + NS];
+        if constexpr (!kAhead) rows(e - e_base, [&](int r, const float* p) { v[r] = __ldcs(reinterpret_cast<const float4*>(p)); });
+        const int64_t rad_base = (e - e_base) * (int64_t)S::kRad * 2 * C + HALF * C + c0;
+        const bool more = k + STEP < ee;
+        if (more) {
+            e = next;
+            request(e - e_base, stage ^ 1);
+            if (k + 2 * STEP < ee) next = edge(k + 2 * STEP);
+        }
+        commit();
         float told = 0.f;
-        if (add_tau && lane < 3) told = tau[e * 4 + lane];
+        if (add_tau && lane < 3) told = tau[ecur * 4 + lane];
         __syncwarp();
         if (lane < WN) w[lane] = w0;
         if (lane + 32 < WN) w[lane + 32] = w1;
         __syncwarp();
-        if (k + STEP < ee) {
-            e = HALF == 0 ? (int64_t)__ldg(perm + k + STEP) : (int64_t)(k + STEP);
+        if (more) {
             w0 = lane < WN ? __ldg(wig + e * S::kW + W0 + lane) : 0.f;
             w1 = lane + 32 < WN ? __ldg(wig + e * S::kW + W0 + 32 + lane) : 0.f;
         }
+        if constexpr (kAhead) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll
+            for (int r = 0; r < NR + NS; ++r) v[r] = ld4(stages + (stage * kGatherRows + r) * C + c0);
+        }
+        float4 go[NR], rd[NS];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) go[r] = v[r];
+#pragma unroll
+        for (int r = 0; r < NS; ++r) rd[r] = v[NR + r];
         float t[3] = {0.f, 0.f, 0.f};
         gather_bwd_degrees<LMAX, LLO, LLO, LHI, NR, NS, 0, 0>(go, rd, grad_radial, rad_base, w, xv, acc, t);
         const float r = reduce4(t[0], t[1], t[2], 0.f, lane);
@@ -524,8 +564,10 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
     grad_radial.load_scale(scale_ptr);
     constexpr int kWarps = WPN == 1 ? 4 : WPN;
     __shared__ float sw[kWarps][48];
-    extern __shared__ float part[];  // WPN > 1: [WPN][9][C]
+    extern __shared__ float4 gather_stages[];  // a warp's two stages; WPN > 1: then its partial sums
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, c0 = lane * 4;
+    constexpr int kMine = 2 * kGatherRows * C;
+    float* stages = reinterpret_cast<float*>(gather_stages) + wid * kMine;
     const int64_t stride = WPN == 1 ? (int64_t)gridDim.x * kWarps : gridDim.x;
     for (int64_t n = n0 + (WPN == 1 ? (int64_t)blockIdx.x * kWarps + wid : blockIdx.x); n < n1; n += stride) {
         const int eb = lo[n], ee = hi[n];
@@ -537,7 +579,7 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
             constexpr int kRows = (LHI + 1) * (LHI + 1) - LLO * LLO;
             float4 acc[kRows];
             gather_bwd_pass<LMAX, LLO, LHI, HALF, WPN>(grad, x_base, wig, radial, grad_radial, perm, tau, add_tau, e_base,
-                                                       eb + (WPN == 1 ? 0 : wid), ee, lane, sw[wid], acc);
+                                                       eb + (WPN == 1 ? 0 : wid), ee, lane, sw[wid], stages, acc);
             if (WPN == 1) {
 #pragma unroll
                 for (int r = 0; r < kRows; ++r) {
@@ -546,13 +588,13 @@ __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
                 }
             } else {
 #pragma unroll
-                for (int r = 0; r < kRows; ++r) st4(part + (wid * kRows + r) * C + c0, acc[r]);
+                for (int r = 0; r < kRows; ++r) st4(stages + r * C + c0, acc[r]);
                 __syncthreads();
                 for (int r = wid; r < kRows; r += WPN) {
                     float* o = g_base + (LLO * LLO + r) * C + c0;
                     float4 v = store_gx ? f4zero() : ld4(o);
 #pragma unroll
-                    for (int i = 0; i < WPN; ++i) v = add4(v, ld4(part + (i * kRows + r) * C + c0));
+                    for (int i = 0; i < WPN; ++i) v = add4(v, ld4(stages + (i - wid) * kMine + r * C + c0));
                     st4(o, v);
                 }
                 __syncthreads();

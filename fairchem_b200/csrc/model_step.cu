@@ -322,10 +322,14 @@ static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, co
                              const float* scale, int64_t e0, int64_t n0, int64_t n1) {
     constexpr int WPN = 8;
     const Layout& L = r.L;
+    constexpr int bytes = 2 * kGatherRows * C * 4, alone = ahead<LMAX, HALF> ? 4 * bytes : 0;  // of a warp, of a block of four nodes
+    static bool done[2][64] = {};
     if (share_node(n1 - n0)) {
-        launch_pdl((gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>), dim3((int)(n1 - n0)), dim3(WPN * 32), WPN * 9 * C * 4, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
+        FCB_TRY(raise_smem(gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>, WPN * bytes, done[0]));
+        launch_pdl((gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>), dim3((int)(n1 - n0)), dim3(WPN * 32), WPN * bytes, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
     } else {
-        launch_pdl((gather_bwd_kernel<LMAX, HALF, 1, OutSplit>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
+        FCB_TRY(raise_smem(gather_bwd_kernel<LMAX, HALF, 1, OutSplit>, alone, done[1]));
+        launch_pdl((gather_bwd_kernel<LMAX, HALF, 1, OutSplit>), dim3(warp_grid(n1 - n0, 4)), dim3(128), alone, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
     }
     return FCB200_OK;
 }
