@@ -155,7 +155,7 @@ def _p(t: Optional[Tensor]):
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream)  # an index: 2 us, no argument 18
 
 
 def _chk(*tensors):

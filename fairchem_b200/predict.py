@@ -104,9 +104,8 @@ def _packed_copy(data: AtomicDataLike, device) -> AtomicDataLike:
     stage = _staging.get(total)
     for _, v, o, n in host:
         stage[o:o + n] = v.detach().reshape(-1).view(torch.uint8).numpy()
-    with torch.cuda.device(device):
-        moved = _staging.block[:total].to(device, non_blocking=True)
-        _staging.copied = torch.cuda.current_stream().record_event()
+    moved = _staging.block[:total].to(device, non_blocking=True)
+    _staging.copied = torch.cuda.current_stream(device.index).record_event()
     out = AtomicDataLike(data)
     for k, v, o, n in host:
         out[k] = moved[o:o + n].view(v.dtype).view(v.shape)
@@ -155,12 +154,16 @@ class B200PredictUnit:
     def _to_device(self, data):
         """Tensors of ``data`` on the device in the base precision; tensors that are already there are not copied."""
         dtype = getattr(self.inference_settings, "base_precision_dtype", None) or torch.float32
-        if all((not torch.is_tensor(v)) or v.device == self.device for _, v in data.items()):
+        device = self.device
+        if device.type == "cuda" and device.index is None:
+            device = torch.device("cuda", torch.cuda.current_device())
+        here = all((not torch.is_tensor(v)) or v.device == device for _, v in data.items())
+        if here and self.device == device:
             out = data
-        elif type(data) is AtomicDataLike and self.device.type == "cuda":
-            out = _packed_copy(data, self.device)
+        elif type(data) is AtomicDataLike and device.type == "cuda":
+            out = AtomicDataLike(data) if here else _packed_copy(data, device)
         else:
-            out = data.to(self.device)
+            out = data.to(device)
         for key, val in list(out.items()):
             if torch.is_tensor(val) and val.is_floating_point() and val.dtype != dtype:
                 out[key] = val.to(dtype)

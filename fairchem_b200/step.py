@@ -166,7 +166,7 @@ class ModelPlan:
     def with_head(self, head):
         """The model struct with the energy head's weights filled in (cached on the head), or None."""
         eb = head.energy_block
-        params = list(eb.parameters())
+        params = [p for i in (0, 2, 4) for p in (eb[i].weight, eb[i].bias)]
         key = (id(self), *_versions(params))
         hit = getattr(head, "_step_model", None)
         if hit is not None and hit[0] == key:
@@ -197,7 +197,7 @@ class ModelPlan:
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream)  # an index: 2 us, no argument 18
 
 
 class BackboneStep:
