@@ -16,11 +16,11 @@ the reference rebuilds the graph on every call.
 
 from __future__ import annotations
 
+import ctypes
 import threading
 from dataclasses import dataclass, field
 from typing import Mapping, Optional
 
-import numpy as np
 import torch
 
 from .synthetic import AtomicDataLike
@@ -76,15 +76,14 @@ class _Staging(threading.local):
     """Pinned block a thread's host inputs are packed into, and the event after its last copy."""
 
     def __init__(self):
-        self.block = self.bytes = self.copied = None
+        self.block = self.copied = None
 
-    def get(self, nbytes: int) -> np.ndarray:
+    def get(self, nbytes: int) -> int:
         if self.block is None or self.block.numel() < nbytes:
             self.block = torch.empty(max(2 * nbytes, 1 << 16), dtype=torch.uint8, pin_memory=True)
-            self.bytes = self.block.numpy()
         elif self.copied is not None:
             self.copied.synchronize()  # the previous call's copy has read the block
-        return self.bytes
+        return self.block.data_ptr()
 
 
 _staging = _Staging()
@@ -97,18 +96,21 @@ def _packed_copy(data: AtomicDataLike, device) -> AtomicDataLike:
     for k, v in data.items():
         if torch.is_tensor(v) and v.device.type == "cpu":
             n = v.numel() * v.element_size()
-            host.append((k, v, total, n))
+            host.append((k, v.detach().contiguous(), total, n))
             total += (n + 255) // 256 * 256
     if total > _PACK_LIMIT:
         return data.to(device)
     stage = _staging.get(total)
     for _, v, o, n in host:
-        stage[o:o + n] = v.detach().reshape(-1).view(torch.uint8).numpy()
+        ctypes.memmove(stage + o, v.data_ptr(), n)
     moved = _staging.block[:total].to(device, non_blocking=True)
     _staging.copied = torch.cuda.current_stream(device.index).record_event()
-    out = AtomicDataLike(data)
-    for k, v, o, n in host:
-        out[k] = moved[o:o + n].view(v.dtype).view(v.shape)
+    out, typed = AtomicDataLike(data), {}
+    for k, v, o, _ in host:
+        block = typed.get(v.dtype)
+        if block is None:
+            block = typed[v.dtype] = moved.view(v.dtype)
+        out[k] = block.as_strided(v.shape, v.stride(), o // v.element_size())
     for k, v in data.items():
         if torch.is_tensor(v) and v.device.type != "cpu" and v.device != device:
             out[k] = v.to(device)
