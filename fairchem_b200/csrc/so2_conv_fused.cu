@@ -259,7 +259,8 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
             // What the rows that follow are multiplied by, made while the tensor core works on the tile.  The values pass
             // through the thread's own slots of the shared tile so that the sigmoids are a loop: unrolled for both chunks,
             // and with row 0 and the gate's gradient unrolled too, the code of a tile outgrew the instruction cache and a
-            // quarter of the epilogue's stalls were instruction fetches (gated backward launches of an evaluation, 62 118 edges: 1.40 -> 1.26 ms; 775 000: 18.9 -> 17.3).
+            // quarter of the epilogue's stalls were instruction fetches (gated backward launches of an evaluation, 62 118 edges:
+            // 1.40 -> 1.26 ms; 775 000: 18.9 -> 17.3).
             if constexpr (KIND == kBackwardKind) {
                 if (mode == kSiluBwd || (t.flags & (kFirst | kSolo))) {
                     const bool slope = mode == kSiluBwd;
@@ -356,34 +357,45 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
                 if (bias) b = ld4(bias + t.w_row + col + c4);
                 const f32x2 b01 = pack(b.x, b.y), b23 = pack(b.z, b.w);
                 // body(i, x01, x23, in): row rr + 4 i of the chunk, four columns
+                auto row_of = [&](int i, auto&& body) {
+                    f32x2 x0, x1;
+                    get(slot(i), x0, x1);
+                    if constexpr (KIND == kBackwardKind) body(i, mul2(x0, os2), mul2(x1, os2), rr + 4 * i < live);
+                    else body(i, fma2(x0, os2, b01), fma2(x1, os2, b23), rr + 4 * i < live);
+                };
                 auto rows = [&](auto&& body) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        f32x2 x0, x1;
-                        get(slot(i), x0, x1);
-                        if constexpr (KIND == kBackwardKind) body(i, mul2(x0, os2), mul2(x1, os2), rr + 4 * i < live);
-                        else body(i, fma2(x0, os2, b01), fma2(x1, os2, b23), rr + 4 * i < live);
-                    }
+                    for (int i = 0; i < 8; ++i) row_of(i, body);
+                };
+                auto loop = [&](auto&& body) {
+#pragma unroll 2
+                    for (int i = 0; i < 8; ++i) row_of(i, body);
                 };
                 float* const yo = yrow + col;
                 __half *const ph = ohi + t.out_col + col, *const pl = olo + t.out_col + col;
                 auto gate_of = [&](float v) { return o_scale * sigmoid_f(gate_silu ? v * sigmoid_f(v) : v); };
                 if (KIND == kPlainKind || mode == kPlain) {
                     const bool inside = t.out_col + col + c4 < prm.y_cols;
-                    rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                    auto store = [&](int i, f32x2 x0, f32x2 x1, bool in) {
                         if (in && inside) store_pair(yo + 4 * i * prm.ldy + t.out_col, x0, x1);
-                        if constexpr (KIND == kForwardKind) {
-                            if (t.flags & kGateSrc) {
-                                keepv[c2][2 * i] = map2(x0, gate_of);
-                                keepv[c2][2 * i + 1] = map2(x1, gate_of);
-                            }
+                    };
+                    if constexpr (KIND == kForwardKind) {  // sigmoids in a loop for the code's size (155 000 edges 4.67 -> 4.55 ms, 3 240: 0.45 -> 0.43)
+                        loop([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                            store(i, x0, x1, in);
+                            put(slot(i), map2(x0, gate_of), map2(x1, gate_of));
+                        });
+                        if (t.flags & kGateSrc) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) get(slot(i), keepv[c2][2 * i], keepv[c2][2 * i + 1]);
                         }
-                    });
+                    } else {
+                        rows(store);
+                    }
                 } else if constexpr (KIND == kForwardKind) {
                     const bool keep = (t.flags & kKeep) != 0;
                     if (mode == kSilu) {
                         auto sig = [&](float v) { return o_scale * sigmoid_f(v); };
-                        rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
+                        loop([&](int i, f32x2 x0, f32x2 x1, bool in) {
                             if (in && keep) store_pair(yo + 4 * i * prm.ldy + t.y_col, x0, x1);
                             store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, map2(x0, sig)), mul2(x1, map2(x1, sig)), in, top);
                         });
