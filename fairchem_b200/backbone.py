@@ -1346,9 +1346,13 @@ class eSCNMDBackboneB200(nn.Module):
             return None
         status = _status(pos.device)
         graph = step.StepGraph(self, data, status, torch.is_grad_enabled() and pos.requires_grad)
-        if self.otf_graph and not self.always_use_pbc and graph.build():
-            edge_index, cell_offsets = graph.edge_index, graph.cell_offsets
-        else:
+        new_step = lambda: step.BackboneStep(plan, graph, plan.dataset_index(self, data["dataset"]), data["charge"], data["spin"],  # noqa: E731
+                                             gamma, self.regress_stress, status)
+        built = self.otf_graph and not self.always_use_pbc and graph.build()
+        if built:
+            run = new_step()  # before finish(), which waits for the graph's kernels
+            built = graph.finish()
+        if not built:
             edge_index, cell_offsets = self._graph(data)
             if edge_index.shape[1] == 0:  # isolated atoms: see _forward
                 edge_index = torch.zeros(2, 1, dtype=torch.long, device=pos.device)
@@ -1357,14 +1361,15 @@ class eSCNMDBackboneB200(nn.Module):
             else:
                 edge_sys = None if data["cell"].shape[0] == 1 else data["batch"][edge_index[1]]
                 graph.from_edges(edge_index[0], edge_index[1], get_pbc_shifts(data["cell"].to(pos.dtype), cell_offsets, edge_sys).contiguous())
-        data["scatter_target"] = edge_index[1]
-        self.last_graph = {"edge_index": edge_index, "cell_offsets": cell_offsets}
-        run = step.BackboneStep(plan, graph, plan.dataset_index(self, data["dataset"]), data["charge"], data["spin"], gamma,
-                                self.regress_stress, status)
+            graph.edge_index, graph.cell_offsets = edge_index, cell_offsets
+            run = new_step()
+        run.set_edges(graph)
         if not run.plan_memory():
             return None
         run.virial = {"num_systems": graph.systems} if self.regress_stress else None
         x = step.BackboneFn.apply(pos, run)
+        data["scatter_target"] = graph.edge_index[1]
+        self.last_graph = {"edge_index": graph.edge_index, "cell_offsets": graph.cell_offsets}
         run.embedding = weakref.ref(x)  # x's autograd node holds the run: a strong reference would be a cycle
         return {"node_embedding": x, "batch": data["batch"], "virial": run.virial, "step": run}
 

@@ -116,8 +116,7 @@ def wrap_positions(pos: np.ndarray, cell: np.ndarray, pbc: np.ndarray) -> np.nda
 def atoms_to_data(atoms, task_name: str, target_dtype: torch.dtype = torch.float32) -> AtomicDataLike:
     pbc = np.array(_field(atoms, "pbc", "get_pbc"), dtype=bool).reshape(3)
     raw_cell = np.array(atoms.cell if not hasattr(atoms, "get_cell") else atoms.get_cell(), dtype=np.float64).reshape(3, 3)
-    volume = abs(np.linalg.det(raw_cell))
-    if pbc.any() and not pbc.all() and volume < 0.1:
+    if pbc.any() and not pbc.all() and abs(np.linalg.det(raw_cell)) < 0.1:
         raise ValueError("atoms must either have a cell or have a cell created by setting <molecule_cell_size>.")
     cell = complete_cell(raw_cell)
     pos = wrap_positions(np.array(_field(atoms, "positions", "get_positions"), dtype=np.float64), cell, pbc)
@@ -129,10 +128,10 @@ def atoms_to_data(atoms, task_name: str, target_dtype: torch.dtype = torch.float
         atomic_numbers=torch.from_numpy(numbers),
         cell=torch.from_numpy(cell).to(target_dtype).view(1, 3, 3),
         pbc=torch.from_numpy(pbc).view(1, 3),
-        natoms=torch.tensor([n], dtype=torch.long),
+        natoms=torch.from_numpy(np.array([n], dtype=np.int64)),
         batch=torch.zeros(n, dtype=torch.long),
-        charge=torch.tensor([int(info.get("charge", 0))], dtype=torch.long),
-        spin=torch.tensor([int(info.get("spin", 0))], dtype=torch.long),
+        charge=torch.from_numpy(np.array([int(info.get("charge", 0))], dtype=np.int64)),
+        spin=torch.from_numpy(np.array([int(info.get("spin", 0))], dtype=np.int64)),
         dataset=[task_name],
     )
 

@@ -73,10 +73,10 @@ def default_tasks(backbone) -> dict:
 
 
 class _Staging(threading.local):
-    """Pinned block a thread's host inputs are packed into, and the event after its last copy."""
+    """Pinned block a thread's host inputs are packed into, and an event per device after its last copy."""
 
     def __init__(self):
-        self.block = self.copied = None
+        self.block, self.copied, self.events = None, None, {}
 
     def get(self, nbytes: int) -> int:
         if self.block is None or self.block.numel() < nbytes:
@@ -84,6 +84,12 @@ class _Staging(threading.local):
         elif self.copied is not None:
             self.copied.synchronize()  # the previous call's copy has read the block
         return self.block.data_ptr()
+
+    def record(self, device: int) -> None:
+        self.copied = self.events.get(device)
+        if self.copied is None:
+            self.copied = self.events[device] = torch.cuda.Event()
+        self.copied.record(torch.cuda.current_stream(device))
 
 
 _staging = _Staging()
@@ -95,8 +101,10 @@ def _packed_copy(data: AtomicDataLike, device) -> AtomicDataLike:
     host, total = [], 0
     for k, v in data.items():
         if torch.is_tensor(v) and v.device.type == "cpu":
+            if not v.is_contiguous():
+                v = v.detach().contiguous()
             n = v.numel() * v.element_size()
-            host.append((k, v.detach().contiguous(), total, n))
+            host.append((k, v, total, n))
             total += (n + 255) // 256 * 256
     if total > _PACK_LIMIT:
         return data.to(device)
@@ -104,7 +112,7 @@ def _packed_copy(data: AtomicDataLike, device) -> AtomicDataLike:
     for _, v, o, n in host:
         ctypes.memmove(stage + o, v.data_ptr(), n)
     moved = _staging.block[:total].to(device, non_blocking=True)
-    _staging.copied = torch.cuda.current_stream(device.index).record_event()
+    _staging.record(device.index)
     out, typed = AtomicDataLike(data), {}
     for k, v, o, _ in host:
         block = typed.get(v.dtype)

@@ -208,8 +208,7 @@ class BackboneStep:
         self.nodes, self.systems, self.device = graph.nodes, graph.systems, graph.device
         e, g = EvalStruct(), graph.g
         self.ev = e
-        e.num_nodes, e.num_edges, e.num_systems = self.nodes, graph.num_edges, self.systems
-        e.num_chunks, e.want_grad = graph.num_chunks, int(graph.want_grad)
+        e.num_nodes, e.num_systems, e.want_grad = self.nodes, self.systems, int(graph.want_grad)
         charge, spin = charge.to(self.device, torch.int64).contiguous(), spin.to(self.device, torch.int64).contiguous()
         gamma = None if gamma is None else gamma.contiguous()
         self.refs = [graph, dataset, charge, spin, gamma, status]
@@ -218,11 +217,15 @@ class BackboneStep:
         e.shift, e.dataset, e.charge, e.spin = graph.shift, dataset.data_ptr(), charge.data_ptr(), spin.data_ptr()
         e.gamma = None if gamma is None else gamma.data_ptr()
         e.status = status.data_ptr()
-        e.chunk_src = g.chunk_src if graph.num_chunks > 1 else None
-        e.chunk_node, e.chunk_edge = ctypes.cast(graph.chunk_node, c_void_p), ctypes.cast(graph.chunk_edge, c_void_p)
         self.want_virial, self.virial = want_virial, None
         self.sizes = (c_int64 * 3)()
         self.keep = self.scratch = None
+
+    def set_edges(self, graph: "StepGraph"):
+        e = self.ev
+        e.num_edges, e.num_chunks = graph.num_edges, graph.num_chunks
+        e.chunk_src = graph.g.chunk_src if graph.num_chunks > 1 else None
+        e.chunk_node, e.chunk_edge = ctypes.addressof(graph.chunk_node), ctypes.addressof(graph.chunk_edge)
 
     def plan_memory(self) -> bool:
         """Decide whether the radial weights are kept too; False when the kept tensors do not fit the free memory."""
@@ -360,6 +363,7 @@ class StepGraph:
         for name, p in self.a.ptr.items():
             setattr(g, name, p)
         self.chunk_src = self.edge_index = self.cell_offsets = self.shift = None
+        self.pending = False
 
     def _call(self, name):
         _lib.call(name, byref(self.g), _stream())
@@ -391,15 +395,11 @@ class StepGraph:
         rows = torch.empty(capacity * 2, dtype=torch.int32, device=self.device)
         g.rows = rows.data_ptr()
         # Few nodes: the edge arrays are sized for every kept-neighbour slot, so that they are filled before the host learns
-        # the edge count instead of after it.
+        # the edge count instead of after it; finish() reads it once the host has nothing else left to prepare.
         if nl is None and self.nodes <= BRUTE_NODES and 2 * capacity < 3 * g.chunk_edges:
             self._call("fcb200_graph_select")
             self._fill(capacity, 1)
-            info = self.a.view("info", 8).tolist()
-            if info[1] or info[0] == 0:
-                return False
-            self._set_chunks(info[0], [0, self.nodes], [0, info[0]])
-            self.edge_index, self.cell_offsets = self.edge_index[:, :info[0]], self.cell_offsets[:info[0]]
+            self.pending = True
             return True
         if nl is not None:
             info = self._select_kept(nl)
@@ -420,6 +420,17 @@ class StepGraph:
             return False
         self._finish_info(info)
         self._fill(self.num_edges, self.num_chunks)
+        return True
+
+    def finish(self) -> bool:
+        """After build: the number of edges where it is not known yet.  False: not for this path."""
+        if self.pending:
+            self.pending = False
+            info = self.a.view("info", 8).tolist()
+            if info[1] or info[0] == 0:
+                return False
+            self._set_chunks(info[0], [0, self.nodes], [0, info[0]])
+            self.edge_index, self.cell_offsets = self.edge_index[:, :info[0]], self.cell_offsets[:info[0]]
         return True
 
     def _fill(self, capacity: int, chunks: int):
