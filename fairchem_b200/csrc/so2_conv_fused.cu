@@ -357,19 +357,29 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
                 if (bias) b = ld4(bias + t.w_row + col + c4);
                 const f32x2 b01 = pack(b.x, b.y), b23 = pack(b.z, b.w);
                 // body(i, x01, x23, in): row rr + 4 i of the chunk, four columns
-                auto row_of = [&](int i, auto&& body) {
-                    f32x2 x0, x1;
-                    get(slot(i), x0, x1);
+                auto row_of = [&](int i, f32x2 x0, f32x2 x1, auto&& body) {
                     if constexpr (KIND == kBackwardKind) body(i, mul2(x0, os2), mul2(x1, os2), rr + 4 * i < live);
                     else body(i, fma2(x0, os2, b01), fma2(x1, os2, b23), rr + 4 * i < live);
                 };
+                // Shared reads of four rows first: a read keeps its place behind another row's stores, and so behind its
+                // arithmetic (gated backward launches of an evaluation, 155 000 edges: 3.45 -> 3.17 ms).
                 auto rows = [&](auto&& body) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) row_of(i, body);
+                    for (int i0 = 0; i0 < 8; i0 += 4) {
+                        f32x2 x[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) get(slot(i0 + i), x[2 * i], x[2 * i + 1]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) row_of(i0 + i, x[2 * i], x[2 * i + 1], body);
+                    }
                 };
                 auto loop = [&](auto&& body) {
 #pragma unroll 2
-                    for (int i = 0; i < 8; ++i) row_of(i, body);
+                    for (int i = 0; i < 8; ++i) {
+                        f32x2 x0, x1;
+                        get(slot(i), x0, x1);
+                        row_of(i, x0, x1, body);
+                    }
                 };
                 float* const yo = yrow + col;
                 __half *const ph = ohi + t.out_col + col, *const pl = olo + t.out_col + col;
@@ -813,14 +823,16 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         const Groups fine = group_tiles(list, num_tiles, rot_begin, kFine);
         if (fine.ok && 10 * makespan(fine, rows_m, sm_count()) < 9 * makespan(grp, rows_m, sm_count())) grp = fine;
     }
-    // backward: the same, if there is room for the raw rows and the second kernel pays: about 5 us, 600 units of K, and its
-    // reads and the raw rows' writes at the memory's rate, 55 KB a unit (without that term 120 000 edges of lmax 4 took the second
-    // kernel: 1.79 + 0.39 ms for 1.46)
+    // backward: the same, if there is room for the raw rows and the second kernel pays: about 3 us, 300 units of K, and its
+    // reads and the raw rows' writes at the memory's rate, 55 KB a unit.  A row on its own costs 1.6 times its estimate (its
+    // factors are made anew and nothing overlaps its epilogue), one in a group 1.1 times.  Natural against row by row, us:
+    // lmax 2, 960 rows 34 / 19, 3 240 rows 37 / 35, 4 320 rows 38 / 45, 7 680 rows 64 / 67; lmax 4, 960 rows 53 / 41, 3 240
+    // rows 60 / 79, 4 320 rows 105 / 96, 7 680 rows 144 / 165.
     GateSums sums{};
     bool solo = backward && raw && grouping != kNatural && split_sums(list, num_tiles, sums);
     if (solo && grouping != kFine) {
-        const int64_t extra = 600 + m * (sums.begin[sums.degrees] + sums.degrees) * (BN * 8) / 55000;
-        solo = makespan(group_tiles(list, num_tiles, rot_begin, kFine), rows_m, sm_count()) + extra < makespan(grp, rows_m, sm_count());
+        const int64_t extra = 300 + m * (sums.begin[sums.degrees] + sums.degrees) * (BN * 8) / 55000;
+        solo = 16 * makespan(group_tiles(list, num_tiles, rot_begin, kFine), rows_m, sm_count()) + 10 * extra < 11 * makespan(grp, rows_m, sm_count());
     }
     if (solo) {
         for (int i = 0; i < num_tiles; ++i)
