@@ -554,7 +554,7 @@ __device__ __forceinline__ void gather_bwd_pass(const float* __restrict__ grad, 
 }
 
 template <int LMAX, int HALF, int WPN, class RadOut>
-__global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 1 ? 3 : 1)
+__global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN, WPN == 8 ? 1 : 3)
     gather_bwd_kernel(const float* __restrict__ grad, const float* __restrict__ x, const int32_t* __restrict__ lo,
                       const int32_t* __restrict__ hi, const int32_t* __restrict__ perm, const float* __restrict__ wig,
                       const float* __restrict__ radial, float* __restrict__ gx, int store_gx, float* __restrict__ tau, int store_tau,

@@ -320,13 +320,24 @@ static int launch_rotate_back(const Run& r, const float* msg, int64_t e_base, co
 template <int LMAX, int HALF>
 static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, const int32_t* hi, const float* radial, float* gx, bool store_gx, bool store_tau,
                              const float* scale, int64_t e0, int64_t n0, int64_t n1) {
-    constexpr int WPN = 8;
     const Layout& L = r.L;
     constexpr int bytes = 2 * kGatherRows * C * 4, alone = ahead<LMAX, HALF> ? 4 * bytes : 0;  // of a warp, of a block of four nodes
-    static bool done[2][64] = {};
-    if (share_node(n1 - n0)) {
-        FCB_TRY(raise_smem(gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>, WPN * bytes, done[0]));
+    static bool done[3][64] = {};
+    auto shared = [&](auto tag, bool (&up)[64]) {
+        constexpr int WPN = decltype(tag)::value;
+        FCB_TRY(raise_smem(gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>, WPN * bytes, up));
         launch_pdl((gather_bwd_kernel<LMAX, HALF, WPN, OutSplit>), dim3((int)(n1 - n0)), dim3(WPN * 32), WPN * bytes, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);
+        return (int)FCB200_OK;
+    };
+    // Twelve warps fit an SM.  Four to a node where whole waves of one node a warp would leave the last one nearly empty
+    // (us of an evaluation, lmax 2: 1 296 nodes 688 -> 656, 1 782 1026 -> 904, 2 000 1198 -> 1002, 2 592 1384 -> 1259, 4 050 2076 ->
+    // 1951; where it does not: 1 440 731 -> 771, 3 120 1496 -> 1529, 5 280 2414 -> 2545; lmax 4, 2 048 nodes 9662 -> 7773).
+    // More nodes come in several chunks, which hold too few edges of a source to share.
+    const int64_t n = n1 - n0, sms = sm_count(), waves = (n + 12 * sms - 1) / (12 * sms), quarters = (n + 3 * sms - 1) / (3 * sms);
+    if (share_node(n)) {
+        FCB_TRY(shared(std::integral_constant<int, 8>{}, done[0]));
+    } else if (waves <= 3 && 11 * quarters < 40 * waves) {
+        FCB_TRY(shared(std::integral_constant<int, 4>{}, done[2]));
     } else {
         FCB_TRY(raise_smem(gather_bwd_kernel<LMAX, HALF, 1, OutSplit>, alone, done[1]));
         launch_pdl((gather_bwd_kernel<LMAX, HALF, 1, OutSplit>), dim3(warp_grid(n1 - n0, 4)), dim3(128), alone, r.st, L.gm, x, lo, hi, r.ev.src_perm, L.wig, radial, gx, (int)store_gx, L.tau_n, (int)store_tau, L.grad.out(), scale, e0, n0, n1);

@@ -1,5 +1,5 @@
 """Whole-model native evaluation (csrc/model_step.cu) against the per-op path, at the sizes where its dispatch changes:
-one atom without neighbours, ragged row tiles, node counts on both sides of the shared-node kernels, several chunks."""
+one atom without neighbours, ragged row tiles, node counts for each way of sharing a node's edges among warps (8, 4, 1), several chunks."""
 
 import pytest
 import torch
@@ -13,6 +13,8 @@ CASES = {
     "fcc_32_chunks": (lambda s: s.fcc_cu((2, 2, 2), seed=4), {"edge_chunk_size": 257}),
     "alloy_stress": (lambda s: s.bcc_alloy((3, 4, 5), seed=5), {"regress_stress": True}),
     "water_2200": (lambda s: s.water_box(2200, seed=6), {"edge_chunk_size": 30000}),
+    "water_1201": (lambda s: s.water_box(1201, seed=7), {}),
+    "alloy_1440": (lambda s: s.bcc_alloy((12, 12, 5), seed=8), {}),
     "batch_stress": (lambda s: s.merge([s.fcc_cu((2, 2, 2), seed=1), s.bcc_alloy((2, 3, 2), seed=2)]), {"regress_stress": True}),
 }
 
