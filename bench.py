@@ -39,7 +39,7 @@ ACC = 9.648533e-3  # (eV/A)/amu -> A/fs^2
 MASS = {1: 1.008, 6: 12.011, 7: 14.007, 8: 15.999, 24: 51.996, 25: 54.938, 26: 55.845, 27: 58.933, 28: 58.693, 29: 63.546}
 CPU_SAMPLE_ATOMS = 1500
 # DRAM bytes (read + write) per edge of one launch of so2_conv_fused_kernel, mean over its four convolution plans, from the
-# ncu capture of 62 118-edge launches summarised in profiles/so2_conv_fused_kernel_bcc_alloy_2000.md:
+# ncu capture of 62 118-edge launches:
 # (886 + 587) + (288 + 235) + (770 + 314) + (355 + 517) MB over 4 launches; traffic grows in proportion to the edges
 FUSED_TRAFFIC_PER_EDGE_LAUNCH = (1473e6 + 523e6 + 1084e6 + 872e6) / 4 / 62118
 
