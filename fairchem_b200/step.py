@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import operator
+from itertools import chain
 from ctypes import POINTER, Structure, byref, c_float, c_int32, c_int64, c_void_p
 
 import torch
@@ -54,10 +55,39 @@ class EvalStruct(Structure):
 
 
 _VERSION = operator.attrgetter("_version")
+_EPS = operator.attrgetter("eps")
+_SCALARS = operator.attrgetter("lmax", "num_distance_basis", "max_num_elements", "cutoff", "rescale_factor", "sphere_channels",
+                               "hidden_channels", "edge_channels")
 
 
 def _versions(params) -> list:
     return [*map(_VERSION, params), *map(torch.Tensor.data_ptr, params)]
+
+
+class _Origin:
+    """What a plan was laid out from: every submodule and parameter a backbone holds, the parameters' versions and
+    addresses, and the plain numbers that went into the plan.  The objects are looked up again on each call, because an
+    assigned parameter (``load_state_dict(assign=True)``, ``functional_call``, ``module.weight = ...``) leaves the old
+    one as it was; that takes 12 us of host time for four layers."""
+
+    def __init__(self, bb):
+        mods = list(bb.modules())
+        self.views = [m._modules.values() for m in mods if m._modules] + [m._parameters.values() for m in mods if m._parameters]
+        self.eps_of = [m for m in mods if hasattr(m, "eps")]
+        self.objects = self._objects()
+        self.params = [o for o in self.objects if isinstance(o, torch.Tensor)]
+        self.versions, self.scalars = _versions(self.params), self._scalars(bb)
+
+    def _objects(self) -> list:
+        return [*chain.from_iterable(self.views)]
+
+    def _scalars(self, bb) -> list:
+        return [*_SCALARS(bb), *map(_EPS, self.eps_of)]
+
+    def unchanged(self, bb) -> bool:
+        now = self._objects()
+        return (len(now) == len(self.objects) and all(map(operator.is_, now, self.objects))
+                and self.versions == _versions(self.params) and self.scalars == self._scalars(bb))
 
 
 class _Weights:
@@ -82,16 +112,16 @@ def _radial_nets(bb):
 
 
 class ModelPlan:
-    """Weights of one backbone in the layout of csrc/model_step.cu, rebuilt when a parameter changes."""
+    """Weights of one backbone in the layout of csrc/model_step.cu, rebuilt when anything they were read from changes."""
 
-    def __init__(self, bb, params):
+    def __init__(self, bb, origin: _Origin):
         from .backbone import _conv_weights
 
-        self.params, self.versions = params, _versions(params)
+        self.origin = origin
         w = self.w = _Weights()
-        self.device = params[0].device
+        self.device = origin.params[0].device
         lmax, nb = bb.lmax, bb.num_distance_basis
-        self.layers = (LayerStruct * bb.num_layers)()
+        self.layers = (LayerStruct * len(bb.blocks))()
         for s, blk in zip(self.layers, bb.blocks):
             ew, ff = blk.edge_wise, blk.atom_wise
             for name, conv in (("conv1", ew.so2_conv_1), ("conv2", ew.so2_conv_2)):
@@ -114,7 +144,7 @@ class ModelPlan:
             s.norm2_w, s.norm2_b = w.ptr(blk.norm_2.affine_weight), w.ptr(blk.norm_2.affine_bias)
             s.eps1, s.eps2 = blk.norm_1.eps, blk.norm_2.eps
         m = self.model = ModelStruct()
-        m.lmax, m.num_layers, m.num_basis, m.num_elements = lmax, bb.num_layers, nb, bb.max_num_elements
+        m.lmax, m.num_layers, m.num_basis, m.num_elements = lmax, len(bb.blocks), nb, bb.max_num_elements
         m.cutoff, m.basis_start, m.basis_stop, m.basis_width = bb.cutoff, 0.0, bb.cutoff, 2.0
         m.rescale, m.norm_eps = bb.rescale_factor, bb.norm.eps
         m.layers = self.layers
@@ -137,14 +167,14 @@ class ModelPlan:
         self.dataset_row = {name: i for i, name in enumerate(emb)}
         m.dataset_emb = w.ptr(torch.cat([e.weight for e in emb.values()]))
         m.csd_w_t, m.csd_b = w.ptr(bb.mix_csd.weight.t()), w.ptr(bb.mix_csd.bias)
-        self.dataset_ids = {}  # (names) -> int32 device tensor of their rows, for batches of one dataset
+        self.dataset_ids = {}  # (row, systems) -> int32 device tensor, for batches of one dataset
 
     @staticmethod
     def supported(bb) -> bool:
         """Shapes that csrc/model_step.cu is written for."""
         nets = _radial_nets(bb)
         return (bb.sphere_channels == C and bb.hidden_channels == C and bb.edge_channels == C and bb.num_distance_basis % 32 == 0
-                and 1 <= bb.num_layers < 40
+                and 1 <= len(bb.blocks) < 40
                 and all(len(n.net) == 7 and n.net[1].eps == n.net[4].eps == nets[0].net[1].eps for n in nets))
 
     @classmethod
@@ -155,12 +185,12 @@ class ModelPlan:
         if not (mode.precision == 2 and mode.fused_conv and mode.native and ops.CONV_VARIANT == -1 and bb.keep_level is None) or ops.generic_kernels():
             return None
         plan = getattr(bb, "_step_plan", None)
-        if plan is not None and plan.versions == _versions(plan.params):
+        if plan is not None and plan.origin.unchanged(bb):
             return plan
-        params = list(bb.parameters())
-        if not cls.supported(bb) or not params[0].is_cuda or any(p.dtype != torch.float32 for p in params):
+        origin = _Origin(bb)
+        if not cls.supported(bb) or not origin.params[0].is_cuda or any(p.dtype != torch.float32 for p in origin.params):
             return None
-        bb._step_plan = plan = cls(bb, params)
+        bb._step_plan = plan = cls(bb, origin)
         return plan
 
     def with_head(self, head):
@@ -185,14 +215,17 @@ class ModelPlan:
         return m
 
     def dataset_index(self, bb, names) -> torch.Tensor:
-        key = names[0] if all(n == names[0] for n in names) else None
-        if key is not None:
-            hit = self.dataset_ids.get((key, len(names)))
-            if hit is not None:
-                return hit
-        idx = torch.tensor([self.dataset_row[bb.dataset_embedding.mapping[n]] for n in names], dtype=torch.int32, device=self.device)
-        if key is not None and len(self.dataset_ids) < 64:
-            self.dataset_ids[(key, len(names))] = idx
+        mapping, key = bb.dataset_embedding.mapping, None
+        if all(n == names[0] for n in names):
+            rows = [self.dataset_row[mapping[names[0]]]] * len(names)
+            key = (rows[0], len(names))
+        else:
+            rows = [self.dataset_row[mapping[n]] for n in names]
+        idx = self.dataset_ids.get(key)
+        if idx is None:
+            idx = torch.tensor(rows, dtype=torch.int32, device=self.device)
+            if key is not None and len(self.dataset_ids) < 64:
+                self.dataset_ids[key] = idx
         return idx
 
 

@@ -101,3 +101,42 @@ def test_out_of_table_charge_is_an_error():
     d["charge"] = torch.tensor([0, 400], device="cuda")
     with pytest.raises(ValueError):
         head(d, bb(d))
+
+
+@pytest.mark.parametrize("how", ["assign", "functional_call", "scalars"])
+def test_replaced_parameters_and_settings_are_used(how):
+    """After an evaluation, other parameter objects and other plain settings: the next one uses them."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S")
+    data = synthetic.molecule_batch(2, 6, 9, seed=3).to("cuda")
+    before = head(data.clone(), bb(data.clone()))["energy"]
+    sd = {k: v.clone() for k, v in bb.state_dict().items()}
+    sd["blocks.2.edge_wise.so2_conv_1.fc_m0.weight"] *= 3.0
+    call = bb
+    if how == "assign":
+        bb.load_state_dict(sd, assign=True)
+    elif how == "functional_call":
+        call = lambda d: torch.func.functional_call(bb, sd, (d,))  # noqa: E731
+    else:
+        bb.cutoff, bb.rescale_factor, bb.blocks[1].norm_2.eps = 4.5, 3.0, 0.1
+    out = []
+    for native in (True, False):
+        B._GemmState.native = native
+        try:
+            d = data.clone()
+            emb = call(d)
+            assert ("step" in emb) == native
+            out.append(emb["node_embedding"].detach())
+            if how != "functional_call":
+                out.append(head(d, emb)["forces"])
+        finally:
+            B._GemmState.native = True
+    half = len(out) // 2
+    for got, ref in zip(out[:half], out[half:]):
+        assert _rel(got, ref) < 2e-5
+    if how == "functional_call":  # and the module's own parameters afterwards
+        d = data.clone()
+        after = head(d, bb(d))["energy"]
+        assert _rel(after, before) < 1e-6
