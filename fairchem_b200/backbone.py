@@ -1100,7 +1100,7 @@ class _RegressConfig:
     hessian: bool = False
 
 
-class eSCNMDBackboneB200(nn.Module):
+class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
     def __init__(
         self,
         max_num_elements: int = 100,
@@ -1445,7 +1445,7 @@ class eSCNMDBackboneB200(nn.Module):
         return {"node_embedding": x, "batch": batch_l, "virial": virial}
 
 
-class MLP_EFS_HeadB200(nn.Module):
+class MLP_EFS_HeadB200(step.HoldsPlan, nn.Module):
     """Energy MLP on the l=0 channels, float64 per-system sum, forces = -dE/dpos
     (src/fairchem/core/models/uma/escn_md.py:1062-1168, src/fairchem/core/models/uma/outputs.py:41-162)."""
 

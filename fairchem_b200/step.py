@@ -107,6 +107,14 @@ class _Weights:
         return Weight(hi.data_ptr(), lo.data_ptr(), scale, w.shape[0], w.shape[1])
 
 
+class HoldsPlan:
+    """Mixin of the modules that keep a plan (``_step_plan``): device addresses of their own weights, which neither a copy nor
+    a file of the module may carry.  Both lay out their own when they are first used."""
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_step_plan"}
+
+
 def _radial_nets(bb):
     return [b.edge_wise.so2_conv_1.rad_func for b in bb.blocks] + [bb.edge_degree_embedding.rad_func]
 
@@ -198,7 +206,7 @@ class ModelPlan:
         eb = head.energy_block
         params = [p for i in (0, 2, 4) for p in (eb[i].weight, eb[i].bias)]
         key = (id(self), *_versions(params))
-        hit = getattr(head, "_step_model", None)
+        hit = getattr(head, "_step_plan", None)
         if hit is not None and hit[0] == key:
             return hit[1]
         if eb[0].weight.shape != (C, C) or eb[2].weight.shape != (C, C) or eb[4].weight.shape != (1, C):
@@ -211,7 +219,7 @@ class ModelPlan:
         from .backbone import _pow2_scale
 
         m.head_scale = w.ptr(_pow2_scale(eb[4].weight.detach().abs().max() * 1.1))  # |d silu| <= 1.1
-        head._step_model = (key, m, w, self)
+        head._step_plan = (key, m, w, self)
         return m
 
     def dataset_index(self, bb, names) -> torch.Tensor:

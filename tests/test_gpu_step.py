@@ -140,3 +140,20 @@ def test_replaced_parameters_and_settings_are_used(how):
         d = data.clone()
         after = head(d, bb(d))["energy"]
         assert _rel(after, before) < 1e-6
+
+
+def test_copies_of_a_used_model_evaluate_on_their_own_weights():
+    import copy
+
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S")
+    data = synthetic.molecule_batch(2, 6, 9, seed=4).to("cuda")
+    run = lambda b, h: (lambda d: h(d, b(d))["forces"])(data.clone())  # noqa: E731
+    first = run(bb, head)
+    bb2, head2 = copy.deepcopy((bb, head))
+    with torch.no_grad():
+        bb2.blocks[0].norm_1.affine_weight.mul_(2.0)
+    assert _rel(run(bb2, head2), first) > 1e-3
+    assert _rel(run(bb, head), first) < 1e-6

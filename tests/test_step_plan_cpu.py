@@ -1,11 +1,16 @@
-"""Host side of the whole-model evaluation (fairchem_b200/step.py) that needs no GPU: when a plan is still good."""
+"""Host side of the whole-model evaluation (fairchem_b200/step.py) that needs no GPU: when a plan is still good, what a
+copy of a used model carries."""
+
+import copy
+import ctypes
+import pickle
 
 import pytest
 import torch
 import torch.nn as nn
 
 from fairchem_b200 import step, weights
-from fairchem_b200.backbone import eSCNMDBackboneB200
+from fairchem_b200.backbone import MLP_EFS_HeadB200, eSCNMDBackboneB200
 
 
 @pytest.fixture()
@@ -62,3 +67,31 @@ def test_plan_is_given_up_inside_functional_call(bb):
     bb.forward = lambda: seen.append(origin.unchanged(bb))
     torch.func.functional_call(bb, {"blocks.0.norm_1.affine_weight": torch.zeros(3, 128)}, ())
     assert seen == [False] and origin.unchanged(bb)
+
+
+def _used_model():
+    """A model as an evaluation leaves it: plans with device addresses on the backbone and the head."""
+    bb = eSCNMDBackboneB200(**dict(weights.UMA_S, num_layers=1))
+    head = MLP_EFS_HeadB200(bb)
+    bb._step_plan, head._step_plan = step.ModelStruct(), (1, step.ModelStruct())
+    bb._step_plan.layers = ctypes.pointer(step.LayerStruct())
+    return nn.ModuleDict({"bb": bb, "head": head})
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "pickle", "save", "copy"])
+def test_a_used_model_can_be_copied_and_saved_whole(how, tmp_path):
+    model = _used_model()
+    if how == "deepcopy":
+        other = copy.deepcopy(model)
+    elif how == "copy":
+        other = nn.ModuleDict({k: copy.copy(m) for k, m in model.items()})
+    elif how == "pickle":
+        other = pickle.loads(pickle.dumps(model))
+    else:
+        torch.save(model, tmp_path / "model.pt")
+        other = torch.load(tmp_path / "model.pt", weights_only=False)
+    assert model["bb"]._step_plan is not None and model["head"]._step_plan is not None
+    for m in other.values():
+        assert not hasattr(m, "_step_plan")
+    for (n, p), (_, q) in zip(model.named_parameters(), other.named_parameters()):
+        assert torch.equal(p, q), n
