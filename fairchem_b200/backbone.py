@@ -1467,6 +1467,7 @@ class MLP_EFS_HeadB200(step.HoldsPlan, nn.Module):
         out = {"energy": run.energy(model)}
         if want:
             out["forces"] = run.backward(model, None, -1.0)
+            run.spent = True
         if self.regress_stress:
             out["stress"] = self._stress(data, run.virial["virial"])
         return out

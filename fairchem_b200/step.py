@@ -253,6 +253,7 @@ class BackboneStep:
         charge, spin = charge.to(self.device, torch.int64).contiguous(), spin.to(self.device, torch.int64).contiguous()
         gamma = None if gamma is None else gamma.contiguous()
         self.refs = [graph, dataset, charge, spin, gamma, status]
+        self.watched = [t for t in (graph.pos, charge, spin, gamma) if t is not None]  # may be the caller's own memory
         for name in ("pos", "z", "batch", "src", "tgt", "row_ptr", "src_ptr", "src_perm"):
             setattr(e, name, getattr(g, name))
         e.shift, e.dataset, e.charge, e.spin = graph.shift, dataset.data_ptr(), charge.data_ptr(), spin.data_ptr()
@@ -260,7 +261,8 @@ class BackboneStep:
         e.status = status.data_ptr()
         self.want_virial, self.virial = want_virial, None
         self.sizes = (c_int64 * 3)()
-        self.keep = self.scratch = None
+        self.keep = None
+        self.spent = False  # the head has computed the forces
 
     def set_edges(self, graph: "StepGraph"):
         e = self.ev
@@ -295,6 +297,10 @@ class BackboneStep:
         return torch.empty(nbytes, dtype=torch.uint8, device=self.device)
 
     def forward(self) -> torch.Tensor:
+        self.inputs = [(t, t._version) for t in self.watched]
+        return self._forward()
+
+    def _forward(self) -> torch.Tensor:
         e = self.ev
         self.keep = self._block(self.sizes[0])
         scratch = self._block(self.sizes[1])
@@ -312,8 +318,10 @@ class BackboneStep:
 
     def backward(self, model: ModelStruct, grad_x, sign: float) -> torch.Tensor:
         """sign * gradient of the energy sum (grad_x None) or of <grad_x, node embedding> with respect to the positions."""
-        if self.keep is None:
-            raise RuntimeError("fairchem_b200: this evaluation's buffers were released by an earlier backward pass")
+        if self.keep is None:  # released by an earlier backward pass over a retained graph: computed again
+            if any(t._version != v for t, v in self.inputs):
+                raise RuntimeError("fairchem_b200: an input of this evaluation was modified in place after its first backward pass")
+            self._forward()
         e = self.ev
         scratch = self._block(self.sizes[2])
         grad = torch.empty(self.nodes, 3, dtype=torch.float32, device=self.device)
@@ -334,11 +342,16 @@ class BackboneFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pos, step: BackboneStep):
         ctx.step = step
+        ctx.save_for_backward(pos)
         return step.forward()
 
     @staticmethod
     def backward(ctx, grad_x):
-        return ctx.step.backward(ctx.step.model, grad_x.contiguous(), 1.0), None
+        ctx.saved_tensors  # raises autograd's own error for a graph that was not retained, or positions modified since
+        step = ctx.step
+        if step.spent:  # the head took its gradient from this evaluation without autograd and did not retain it
+            raise RuntimeError("fairchem_b200: the forces of this evaluation were computed already; its graph was not retained")
+        return step.backward(step.model, grad_x.contiguous(), 1.0), None
 
 
 class GraphStruct(Structure):

@@ -157,3 +157,52 @@ def test_copies_of_a_used_model_evaluate_on_their_own_weights():
         bb2.blocks[0].norm_1.affine_weight.mul_(2.0)
     assert _rel(run(bb2, head2), first) > 1e-3
     assert _rel(run(bb, head), first) < 1e-6
+
+
+@pytest.mark.parametrize("wants", ["forces", "stress"])
+def test_repeated_backward_over_a_retained_graph(wants):
+    """Several vector-Jacobian products of one node embedding, then the head's forces, as autograd allows them."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S", regress_stress=wants == "stress")
+    data = synthetic.bcc_alloy((2, 2, 3), seed=5).to("cuda")
+    out = {}
+    for native in (True, False):
+        B._GemmState.native = native
+        try:
+            d = data.clone()
+            emb = bb(d)
+            x = emb["node_embedding"]
+            gen = torch.Generator("cuda").manual_seed(2)
+            grads = [torch.autograd.grad((x * torch.randn(x.shape, generator=gen, device="cuda")).sum(), d["pos"], retain_graph=True)[0]
+                     for _ in range(3)]
+            res = head(d, emb)
+            out[native] = grads + [res[k] for k in sorted(res)]
+            with pytest.raises(RuntimeError):  # the head did not retain the graph
+                torch.autograd.grad(x.sum(), d["pos"])
+        finally:
+            B._GemmState.native = True
+    for got, ref in zip(out[True], out[False]):
+        assert _rel(got, ref) < 2e-5
+
+
+def test_backward_again_without_a_retained_graph_or_after_a_change_is_an_error():
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, _ = _model(B, "UMA_S")
+    data = synthetic.molecule_batch(2, 5, 8, seed=6).to("cuda")
+    d = data.clone()
+    x = bb(d)["node_embedding"]
+    torch.autograd.grad(x.sum(), d["pos"])
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(x.sum(), d["pos"])
+    for key in ("pos", "charge"):
+        d = data.clone()
+        x = bb(d)["node_embedding"]
+        torch.autograd.grad(x.sum(), d["pos"], retain_graph=True)
+        with torch.no_grad():
+            d[key].add_(1)
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(x.sum(), d["pos"])
