@@ -1171,6 +1171,7 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
         self.blocks = nn.ModuleList([_Block(c, h, lmax, mmax, self.edge_channels_list) for _ in range(num_layers)])
         self.norm = RMSNormSH(lmax, c)
         self.register_buffer("_wig_transpose", torch.tensor(_transpose_index()), persistent=False)
+        self._built_as = step.structure_of(self)  # another module put in later sends an evaluation down the per-op path
         self.last_graph = None
         self.neighbor_list = None  # optional SkinNeighborList: reuse of the candidate list while atoms move less than skin / 2
 
@@ -1457,8 +1458,10 @@ class MLP_EFS_HeadB200(step.HoldsPlan, nn.Module):
 
     def _forward_native(self, data, emb):
         """Energy and forces straight from the evaluation that made ``emb`` (no autograd graph in between)."""
-        run = emb.get("step", None)
-        if run is None or run.keep is None or emb["node_embedding"] is not run.embedding() or emb["node_embedding"]._version != 0:
+        run, x = emb.get("step", None), emb["node_embedding"]
+        if run is None or run.keep is None or x is not run.embedding() or x._version != 0:
+            return None
+        if x._backward_hooks or x.retains_grad or run.leaf._backward_hooks:  # autograd has more to do than the forces
             return None
         want = self.regress_forces or self.regress_stress
         model = run.plan.with_head(self)

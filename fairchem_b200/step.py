@@ -14,6 +14,7 @@ from itertools import chain
 from ctypes import POINTER, Structure, byref, c_float, c_int32, c_int64, c_void_p
 
 import torch
+import torch.nn.modules.module as _nn_module
 
 from . import _lib, ops
 
@@ -90,6 +91,34 @@ class _Origin:
                 and self.versions == _versions(self.params) and self.scalars == self._scalars(bb))
 
 
+def structure_of(bb) -> tuple:
+    """Module types and parameter shapes by name."""
+    return ({n: type(m) for n, m in bb.named_modules(remove_duplicate=False) if n},
+            {n: p.shape for n, p in bb.named_parameters(remove_duplicate=False)})
+
+
+_METHODS = ("csd_embedding", "_tables", "_graph")  # what the native evaluation does in their place
+_HOOK_DICTS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+_GLOBAL_HOOKS = [getattr(_nn_module, "_global" + n) for n in _HOOK_DICTS]
+
+
+class _Calls:
+    """The submodules that the per-op path calls as modules, and the hooks it would run.  A hook, or a forward of an
+    instance's own, sends an evaluation down that path."""
+
+    def __init__(self, bb):
+        mods = [bb.norm, bb.sphere_embedding, bb.charge_embedding, bb.charge_embedding.rand_emb, bb.spin_embedding,
+                bb.spin_embedding.rand_emb, bb.dataset_embedding, bb.mix_csd]
+        for blk in bb.blocks:
+            mods += [blk.norm_1, blk.norm_2, blk.atom_wise, blk.atom_wise.so3_linear_1, blk.atom_wise.so3_linear_2]
+        self.hooks = [*_GLOBAL_HOOKS, *(getattr(m, n) for m in mods for n in _HOOK_DICTS)]
+        self.attributes = [m.__dict__ for m in mods]
+        self.own = bb.__dict__
+
+    def watched(self) -> bool:
+        return any(map(len, self.hooks)) or any("forward" in d for d in self.attributes) or any(n in self.own for n in _METHODS)
+
+
 class _Weights:
     """Half-split device copies of a module's matrices; keeps every tensor whose address is handed out alive."""
 
@@ -125,7 +154,7 @@ class ModelPlan:
     def __init__(self, bb, origin: _Origin):
         from .backbone import _conv_weights
 
-        self.origin = origin
+        self.origin, self.calls = origin, _Calls(bb)
         w = self.w = _Weights()
         self.device = origin.params[0].device
         lmax, nb = bb.lmax, bb.num_distance_basis
@@ -179,11 +208,15 @@ class ModelPlan:
 
     @staticmethod
     def supported(bb) -> bool:
-        """Shapes that csrc/model_step.cu is written for."""
+        """Shapes that csrc/model_step.cu is written for, of the modules and methods that it stands for."""
+        from .backbone import eSCNMDBackboneB200 as plain
+
+        if not (bb.sphere_channels == C and bb.hidden_channels == C and bb.edge_channels == C and bb.num_distance_basis % 32 == 0
+                and 1 <= len(bb.blocks) < 40 and all(getattr(type(bb), n) is getattr(plain, n) for n in _METHODS)):
+            return False
         nets = _radial_nets(bb)
-        return (bb.sphere_channels == C and bb.hidden_channels == C and bb.edge_channels == C and bb.num_distance_basis % 32 == 0
-                and 1 <= len(bb.blocks) < 40
-                and all(len(n.net) == 7 and n.net[1].eps == n.net[4].eps == nets[0].net[1].eps for n in nets))
+        return (bb.__dict__.get("_built_as") in (None, structure_of(bb))
+                and all(n.net[1].eps == n.net[4].eps == nets[0].net[1].eps for n in nets))
 
     @classmethod
     def of(cls, bb):
@@ -194,12 +227,12 @@ class ModelPlan:
             return None
         plan = getattr(bb, "_step_plan", None)
         if plan is not None and plan.origin.unchanged(bb):
-            return plan
+            return None if plan.calls.watched() else plan
         origin = _Origin(bb)
         if not cls.supported(bb) or not origin.params[0].is_cuda or any(p.dtype != torch.float32 for p in origin.params):
             return None
         bb._step_plan = plan = cls(bb, origin)
-        return plan
+        return None if plan.calls.watched() else plan
 
     def with_head(self, head):
         """The model struct with the energy head's weights filled in (cached on the head), or None."""
@@ -252,6 +285,7 @@ class BackboneStep:
         e.num_nodes, e.num_systems, e.want_grad = self.nodes, self.systems, int(graph.want_grad)
         charge, spin = charge.to(self.device, torch.int64).contiguous(), spin.to(self.device, torch.int64).contiguous()
         gamma = None if gamma is None else gamma.contiguous()
+        self.leaf = graph.leaf
         self.refs = [graph, dataset, charge, spin, gamma, status]
         self.watched = [t for t in (graph.pos, charge, spin, gamma) if t is not None]  # may be the caller's own memory
         for name in ("pos", "z", "batch", "src", "tgt", "row_ptr", "src_ptr", "src_perm"):
@@ -398,6 +432,7 @@ class StepGraph:
     def __init__(self, bb, data, status, want_grad: bool):
         self.bb, self.data, self.want_grad = bb, data, want_grad
         pos = self.pos = data["pos"].detach().contiguous()
+        self.leaf = data["pos"]
         self.device, self.nodes, self.systems = pos.device, pos.shape[0], len(data["natoms"])
         n, b = self.nodes, self.systems
         self.a = _Carve(self.device, sys=b * 24, bbox=b * 6, z=n, batch=n, count=n, row_ptr=n + 1, info=INFO_WORDS)

@@ -206,3 +206,52 @@ def test_backward_again_without_a_retained_graph_or_after_a_change_is_an_error()
             d[key].add_(1)
         with pytest.raises(RuntimeError):
             torch.autograd.grad(x.sum(), d["pos"])
+
+
+@pytest.mark.parametrize("what", ["module_hook", "foreign_module", "tensor_hook", "position_hook", "retain_grad"])
+def test_hooks_and_foreign_modules_take_part(what):
+    """What the per-op path calls and autograd runs is called and run, and the model goes back to the native path after."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S")
+    data = synthetic.molecule_batch(2, 5, 8, seed=7).to("cuda")
+    plain = head(data.clone(), bb(data.clone()))["energy"]
+    d = data.clone()
+    ref = head(d, bb(d))["forces"]
+    d, seen = data.clone(), []
+    if what == "module_hook":
+        handle = bb.blocks[1].norm_2.register_forward_hook(lambda m, i, o: seen.append(o) or 2.0 * o)
+    elif what == "foreign_module":
+        class Doubled(B.RMSNormSH):
+            def forward(self, x, extra=None):
+                seen.append(x)
+                return 2.0 * super().forward(x, extra)
+
+        old = bb.blocks[1].norm_2
+        bb.blocks[1].norm_2 = new = Doubled(2, 128).cuda()
+        new.load_state_dict(old.state_dict())
+    emb = bb(d)
+    if what == "tensor_hook":
+        emb["node_embedding"].register_hook(lambda g: seen.append(g) or 2.0 * g)
+    elif what == "position_hook":
+        d["pos"].register_hook(lambda g: seen.append(g) or 2.0 * g)
+    elif what == "retain_grad":
+        emb["node_embedding"].retain_grad()
+    out = head(d, emb)
+    if what == "retain_grad":
+        assert emb["node_embedding"].grad is not None
+        assert _rel(out["forces"], ref) < 2e-5
+    else:
+        assert len(seen) == 1
+        if what in ("tensor_hook", "position_hook"):
+            assert _rel(out["forces"], 2.0 * ref) < 2e-5
+        else:
+            assert _rel(out["energy"], plain) > 1e-4
+            if what == "module_hook":
+                handle.remove()
+            else:
+                bb.blocks[1].norm_2 = old
+    d = data.clone()
+    emb = bb(d)
+    assert "step" in emb and _rel(head(d, emb)["forces"], ref) < 1e-6

@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from fairchem_b200 import step, weights
-from fairchem_b200.backbone import MLP_EFS_HeadB200, eSCNMDBackboneB200
+from fairchem_b200.backbone import MLP_EFS_HeadB200, RMSNormSH, eSCNMDBackboneB200
 
 
 @pytest.fixture()
@@ -95,3 +95,53 @@ def test_a_used_model_can_be_copied_and_saved_whole(how, tmp_path):
         assert not hasattr(m, "_step_plan")
     for (n, p), (_, q) in zip(model.named_parameters(), other.named_parameters()):
         assert torch.equal(p, q), n
+
+
+class _OtherNorm(RMSNormSH):
+    pass
+
+
+def _foreign_module(bb):
+    bb.blocks[1].norm_2 = _OtherNorm(2, 128)
+
+
+def _other_shape(bb):
+    bb.blocks[0].edge_wise.so2_conv_1.fc_m0 = nn.Linear(768, 512)
+
+
+def test_other_modules_are_not_for_the_native_path(bb):
+    assert step.ModelPlan.supported(bb)
+    for change in (_foreign_module, _other_shape):
+        other = copy.deepcopy(bb)
+        change(other)
+        assert step.ModelPlan.supported(bb) and not step.ModelPlan.supported(other)
+
+    class Sub(eSCNMDBackboneB200):
+        def csd_embedding(self, charge, spin, dataset):
+            return super().csd_embedding(charge, spin, dataset)
+
+    assert not step.ModelPlan.supported(Sub(**dict(weights.UMA_S, num_layers=1)))
+
+
+@pytest.mark.parametrize("kind", ["forward_hook", "pre_hook", "backward_hook", "global_hook", "own_forward", "own_method"])
+def test_hooks_send_an_evaluation_down_the_per_op_path(bb, kind):
+    calls, undo = step._Calls(bb), None
+    assert not calls.watched()
+    mod = bb.blocks[2].atom_wise.so3_linear_2
+    if kind == "forward_hook":
+        undo = mod.register_forward_hook(lambda *a: None).remove
+    elif kind == "pre_hook":
+        undo = bb.norm.register_forward_pre_hook(lambda *a: None).remove
+    elif kind == "backward_hook":
+        undo = bb.blocks[0].norm_1.register_full_backward_hook(lambda *a: None).remove
+    elif kind == "global_hook":
+        undo = nn.modules.module.register_module_forward_hook(lambda *a: None).remove
+    elif kind == "own_forward":
+        mod.forward = lambda x: x
+        undo = lambda: delattr(mod, "forward")  # noqa: E731
+    else:
+        bb.csd_embedding = lambda *a: None
+        undo = lambda: delattr(bb, "csd_embedding")  # noqa: E731
+    assert calls.watched()
+    undo()
+    assert not calls.watched()
