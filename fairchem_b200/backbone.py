@@ -1340,11 +1340,12 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
             return self._forward(data, gamma)
 
     def _forward_native(self, data, gamma):
-        """The whole evaluation from native code (fairchem_b200.step); None when it does not apply."""
+        """The whole evaluation from native code (fairchem_b200.step), and the graph (edge_index, cell_offsets) it ran on.
+        No evaluation when the native path does not apply or the GPU lacks the memory; no graph when none was built."""
         plan = step.ModelPlan.of(self)
         pos = data["pos"]
         if plan is None or pos.dtype != torch.float32 or not pos.is_cuda or pos.device != plan.device or pos.shape[0] == 0:
-            return None
+            return None, None
         status = _status(pos.device)
         graph = step.StepGraph(self, data, status, torch.is_grad_enabled() and pos.requires_grad)
         new_step = lambda: step.BackboneStep(plan, graph, plan.dataset_index(self, data["dataset"]), data["charge"], data["spin"],  # noqa: E731
@@ -1353,8 +1354,9 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
         if built:
             run = new_step()  # before finish(), which waits for the graph's kernels
             built = graph.finish()
+            found = graph.edge_index, graph.cell_offsets
         if not built:
-            edge_index, cell_offsets = self._graph(data)
+            found = edge_index, cell_offsets = self._graph(data)
             if edge_index.shape[1] == 0:  # isolated atoms: see _forward
                 edge_index = torch.zeros(2, 1, dtype=torch.long, device=pos.device)
                 cell_offsets = torch.zeros(1, 3, dtype=pos.dtype, device=pos.device)
@@ -1366,13 +1368,13 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
             run = new_step()
         run.set_edges(graph)
         if not run.plan_memory():
-            return None
+            return None, found
         run.virial = {"num_systems": graph.systems} if self.regress_stress else None
         x = step.BackboneFn.apply(pos, run)
         data["scatter_target"] = graph.edge_index[1]
         self.last_graph = {"edge_index": graph.edge_index, "cell_offsets": graph.cell_offsets}
         run.embedding = weakref.ref(x)  # x's autograd node holds the run: a strong reference would be a cycle
-        return {"node_embedding": x, "batch": data["batch"], "virial": run.virial, "step": run}
+        return {"node_embedding": x, "batch": data["batch"], "virial": run.virial, "step": run}, found
 
     def _forward(self, data, gamma):
         from .parallel import halo_collect
@@ -1385,8 +1387,9 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
         if (self.regress_forces or self.regress_stress) and not self.direct_forces:
             pos.requires_grad_(True)
         c, nb = self.sphere_channels, self.num_distance_basis
+        found = None
         if data.get("gp_plan", None) is None:
-            out = self._forward_native(data, gamma)
+            out, found = self._forward_native(data, gamma)
             if out is not None:
                 return out
         csd = self.csd_embedding(data["charge"], data["spin"], data.get("dataset", None))
@@ -1394,7 +1397,7 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
         # graph-parallel run: this rank owns plan.node_partition and reads plan.halo_ids from its peers
         plan = data.get("gp_plan", None)
         if plan is None:
-            edge_index, cell_offsets = self._graph(data)
+            edge_index, cell_offsets = found or self._graph(data)
             pos_e, z_e, batch_l = pos, z, batch
         else:
             edge_index, cell_offsets = plan.edge_index_local, plan.cell_offsets

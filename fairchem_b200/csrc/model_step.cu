@@ -48,7 +48,7 @@ struct Dims {
 
 struct Layer {
     float *x0, *xn1, *st1, *x1, *st2, *ffn_y;  // inputs of the two norms, first norm's output, feed-forward pre-activation
-    float *y, *msg, *rad;                      // conv-1 output, messages, radial weights (per edge)
+    float *y, *msg, *rad;                      // conv-1 output, messages, radial weights (per edge); null: not kept
 };
 
 struct Layout {
@@ -124,9 +124,10 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         q.x1 = k.take<float>(n * d.nl * C);
         q.st2 = k.take<float>(n * 2);
         q.ffn_y = k.take<float>(n * (md.lmax + d.nl) * C);
-        q.y = keep ? k.take<float>(er * d.yw) : nullptr;
-        q.msg = keep ? k.take<float>(er * d.nm * C) : nullptr;
-        q.rad = keep && ev.keep_radial ? k.take<float>(er * d.nrad * 2 * C) : nullptr;
+        const bool edges = keep && l >= ev.drop_layers;
+        q.y = edges ? k.take<float>(er * d.yw) : nullptr;
+        q.msg = edges ? k.take<float>(er * d.nm * C) : nullptr;
+        q.rad = edges && ev.keep_radial ? k.take<float>(er * d.nrad * 2 * C) : nullptr;
     }
     L.keep_bytes = k.off;
 
@@ -138,8 +139,9 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         L.radial = b.take<float>(ec * d.nrad * 2 * C);
         L.m = planes(b, ec, d.nm * 2 * C);
         L.a = planes(b, ec, d.nm * C);
-        L.y_c = keep ? nullptr : b.take<float>(ec * d.gates);
-        L.msg_c = keep ? nullptr : b.take<float>(ec * d.nm * C);
+        const bool all = keep && ev.drop_layers <= 0;
+        L.y_c = all ? nullptr : b.take<float>(ec * d.gates);
+        L.msg_c = all ? nullptr : b.take<float>(ec * d.nm * C);
         L.xn2 = planes(b, n, d.nl * C);
         L.a2 = planes(b, n, d.nl * C);
         L.ffn_out = b.take<float>(n * d.nl * C);
@@ -166,6 +168,14 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
     L.gm = b.take<float>(ec * d.nm * 2 * C);
     L.grad = planes(b, ec, d.nrad * 2 * C);
     const int64_t layers_end = b.off;
+    // A layer that keeps nothing per edge is computed again on the memory of gradients that come later in its chunk:
+    // the rotated rows where theirs go, the gated rows in the message gradient, the messages and the conv-1 output in the
+    // planes of the conv-1 output's and the radial weights' gradients (4 bytes an element each, like float32).
+    L.m.hi = reinterpret_cast<__half*>(L.gm), L.m.lo = L.m.hi + ec * d.nm * 2 * C, L.m.ld = d.nm * 2 * C;
+    L.a = L.gmsg;
+    L.msg_c = reinterpret_cast<float*>(L.gy.hi);
+    L.y_c = reinterpret_cast<float*>(L.grad.hi);
+    static_assert(2 + 9 <= 6 * 2 && 4 + 19 <= 12 * 2, "yw fits the radial gradient of lmax 2 and 4");
     b.off = edge_part;  // the radial MLPs' backward runs after the layers, on the same memory
     L.r3 = b.take<float>(ec * (md.lmax + 1) * C);
     L.gr3 = planes(b, ec, (md.lmax + 1) * C);
@@ -262,6 +272,8 @@ struct Run {
         if (r < 2 * d.lmax) return r % d.lmax + 1;
         return (r - 2 * d.lmax) % (d.lmax - 1) + 2;
     }
+    Conv conv1_gate(int l, bool keep) const;
+    int messages(int l, const Conv& c1, int64_t e0, int64_t ec, float* y, int64_t yw, float* msg) const;
     int forward();
     int energy();
     int backward();
@@ -375,6 +387,40 @@ int Run::radial_hidden_forward() {
     });
 }
 
+// conv 1 with the gate in its epilogue: gate tiles first, then the rows; keep: the rows' raw values too
+Conv Run::conv1_gate(int l, bool keep) const {
+    Conv c = blocks(md.layers[l].conv1);
+    c.bias[0] = md.layers[l].conv1_bias;
+    for (int i = d.lmax; i < c.count(); ++i) {
+        int32_t* t = &c.t[9 * i];
+        const int r = i - d.lmax;
+        t[4] = r * C;
+        t[5] = r == 0 ? kSilu : kGated;
+        t[6] = (d.lmax + r) * C;
+        t[7] = r == 0 ? 0 : (degree_of_row(r) - 1) * C;
+        t[8] = keep ? kKeep : 0;
+    }
+    return c;
+}
+
+// messages of a chunk's edges: radial weights, gather + rotate, conv 1 + gate, conv 2; y [ec, yw] takes conv 1's raw values
+int Run::messages(int l, const Conv& c1, int64_t e0, int64_t ec, float* y, int64_t yw, float* msg) const {
+    const Layer& q = L.layer[l];
+    FCB_TRY(radial_out(l, e0, ec));
+    const int64_t gb = ec * (4LL * (2 * d.nl * C + 2 * d.nm * C + d.nw + d.nrad * 2 * C) + 8);
+    FCB_TRY(op("gather_rotate_fwd", gb, [&] {
+        return by_lmax([&](auto lm) {
+            constexpr int LM = decltype(lm)::value;
+            launch_pdl(gather_fwd_kernel<LM>, dim3(warp_grid(2 * ec, 4, 148 * (LM == 2 ? 5 : 3) * 4)), dim3(128), 0, st, q.xn1, ev.src + e0, ev.tgt + e0, L.wig + e0 * d.nw, radial_of(l, e0), L.m.out(), ec);
+            return 0;
+        });
+    }));
+    FCB_TRY(conv("so2_conv_fused_conv1_gate", c1, L.m.hi, L.m.lo, L.m.ld, L.m.ld, d.lmax, y, yw, yw, &L.a, L.a.ld, nullptr, nullptr, ec));
+    Conv c2 = blocks(md.layers[l].conv2);
+    c2.bias[0] = md.layers[l].conv2_bias;
+    return conv("so2_conv_fused_conv2", c2, L.a.hi, L.a.lo, L.a.ld, L.a.ld, 0, msg, d.nm * C, d.nm * C, nullptr, 0, nullptr, nullptr, ec);
+}
+
 int Run::layer_forward(int l, const float* ffn_prev) {
     const fcb200_layer& w = md.layers[l];
     const Layer& q = L.layer[l];
@@ -387,33 +433,10 @@ int Run::layer_forward(int l, const float* ffn_prev) {
             return 0;
         });
     }));
-    const bool keep = ev.want_grad != 0;
-    Conv c1 = blocks(w.conv1), c2 = blocks(w.conv2);  // conv 1: gate tiles first, then the rows
-    c1.bias[0] = w.conv1_bias, c2.bias[0] = w.conv2_bias;
-    for (int i = d.lmax; i < c1.count(); ++i) {
-        int32_t* t = &c1.t[9 * i];
-        const int r = i - d.lmax;
-        t[4] = r * C;
-        t[5] = r == 0 ? kSilu : kGated;
-        t[6] = (d.lmax + r) * C;
-        t[7] = r == 0 ? 0 : (degree_of_row(r) - 1) * C;
-        t[8] = keep ? kKeep : 0;
-    }
+    const Conv c1 = conv1_gate(l, q.y != nullptr);
     return chunks([&](int, int64_t e0, int64_t ec, int64_t n0, int64_t n1) {
-        FCB_TRY(radial_out(l, e0, ec));
-        const int64_t gb = ec * (4LL * (2 * d.nl * C + 2 * d.nm * C + d.nw + d.nrad * 2 * C) + 8);
-        FCB_TRY(op("gather_rotate_fwd", gb, [&] {
-            return by_lmax([&](auto lm) {
-                constexpr int LM = decltype(lm)::value;
-                launch_pdl(gather_fwd_kernel<LM>, dim3(warp_grid(2 * ec, 4, 148 * (LM == 2 ? 5 : 3) * 4)), dim3(128), 0, st, q.xn1, ev.src + e0, ev.tgt + e0, L.wig + e0 * d.nw, radial_of(l, e0), L.m.out(), ec);
-                return 0;
-            });
-        }));
-        float* y = keep ? q.y + e0 * d.yw : L.y_c;
-        const int64_t yw = keep ? d.yw : d.gates;
-        FCB_TRY(conv("so2_conv_fused_conv1_gate", c1, L.m.hi, L.m.lo, L.m.ld, L.m.ld, d.lmax, y, yw, yw, &L.a, L.a.ld, nullptr, nullptr, ec));
-        float* msg = keep ? q.msg + e0 * d.nm * C : L.msg_c;
-        FCB_TRY(conv("so2_conv_fused_conv2", c2, L.a.hi, L.a.lo, L.a.ld, L.a.ld, 0, msg, d.nm * C, d.nm * C, nullptr, 0, nullptr, nullptr, ec));
+        float* msg = q.msg ? q.msg + e0 * d.nm * C : L.msg_c;
+        FCB_TRY(messages(l, c1, e0, ec, q.y ? q.y + e0 * d.yw : L.y_c, q.y ? d.yw : d.gates, msg));
         return op("rotate_back_reduce_fwd", ec * 4 * (d.nm * C + d.nw) + (n1 - n0) * row * 8,
                   [&] { return by_lmax([&](auto lm) { return launch_rotate_back<decltype(lm)::value, 0>(*this, msg, e0, q.x0, q.x1, n0, n1); }); });
     });
@@ -549,13 +572,19 @@ int Run::layer_backward(int l) {
         }
     }
     const bool first_layer = l == md.num_layers - 1;
+    const Conv again = q.y ? Conv{} : conv1_gate(l, true);
     FCB_TRY(chunks([&](int c, int64_t e0, int64_t ec, int64_t n0, int64_t n1) {
-        if (!q.rad) FCB_TRY(radial_out(l, e0, ec));
+        float* y = q.y ? q.y + e0 * d.yw : L.y_c;
+        float* msg = q.msg ? q.msg + e0 * d.nm * C : L.msg_c;
+        if (!q.y) {
+            FCB_TRY(messages(l, again, e0, ec, y, d.yw, msg));
+        } else if (!q.rad) {
+            FCB_TRY(radial_out(l, e0, ec));
+        }
         const float* rad = radial_of(l, e0);
-        float* y = q.y + e0 * d.yw;
         FCB_TRY(op("rotate_back_bwd", ec * 4 * (d.nl * C + 2 * d.nm * C + d.nw + 9), [&] {
             return by_lmax([&](auto lm) {
-                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 0, OutSplit>), dim3(warp_grid(ec, 4, 148 * 12)), dim3(128), 0, st, L.g1, q.msg + e0 * d.nm * C, L.wig, L.env, ev.tgt, L.gmsg.out(), scale, L.tau_e, !first_layer, 1.0f, e0, ec);
+                launch_pdl((rotate_back_bwd_kernel<decltype(lm)::value, 0, OutSplit>), dim3(warp_grid(ec, 4, 148 * 12)), dim3(128), 0, st, L.g1, msg, L.wig, L.env, ev.tgt, L.gmsg.out(), scale, L.tau_e, !first_layer, 1.0f, e0, ec);
                 return 0;
             });
         }));

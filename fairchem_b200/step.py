@@ -48,7 +48,7 @@ class ModelStruct(Structure):
 
 class EvalStruct(Structure):
     _fields_ = ([("num_nodes", c_int64), ("num_edges", c_int64)]
-                + [(n, c_int32) for n in ("num_systems", "num_chunks", "want_grad", "keep_radial")]
+                + [(n, c_int32) for n in ("num_systems", "num_chunks", "want_grad", "keep_radial", "drop_layers")]
                 + [(n, c_void_p) for n in ("pos", "shift", "gamma", "src", "tgt", "row_ptr", "src_ptr", "src_perm", "chunk_src", "z",
                                            "batch", "dataset", "charge", "spin", "chunk_node", "chunk_edge", "keep", "scratch", "x_out",
                                            "energy", "grad_x", "grad_pos")]
@@ -274,6 +274,9 @@ def _stream():
     return c_void_p(torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream)  # an index: 2 us, no argument 18
 
 
+ALWAYS_THERE = 1 << 28  # bytes that any GPU in use has; more: what the allocator already holds, or the driver is asked
+
+
 class BackboneStep:
     """One evaluation: graph arrays, outputs and the memory that the backward pass reads."""
 
@@ -305,13 +308,14 @@ class BackboneStep:
         e.chunk_node, e.chunk_edge = ctypes.addressof(graph.chunk_node), ctypes.addressof(graph.chunk_edge)
 
     def plan_memory(self) -> bool:
-        """Decide whether the radial weights are kept too; False when the kept tensors do not fit the free memory."""
-        e, sizes = self.ev, self.sizes
-        for keep_radial in (1, 0) if e.want_grad else (0,):
-            e.keep_radial = keep_radial
+        """Decide what is kept for the backward pass: everything, all but the radial weights, or, layer by layer, no conv-1
+        output and messages either.  False when not even the smallest set fits the free memory."""
+        e, sizes, layers = self.ev, self.sizes, self.model.num_layers
+        for keep_radial, drop in [(1, 0), *((0, n) for n in range(layers + 1))] if e.want_grad else [(0, 0)]:
+            e.keep_radial, e.drop_layers = keep_radial, drop
             _lib.call("fcb200_model_sizes", byref(self.model), byref(e), sizes)
             need = sizes[0] + max(sizes[1], sizes[2] if e.want_grad else 0)
-            if need < (1 << 28) or need < self._cached():  # what any GPU in use has, or what the allocator already holds
+            if need < ALWAYS_THERE or need < self._cached():
                 return True
             if not hasattr(self, "avail"):
                 free, self.total = torch.cuda.mem_get_info(self.device)

@@ -594,6 +594,8 @@ typedef struct {
     int32_t num_systems, num_chunks;
     int32_t want_grad;   /* keep what the backward pass needs */
     int32_t keep_radial; /* also keep the radial weights (else recomputed per chunk) */
+    int32_t drop_layers; /* the first layers, as many, keep no conv-1 output, messages and radial weights either: the
+                            backward pass computes them again per chunk */
     const float *pos, *shift, *gamma; /* [N,3]; [E,3] or null; [E] or null */
     const int32_t *src, *tgt, *row_ptr, *src_ptr, *src_perm;
     const int32_t* chunk_src; /* [(num_chunks+1), N]: per node, first position of src_perm with an edge id >= the chunk's first

@@ -255,3 +255,54 @@ def test_hooks_and_foreign_modules_take_part(what):
     d = data.clone()
     emb = bb(d)
     assert "step" in emb and _rel(head(d, emb)["forces"], ref) < 1e-6
+
+
+@pytest.mark.parametrize("cfg,drop", [("UMA_S", 1), ("UMA_S", 4), ("ESCN_MD_L4", 1), ("ESCN_MD_L4", 2)])
+@pytest.mark.parametrize("wants", ["forces", "stress"])
+def test_layers_that_keep_nothing_per_edge_give_the_same_result(cfg, drop, wants, monkeypatch):
+    """Less free memory: some layers are computed again in the backward pass, with the same kernels on the same inputs."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import step, synthetic
+
+    bb, head = _model(B, cfg, regress_stress=wants == "stress", edge_chunk_size=700)
+    data = synthetic.merge([synthetic.fcc_cu((2, 2, 3), seed=8), synthetic.molecule_batch(2, 5, 30, seed=9)]).to("cuda")
+    d = data.clone()
+    ref = head(d, bb(d))
+    runs = []
+
+    def short(run):
+        run.ev.keep_radial, run.ev.drop_layers = 0, drop
+        step._lib.call("fcb200_model_sizes", step.byref(run.model), step.byref(run.ev), run.sizes)
+        runs.append(run)
+        return True
+
+    monkeypatch.setattr(step.BackboneStep, "plan_memory", short)
+    d = data.clone()
+    emb = bb(d)
+    got = head(d, emb)
+    assert len(runs) == 1 and runs[0].ev.num_chunks > 1
+    for k in ref:
+        assert _rel(got[k], ref[k]) < 1e-6, k
+
+
+@pytest.mark.parametrize("skin", [0.0, 0.5])
+def test_without_the_memory_the_per_op_path_takes_over_the_graph(skin, monkeypatch):
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import graph, step, synthetic
+
+    bb, head = _model(B, "UMA_S")
+    data = synthetic.water_box(300, seed=1).to("cuda")
+    d = data.clone()
+    ref = head(d, bb(d))
+    if skin:
+        bb.neighbor_list = graph.SkinNeighborList(bb.cutoff, bb.max_neighbors, skin)
+    monkeypatch.setattr(step.BackboneStep, "plan_memory", lambda run: False)
+    monkeypatch.setattr(B.eSCNMDBackboneB200, "_graph", lambda *a: pytest.fail("the graph was built a second time"))
+    d = data.clone()
+    emb = bb(d)
+    assert "step" not in emb
+    got = head(d, emb)
+    for k in ref:
+        assert _rel(got[k], ref[k]) < 2e-5
+    if skin:
+        assert (bb.neighbor_list.searches, bb.neighbor_list.refreshes) == (1, 0)

@@ -145,3 +145,45 @@ def test_hooks_send_an_evaluation_down_the_per_op_path(bb, kind):
     assert calls.watched()
     undo()
     assert not calls.watched()
+
+
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+def test_what_is_kept_follows_the_free_memory_layer_by_layer(cfg, monkeypatch):
+    """The 100 000-atom box and beyond: less free memory, fewer layers with per-edge tensors, and only then no evaluation."""
+    cfg = getattr(weights, cfg)
+    run = object.__new__(step.BackboneStep)
+    layers = (step.LayerStruct * cfg["num_layers"])()
+    run.model = m = step.ModelStruct()
+    m.lmax, m.num_layers, m.num_basis, m.layers = cfg["lmax"], cfg["num_layers"], cfg["num_distance_basis"], layers
+    run.ev = e = step.EvalStruct()
+    nodes, edges, chunks = 100_000, 3_100_000, 24
+    node, edge = ((ctypes.c_int64 * (chunks + 1))(*(n * i // chunks for i in range(chunks + 1))) for n in (nodes, edges))
+    e.num_nodes, e.num_edges, e.num_systems, e.num_chunks, e.want_grad = nodes, edges, 1, chunks, 1
+    e.chunk_node, e.chunk_edge = ctypes.addressof(node), ctypes.addressof(edge)
+    run.sizes, run.device = (ctypes.c_int64 * 3)(), torch.device("cuda", 0)
+    total = 183 * 2 ** 30
+    monkeypatch.setattr(step.BackboneStep, "_cached", lambda self: 0)
+
+    def kept(avail):
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (avail, total))
+        run.__dict__.pop("avail", None)
+        if not run.plan_memory():
+            return None
+        need = run.sizes[0] + max(run.sizes[1], run.sizes[2])
+        return e.keep_radial, e.drop_layers, need
+
+    seen, avail = [], 10 ** 13
+    while (got := kept(int(avail))) is not None:
+        seen.append(got)
+        avail = got[2] + 0.03 * total  # what this choice needs: the next one has to do with less
+    want = [(1, 0), *((0, n) for n in range(cfg["num_layers"] + 1))]
+    assert [s[:2] for s in seen] == want
+    lmax = cfg["lmax"]
+    rows = 5 * lmax - 1  # of a message
+    per_layer = edges * (lmax + 2 * rows) * 512  # conv-1 output and messages
+    no_radial = [s[2] for s in seen if s[0] == 0]
+    for a, b in zip(no_radial, no_radial[1:]):
+        # the row counts are rounded up by at most 1/32; the first dropped layer adds two chunk-sized buffers
+        assert a - b < per_layer * 33 / 32 + 4096 and a - b > 0.75 * per_layer
+    e.want_grad = 0
+    assert kept(10 ** 12)[:2] == (0, 0)
