@@ -1467,12 +1467,12 @@ class MLP_EFS_HeadB200(step.HoldsPlan, nn.Module):
         if x._backward_hooks or x.retains_grad or run.leaf._backward_hooks:  # autograd has more to do than the forces
             return None
         want = self.regress_forces or self.regress_stress
-        model = run.plan.with_head(self)
-        if model is None or (want and not run.ev.want_grad):
+        plan = run.plan.with_head(self)
+        if plan is None or (want and not run.ev.want_grad):
             return None
-        out = {"energy": run.energy(model)}
+        out = {"energy": run.energy(plan)}
         if want:
-            out["forces"] = run.backward(model, None, -1.0)
+            out["forces"] = run.backward(plan, None, -1.0)
             run.spent = True
         if self.regress_stress:
             out["stress"] = self._stress(data, run.virial["virial"])

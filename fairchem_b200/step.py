@@ -10,8 +10,9 @@ from __future__ import annotations
 
 import ctypes
 import operator
-from itertools import chain
 from ctypes import POINTER, Structure, byref, c_float, c_int32, c_int64, c_void_p
+from itertools import chain
+from typing import Optional
 
 import torch
 import torch.nn.modules.module as _nn_module
@@ -120,10 +121,28 @@ class _Calls:
 
 
 class _Weights:
-    """Half-split device copies of a module's matrices; keeps every tensor whose address is handed out alive."""
+    """Half-split device copies of a module's matrices; keeps every tensor whose address is handed out alive.
 
-    def __init__(self):
+    They are written on the stream that was current then.  Another stream waits for that before its first use, and the
+    memory goes back only behind what other streams were still doing with it."""
+
+    def __init__(self, device):
         self.alive = []
+        self.device, self.home, self.ready, self.last_use = device, torch.cuda.current_stream(device), None, {}
+
+    def laid_out(self):
+        self.ready = self.home.record_event()
+
+    def before_use(self, stream):
+        if stream.cuda_stream not in self.last_use:
+            stream.wait_event(self.ready)
+
+    def after_use(self, stream):
+        self.last_use[stream.cuda_stream] = stream.record_event(self.last_use.get(stream.cuda_stream))
+
+    def __del__(self):
+        for event in self.last_use.values():
+            self.home.wait_event(event)
 
     def ptr(self, t: torch.Tensor) -> int:
         t = t.detach().float().contiguous()
@@ -155,8 +174,8 @@ class ModelPlan:
         from .backbone import _conv_weights
 
         self.origin, self.calls = origin, _Calls(bb)
-        w = self.w = _Weights()
         self.device = origin.params[0].device
+        w = self.w = _Weights(self.device)
         lmax, nb = bb.lmax, bb.num_distance_basis
         self.layers = (LayerStruct * len(bb.blocks))()
         for s, blk in zip(self.layers, bb.blocks):
@@ -204,6 +223,7 @@ class ModelPlan:
         self.dataset_row = {name: i for i, name in enumerate(emb)}
         m.dataset_emb = w.ptr(torch.cat([e.weight for e in emb.values()]))
         m.csd_w_t, m.csd_b = w.ptr(bb.mix_csd.weight.t()), w.ptr(bb.mix_csd.bias)
+        w.laid_out()
         self.dataset_ids = {}  # (row, systems) -> int32 device tensor, for batches of one dataset
 
     @staticmethod
@@ -234,26 +254,18 @@ class ModelPlan:
         bb._step_plan = plan = cls(bb, origin)
         return None if plan.calls.watched() else plan
 
-    def with_head(self, head):
-        """The model struct with the energy head's weights filled in (cached on the head), or None."""
+    def with_head(self, head) -> Optional["HeadPlan"]:
+        """This plan with the energy head's weights (cached on the head), or None."""
         eb = head.energy_block
         params = [p for i in (0, 2, 4) for p in (eb[i].weight, eb[i].bias)]
-        key = (id(self), *_versions(params))
+        key = _versions(params)
         hit = getattr(head, "_step_plan", None)
-        if hit is not None and hit[0] == key:
-            return hit[1]
+        if hit is not None and hit.backbone is self and hit.key == key:
+            return hit
         if eb[0].weight.shape != (C, C) or eb[2].weight.shape != (C, C) or eb[4].weight.shape != (1, C):
             return None
-        w, m = _Weights(), ModelStruct()
-        ctypes.pointer(m)[0] = self.model
-        m.head_w1, m.head_w1_t = w.split(eb[0].weight), w.split(eb[0].weight.detach().t().contiguous())
-        m.head_w2, m.head_w2_t = w.split(eb[2].weight), w.split(eb[2].weight.detach().t().contiguous())
-        m.head_b1, m.head_b2, m.head_w3, m.head_b3 = w.ptr(eb[0].bias), w.ptr(eb[2].bias), w.ptr(eb[4].weight), w.ptr(eb[4].bias)
-        from .backbone import _pow2_scale
-
-        m.head_scale = w.ptr(_pow2_scale(eb[4].weight.detach().abs().max() * 1.1))  # |d silu| <= 1.1
-        head._step_plan = (key, m, w, self)
-        return m
+        head._step_plan = hit = HeadPlan(self, eb, key)
+        return hit
 
     def dataset_index(self, bb, names) -> torch.Tensor:
         mapping, key = bb.dataset_embedding.mapping, None
@@ -267,7 +279,24 @@ class ModelPlan:
             idx = torch.tensor(rows, dtype=torch.int32, device=self.device)
             if key is not None and len(self.dataset_ids) < 64:
                 self.dataset_ids[key] = idx
+                self.w.alive.append(idx)
         return idx
+
+
+class HeadPlan:
+    """A backbone's plan with an energy head's weights filled in."""
+
+    def __init__(self, backbone: ModelPlan, eb, key):
+        from .backbone import _pow2_scale
+
+        self.backbone, self.key = backbone, key
+        w, m = self.w, self.model = _Weights(backbone.device), ModelStruct()
+        ctypes.pointer(m)[0] = backbone.model
+        m.head_w1, m.head_w1_t = w.split(eb[0].weight), w.split(eb[0].weight.detach().t().contiguous())
+        m.head_w2, m.head_w2_t = w.split(eb[2].weight), w.split(eb[2].weight.detach().t().contiguous())
+        m.head_b1, m.head_b2, m.head_w3, m.head_b3 = w.ptr(eb[0].bias), w.ptr(eb[2].bias), w.ptr(eb[4].weight), w.ptr(eb[4].bias)
+        m.head_scale = w.ptr(_pow2_scale(eb[4].weight.detach().abs().max() * 1.1))  # |d silu| <= 1.1
+        w.laid_out()
 
 
 def _stream():
@@ -288,8 +317,8 @@ class BackboneStep:
         e.num_nodes, e.num_systems, e.want_grad = self.nodes, self.systems, int(graph.want_grad)
         charge, spin = charge.to(self.device, torch.int64).contiguous(), spin.to(self.device, torch.int64).contiguous()
         gamma = None if gamma is None else gamma.contiguous()
-        self.leaf = graph.leaf
-        self.refs = [graph, dataset, charge, spin, gamma, status]
+        self.leaf, self.graph = graph.leaf, graph
+        self.refs = [t for t in (dataset, charge, spin, gamma, status, *graph.alive) if t is not None]
         self.watched = [t for t in (graph.pos, charge, spin, gamma) if t is not None]  # may be the caller's own memory
         for name in ("pos", "z", "batch", "src", "tgt", "row_ptr", "src_ptr", "src_perm"):
             setattr(e, name, getattr(g, name))
@@ -298,7 +327,7 @@ class BackboneStep:
         e.status = status.data_ptr()
         self.want_virial, self.virial = want_virial, None
         self.sizes = (c_int64 * 3)()
-        self.keep = None
+        self.keep = self.home = None
         self.spent = False  # the head has computed the forces
 
     def set_edges(self, graph: "StepGraph"):
@@ -338,6 +367,22 @@ class BackboneStep:
         self.inputs = [(t, t._version) for t in self.watched]
         return self._forward()
 
+    def _launch(self, name: str, *plans):
+        """One native call on the current stream, which need not be the one that the evaluation began on."""
+        stream = torch.cuda.current_stream(self.device.index)
+        if self.home is None:
+            self.home = stream
+        elif stream.cuda_stream != self.home.cuda_stream:
+            stream.wait_stream(self.home)
+            for t in (self.keep, self.graph.a.block, self.graph.b.block, *self.refs):
+                t.record_stream(stream)
+        foreign = [p.w for p in plans if p.w.home.cuda_stream != stream.cuda_stream]
+        for w in foreign:
+            w.before_use(stream)
+        _lib.call(name, byref(plans[-1].model), byref(self.ev), c_void_p(stream.cuda_stream))
+        for w in foreign:
+            w.after_use(stream)
+
     def _forward(self) -> torch.Tensor:
         e = self.ev
         self.keep = self._block(self.sizes[0])
@@ -345,16 +390,16 @@ class BackboneStep:
         nl = (self.model.lmax + 1) ** 2
         x = torch.empty(self.nodes, nl, C, dtype=torch.float32, device=self.device)
         e.keep, e.scratch, e.x_out = self.keep.data_ptr(), scratch.data_ptr(), x.data_ptr()
-        _lib.call("fcb200_model_forward", byref(self.model), byref(e), _stream())
+        self._launch("fcb200_model_forward", self.plan)
         return x
 
-    def energy(self, model: ModelStruct) -> torch.Tensor:
+    def energy(self, head: HeadPlan) -> torch.Tensor:
         out = torch.zeros(self.systems, dtype=torch.float64, device=self.device)
         self.ev.energy = out.data_ptr()
-        _lib.call("fcb200_model_energy", byref(model), byref(self.ev), _stream())
+        self._launch("fcb200_model_energy", self.plan, head)
         return out
 
-    def backward(self, model: ModelStruct, grad_x, sign: float) -> torch.Tensor:
+    def backward(self, head: Optional[HeadPlan], grad_x, sign: float) -> torch.Tensor:
         """sign * gradient of the energy sum (grad_x None) or of <grad_x, node embedding> with respect to the positions."""
         if self.keep is None:  # released by an earlier backward pass over a retained graph: computed again
             if any(t._version != v for t, v in self.inputs):
@@ -369,7 +414,7 @@ class BackboneStep:
             v = torch.zeros(self.systems, 3, 3, dtype=torch.float64, device=self.device)
             e.virial = v.data_ptr()
             self.virial["virial"] = v
-        _lib.call("fcb200_model_backward", byref(model), byref(e), _stream())
+        self._launch("fcb200_model_backward", self.plan, *([] if head is None else [head]))
         self.keep = None
         return grad
 
@@ -389,7 +434,7 @@ class BackboneFn(torch.autograd.Function):
         step = ctx.step
         if step.spent:  # the head took its gradient from this evaluation without autograd and did not retain it
             raise RuntimeError("fairchem_b200: the forces of this evaluation were computed already; its graph was not retained")
-        return step.backward(step.model, grad_x.contiguous(), 1.0), None
+        return step.backward(None, grad_x.contiguous(), 1.0), None
 
 
 class GraphStruct(Structure):

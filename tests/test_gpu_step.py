@@ -306,3 +306,62 @@ def test_without_the_memory_the_per_op_path_takes_over_the_graph(skin, monkeypat
         assert _rel(got[k], ref[k]) < 2e-5
     if skin:
         assert (bb.neighbor_list.searches, bb.neighbor_list.refreshes) == (1, 0)
+
+
+def test_head_on_another_stream_and_memory_reused_on_the_first():
+    """The evaluation's memory is allocated on the backbone's stream; a head on another one frees it there while its kernels
+    are still queued, and the first stream's next allocations must not get it before they are done."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S", regress_stress=True)
+    data = synthetic.bcc_alloy((6, 6, 6), seed=2).to("cuda")
+    d = data.clone()
+    ref = head(d, bb(d))
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    junk, got = [], []
+    for _ in range(4):
+        with torch.cuda.stream(first):
+            d = data.clone()
+            emb = bb(d)
+            nbytes = emb["step"].keep.numel()
+        with torch.cuda.stream(second):
+            got.append(head(d, emb, check_status=False))
+        del emb, d
+        with torch.cuda.stream(first):
+            junk = [torch.full((nbytes // 2,), 255, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    assert len(junk) == 2
+    for out in got:
+        for k in ref:
+            assert _rel(out[k], ref[k]) < 1e-6, k
+
+
+def test_threads_with_streams_of_their_own_share_a_model():
+    import threading
+
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S")
+    systems = [synthetic.molecule_batch(3, 10, 20, seed=20 + i).to("cuda") for i in range(3)]
+    refs = [head(d, bb(d))["forces"] for d in (s.clone() for s in systems)]
+    del bb._step_plan, head._step_plan
+    torch.cuda.synchronize()
+    worst = [1.0] * len(systems)
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            rel = []
+            for _ in range(10):
+                d = systems[i].clone()
+                rel.append(_rel(head(d, bb(d))["forces"], refs[i]))
+            worst[i] = max(rel)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(systems))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert max(worst) < 1e-6

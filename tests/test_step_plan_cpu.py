@@ -4,6 +4,7 @@ copy of a used model carries."""
 import copy
 import ctypes
 import pickle
+from types import SimpleNamespace as NS
 
 import pytest
 import torch
@@ -187,3 +188,42 @@ def test_what_is_kept_follows_the_free_memory_layer_by_layer(cfg, monkeypatch):
         assert a - b < per_layer * 33 / 32 + 4096 and a - b > 0.75 * per_layer
     e.want_grad = 0
     assert kept(10 ** 12)[:2] == (0, 0)
+
+
+class _Stream:
+    def __init__(self, handle, log):
+        self.cuda_stream, self.log = handle, log
+
+    def wait_stream(self, other):
+        self.log.append((self.cuda_stream, "waits for", other.cuda_stream))
+
+    def wait_event(self, event):
+        self.log.append((self.cuda_stream, "waits for", event))
+
+    def record_event(self, event=None):
+        return f"event of {self.cuda_stream}"
+
+
+def test_memory_and_weights_used_on_another_stream_are_tied_to_it(monkeypatch):
+    log, used = [], []
+    one, two = _Stream(1, log), _Stream(2, log)
+    now = [one]
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: now[0])
+    monkeypatch.setattr(step._lib, "call", lambda name, *args: log.append((args[-1].value, name)))
+    tensor = lambda name: NS(record_stream=lambda s: used.append((name, s.cuda_stream)))  # noqa: E731
+    plan, head = NS(w=step._Weights(0), model=step.ModelStruct()), NS(w=step._Weights(0), model=step.ModelStruct())
+    plan.w.laid_out(), head.w.laid_out()
+    run = object.__new__(step.BackboneStep)
+    run.device, run.ev, run.home, run.plan = torch.device("cuda", 0), step.EvalStruct(), None, plan
+    run.keep, run.graph, run.refs = tensor("keep"), NS(a=NS(block=tensor("a")), b=NS(block=tensor("b"))), [tensor("charge")]
+    run._launch("forward", plan)
+    run._launch("energy", plan, head)
+    assert log == [(1, "forward"), (1, "energy")] and not used
+    now[0] = two
+    run._launch("backward", plan, head)
+    assert log[2:] == [(2, "waits for", 1), *2 * [(2, "waits for", "event of 1")], (2, "backward")]
+    assert sorted(used) == [("a", 2), ("b", 2), ("charge", 2), ("keep", 2)]
+    del log[:], plan, run
+    head.w.__del__()  # both blocks of weights go back behind what the second stream did with them
+    assert log == 2 * [(1, "waits for", "event of 2")]
+    head.w.last_use.clear()
