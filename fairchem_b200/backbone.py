@@ -361,8 +361,8 @@ class HalfRangeError(RuntimeError):
 
 def read_gemm_status() -> int:
     """The contraction kernels' device status word, read and cleared: 0 = fine, 1 = a bounded wait expired inside a
-    kernel, 2 = an operand or output left the half-precision range (precision 2 only), 3 = charge, spin or atomic number
-    outside the embedding tables."""
+    kernel, 2 = an operand or output left the half-precision range (precision 2 only), 3 = charge or spin outside the
+    embedding tables (of callers of the C entry points; the backbone refuses them before it evaluates)."""
     if _GemmState.status is None:
         return 0
     code = int(_GemmState.status.item())
@@ -375,7 +375,7 @@ def raise_gemm_status(code: int) -> None:
     if code == 0:
         return
     if code == 3:
-        raise ValueError("charge outside [-100, 100], spin outside [0, 100] or atomic number outside the embedding table")
+        raise ValueError("charge outside [-100, 100] or spin outside [0, 100]")
     if code == 2:
         raise HalfRangeError("tcgen05 GEMM: an operand left the half-precision range; results are invalid "
                              "(use set_gemm_precision(3), or energy_forces(), which falls back by itself)")
@@ -1347,10 +1347,14 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
         if plan is None or pos.dtype != torch.float32 or not pos.is_cuda or pos.device != plan.device or pos.shape[0] == 0:
             return None, None
         status = _status(pos.device)
-        graph = step.StepGraph(self, data, status, torch.is_grad_enabled() and pos.requires_grad)
-        new_step = lambda: step.BackboneStep(plan, graph, plan.dataset_index(self, data["dataset"]), data["charge"], data["spin"],  # noqa: E731
-                                             gamma, self.regress_stress, status)
-        built = self.otf_graph and not self.always_use_pbc and graph.build()
+        graph = step.StepGraph(self, data, torch.is_grad_enabled() and pos.requires_grad)
+        new_step = lambda: step.BackboneStep(plan, graph, plan.dataset_index(self, data["dataset"]), gamma,  # noqa: E731
+                                             self.regress_stress, status)
+        built = False
+        if self.otf_graph and not self.always_use_pbc:
+            built = graph.build()
+        else:
+            graph.check_inputs()
         if built:
             run = new_step()  # before finish(), which waits for the graph's kernels
             built = graph.finish()

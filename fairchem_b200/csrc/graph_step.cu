@@ -13,7 +13,7 @@ namespace step {
 
 constexpr int kCap = 512;        // candidates of one target held in shared memory
 constexpr int kMaxChunks = 512;  // chunk boundaries in the info block
-enum { kInfoEdges = 0, kInfoFlag = 1, kInfoChunks = 2, kInfoMoved = 3, kInfoSources = 4, kInfoCells = 5, kInfoPairs = 6, kInfoNodes = 8,
+enum { kInfoEdges = 0, kInfoFlag = 1, kInfoChunks = 2, kInfoMoved = 3, kInfoSources = 4, kInfoCells = 5, kInfoPairs = 6, kInfoInput = 7, kInfoNodes = 8,
        kInfoEdgeCut = 8 + kMaxChunks + 1 };
 static_assert(FCB200_GRAPH_INFO_WORDS >= 8 + 2 * (kMaxChunks + 1), "info block");
 
@@ -32,13 +32,31 @@ __device__ int image_repeats(const float* cr, float vol, float radius, int* __re
     return (int)r;
 }
 
+// what of the inputs lies outside the embedding tables, the host's to report: a sweep of all blocks over the atoms
+__device__ __forceinline__ void check_inputs(const int64_t* __restrict__ z64, const int64_t* __restrict__ batch64, int64_t num_nodes,
+                                             int num_elements, const int64_t* __restrict__ charge, const int64_t* __restrict__ spin,
+                                             int nsys, int32_t* __restrict__ info) {
+    int bits = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < num_nodes; i += (int64_t)gridDim.x * blockDim.x) {
+        if (z64[i] < 0 || z64[i] >= num_elements) bits |= FCB200_INPUT_ELEMENT;
+        if (batch64[i] < 0 || batch64[i] >= nsys) bits |= FCB200_INPUT_BATCH;
+    }
+    if (threadIdx.x == 0) {
+        if (charge && (charge[blockIdx.x] < -100 || charge[blockIdx.x] > 100)) bits |= FCB200_INPUT_CHARGE;
+        if (spin && (spin[blockIdx.x] < 0 || spin[blockIdx.x] > 100)) bits |= FCB200_INPUT_SPIN;
+    }
+    if (bits) atomicOr(info + kInfoInput, bits);
+}
+
 // One block per system: atom range, bounding box, image counts -> system table.  Grid cells as build_system_table sizes
 // them (edge radius / 1.99, coarser when the product of the dimensions would exceed the limit).
 __global__ void __launch_bounds__(1024)
     graph_systems_kernel(int64_t num_nodes, const float* __restrict__ pos, const float* __restrict__ cell, const uint8_t* __restrict__ pbc,
-                         const int64_t* __restrict__ natoms, int nsys, float radius, int32_t* __restrict__ sys, float* __restrict__ bbox,
-                         int32_t* __restrict__ info) {
+                         const int64_t* __restrict__ natoms, int nsys, float radius, const int64_t* __restrict__ z64,
+                         const int64_t* __restrict__ batch64, int num_elements, const int64_t* __restrict__ charge,
+                         const int64_t* __restrict__ spin, int32_t* __restrict__ sys, float* __restrict__ bbox, int32_t* __restrict__ info) {
     pdl_sync();
+    check_inputs(z64, batch64, num_nodes, num_elements, charge, spin, nsys, info);
     __shared__ long long s_begin[32];
     __shared__ float s_lo[32][3], s_hi[32][3];
     const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, threads = blockDim.x, warps = threads >> 5;
@@ -126,15 +144,13 @@ __global__ void __launch_bounds__(32) graph_offsets_kernel(int32_t* __restrict__
 }
 
 __global__ void graph_convert_kernel(const int64_t* __restrict__ z64, const int64_t* __restrict__ batch64, int32_t* __restrict__ z,
-                                     int32_t* __restrict__ batch, int64_t n, int num_elements, int nsys, int32_t* __restrict__ info,
-                                     int32_t* __restrict__ status) {
+                                     int32_t* __restrict__ batch, int64_t n, int num_elements, int nsys, int32_t* __restrict__ info) {
     pdl_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 8) info[i] = 0;  // the kernels that raise words of it run after this one
     if (i >= n) return;
     const int64_t a = z64[i], b = batch64[i];
-    const bool bad = a < 0 || a >= num_elements || b < 0 || b >= nsys;
-    if (bad) atomicExch(status, 3);
+    const bool bad = a < 0 || a >= num_elements || b < 0 || b >= nsys;  // reported by the next kernel
     z[i] = bad ? 0 : (int)a;
     batch[i] = bad ? 0 : (int)b;
 }
@@ -442,15 +458,15 @@ extern "C" {
 
 int fcb200_graph_systems(const fcb200_graph* g, void* stream) {
     if (!g || g->num_nodes < 1 || g->num_systems < 1 || !(g->radius > 0.f)) return FCB200_EINVAL;
-    if (!g->pos || !g->cell || !g->pbc || !g->natoms || !g->batch64 || !g->z64 || !g->sys || !g->bbox || !g->z || !g->batch || !g->info || !g->status)
+    if (!g->pos || !g->cell || !g->pbc || !g->natoms || !g->batch64 || !g->z64 || !g->sys || !g->bbox || !g->z || !g->batch || !g->info)
         return FCB200_EINVAL;
     const step::PdlScope scope(g->num_nodes);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     launch_pdl(step::graph_convert_kernel, dim3((unsigned)((g->num_nodes + 255) / 256)), dim3(256), 0, st, g->z64, g->batch64, g->z, g->batch, g->num_nodes,
-                                                                                      g->num_elements, g->num_systems, g->info, g->status);
+                                                                                      g->num_elements, g->num_systems, g->info);
     // few systems: a block each has to sweep many atoms
-    launch_pdl(step::graph_systems_kernel, dim3(g->num_systems), dim3(g->num_systems < 148 ? 1024 : 128), 0, st, g->num_nodes, g->pos, g->cell, g->pbc, g->natoms, g->num_systems, g->radius, g->sys, g->bbox,
-                                                               g->info);
+    launch_pdl(step::graph_systems_kernel, dim3(g->num_systems), dim3(g->num_systems < 148 ? 1024 : 128), 0, st, g->num_nodes, g->pos, g->cell, g->pbc, g->natoms, g->num_systems, g->radius, g->z64,
+                                                               g->batch64, g->num_elements, g->charge, g->spin, g->sys, g->bbox, g->info);
     if (g->want_totals) launch_pdl(step::graph_offsets_kernel, dim3(1), dim3(32), 0, st, g->sys, g->num_systems, g->info);
     return launch_status();
 }

@@ -309,20 +309,19 @@ ALWAYS_THERE = 1 << 28  # bytes that any GPU in use has; more: what the allocato
 class BackboneStep:
     """One evaluation: graph arrays, outputs and the memory that the backward pass reads."""
 
-    def __init__(self, plan: ModelPlan, graph: "StepGraph", dataset, charge, spin, gamma, want_virial: bool, status):
+    def __init__(self, plan: ModelPlan, graph: "StepGraph", dataset, gamma, want_virial: bool, status):
         self.plan, self.model = plan, plan.model
         self.nodes, self.systems, self.device = graph.nodes, graph.systems, graph.device
         e, g = EvalStruct(), graph.g
         self.ev = e
         e.num_nodes, e.num_systems, e.want_grad = self.nodes, self.systems, int(graph.want_grad)
-        charge, spin = charge.to(self.device, torch.int64).contiguous(), spin.to(self.device, torch.int64).contiguous()
         gamma = None if gamma is None else gamma.contiguous()
         self.leaf, self.graph = graph.leaf, graph
-        self.refs = [t for t in (dataset, charge, spin, gamma, status, *graph.alive) if t is not None]
-        self.watched = [t for t in (graph.pos, charge, spin, gamma) if t is not None]  # may be the caller's own memory
+        self.refs = [t for t in (dataset, gamma, status, *graph.alive) if t is not None]
+        self.watched = [t for t in (graph.pos, graph.charge, graph.spin, gamma) if t is not None]  # may be the caller's own memory
         for name in ("pos", "z", "batch", "src", "tgt", "row_ptr", "src_ptr", "src_perm"):
             setattr(e, name, getattr(g, name))
-        e.shift, e.dataset, e.charge, e.spin = graph.shift, dataset.data_ptr(), charge.data_ptr(), spin.data_ptr()
+        e.shift, e.dataset, e.charge, e.spin = graph.shift, dataset.data_ptr(), g.charge, g.spin
         e.gamma = None if gamma is None else gamma.data_ptr()
         e.status = status.data_ptr()
         self.want_virial, self.virial = want_virial, None
@@ -441,8 +440,8 @@ class GraphStruct(Structure):
     _fields_ = ([("num_nodes", c_int64)]
                 + [(n, c_int32) for n in ("num_systems", "num_elements", "max_neighbors", "stride", "chunk_edges", "want_totals")]
                 + [("radius", c_float), ("radius_sq", c_float)]
-                + [(n, c_void_p) for n in ("pos", "cell", "pbc", "natoms", "batch64", "z64", "sys", "bbox", "z", "batch", "rows", "count",
-                                           "row_ptr", "info", "status")]
+                + [(n, c_void_p) for n in ("pos", "cell", "pbc", "natoms", "batch64", "z64", "charge", "spin", "sys", "bbox", "z", "batch",
+                                           "rows", "count", "row_ptr", "info")]
                 + [("num_sources", c_int64), ("num_cells", c_int64)]
                 + [(n, c_void_p) for n in ("cell_count", "source_cell", "cell_ptr", "cell_fill", "bucket", "cand_ptr", "cand_id",
                                            "cand_sys", "pos0", "cell0", "pbc0", "natoms0")]
@@ -451,7 +450,9 @@ class GraphStruct(Structure):
                                            "src_perm", "chunk_src")])
 
 
-INFO_WORDS, INFO_NODES, INFO_EDGES = 1040, 8, 8 + 513
+INFO_WORDS, INFO_INPUT, INFO_NODES, INFO_EDGES = 1040, 7, 8, 8 + 513
+INPUT_ERRORS = ((1, "atomic number outside the embedding table"), (2, "system index (batch) outside the batch"),
+                (4, "charge outside [-100, 100]"), (8, "spin outside [0, 100]"))
 STRIDE_MAX = 512     # kept neighbours of one target that graph_select_kernel can hold
 BRUTE_NODES = 8192   # below: every periodic image in reach is tried, no grid and no host read to size one
 BRUTE_PAIRS = 4e9    # above that, still the faster way while the systems of a batch are small
@@ -478,7 +479,7 @@ class StepGraph:
     """Index arrays of one evaluation for csrc/model_step.cu (edges sorted by target; ``None`` from ``build`` when the
     general path has to decide: too many neighbours, a degenerate cell)."""
 
-    def __init__(self, bb, data, status, want_grad: bool):
+    def __init__(self, bb, data, want_grad: bool):
         self.bb, self.data, self.want_grad = bb, data, want_grad
         pos = self.pos = data["pos"].detach().contiguous()
         self.leaf = data["pos"]
@@ -491,13 +492,15 @@ class StepGraph:
         g.radius, g.radius_sq = bb.cutoff, bb.cutoff * bb.cutoff
         pbc = data["pbc"] if data["pbc"].dtype == torch.bool else data["pbc"].bool()
         cell = data["cell"].detach().to(torch.float32)
-        self.alive = [cell.contiguous(), pbc.contiguous(), *(data[k].long().contiguous() for k in ("natoms", "batch", "atomic_numbers")), status]
+        self.alive = [cell.contiguous(), pbc.contiguous(),
+                      *(data[k].long().contiguous() for k in ("natoms", "batch", "atomic_numbers", "charge", "spin"))]
         if any(t.device != self.device for t in self.alive):  # small host tensors next to device positions
             self.alive = [t.to(self.device) for t in self.alive]
         if self.alive[1].numel() != 3 * b:
             self.alive[1] = self.alive[1].reshape(-1, 3).expand(b, 3).contiguous()
         g.pos = pos.data_ptr()
-        g.cell, g.pbc, g.natoms, g.batch64, g.z64, g.status = (t.data_ptr() for t in self.alive)
+        g.cell, g.pbc, g.natoms, g.batch64, g.z64, g.charge, g.spin = (t.data_ptr() for t in self.alive)
+        self.charge, self.spin = self.alive[-2:]
         for name, p in self.a.ptr.items():
             setattr(g, name, p)
         self.chunk_src = self.edge_index = self.cell_offsets = self.shift = None
@@ -506,8 +509,18 @@ class StepGraph:
     def _call(self, name):
         _lib.call(name, byref(self.g), _stream())
 
-    def _info(self):
-        return self.a.view("info", INFO_WORDS).cpu()
+    def _info(self, words: int = INFO_WORDS):
+        """The info block on the host, in which the kernels have noted inputs that the model has no embedding for."""
+        info = self.a.view("info", words).cpu()
+        bad = int(info[INFO_INPUT])
+        if bad:
+            raise ValueError(", ".join(what for bit, what in INPUT_ERRORS if bad & bit))
+        return info
+
+    def check_inputs(self):
+        """Before other code indexes by them: raise for inputs outside the tables."""
+        self._call("fcb200_graph_systems")
+        self._info(8)
 
     def _set_chunks(self, edges: int, node_cut: list, edge_cut: list):
         self.num_edges, n = edges, len(node_cut) - 1
@@ -543,7 +556,7 @@ class StepGraph:
             info = self._select_kept(nl)
         else:
             if g.want_totals:
-                head = self.a.view("info", 8).cpu()
+                head = self._info(8)
                 if int(head[1]):
                     return False
                 g.num_sources, g.num_cells = int(head[4]), int(head[5])
@@ -564,7 +577,7 @@ class StepGraph:
         """After build: the number of edges where it is not known yet.  False: not for this path."""
         if self.pending:
             self.pending = False
-            info = self.a.view("info", 8).tolist()
+            info = self._info(8).tolist()
             if info[1] or info[0] == 0:
                 return False
             self._set_chunks(info[0], [0, self.nodes], [0, info[0]])
@@ -592,6 +605,7 @@ class StepGraph:
             if not int(info[3]):
                 nl.refreshes += 1
                 return info
+        self._info(8)  # the search indexes by the batch
         nl.search(data, data["pbc"])
         nl.origin = (nl._pos0, self.alive[0].clone(), self.alive[1].clone(), self.alive[2].clone())
         g.pos0 = None

@@ -623,7 +623,12 @@ int fcb200_model_backward(const fcb200_model* model_host, const fcb200_eval* eva
 
 /* Graph of an evaluation (csrc/graph_step.cu): fcb200_graph_systems, then fcb200_graph_select, one host read of `info`,
  * then fcb200_graph_fill.  `info` words: 0 edges, 1 nonzero = left to the general path, 2 chunks, 3 nonzero = kept
- * candidates expired, 4 / 5 source and cell totals, 6 candidate pairs (float), 8.. chunk nodes, 8 + 513.. chunk edges. */
+ * candidates expired, 4 / 5 source and cell totals, 6 candidate pairs (float), 7 FCB200_INPUT_* bits of inputs outside the
+ * model's tables (the kernels go on with row 0 for them), 8.. chunk nodes, 8 + 513.. chunk edges. */
+#define FCB200_INPUT_ELEMENT 1 /* atomic number outside [0, num_elements) */
+#define FCB200_INPUT_BATCH 2   /* system index outside [0, num_systems) */
+#define FCB200_INPUT_CHARGE 4  /* charge outside [-100, 100] */
+#define FCB200_INPUT_SPIN 8    /* spin outside [0, 100] */
 #define FCB200_GRAPH_INFO_WORDS 1040
 typedef struct {
     int64_t num_nodes;
@@ -631,12 +636,11 @@ typedef struct {
     float radius, radius_sq;
     const float *pos, *cell;
     const uint8_t* pbc;
-    const int64_t *natoms, *batch64, *z64;
+    const int64_t *natoms, *batch64, *z64, *charge, *spin; /* [num_systems], [N], [N], [num_systems] x 2 (null: not checked) */
     int32_t* sys;            /* [num_systems, FCB200_SYS_WORDS] out */
     float* bbox;             /* [num_systems, 6] out */
     int32_t *z, *batch;      /* [N] out */
     int32_t *rows, *count, *row_ptr, *info; /* [N, stride, 2], [N], [N+1], [FCB200_GRAPH_INFO_WORDS] out */
-    int32_t* status;
     /* cell-list search (cell_ptr set) */
     int64_t num_sources, num_cells;
     int32_t *cell_count, *source_cell, *cell_ptr, *cell_fill;

@@ -365,3 +365,42 @@ def test_threads_with_streams_of_their_own_share_a_model():
     for t in threads:
         t.join()
     assert max(worst) < 1e-6
+
+
+@pytest.mark.parametrize("what", ["atomic number", "batch", "charge", "spin"])
+@pytest.mark.parametrize("graph", ["own", "own_chunked", "own_counted", "kept_list", "given", "all_periodic"])
+def test_inputs_outside_the_tables_are_reported_by_the_backbone(what, graph, monkeypatch):
+    """The backbone's own call raises and names them; nothing is left behind for the next evaluation."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import step, synthetic
+    from fairchem_b200.graph import SkinNeighborList
+
+    kw = {"own_chunked": {"edge_chunk_size": 40}, "all_periodic": {"always_use_pbc": True}}.get(graph, {})
+    bb, head = _model(B, "UMA_S", **kw)
+    data = synthetic.merge([synthetic.fcc_cu((2, 2, 2), seed=i) for i in range(3)]).to("cuda")
+    if graph == "own_counted":
+        monkeypatch.setattr(step, "BRUTE_NODES", 0)
+    if graph == "kept_list":
+        bb.neighbor_list = SkinNeighborList(bb.cutoff, bb.max_neighbors, 0.5)
+    if graph == "given":
+        bb(data.clone())
+        bb.otf_graph = False
+        data["edge_index"], data["cell_offsets"] = bb.last_graph["edge_index"].clone(), bb.last_graph["cell_offsets"].clone()
+    d = data.clone()
+    ref = head(d, bb(d))["forces"]
+    key = "atomic_numbers" if what == "atomic number" else what
+    for value in (-101, 1000):
+        d = data.clone()
+        d[key] = d[key].clone()
+        d[key][-1] = value
+        with pytest.raises(ValueError, match=what):
+            bb(d)
+        assert B.read_gemm_status() == 0
+    d = data.clone()
+    assert _rel(head(d, bb(d))["forces"], ref) < 1e-6
+    if graph == "kept_list":  # a list that has expired is searched for again, by code that indexes by the batch
+        bb.neighbor_list = SkinNeighborList(bb.cutoff, bb.max_neighbors, 0.5)
+        d[key] = d[key].clone()
+        d[key][0] = 1000
+        with pytest.raises(ValueError, match=what):
+            bb(d)
