@@ -261,8 +261,9 @@ __global__ void __launch_bounds__(256)
             const int i = i0 + lane;
             float d2 = 0.f;
             int atom = 0, code = 0;
-            if (i < e) {
-                const int local = cand_id[i] - s.source_begin;
+            const int local = i < e ? cand_id[i] - s.source_begin : -1;
+            // an expired list, whose result the host discards, may name sources that this system does not have
+            if (local >= 0 && local < (s.atom_end - s.atom_begin) * s.nimg) {
                 int n0, n1, n2;
                 decode_image(s, local % s.nimg, n0, n1, n2);
                 atom = s.atom_begin + local / s.nimg;

@@ -404,3 +404,26 @@ def test_inputs_outside_the_tables_are_reported_by_the_backbone(what, graph, mon
         d[key][0] = 1000
         with pytest.raises(ValueError, match=what):
             bb(d)
+
+
+def test_kept_list_of_another_split_is_not_used():
+    """The same atoms and the same number of systems, divided differently: the kept candidates name periodic sources that a
+    target's new system does not have, and the list is searched for again."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+    from fairchem_b200.graph import SkinNeighborList
+
+    bb, head = _model(B, "UMA_S")
+    bb.neighbor_list = SkinNeighborList(bb.cutoff, bb.max_neighbors, 0.5)
+    mol, cu = synthetic.molecule_batch(1, 20, 20, seed=2), synthetic.fcc_cu((2, 2, 2), seed=1)
+    a, b = synthetic.merge([mol, cu]), synthetic.merge([cu, mol])  # 20 + 32 atoms, images 1 and 27; then the other way round
+    for data in (a, b, a):
+        d = data.to("cuda")
+        emb = bb(d)
+        got, kept = head(d, emb), bb.neighbor_list
+        bb.neighbor_list = None
+        d = data.to("cuda")
+        ref = head(d, bb(d))
+        bb.neighbor_list = kept
+        assert _rel(got["forces"], ref["forces"]) < 1e-6
+    assert (kept.searches, kept.refreshes) == (3, 0)
