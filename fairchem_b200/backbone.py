@@ -1331,6 +1331,12 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
                     edge_index, cell_offsets, neighbors = radius_graph_pbc_b200(data, self.cutoff, self.max_neighbors, False, pbc)
         else:
             edge_index, cell_offsets = data["edge_index"], data["cell_offsets"]
+            if edge_index.dim() != 2 or edge_index.shape[0] != 2 or cell_offsets.shape != (edge_index.shape[1], 3):
+                raise ValueError(f"edge_index of shape {tuple(edge_index.shape)} with cell_offsets of shape {tuple(cell_offsets.shape)}")
+            if edge_index.numel():
+                lo, hi = torch.stack(torch.aminmax(edge_index)).tolist()
+                if lo < 0 or hi >= len(data["pos"]):
+                    raise ValueError(f"edge_index names atoms {lo} to {hi} of {len(data['pos'])}")
             order = torch.sort(edge_index[1], stable=True).indices
             edge_index, cell_offsets = edge_index[:, order], cell_offsets[order]
         return edge_index, cell_offsets

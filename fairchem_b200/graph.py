@@ -68,6 +68,8 @@ def build_system_table(pos: torch.Tensor, cell: torch.Tensor, pbc: torch.Tensor,
     """
     nsys = int(natoms.shape[0])
     natoms_h = natoms.detach().cpu().numpy().astype(np.int64)
+    if (natoms_h < 0).any() or int(natoms_h.sum()) > int(pos.shape[0]):
+        raise _lib.FairchemB200Error(f"radius graph: systems of {natoms_h.tolist()[:8]}... atoms with {int(pos.shape[0])} positions")
     cell_h = cell.detach().float().cpu().numpy().reshape(nsys, 3, 3)
     pbc_h = torch.atleast_2d(pbc).detach().cpu().numpy().astype(bool)
     if pbc_h.shape[0] == 1 and nsys > 1:

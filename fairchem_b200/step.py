@@ -258,11 +258,15 @@ class ModelPlan:
         """This plan with the energy head's weights (cached on the head), or None."""
         eb = head.energy_block
         params = [p for i in (0, 2, 4) for p in (eb[i].weight, eb[i].bias)]
+        if any(p is None for p in params):
+            return None
         key = _versions(params)
         hit = getattr(head, "_step_plan", None)
         if hit is not None and hit.backbone is self and hit.key == key:
             return hit
         if eb[0].weight.shape != (C, C) or eb[2].weight.shape != (C, C) or eb[4].weight.shape != (1, C):
+            return None
+        if any(p.device != self.device or p.dtype != torch.float32 for p in params):
             return None
         head._step_plan = hit = HeadPlan(self, eb, key)
         return hit
@@ -315,7 +319,12 @@ class BackboneStep:
         e, g = EvalStruct(), graph.g
         self.ev = e
         e.num_nodes, e.num_systems, e.want_grad = self.nodes, self.systems, int(graph.want_grad)
-        gamma = None if gamma is None else gamma.contiguous()
+        if dataset.numel() != self.systems:
+            raise ValueError(f"dataset has {dataset.numel()} entries, expected {self.systems}")
+        gamma = None if gamma is None or gamma.numel() == 0 else gamma.contiguous()
+        ops._chk(gamma)
+        ops._f32(gamma)
+        self.gamma = gamma
         self.leaf, self.graph = graph.leaf, graph
         self.refs = [t for t in (dataset, gamma, status, *graph.alive) if t is not None]
         self.watched = [t for t in (graph.pos, graph.charge, graph.spin, gamma) if t is not None]  # may be the caller's own memory
@@ -331,6 +340,8 @@ class BackboneStep:
 
     def set_edges(self, graph: "StepGraph"):
         e = self.ev
+        if self.gamma is not None and self.gamma.numel() != graph.num_edges:
+            raise ValueError(f"gamma has {self.gamma.numel()} entries for {graph.num_edges} edges")
         e.num_edges, e.num_chunks = graph.num_edges, graph.num_chunks
         e.chunk_src = graph.g.chunk_src if graph.num_chunks > 1 else None
         e.chunk_node, e.chunk_edge = ctypes.addressof(graph.chunk_node), ctypes.addressof(graph.chunk_edge)
@@ -485,6 +496,11 @@ class StepGraph:
         self.leaf = data["pos"]
         self.device, self.nodes, self.systems = pos.device, pos.shape[0], len(data["natoms"])
         n, b = self.nodes, self.systems
+        if pos.dim() != 2 or pos.shape[1] != 3:
+            raise ValueError(f"positions of shape {tuple(pos.shape)}, expected [atoms, 3]")
+        for key, want in (("batch", n), ("atomic_numbers", n), ("cell", 9 * b), ("charge", b), ("spin", b)):
+            if data[key].numel() != want:  # the kernels read as many
+                raise ValueError(f"{key} has {data[key].numel()} entries, expected {want} for {n} atoms in {b} systems")
         self.a = _Carve(self.device, sys=b * 24, bbox=b * 6, z=n, batch=n, count=n, row_ptr=n + 1, info=INFO_WORDS)
         g = self.g = GraphStruct()
         g.num_nodes, g.num_systems, g.num_elements = n, b, bb.max_num_elements

@@ -10,8 +10,9 @@ import pytest
 import torch
 import torch.nn as nn
 
-from fairchem_b200 import step, weights
+from fairchem_b200 import _lib, step, synthetic, weights
 from fairchem_b200.backbone import MLP_EFS_HeadB200, RMSNormSH, eSCNMDBackboneB200
+from fairchem_b200.graph import build_system_table
 
 
 @pytest.fixture()
@@ -227,3 +228,33 @@ def test_memory_and_weights_used_on_another_stream_are_tied_to_it(monkeypatch):
     head.w.__del__()  # both blocks of weights go back behind what the second stream did with them
     assert log == 2 * [(1, "waits for", "event of 2")]
     head.w.last_use.clear()
+
+
+def test_inputs_of_another_length_than_the_kernels_read_are_refused(bb):
+    data = synthetic.molecule_batch(3, 5, 8, seed=1)
+    step.StepGraph(bb, data, True)
+    for key in ("batch", "atomic_numbers", "cell", "charge", "spin"):
+        for wrong in (data[key][:-1], torch.cat([data[key], data[key]])):
+            d = data.clone()
+            d[key] = wrong
+            with pytest.raises(ValueError, match=key):
+                step.StepGraph(bb, d, True)
+    d = data.clone()
+    d["pos"] = d["pos"][:, :2]
+    with pytest.raises(ValueError, match="positions"):
+        step.StepGraph(bb, d, True)
+    with pytest.raises(_lib.FairchemB200Error, match="positions"):
+        build_system_table(data.pos, data.cell, data.pbc, data.natoms + 1, 6.0)
+
+
+def test_a_given_graph_that_names_other_atoms_is_refused(bb):
+    bb.otf_graph = False
+    data = synthetic.molecule_batch(1, 5, 5, seed=1)
+    good = dict(edge_index=torch.tensor([[0, 4], [1, 0]]), cell_offsets=torch.zeros(2, 3))
+    data.update(good)
+    bb._graph(data)
+    for key, wrong in (("edge_index", torch.tensor([[0, 5], [1, 0]])), ("edge_index", torch.tensor([[0, 4], [-1, 0]])),
+                       ("cell_offsets", torch.zeros(1, 3)), ("edge_index", torch.zeros(3, 2, dtype=torch.long))):
+        data.update({**good, key: wrong})
+        with pytest.raises(ValueError, match="edge_index"):
+            bb._graph(data)
