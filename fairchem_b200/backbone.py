@@ -1348,8 +1348,7 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
     def _forward_native(self, data, gamma):
         """The whole evaluation from native code (fairchem_b200.step), and the graph (edge_index, cell_offsets) it ran on.
         No evaluation when the native path does not apply or the GPU lacks the memory; no graph when none was built."""
-        plan = step.ModelPlan.of(self)
-        pos = data["pos"]
+        plan, pos = step.ModelPlan.likely(self, data["pos"].device), data["pos"]
         if plan is None or pos.dtype != torch.float32 or not pos.is_cuda or pos.device != plan.device or pos.shape[0] == 0:
             return None, None
         status = _status(pos.device)
@@ -1361,12 +1360,12 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
             built = graph.build()
         else:
             graph.check_inputs()
-        if built:
-            run = new_step()  # before finish(), which waits for the graph's kernels
-            built = graph.finish()
+        run = new_step() if built else None  # before finish(), which waits for the graph's kernels
+        if built and graph.finish():
             found = graph.edge_index, graph.cell_offsets
-        if not built:
-            found = edge_index, cell_offsets = self._graph(data)
+        else:
+            run, found = None, self._graph(data)
+            edge_index, cell_offsets = found
             if edge_index.shape[1] == 0:  # isolated atoms: see _forward
                 edge_index = torch.zeros(2, 1, dtype=torch.long, device=pos.device)
                 cell_offsets = torch.zeros(1, 3, dtype=pos.dtype, device=pos.device)
@@ -1375,13 +1374,22 @@ class eSCNMDBackboneB200(step.HoldsPlan, nn.Module):
                 edge_sys = None if data["cell"].shape[0] == 1 else data["batch"][edge_index[1]]
                 graph.from_edges(edge_index[0], edge_index[1], get_pbc_shifts(data["cell"].to(pos.dtype), cell_offsets, edge_sys).contiguous())
             graph.edge_index, graph.cell_offsets = edge_index, cell_offsets
-            run = new_step()
-        run.set_edges(graph)
-        if not run.plan_memory():
-            return None, found
-        run.virial = {"num_systems": graph.systems} if self.regress_stress else None
-        x = step.BackboneFn.apply(pos, run)
-        data["scatter_target"] = graph.edge_index[1]
+        while True:
+            run = run or new_step()
+            run.set_edges(graph)
+            if not run.plan_memory():
+                return None, found
+            run.virial = {"num_systems": graph.systems} if self.regress_stress else None
+            x = step.BackboneFn.apply(pos, run)
+            # whether the plan still holds is looked at while its launches run; one that does not costs them again
+            now = step.ModelPlan.of(self)
+            if now is plan:
+                break
+            status.zero_()
+            if now is None or now.device != pos.device:
+                return None, found
+            plan, run, x = now, None, None
+        data["scatter_target"] = found[0][1]
         self.last_graph = {"edge_index": graph.edge_index, "cell_offsets": graph.cell_offsets}
         run.embedding = weakref.ref(x)  # x's autograd node holds the run: a strong reference would be a cycle
         return {"node_embedding": x, "batch": data["batch"], "virial": run.virial, "step": run}, found
