@@ -64,6 +64,36 @@ __device__ __forceinline__ int warp_sum_i(int v) {
     return v;
 }
 
+// v[i] = its sum over the warp, in every lane, for N = 2, 4, 8: at the first offsets every lane hands over the half it will
+// not own, which leaves N - 1 + (5 - log2 N) shuffles and N to hand the sums round (N = 4: 10, not 20).  Added in the order of
+// warp_sum: the same bits.
+template <int N> __device__ __forceinline__ void warp_sums(float (&v)[N], int lane) {
+    int n = N;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i)
+                if (i < n) {
+                    const float send = upper ? v[i] : v[i + n], keep = upper ? v[i + n] : v[i];
+                    v[i] = keep + __shfl_xor_sync(kFull, send, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(kFull, v[0], o);
+        }
+    }
+    const float total = v[0];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        int from = 0;
+#pragma unroll
+        for (int m = N >> 1, o = 16; m > 0; m >>= 1, o >>= 1) from |= (i & m) ? o : 0;
+        v[i] = __shfl_sync(kFull, total, from);
+    }
+}
+
 // Sum each of 35 per-lane partial values over the warp.  The first 32 go through a transposed butterfly
 // (at offset h every lane hands over the half it will not own: 16+8+4+2+1 = 31 shuffles, after which
 // lane l holds the total of value l); the last 3 use plain warp sums.  46 shuffles instead of 175.

@@ -371,17 +371,17 @@ int Run::radial_hidden_forward() {
         float *pre1 = L.pre1 + k0 * L.rw, *pre2 = L.pre2 + k0 * L.rw;
         FCB_TRY(conv("so2_conv_fused_radial_in", c0, L.gauss.hi + e0 * md.num_basis, L.gauss.lo + e0 * md.num_basis, md.num_basis, md.num_basis,
                      0, pre1, L.rw, L.rw, nullptr, 0, nullptr, nullptr, ec));
-        const int grid = warp_grid(radial_items(ec, nets), 8);
+        const int grid = warp_grid(radial_items(ec, nets, kRadialFwdRows), 8);
         FCB_TRY(op("radial_act_fwd", ec * nets * 1040, [&] {
-            launch_pdl(radial_fwd_kernel, dim3(grid), dim3(256), 0, st, pre1, md.table_src, md.table_tgt, ev.z, ev.src, ev.tgt, md.ln1_w, md.ln1_b, md.radial_eps,
-                                                    L.h1.out(), L.rw, C, L.rst1 + k0 * nets * 2, e0, ec, nets);
+            launch_pdl(radial_fwd_kernel, dim3(grid), dim3(256), 0, st, pre1, md.table_src, md.table_tgt, ev.z, ev.src + e0, ev.tgt + e0, md.ln1_w, md.ln1_b, md.radial_eps,
+                                                    L.h1.out(), C, L.rst1 + k0 * nets * 2, ec * nets, nets);
             return 0;
         }));
         FCB_TRY(conv("so2_conv_fused_radial_in", c1, L.h1.hi, L.h1.lo, L.rw, L.rw, 0, pre2, L.rw, L.rw, nullptr, 0, nullptr, nullptr, ec));
         __half* h = L.h2 + e0 * L.rw * 2;
         return op("radial_act_fwd", ec * nets * 1032, [&] {
-            launch_pdl(radial_fwd_kernel, dim3(grid), dim3(256), 0, st, pre2, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b, md.radial_eps,
-                                                    OutSplit{h, h + C, 1.0f}, L.rw * 2, 2 * C, L.rst2 + k0 * nets * 2, e0, ec, nets);
+            launch_pdl(radial_fwd_kernel, dim3(grid), dim3(256), 0, st, pre2, nullptr, nullptr, ev.z, ev.src + e0, ev.tgt + e0, md.ln2_w, md.ln2_b, md.radial_eps,
+                                                    OutSplit{h, h + C, 1.0f}, 2 * C, L.rst2 + k0 * nets * 2, ec * nets, nets);
             return 0;
         });
     });
@@ -653,16 +653,16 @@ int Run::backward() {
         }));
         float* gh = reinterpret_cast<float*>(L.h2) + e0 * L.rw;
         FCB_TRY(gemm("so2_conv_fused_radial_out_bwd", L.gr3, md.degree_out_t, scale, gh + (int64_t)md.num_layers * C, L.rw, ec));
-        const int grid = warp_grid(radial_items(ec, nets), 8);
+        const int grid = warp_grid(radial_items(ec, nets, kRadialBwdRows), 8);
         FCB_TRY(op("radial_act_bwd", ec * nets * 1544, [&] {
-            launch_pdl(radial_bwd_kernel, dim3(grid), dim3(256), 0, st, gh, L.pre2 + e0 * L.rw, nullptr, nullptr, ev.z, ev.src, ev.tgt, md.ln2_w, md.ln2_b,
-                                                    L.rst2 + e0 * nets * 2, L.rp.out(), L.rw, C, L.scales, nscale, L.rad_scale, e0, ec, nets);
+            launch_pdl(radial_bwd_kernel, dim3(grid), dim3(256), 0, st, gh, L.pre2 + e0 * L.rw, nullptr, nullptr, ev.z, ev.src + e0, ev.tgt + e0, md.ln2_w, md.ln2_b,
+                                                    L.rst2 + e0 * nets * 2, L.rp.out(), C, L.scales, nscale, L.rad_scale, ec * nets, nets);
             return 0;
         }));
         FCB_TRY(conv("so2_conv_fused_radial_in", c1, L.rp.hi, L.rp.lo, L.rw, L.rw, 0, L.rh, L.rw, L.rw, nullptr, 0, L.rad_scale, nullptr, ec));
         FCB_TRY(op("radial_act_bwd", ec * nets * 1544, [&] {
-            launch_pdl(radial_bwd_kernel, dim3(grid), dim3(256), 0, st, L.rh, L.pre1 + e0 * L.rw, md.table_src, md.table_tgt, ev.z, ev.src, ev.tgt, md.ln1_w, md.ln1_b,
-                                                    L.rst1 + e0 * nets * 2, L.rp.out(), L.rw, C, L.scales, nscale, L.rad_scale, e0, ec, nets);
+            launch_pdl(radial_bwd_kernel, dim3(grid), dim3(256), 0, st, L.rh, L.pre1 + e0 * L.rw, md.table_src, md.table_tgt, ev.z, ev.src + e0, ev.tgt + e0, md.ln1_w, md.ln1_b,
+                                                    L.rst1 + e0 * nets * 2, L.rp.out(), C, L.scales, nscale, L.rad_scale, ec * nets, nets);
             return 0;
         }));
         FCB_TRY(gemm("so2_conv_fused_radial_in", L.rp, md.rad_w0_t, L.rad_scale, L.ggauss, md.num_basis, ec));

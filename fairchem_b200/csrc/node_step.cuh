@@ -146,114 +146,124 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- hidden activations of the radial MLPs ------------------------------------------------------------------------
-// SiLU(LayerNorm(pre + element tables)) for `nets` MLPs side by side.  Rows: pre [E, nets*C], stats [E, nets, 2]; output
-// planes at i * out_ld + net * out_net.  One warp per edge and kNetBatch nets: one row of 512 bytes per warp left the
-// loads and the two reductions of a row in series (3.1 M edges x 5 nets: 10.8 ms forward, 14.0 ms backward).
-constexpr int kNetBatch = 3;
+// SiLU(LayerNorm(pre + element tables)) for `nets` MLPs side by side.  Rows (edge, net) of 128: pre [E, nets*C], stats
+// [E, nets, 2]; output planes out_row apart.  A warp takes R rows that follow one another, whatever edges they belong to.
+// Bound by instruction issue (exponential, division, reductions), which the backward pass needs warps for and the forward
+// pass independent rows: 1.55 M edges x 5 nets, ms, backward with 4 rows / 3 blocks on an SM 7.2, 4 / 4 6.6, 2 / 4 6.5, 2 / 5
+// 6.2, 1 / 8 6.0; forward with 1 / 8 5.4, 2 / 5 5.4, 4 / 5 4.9.  One edge's nets three at a time, a sixth of the slots empty
+// at five nets: 7.8 and 5.6.
+constexpr int kRadialFwdRows = 4, kRadialBwdRows = 1;
 
-struct RadialItem {
-    int64_t i;
-    int net0, n;
-};
-__device__ __forceinline__ RadialItem radial_item(int64_t it, int nets) {
-    const int groups = (nets + kNetBatch - 1) / kNetBatch;
-    const int64_t i = it / groups;
-    const int net0 = (int)(it - i * groups) * kNetBatch;
-    return {i, net0, min(kNetBatch, nets - net0)};
-}
-__host__ __device__ inline int64_t radial_items(int64_t edges, int nets) { return edges * ((nets + kNetBatch - 1) / kNetBatch); }
+inline int64_t radial_items(int64_t edges, int nets, int rows) { return (edges * nets + rows - 1) / rows; }
 
-__device__ __forceinline__ void radial_rows(float4 (&y)[kNetBatch], const RadialItem& q, const float* __restrict__ pre, const float* __restrict__ ts,
-                                            const float* __restrict__ tt, const int32_t* __restrict__ z, const int32_t* __restrict__ src,
-                                            const int32_t* __restrict__ tgt, int64_t e_base, int64_t width, int c) {
+// rows [row0, row0 + n) of the pre-activation, tables added, and the nets they belong to
+template <int R>
+__device__ __forceinline__ void radial_rows(float4 (&y)[R], int (&net)[R], uint32_t row0, int n, const float* __restrict__ pre,
+                                            const float* __restrict__ ts, const float* __restrict__ tt, const int32_t* __restrict__ z,
+                                            const int32_t* __restrict__ src, const int32_t* __restrict__ tgt, int nets, int c) {
+    uint32_t i = row0 / (uint32_t)nets;
+    net[0] = (int)(row0 - i * nets);
 #pragma unroll
-    for (int b = 0; b < kNetBatch; ++b) y[b] = b < q.n ? ld4(pre + q.i * width + (q.net0 + b) * C + c) : f4zero();
-    if (ts) {
-        const float* s0 = ts + z[src[e_base + q.i]] * width + q.net0 * C + c;
-        const float* t0 = tt + z[tgt[e_base + q.i]] * width + q.net0 * C + c;
-#pragma unroll
-        for (int b = 0; b < kNetBatch; ++b)
-            if (b < q.n) y[b] = add4(y[b], add4(ld4(s0 + b * C), ld4(t0 + b * C)));
+    for (int b = 0; b < R; ++b) {
+        if (b > 0) {
+            const bool next = net[b - 1] + 1 == nets;
+            net[b] = next ? 0 : net[b - 1] + 1;
+            i += next ? 1 : 0;
+        }
+        y[b] = f4zero();
+        if (b >= n) continue;
+        y[b] = ld4(pre + (int64_t)(row0 + b) * C + c);
+        if (ts) {
+            const int64_t col = net[b] * C + c, width = (int64_t)nets * C;
+            y[b] = add4(y[b], add4(ld4(ts + z[src[i]] * width + col), ld4(tt + z[tgt[i]] * width + col)));
+        }
     }
 }
 
 __global__ void __launch_bounds__(256)
     radial_fwd_kernel(const float* __restrict__ pre, const float* __restrict__ ts, const float* __restrict__ tt,
                       const int32_t* __restrict__ z, const int32_t* __restrict__ src, const int32_t* __restrict__ tgt,
-                      const float* __restrict__ gamma, const float* __restrict__ beta, float eps, OutSplit out, int64_t out_ld,
-                      int out_net, float* __restrict__ stats, int64_t e_base, int64_t num_edges, int nets) {
+                      const float* __restrict__ gamma, const float* __restrict__ beta, float eps, OutSplit out, int64_t out_row,
+                      float* __restrict__ stats, uint32_t rows, int nets) {
     pdl_sync();
+    constexpr int R = kRadialFwdRows;
     out.s = 1.0f;
     const int lane = threadIdx.x & 31, c = lane * 4;
-    const int64_t items = radial_items(num_edges, nets), width = (int64_t)nets * C;
-    for (int64_t it = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); it < items; it += (int64_t)gridDim.x * 8) {
-        const RadialItem q = radial_item(it, nets);
-        float4 y[kNetBatch];
-        radial_rows(y, q, pre, ts, tt, z, src, tgt, e_base, width, c);
-        float mean[kNetBatch], rstd[kNetBatch];
+    for (uint32_t row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * R; row0 < rows; row0 += gridDim.x * 8 * R) {
+        const int n = min((uint32_t)R, rows - row0);
+        float4 y[R];
+        int net[R];
+        radial_rows(y, net, row0, n, pre, ts, tt, z, src, tgt, nets, c);
+        float mean[R], rstd[R];
 #pragma unroll
-        for (int b = 0; b < kNetBatch; ++b) mean[b] = warp_sum(hsum4(y[b])) * (1.0f / C);
+        for (int b = 0; b < R; ++b) mean[b] = hsum4(y[b]);
+        warp_sums(mean, lane);
 #pragma unroll
-        for (int b = 0; b < kNetBatch; ++b) {
+        for (int b = 0; b < R; ++b) {
+            mean[b] *= 1.0f / C;
             y[b] = make_float4(y[b].x - mean[b], y[b].y - mean[b], y[b].z - mean[b], y[b].w - mean[b]);
-            rstd[b] = rsqrtf(warp_sum(dot4(y[b], y[b])) * (1.0f / C) + eps);
+            rstd[b] = dot4(y[b], y[b]);
         }
+        warp_sums(rstd, lane);
 #pragma unroll
-        for (int b = 0; b < kNetBatch; ++b) {
-            if (b >= q.n) break;
-            const int col = (q.net0 + b) * C + c;
+        for (int b = 0; b < R; ++b) {
+            if (b >= n) break;
+            rstd[b] = rsqrtf(rstd[b] * (1.0f / C) + eps);
+            const int col = net[b] * C + c;
             const float4 gm = ld4(gamma + col), bt = ld4(beta + col), d = y[b];
             const float4 v = make_float4(fmaf(d.x * rstd[b], gm.x, bt.x), fmaf(d.y * rstd[b], gm.y, bt.y), fmaf(d.z * rstd[b], gm.z, bt.z),
                                          fmaf(d.w * rstd[b], gm.w, bt.w));
-            out.st(q.i * out_ld + (q.net0 + b) * out_net + c, make_float4(v.x * sigm(v.x), v.y * sigm(v.y), v.z * sigm(v.z), v.w * sigm(v.w)));
-            if (lane == 0) *reinterpret_cast<float2*>(stats + (q.i * nets + q.net0 + b) * 2) = make_float2(mean[b], rstd[b]);
+            out.st((row0 + b) * out_row + c, make_float4(v.x * sigm(v.x), v.y * sigm(v.y), v.z * sigm(v.z), v.w * sigm(v.w)));
+            if (lane == 0) *reinterpret_cast<float2*>(stats + (int64_t)(row0 + b) * 2) = make_float2(mean[b], rstd[b]);
         }
     }
 }
 
 // backward of the same; the planes are written with the smallest of the nets' gradient scales (block 0 leaves it at
 // scale_out), so that one contraction may sum over the nets
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)
     radial_bwd_kernel(const float* __restrict__ grad_out, const float* __restrict__ pre, const float* __restrict__ ts,
                       const float* __restrict__ tt, const int32_t* __restrict__ z, const int32_t* __restrict__ src,
                       const int32_t* __restrict__ tgt, const float* __restrict__ gamma, const float* __restrict__ beta,
-                      const float* __restrict__ stats, OutSplit out, int64_t out_ld, int out_net, const Scale* __restrict__ scales,
-                      int num_scales, float* __restrict__ scale_out, int64_t e_base, int64_t num_edges, int nets) {
+                      const float* __restrict__ stats, OutSplit out, int64_t out_row, const Scale* __restrict__ scales,
+                      int num_scales, float* __restrict__ scale_out, uint32_t rows, int nets) {
     pdl_sync();
+    constexpr int R = kRadialBwdRows;
     float s = scales[0].scale;
     for (int i = 1; i < num_scales; ++i) s = fminf(s, scales[i].scale);
     out.s = s;
     if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = s;
     const int lane = threadIdx.x & 31, c = lane * 4;
-    const int64_t items = radial_items(num_edges, nets), width = (int64_t)nets * C;
-    for (int64_t it = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); it < items; it += (int64_t)gridDim.x * 8) {
-        const RadialItem q = radial_item(it, nets);
-        float4 y[kNetBatch], go[kNetBatch];
-        float2 st[kNetBatch];
+    for (uint32_t row0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * R; row0 < rows; row0 += gridDim.x * 8 * R) {
+        const int n = min((uint32_t)R, rows - row0);
+        float4 y[R], go[R];
+        float2 st[R];
+        int net[R];
 #pragma unroll
-        for (int b = 0; b < kNetBatch; ++b) {
-            go[b] = b < q.n ? ld4(grad_out + q.i * width + (q.net0 + b) * C + c) : f4zero();
-            st[b] = b < q.n ? *reinterpret_cast<const float2*>(stats + (q.i * nets + q.net0 + b) * 2) : make_float2(0.f, 0.f);
+        for (int b = 0; b < R; ++b) {
+            go[b] = b < n ? ld4(grad_out + (int64_t)(row0 + b) * C + c) : f4zero();
+            st[b] = b < n ? *reinterpret_cast<const float2*>(stats + (int64_t)(row0 + b) * 2) : make_float2(0.f, 0.f);
         }
-        radial_rows(y, q, pre, ts, tt, z, src, tgt, e_base, width, c);
-        float s1[kNetBatch], s2[kNetBatch];
+        radial_rows(y, net, row0, n, pre, ts, tt, z, src, tgt, nets, c);
+        float sum[2 * R];
 #pragma unroll
-        for (int b = 0; b < kNetBatch; ++b) {
-            const int col = (q.net0 + (b < q.n ? b : 0)) * C + c;
+        for (int b = 0; b < R; ++b) {
+            const int col = net[b] * C + c;
             const float4 gm = ld4(gamma + col), bt = ld4(beta + col);
             const float4 xh = make_float4((y[b].x - st[b].x) * st[b].y, (y[b].y - st[b].x) * st[b].y, (y[b].z - st[b].x) * st[b].y, (y[b].w - st[b].x) * st[b].y);
             go[b] = make_float4(go[b].x * dsilu(fmaf(xh.x, gm.x, bt.x)) * gm.x, go[b].y * dsilu(fmaf(xh.y, gm.y, bt.y)) * gm.y,
                                 go[b].z * dsilu(fmaf(xh.z, gm.z, bt.z)) * gm.z, go[b].w * dsilu(fmaf(xh.w, gm.w, bt.w)) * gm.w);
             y[b] = xh;
-            s1[b] = warp_sum(hsum4(go[b])) * (1.0f / C);
-            s2[b] = warp_sum(dot4(go[b], xh)) * (1.0f / C);
+            sum[b] = hsum4(go[b]);
+            sum[R + b] = dot4(go[b], xh);
         }
+        warp_sums(sum, lane);
 #pragma unroll
-        for (int b = 0; b < kNetBatch; ++b) {
-            if (b >= q.n) break;
-            out.st(q.i * out_ld + (q.net0 + b) * out_net + c,
-                   make_float4(st[b].y * (go[b].x - s1[b] - y[b].x * s2[b]), st[b].y * (go[b].y - s1[b] - y[b].y * s2[b]),
-                               st[b].y * (go[b].z - s1[b] - y[b].z * s2[b]), st[b].y * (go[b].w - s1[b] - y[b].w * s2[b])));
+        for (int b = 0; b < R; ++b) {
+            if (b >= n) break;
+            const float s1 = sum[b] * (1.0f / C), s2 = sum[R + b] * (1.0f / C);
+            out.st((row0 + b) * out_row + c, make_float4(st[b].y * (go[b].x - s1 - y[b].x * s2), st[b].y * (go[b].y - s1 - y[b].y * s2),
+                                                         st[b].y * (go[b].z - s1 - y[b].z * s2), st[b].y * (go[b].w - s1 - y[b].w * s2)));
         }
     }
 }
