@@ -115,10 +115,9 @@ class _Calls:
             mods += [blk.norm_1, blk.norm_2, blk.atom_wise, blk.atom_wise.so3_linear_1, blk.atom_wise.so3_linear_2]
         self.hooks = [*_GLOBAL_HOOKS, *(getattr(m, n) for m in mods for n in _HOOK_DICTS)]
         self.attributes = [m.__dict__ for m in mods]
-        self.own = bb.__dict__
 
-    def watched(self) -> bool:
-        return any(map(len, self.hooks)) or any("forward" in d for d in self.attributes) or any(n in self.own for n in _METHODS)
+    def watched(self, bb) -> bool:  # the backbone is passed in: held here it would be a cycle through its own plan
+        return any(map(len, self.hooks)) or any("forward" in d for d in self.attributes) or any(n in bb.__dict__ for n in _METHODS)
 
 
 class _Weights:
@@ -271,7 +270,7 @@ class ModelPlan:
             if not cls.supported(bb) or not origin.params[0].is_cuda or any(p.dtype != torch.float32 for p in origin.params):
                 return None
             bb._step_plan = plan = cls(bb, origin)
-        plan.in_doubt = plan.calls.watched()
+        plan.in_doubt = plan.calls.watched(bb)
         return None if plan.in_doubt else plan
 
     def with_head(self, head) -> Optional["HeadPlan"]:

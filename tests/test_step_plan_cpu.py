@@ -3,7 +3,9 @@ copy of a used model carries."""
 
 import copy
 import ctypes
+import gc
 import pickle
+import weakref
 from types import SimpleNamespace as NS
 
 import pytest
@@ -128,7 +130,7 @@ def test_other_modules_are_not_for_the_native_path(bb):
 @pytest.mark.parametrize("kind", ["forward_hook", "pre_hook", "backward_hook", "global_hook", "own_forward", "own_method"])
 def test_hooks_send_an_evaluation_down_the_per_op_path(bb, kind):
     calls, undo = step._Calls(bb), None
-    assert not calls.watched()
+    assert not calls.watched(bb)
     mod = bb.blocks[2].atom_wise.so3_linear_2
     if kind == "forward_hook":
         undo = mod.register_forward_hook(lambda *a: None).remove
@@ -144,9 +146,9 @@ def test_hooks_send_an_evaluation_down_the_per_op_path(bb, kind):
     else:
         bb.csd_embedding = lambda *a: None
         undo = lambda: delattr(bb, "csd_embedding")  # noqa: E731
-    assert calls.watched()
+    assert calls.watched(bb)
     undo()
-    assert not calls.watched()
+    assert not calls.watched(bb)
 
 
 @pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
@@ -258,3 +260,16 @@ def test_a_given_graph_that_names_other_atoms_is_refused(bb):
         data.update({**good, key: wrong})
         with pytest.raises(ValueError, match="edge_index"):
             bb._graph(data)
+
+
+def test_a_model_and_its_plan_go_without_the_garbage_collector():
+    """Their device memory has to come back when the last reference goes, not at some later collection."""
+    gc.disable()
+    try:
+        other = eSCNMDBackboneB200(**dict(weights.UMA_S, num_layers=1))
+        other._step_plan = NS(origin=step._Origin(other), calls=step._Calls(other))
+        inner = weakref.ref(other.norm)
+        del other
+        assert inner() is None
+    finally:
+        gc.enable()
