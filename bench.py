@@ -151,8 +151,8 @@ def run_b200(args):
         os.environ.setdefault("NCCL_NVLS_ENABLE", "0")
         dist.init_process_group("nccl", device_id=dev)
     B.set_gemm_precision(args.precision)
-    if args.conv_variant is not None:
-        ops.CONV_VARIANT = args.conv_variant
+    if args.per_op:
+        B._GemmState.native = False
     if args.edge_source_sums:
         from fairchem_b200 import backbone as _bb
 
@@ -479,9 +479,8 @@ def main():
                     help="gather backward with the source half per edge plus a segmented sum instead of per-node sums (A/B measurement)")
     ap.add_argument("--generic-kernels", action="store_true",
                     help="route the lmax=2 model through the any-lmax edge-block kernels (A/B measurement)")
-    ap.add_argument("--conv-variant", type=int, default=None, choices=[-1, 0, 1, 2],
-                    help="accepted for earlier launch forms of the fused convolution kernel, which now has one; any value but -1 "
-                         "takes the per-op path (A/B measurement)")
+    ap.add_argument("--per-op", action="store_true",
+                    help="the per-op path (backbone.py) instead of the evaluation issued from native code (A/B measurement)")
     ap.add_argument("--profile-run", action="store_true",
                     help="for runs under a profiler: allows fewer than 3 warm-up steps; the printed number is not a bench value")
     args = ap.parse_args()

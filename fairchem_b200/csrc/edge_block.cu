@@ -27,7 +27,6 @@ __global__ void __launch_bounds__(kWarpsPerBlock* kWarp, 2)
     gather_rotate_fwd_kernel(const float* __restrict__ x, const int32_t* __restrict__ src, const int32_t* __restrict__ tgt,
                              const float* __restrict__ wig, const float* __restrict__ radial, Out out,
                              const float* __restrict__ scale_ptr, int64_t num_edges, int channels) {
-    pdl_sync();
     out.load_scale(scale_ptr);
     const int lane = threadIdx.x & 31;
     const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -708,9 +707,9 @@ int fcb200_gather_rotate_fwd(const float* x, const int32_t* src, const int32_t* 
     if (radial && !aligned16(radial)) return FCB200_EALIGN;
     if (num_edges == 0) return FCB200_OK;
     if (radial)
-        launch_pdl((gather_rotate_fwd_kernel<true, OutF32>), dim3(warp_grid(num_edges, kWarpsPerBlock)), dim3(kWarpsPerBlock * kWarp), 0, FCB_STREAM, x, src, tgt, wig, radial, OutF32{out}, nullptr, num_edges, channels);
+        gather_rotate_fwd_kernel<true, OutF32><<<FCB_LAUNCH(num_edges)>>>(x, src, tgt, wig, radial, OutF32{out}, nullptr, num_edges, channels);
     else
-        launch_pdl((gather_rotate_fwd_kernel<false, OutF32>), dim3(warp_grid(num_edges, kWarpsPerBlock)), dim3(kWarpsPerBlock * kWarp), 0, FCB_STREAM, x, src, tgt, wig, nullptr, OutF32{out}, nullptr, num_edges, channels);
+        gather_rotate_fwd_kernel<false, OutF32><<<FCB_LAUNCH(num_edges)>>>(x, src, tgt, wig, nullptr, OutF32{out}, nullptr, num_edges, channels);
     return launch_status();
 }
 
@@ -931,9 +930,9 @@ int fcb200_gather_rotate_fwd_h(const float* x, const int32_t* src, const int32_t
     if (num_edges == 0) return FCB200_OK;
     const OutSplit out{static_cast<__half*>(out_hi), static_cast<__half*>(out_lo), 1.0f};
     if (radial)
-        launch_pdl((gather_rotate_fwd_kernel<true, OutSplit>), dim3(warp_grid(num_edges, kWarpsPerBlock)), dim3(kWarpsPerBlock * kWarp), 0, FCB_STREAM, x, src, tgt, wig, radial, out, scale, num_edges, channels);
+        gather_rotate_fwd_kernel<true, OutSplit><<<FCB_LAUNCH(num_edges)>>>(x, src, tgt, wig, radial, out, scale, num_edges, channels);
     else
-        launch_pdl((gather_rotate_fwd_kernel<false, OutSplit>), dim3(warp_grid(num_edges, kWarpsPerBlock)), dim3(kWarpsPerBlock * kWarp), 0, FCB_STREAM, x, src, tgt, wig, nullptr, out, scale, num_edges, channels);
+        gather_rotate_fwd_kernel<false, OutSplit><<<FCB_LAUNCH(num_edges)>>>(x, src, tgt, wig, nullptr, out, scale, num_edges, channels);
     return launch_status();
 }
 

@@ -59,7 +59,6 @@ __global__ void __launch_bounds__(kLxWarps* kWarp)
     lx_gather_rotate_fwd_kernel(const float* __restrict__ x, const int32_t* __restrict__ src, const int32_t* __restrict__ tgt,
                                 const float* __restrict__ wig, const float* __restrict__ radial, Out out,
                                 const float* __restrict__ scale_ptr, int64_t num_edges, int channels) {
-    pdl_sync();
     using S = Shape<LMAX>;
     out.load_scale(scale_ptr);
     __shared__ float sw[kLxWarps][kWigSlot];

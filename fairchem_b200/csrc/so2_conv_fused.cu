@@ -40,8 +40,7 @@ namespace fused {
 using namespace f16;
 
 enum Mode : int32_t {
-    kPlain = 0,     // float32 tile -> y[:, out_col ...]
-    kGateRaw = 1,   // (unused: gate scalars are kPlain tiles with kGateSrc)
+    kPlain = 0,     // float32 tile -> y[:, out_col ...]; 1 is not assigned
     kSilu = 2,      // planes[:, out_col ...] = split(v * sigmoid(v));                       keep: y[:, y_col ...] = v
     kGated = 3,     // planes[:, out_col ...] = split(v * sigmoid(gate));                    keep: y[:, y_col ...] = v
     kSiluBwd = 4,   // planes[:, out_col ...] = split(v * d/dy silu(y[:, y_col ...]))
@@ -789,7 +788,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         if (t.w < 0 || t.w > 2 || !w_hi[t.w] || !w_lo[t.w]) return FCB200_EINVAL;
         if (t.k <= 0 || t.k % 32 || t.k > w_cols[t.w] || t.a_col < 0 || t.a_col % 8 || t.a_col + t.k > a_cols) return FCB200_EINVAL;
         if (t.w_row % BN || t.w_row >= w_rows[t.w]) return FCB200_EINVAL;
-        if (t.mode > kGatedBwd || t.mode == kGateRaw || t.out_col % 8) return FCB200_EINVAL;
+        if (t.mode > kGatedBwd || t.mode == 1 || t.out_col % 8) return FCB200_EINVAL;
         const bool split = t.mode >= kSilu;
         if (w_rows[t.w] - t.w_row < BN && (split || w_rows[t.w] % 4 || t.out_col + (w_rows[t.w] - t.w_row) != y_cols)) return FCB200_EINVAL;
         if (split && (!o_hi || t.out_col + BN > o_cols)) return FCB200_EINVAL;

@@ -655,11 +655,9 @@ def gemm_f16x2_presplit_(a_hi: Tensor, a_lo: Tensor, w_hi: Tensor, w_lo: Tensor,
 
 
 # epilogue modes and flags of so2_conv_fused_ (csrc/so2_conv_fused.cu)
-CONV_PLAIN, CONV_GATE_RAW, CONV_SILU, CONV_GATED, CONV_SILU_BWD, CONV_GATED_BWD = range(6)
+CONV_PLAIN, CONV_SILU, CONV_GATED, CONV_SILU_BWD, CONV_GATED_BWD = 0, 2, 3, 4, 5
 CONV_FIRST, CONV_LAST, CONV_KEEP = 1, 2, 4
 CONV_MAX_TILES = 40
-# Accepted for earlier launch forms (0, 1, 2; -1 = none); there is one form now.
-CONV_VARIANT = -1
 # How a launch's tile list is cut into work items: 0 the choice of the library, 1 natural groups, 2 fine (csrc/so2_conv_fused.cu)
 CONV_GROUPING = 0
 
@@ -704,9 +702,7 @@ def so2_conv_fused_(a_hi: Tensor, a_lo: Tensor, w_hi: List[Tensor], w_lo: List[T
     scales = (c_float * 3)(*(list(w_scale) + [1.0] * (3 - nw)))
     biases = (c_void_p * 3)(None if bias0 is None else bias0.data_ptr(), None, None)
     tl = (c_int32 * len(tiles))(*tiles)
-    if variant < 0:
-        variant = max(CONV_VARIANT, 0)
-    variant += 16 * CONV_GROUPING
+    variant = max(variant, 0) + 16 * CONV_GROUPING
     flops = 2 * m * 128 * sum(tiles[9 * i + 1] for i in range(nt))
     nbytes = 4 * m * (a_hi.shape[1] + 128 * nt)
     _launch("so2_conv_fused" + label, "fcb200_so2_conv_fused",

@@ -243,7 +243,7 @@ class ModelPlan:
     def wanted(bb) -> bool:
         from .backbone import _GemmState as mode
 
-        return (mode.precision == 2 and mode.fused_conv and mode.native and ops.CONV_VARIANT == -1 and bb.keep_level is None
+        return (mode.precision == 2 and mode.fused_conv and mode.native and bb.keep_level is None
                 and not ops.generic_kernels())
 
     @classmethod

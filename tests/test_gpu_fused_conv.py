@@ -27,18 +27,18 @@ def _unplane(p, scale=1.0):
     return (p[0].float() + p[1].float() / 2048.0) / scale
 
 
-@pytest.fixture(params=[0, 1, 2, -1], ids=["single_cta", "cta_pairs", "single_cta_k64", "per_launch_choice"])
-def variant(request, ops):
-    """The launch forms of the fused kernel: one CTA per 128 edges with 32- or 64-deep ring stages, and CTA pairs
-    (cta_group::2) per 256 edges."""
-    saved = ops.CONV_VARIANT
-    ops.CONV_VARIANT = request.param
+@pytest.fixture(params=[0, 1, 2], ids=["per_launch_choice", "natural_groups", "row_by_row"])
+def grouping(request, ops):
+    """How the tile list of a launch is cut into work items (forward; row by row, the gate is computed again for each).  A
+    backward launch cuts its rows one by one only with the scratch block that the whole-model evaluation gives it:
+    tests/test_gpu_step.py has systems on both sides of that rule."""
+    ops.CONV_GROUPING = request.param
     yield request.param
-    ops.CONV_VARIANT = saved
+    ops.CONV_GROUPING = 0
 
 
 @pytest.mark.parametrize("lmax,e", [(2, 77), (2, 1000), (4, 300), (2, 40000)])
-def test_fused_convolutions_match_the_separate_kernels(ops, variant, lmax, e):
+def test_fused_convolutions_match_the_separate_kernels(ops, grouping, lmax, e):
     from fairchem_b200 import backbone as B
 
     torch.manual_seed(lmax)
@@ -83,7 +83,7 @@ def test_fused_convolutions_match_the_separate_kernels(ops, variant, lmax, e):
     torch.testing.assert_close(gm, gm_ref, rtol=1e-5, atol=1e-5 * float(gm_ref.abs().max()))
 
 
-def test_edge_block_is_the_same_with_and_without_the_fused_launches(ops, variant):
+def test_edge_block_is_the_same_with_and_without_the_fused_launches(ops, grouping):
     """Energy and forces of a small periodic system with the fused convolution launches on and off."""
     from fairchem_b200 import backbone as B
     from fairchem_b200 import synthetic, weights

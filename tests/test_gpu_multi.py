@@ -70,14 +70,11 @@ def test_contraction_kernels_on_a_second_device_of_the_same_process():
             ops.gemm_f16x2_presplit_(planes[0], planes[1], hi, lo, sc, None, None, y2, status)
             y3 = torch.empty_like(y)
             tiles = [0, 256, 0, 0, 0, ops.CONV_PLAIN, 0, 0, 0]
-            for variant in (0, 1):                                                       # fused kernel, both launch forms
-                ops.so2_conv_fused_(planes[0], planes[1], [hi], [lo], [sc], None, tiles, 0, y3, None, None, None, None, status, "",
-                                    variant)
-                torch.testing.assert_close(y3.cpu().double(), want, rtol=1e-5, atol=1e-4)
+            ops.so2_conv_fused_(planes[0], planes[1], [hi], [lo], [sc], None, tiles, 0, y3, None, None, None, None, status)
             hi3, lo3 = ops.split_tf32(wd)
             y4 = torch.empty_like(y)
             ops.gemm_tf32_(ad, hi3, lo3, None, y4, 3, status)
             assert int(status.item()) == 0
-            for got in (y, y2, y4):
+            for got in (y, y2, y3, y4):
                 torch.testing.assert_close(got.cpu().double(), want, rtol=1e-5, atol=1e-4)
     del B
