@@ -34,10 +34,13 @@ def _rel(a, b):
 
 @pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
 @pytest.mark.parametrize("name", list(CASES))
-def test_native_evaluation_matches_per_op_path(cfg, name):
+def test_native_evaluation_matches_per_op_path(cfg, name, monkeypatch):
     from fairchem_b200 import backbone as B
-    from fairchem_b200 import synthetic
+    from fairchem_b200 import step, synthetic
 
+    general = []
+    from_edges = step.StepGraph.from_edges
+    monkeypatch.setattr(step.StepGraph, "from_edges", lambda self, *a: general.append(1) or from_edges(self, *a))
     make, kw = CASES[name]
     bb, head = _model(B, cfg, **kw)
     data = make(synthetic).to("cuda")
@@ -51,6 +54,7 @@ def test_native_evaluation_matches_per_op_path(cfg, name):
             out[native] = head(d, emb)
         finally:
             B._GemmState.native = True
+    assert len(general) == (name == "one_atom")  # the evaluation's own graph, but for the atom without neighbours
     assert set(out[True]) == set(out[False])
     # energies are sums of per-atom terms of order 0.1 that may cancel
     e, ref = out[True]["energy"], out[False]["energy"]
