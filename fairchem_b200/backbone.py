@@ -1480,7 +1480,7 @@ class MLP_EFS_HeadB200(step.HoldsPlan, nn.Module):
     def _forward_native(self, data, emb):
         """Energy and forces straight from the evaluation that made ``emb`` (no autograd graph in between)."""
         run, x = emb.get("step", None), emb["node_embedding"]
-        if run is None or run.keep is None or x is not run.embedding() or x._version != 0:
+        if run is None or run.keep is None or x is not run.embedding() or not (x.is_inference() or x._version == 0):
             return None
         if x._backward_hooks or x.retains_grad or run.leaf._backward_hooks:  # autograd has more to do than the forces
             return None

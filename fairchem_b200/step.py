@@ -393,7 +393,8 @@ class BackboneStep:
         return torch.empty(nbytes, dtype=torch.uint8, device=self.device)
 
     def forward(self) -> torch.Tensor:
-        self.inputs = [(t, t._version) for t in self.watched]
+        if self.ev.want_grad:  # tensors of inference mode have no versions, and no second backward pass either
+            self.inputs = [(t, t._version) for t in self.watched if not t.is_inference()]
         return self._forward()
 
     def _launch(self, name: str, *plans):

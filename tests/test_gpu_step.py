@@ -431,3 +431,21 @@ def test_kept_list_of_another_split_is_not_used():
         bb.neighbor_list = kept
         assert _rel(got["forces"], ref["forces"]) < 1e-6
     assert (kept.searches, kept.refreshes) == (3, 0)
+
+
+@pytest.mark.parametrize("forces", [False, True])
+@pytest.mark.parametrize("mode", ["inference_mode", "no_grad"])
+def test_evaluation_inside_inference_mode(forces, mode):
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, "UMA_S", regress_forces=forces)
+    data = synthetic.molecule_batch(2, 6, 9, seed=8).to("cuda")
+    d = data.clone()
+    ref = head(d, bb(d))
+    with getattr(torch, mode)():
+        d = data.clone() if not (forces and mode == "inference_mode") else data
+        out = head(d, bb(d))
+    assert set(out) == set(ref)
+    for k in ref:
+        assert _rel(out[k], ref[k]) < 1e-6
