@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(128)
 }
 
 // Memory-bound: 100 000 nodes of lmax 2, 4.2 -> 6.6 TB/s, the residual's gradient and the largest value in the same pass.
+// lmax 4 holds 25 rows twice in 255 registers and spills 40 bytes; 20 000 nodes 5.9 TB/s.
 // grad_x = residual + d norm; g has all rows, or (ROW0) only row 0 of every node, [N, C]
 template <int LMAX, bool ROW0>
 __global__ void __launch_bounds__(128)

@@ -28,10 +28,12 @@
 // accumulator block in that tile from a row per lane to whole lines per instruction and does everything else on registers
 // and global memory directly (the forms with TMA-fed input and output tiles needed 64-96 KiB and two or five operand
 // stages of half the depth).
-// us per launch at M = 131 072, lmax 2, four 32-deep or two 64-deep stages with TMA epilogues -> this: conv 1 + gate
-// 1219 -> 985, conv 2 499 -> 377, its backward + gate 780 -> 655, conv 1 backward 1050 -> 890, radial output layer
-// 263 -> 243.  Still above the main loop's own time: the epilogues' instruction stream (the gate's backward: 1500 per
-// 32 x 32 chunk) and 64-byte plane stores share the SM with it.
+// us per launch by itself at M = 131 072, lmax 2, four 32-deep or two 64-deep stages with TMA epilogues -> this: conv 1 +
+// gate 1219 -> 985, conv 2 499 -> 377, its backward + gate 780 -> 655, conv 1 backward 1050 -> 890, radial output layer
+// 263 -> 243.  Among the other launches of a 100 000-atom evaluation (129 000 edges each): 1184 -> 1003, 457 -> 395, 642 ->
+// 652 (no gain: its epilogue, not its loop, is what there is to wait for), 1011 -> 891, 220 -> 216.  Still above the main
+// loop's own time: the epilogues' instruction stream (the gate's backward: 1500 per 32 x 32 chunk) and 64-byte plane stores
+// share the SM with it.
 #include "gemm_f16_common.cuh"
 
 namespace fcb200 {

@@ -1,4 +1,4 @@
-// Pieces shared by the kernels of the whole-model evaluation (edge_step.cu, node_step.cu, graph_step.cu) and the host
+// Pieces shared by the kernels of the whole-model evaluation (edge_step.cuh, node_step.cuh, graph_step.cu) and the host
 // code that issues them (model_step.cu).
 #pragma once
 
