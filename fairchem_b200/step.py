@@ -59,7 +59,7 @@ class EvalStruct(Structure):
 _VERSION = operator.attrgetter("_version")
 _EPS = operator.attrgetter("eps")
 _SCALARS = operator.attrgetter("lmax", "num_distance_basis", "max_num_elements", "cutoff", "rescale_factor", "sphere_channels",
-                               "hidden_channels", "edge_channels")
+                               "hidden_channels", "edge_channels", "charge_embedding.offset", "spin_embedding.offset")
 
 
 def _versions(params) -> list:
@@ -233,6 +233,7 @@ class ModelPlan:
         from .backbone import eSCNMDBackboneB200 as plain
 
         if not (bb.sphere_channels == C and bb.hidden_channels == C and bb.edge_channels == C and bb.num_distance_basis % 32 == 0
+                and (bb.charge_embedding.offset, bb.spin_embedding.offset) == (100, 0)  # as csrc/node_step.cuh indexes the tables
                 and 1 <= len(bb.blocks) < 40 and all(getattr(type(bb), n) is getattr(plain, n) for n in _METHODS)):
             return False
         nets = _radial_nets(bb)

@@ -52,6 +52,7 @@ CHANGES = {
     "load_state_dict_assign": _assign_state, "parameter": _new_parameter, "module": _new_module, "in_place": _in_place, "storage": _moved_storage,
     "block_order": _swap, "fewer_blocks": lambda bb: bb.blocks.__delitem__(3),
     "cutoff": lambda bb: setattr(bb, "cutoff", 5.0), "rescale": lambda bb: setattr(bb, "rescale_factor", 4.0),
+    "charge_offset": lambda bb: setattr(bb.charge_embedding, "offset", 90),
     "norm_eps": lambda bb: setattr(bb.blocks[2].norm_2, "eps", 1e-4),
     "radial_eps": lambda bb: setattr(bb.edge_degree_embedding.rad_func.net[4], "eps", 1e-3),
 }
@@ -115,7 +116,7 @@ def _other_shape(bb):
 
 def test_other_modules_are_not_for_the_native_path(bb):
     assert step.ModelPlan.supported(bb)
-    for change in (_foreign_module, _other_shape):
+    for change in (_foreign_module, _other_shape, CHANGES["charge_offset"]):
         other = copy.deepcopy(bb)
         change(other)
         assert step.ModelPlan.supported(bb) and not step.ModelPlan.supported(other)
