@@ -34,51 +34,21 @@
 // 652 (no gain: its epilogue, not its loop, is what there is to wait for), 1011 -> 891, 220 -> 216.  Still above the main
 // loop's own time: the epilogues' instruction stream (the gate's backward: 1500 per 32 x 32 chunk) and 64-byte plane stores
 // share the SM with it.
-#include "gemm_f16_common.cuh"
+#include "so2_conv.cuh"
 
 namespace fcb200 {
 namespace fused {
 
-using namespace f16;
-
-enum Mode : int32_t {
-    kPlain = 0,     // float32 tile -> y[:, out_col ...]; 1 is not assigned
-    kSilu = 2,      // planes[:, out_col ...] = split(v * sigmoid(v));                       keep: y[:, y_col ...] = v
-    kGated = 3,     // planes[:, out_col ...] = split(v * sigmoid(gate));                    keep: y[:, y_col ...] = v
-    kSiluBwd = 4,   // planes[:, out_col ...] = split(v * d/dy silu(y[:, y_col ...]))
-    kGatedBwd = 5,  // planes[:, out_col ...] = split(v * sigmoid(gate)); gate gradient summed over consecutive tiles
-};
-// kGateSilu: the gate is sigmoid(silu(g)), the scalar MLP of the node-wise feed-forward, instead of sigmoid(g).
-// kGateSrc (set on the host): a gate tile of the rows that follow.  kSolo (host): a backward gated row on its own; its raw
-// value goes to Params::raw and gate_sum_kernel adds up the rows of a degree.
-enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8, kGateSrc = 16, kSolo = 32 };
-
-struct Tile {
-    int16_t a_col;     // first input column of this tile's K range
-    int16_t k;         // K extent (multiple of 32)
-    int16_t w;         // weight matrix 0..2
-    int16_t w_row;     // first output row of the weight matrix (multiple of 128)
-    int16_t out_col;   // where the result goes (column of y for float32 modes, of the planes for split modes)
-    int16_t mode;
-    int16_t y_col;     // column of y holding this row's raw value (kSilu/kGated keep, kSiluBwd/kGatedBwd read)
-    int16_t gate_col;  // column of y (and of the gradient planes) of the gate scalars of this row's degree
-    int16_t flags;
-    int16_t raw_col;   // kSolo: column of Params::raw
-};
-constexpr int kMaxTiles = 40;   // tiles a caller may list; lmax 4: 19 rows x 2C = 38 column tiles in the conv-1 backward
-constexpr int kMaxPlan = 80;    // tiles of a plan: a gate tile may be repeated for each of its rows
 // A work item is one row tile times one group of consecutive tiles [begin[g], begin[g + 1]): what has to pass through one
 // CTA in order.  See group_tiles() on the host.
 struct Plan {
-    int32_t groups;
+    Order order;
     int16_t begin[kMaxPlan + 1];
     Tile t[kMaxPlan];
 };
 
-constexpr int KB = 64;                               // k extent of a ring stage: 128-byte rows, 128-byte swizzle
 constexpr int kStages = 3;
-constexpr int kPart = BM * KB * 2;                   // A_hi | A_lo | W_hi | W_lo, 16 KiB each
-constexpr int kStageBytes = 4 * kPart;
+constexpr int kStageBytes = 4 * kPart;               // A_hi | A_lo | W_hi | W_lo
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 128 + 32 * kEpiWarps;       // warp 0 TMA, warp 1 MMA, 2-3 idle, warps 4-11 epilogue
 // Registers: launched with 168 a thread (12 warps on 4 schedulers); the first warpgroup gives up what the two epilogue
@@ -88,73 +58,6 @@ static_assert(128 * kIdleRegs + 32 * kEpiWarps * kEpiRegs <= kThreads * 168, "re
 constexpr int kAccCols = 2 * BN, kTmemCols = 2 * kAccCols;
 constexpr int kSmemBytes = kStages * kStageBytes + kEpiWarps * 4096 + 1024 + 256;
 
-// K-major, 128-byte swizzle: rows at a 128 B pitch, 8-row groups 1024 B apart
-__device__ __forceinline__ uint64_t smem_desc128(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;  // SWIZZLE_128B
-    return d;
-}
-
-struct Params {
-    const float* bias[3];
-    float w_scale[3];
-    float* y;          // raw conv-1 output / float32 output
-    int32_t ldy, y_cols;
-    __half *o_hi, *o_lo;
-    int32_t ldo;
-    const float* a_scale;  // power of two the A planes were written with (null = 1)
-    const float* o_scale;  // power of two the output planes are written with (null = 1)
-    int64_t m_total;
-    int32_t* status;
-    float* raw;        // [m, raw_ld] values of the kSolo tiles
-    int32_t raw_ld;
-};
-
-// 1 / (1 + e^-v) on the special-function unit (ex2.approx, rcp.approx): relative error ~2^-22, a few instructions
-// instead of the ~20 of expf and an IEEE division -- the epilogue evaluates it for every output element
-__device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
-
-// Two float32 in a register pair; the packed instructions halve the epilogue's multiply and add count.
-typedef uint64_t f32x2;
-__device__ __forceinline__ f32x2 pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-template <class F> __device__ __forceinline__ f32x2 map2(f32x2 v, F f) {
-    float a, b;
-    unpack(v, a, b);
-    return pack(f(a), f(b));
-}
-
-// Two values -> packed halves hi and lo.  `top`: largest |hi| so far, NaN-propagating: an overflowed or invalid value
-// becomes inf or NaN as a half, so one packed maximum per pair replaces range checks on the float32 values.
-__device__ __forceinline__ void split2(f32x2 v, uint32_t& hi, uint32_t& lo, __half2& top) {
-    float a, b;
-    unpack(v, a, b);
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 hf = __half22float2(h);
-    unpack(mul2(fma2(pack(hf.x, hf.y), pack(-1.f, -1.f), v), pack(kLoScale, kLoScale)), a, b);
-    const __half2 l = __floats2half2_rn(a, b);
-    top = __hmax2_nan(top, __habs2(h));
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
 __device__ __forceinline__ void store_split(__half* hi, __half* lo, int off, f32x2 o0, f32x2 o1, bool in, __half2& top) {
     uint2 h, l;
     split2(o0, h.x, l.x, top);
@@ -171,23 +74,12 @@ __device__ __forceinline__ void load_pair(const float* p, f32x2& a, f32x2& b) {
     asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
 }
 
-#define FCB_TMEM_LD16(r, taddr)                                                                                           \
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "                                                                \
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"                         \
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),        \
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])   \
-                 : "r"(taddr)                                                                                             \
-                 : "memory")
-
-// What the epilogue of a launch has to be able to do; fixes how many registers it keeps between tiles.
-enum Kind { kPlainKind = 0, kForwardKind = 1, kBackwardKind = 2 };
-
 // Epilogue warps 4..11: warp w reads TMEM lanes [32 (w % 4), +32) -- one accumulator row per lane -- and takes the columns
 // [64 h, 64 h + 64) of every tile, h = (w - 4) / 4, in two chunks of 32.  A chunk is turned in the warp's shared tile to
 // "lane = row 4 i + lane / 8, columns 4 (lane % 8)": 128-byte lines per row for every global access, and the same
 // (row, column) in the same thread for every tile, so gates and gate-gradient sums stay in registers.
 template <int KIND>
-__device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, int64_t items, uint32_t tmem_base, uint32_t tile,
+__device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, uint32_t tmem_base, uint32_t tile,
                                          uint32_t tfull0, uint32_t tempty0, volatile int* abort_flag, volatile int* range_flag) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = warp & 3, half = (warp - 4) >> 2;
@@ -206,9 +98,9 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
     auto put = [](uint32_t at, f32x2 a, f32x2 b) { asm volatile("st.shared.v2.b64 [%0], {%1,%2};" ::"r"(at), "l"(a), "l"(b) : "memory"); };
     auto get = [](uint32_t at, f32x2& a, f32x2& b) { asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "r"(at) : "memory"); };
     // y lines of a backward tile on their way to L2 one tile early (lane = row; a warp's 64 columns are two lines)
-    auto prefetch = [&](int64_t item2, int ti2) {
+    auto prefetch = [&](int64_t mt2, int ti2) {
         if constexpr (KIND == kBackwardKind) {
-            const int64_t row = item2 / plan.groups * BM + q * 32 + lane;
+            const int64_t row = mt2 * BM + q * 32 + lane;
             if (row < prm.m_total) {
                 const Tile& t2 = plan.t[ti2];
                 const float* p = prm.y + row * prm.ldy + t2.y_col + half * 64;
@@ -223,10 +115,9 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
         }
     };
     uint32_t r[kAhead ? 32 : 1], c[kAhead ? 32 : 1];
-    int64_t tcount = 0;
-    for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
-        const int64_t mt = item / plan.groups;
-        const int g = (int)(item - mt * plan.groups);
+    int64_t tcount = 0, mt;
+    int g;
+    for (int64_t n = 0; plan.order.item(n, gridDim.x, blockIdx.x, mt, g); ++n) {
         const int64_t row0 = mt * BM + q * 32;
         const int live = (int)(prm.m_total - row0 < 32 ? prm.m_total - row0 : 32);  // rows of this warp inside the matrix
         // 32 rows of at most 32 767 columns: offsets inside a warp's block fit 32 bits
@@ -252,8 +143,10 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, in
             const int buf = (int)(tcount & 1);
             const uint32_t use = (uint32_t)((tcount >> 1) & 1);
             if constexpr (KIND == kBackwardKind) {
-                if (ti + 1 < plan.begin[g + 1]) prefetch(item, ti + 1);
-                else if (item + gridDim.x < items) prefetch(item + gridDim.x, plan.begin[(int)((item + gridDim.x) % plan.groups)]);
+                int64_t mt2;
+                int g2;
+                if (ti + 1 < plan.begin[g + 1]) prefetch(mt, ti + 1);
+                else if (plan.order.item(n + 1, gridDim.x, blockIdx.x, mt2, g2)) prefetch(mt2, plan.begin[g2]);
             }
             const bool gate_silu = (t.flags & kGateSilu) != 0;
             const bool solo = (t.flags & kSolo) != 0;
@@ -462,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                           const __grid_constant__ CUtensorMap map_whi0, const __grid_constant__ CUtensorMap map_wlo0,
                           const __grid_constant__ CUtensorMap map_whi1, const __grid_constant__ CUtensorMap map_wlo1,
                           const __grid_constant__ CUtensorMap map_whi2, const __grid_constant__ CUtensorMap map_wlo2,
-                          const __grid_constant__ Plan plan, const __grid_constant__ Params prm, int64_t items) {
+                          const __grid_constant__ Plan plan, const __grid_constant__ Params prm) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t epi_base = base + kStages * kStageBytes;
@@ -509,7 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (warp >= 4) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
-        epilogue<KIND>(plan, prm, items, tmem_base, epi_base + (uint32_t)((warp - 4) * 4096), tfull_bar(0), tempty_bar(0), abort_flag, range_flag);
+        epilogue<KIND>(plan, prm, tmem_base, epi_base + (uint32_t)((warp - 4) * 4096), tfull_bar(0), tempty_bar(0), abort_flag, range_flag);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIdleRegs));
         if (warp == 0 && lane == 0) {
@@ -518,9 +411,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             // an A tile is fetched again for each of the output tiles of its m-block, the weights by every CTA: keep
             // both in L2 ahead of the streamed outputs
             const uint64_t keep = l2_policy_evict_last();
-            for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
-                const int64_t mt = item / plan.groups;
-                const int g = (int)(item - mt * plan.groups);
+            int64_t mt;
+            int g;
+            for (int64_t n = 0; ok && plan.order.item(n, gridDim.x, blockIdx.x, mt, g); ++n) {
                 for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti) {
                     const Tile& t = plan.t[ti];
                     const CUtensorMap* whi = t.w == 0 ? &map_whi0 : (t.w == 1 ? &map_whi1 : &map_whi2);
@@ -541,10 +434,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         if (warp == 1 && lane == 0) {
-            int64_t it = 0, tcount = 0;
+            int64_t it = 0, tcount = 0, mt;
+            int g;
             bool ok = true;
-            for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
-                const int g = (int)(item % plan.groups);
+            for (int64_t n = 0; ok && plan.order.item(n, gridDim.x, blockIdx.x, mt, g); ++n) {
                 for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti, ++tcount) {
                     const int k = plan.t[ti].k, num_kb = (k + KB - 1) / KB;
                     const int buf = (int)(tcount & 1);
@@ -653,7 +546,8 @@ static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t col
 //            or their gate-gradient sum (backward)
 //   fine     gated rows one by one: forward each after its own copy of the gate tile (the gate is computed again), backward
 //            with the gate-gradient sums left to a second kernel
-enum Grouping { kAuto = 0, kNatural = 1, kFine = 2 };
+//   pair     natural groups on CTA pairs, tiles that read the same columns side by side (so2_conv_pair.cu)
+enum Grouping { kAuto = 0, kNatural = 1, kFine = 2, kPair = 3 };
 
 struct Groups {
     int n = 0;           // tiles
@@ -664,8 +558,9 @@ struct Groups {
     bool ok = true;
 };
 
-// a tile's fixed share (epilogue, ring start-up) in units of its K extent, from launches of one row tile
-constexpr int kTileCost = 192;
+// a tile's fixed share (epilogue, ring start-up) in units of its K extent, from launches of one row tile; of a tile on a pair
+// of CTAs, whose K extent counts 0.8 where it has a partner (see the choice of the form)
+constexpr int kTileCost = 192, kPairTileCost = 230;
 
 static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
     Groups g;
@@ -735,20 +630,103 @@ static bool split_sums(Tile* t, int n, GateSums& g) {
     return g.degrees > 0;
 }
 
-// longest CTA of a static round-robin over rows x groups items, in units of K
-static int64_t makespan(const Groups& g, int64_t rows, int ctas) {
-    const int64_t items = rows * g.groups;
+// Natural groups for CTA pairs: tiles of a group two by two where they follow one another and read the same columns; groups
+// of a single tile that no order binds to others are joined the same way.
+struct PairGroups {
+    PairPlan plan{};
+    int cost[kMaxTiles] = {};
+};
+static PairGroups pair_tiles(const Tile* t, const Groups& g) {
+    PairGroups out;
+    PairPlan& p = out.plan;
+    int n = 0, groups = 0;
+    auto joins = [&](const PairTile& a, const Tile& b) { return a.n == 1 && a.a_col == b.a_col && a.k == b.k && a.w == b.w; };
+    bool open = false;  // the last group is one lone tile
+    for (int i = 0; i < g.groups; ++i) {
+        const bool lone = g.begin[i + 1] - g.begin[i] == 1;
+        if (!(lone && open && joins(p.t[n - 1], t[g.tile[g.begin[i]]]))) p.begin[groups++] = (int16_t)n;
+        for (int j = g.begin[i]; j < g.begin[i + 1]; ++j) {
+            const Tile& s = t[g.tile[j]];
+            if (n == p.begin[groups - 1] || !joins(p.t[n - 1], s)) {
+                p.t[n] = PairTile{};
+                p.t[n].a_col = s.a_col, p.t[n].k = s.k, p.t[n].w = s.w;
+                ++n;
+            }
+            PairTile& d = p.t[n - 1];
+            d.w_row[d.n] = s.w_row, d.out_col[d.n] = s.out_col, d.mode[d.n] = s.mode, d.y_col[d.n] = s.y_col, d.flags[d.n] = s.flags;
+            ++d.n;
+        }
+        open = lone && n - p.begin[groups - 1] == 1 && p.t[n - 1].n == 1;
+        p.begin[groups] = (int16_t)n;
+    }
+    p.order.groups = groups;
+    for (int i = 0; i < groups; ++i)
+        for (int j = p.begin[i]; j < p.begin[i + 1]; ++j) out.cost[i] += p.t[j].n == 2 ? 2 * (8 * p.t[j].k / 10 + kPairTileCost) : p.t[j].k + kPairTileCost;
+    return out;
+}
+
+// longest of `units` CTAs or pairs, in units of K
+static int64_t makespan(const Order& order, const int* cost, int units) {
+    const int64_t items = order.rows * order.groups;
     int64_t total = 0, most = 0;
-    for (int i = 0; i < g.groups; ++i) total += g.cost[i], most = g.cost[i] > most ? g.cost[i] : most;
-    if (items > 16LL * ctas * g.groups) return rows * total / ctas + most;
-    int64_t worst = 0;
-    for (int c = 0; c < ctas && c < items; ++c) {
+    for (int i = 0; i < order.groups; ++i) total += cost[i], most = cost[i] > most ? cost[i] : most;
+    if (items > 16LL * units * order.groups) return order.rows * total / units + most;
+    int64_t worst = 0, row;
+    int g;
+    for (int c = 0; c < units && c < items; ++c) {
         int64_t sum = 0;
-        for (int64_t i = c; i < items; i += ctas) sum += g.cost[i % g.groups];
+        for (int64_t n = 0; order.item(n, units, c, row, g); ++n) sum += cost[g];
         worst = sum > worst ? sum : worst;
     }
     return worst;
 }
+
+// The order of a launch's items and its makespan.  perm: the groups by falling cost.  Group by group an A tile leaves L2
+// between its groups when there are many rows, so that has to gain more than the extra reads cost (first convolution, lmax 2,
+// us row by row / group by group: 7 680 rows 90 / 68, 20 580 rows 188 / 182, 40 000 rows 332 / 353).
+static int64_t choose_order(Order& order, int* cost, int* perm, int units) {
+    for (int i = 0; i < order.groups; ++i) perm[i] = i;
+    const int64_t by_row = makespan(order, cost, units), items = order.rows * order.groups;
+    if (items > 8LL * units || items <= units) return by_row;
+    int sorted[kMaxPlan], at[kMaxPlan];
+    for (int i = 0; i < order.groups; ++i) {
+        int j = i;
+        for (; j > 0 && cost[i] > sorted[j - 1]; --j) sorted[j] = sorted[j - 1], at[j] = at[j - 1];
+        sorted[j] = cost[i], at[j] = i;
+    }
+    Order snake = order;
+    snake.snake = 1;
+    const int64_t by_group = makespan(snake, sorted, units);
+    if (100 * by_group >= 96 * by_row) return by_row;
+    order = snake;
+    for (int i = 0; i < order.groups; ++i) cost[i] = sorted[i], perm[i] = at[i];
+    return by_group;
+}
+static PairPlan reordered(const PairPlan& p, const int* perm) {
+    PairPlan q = p;
+    int n = 0;
+    for (int g = 0; g < p.order.groups; ++g) {
+        for (int i = p.begin[perm[g]]; i < p.begin[perm[g] + 1]; ++i) q.t[n++] = p.t[i];
+        q.begin[g + 1] = (int16_t)n;
+    }
+    return q;
+}
+// Groups on single CTAs with the order of their items.
+struct Schedule {
+    Groups g;
+    Order order;
+    int perm[kMaxPlan];
+    int64_t span;
+    Schedule(const Groups& groups, int64_t rows) : g(groups), order{rows, groups.groups, 0} { span = choose_order(order, g.cost, perm, sm_count()); }
+    void fill(Plan& plan, const Tile* list) const {
+        plan.order = order;
+        int n = 0;
+        for (int i = 0; i < order.groups; ++i) {
+            for (int j = g.begin[perm[i]]; j < g.begin[perm[i] + 1]; ++j) plan.t[n++] = list[g.tile[j]];
+            plan.begin[i + 1] = (int16_t)n;
+        }
+    }
+};
 
 }  // namespace fused
 }  // namespace fcb200
@@ -769,7 +747,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
     Params prm{};
     Tile list[kMaxTiles] = {};
     const int grouping = variant >> 4;
-    if ((variant & 15) > 2 || grouping < kAuto || grouping > kFine) return FCB200_EINVAL;
+    if ((variant & 15) > 2 || grouping < kAuto || grouping > kPair) return FCB200_EINVAL;
     if (num_tiles <= 0 || num_tiles > kMaxTiles) return FCB200_ERANGE;
     if (lda % 8 || lda < a_cols || ldy % 4 || ldy < y_cols || y_cols % 4) return FCB200_EINVAL;
     if (!aligned16(a_hi) || !aligned16(a_lo) || !aligned16(y)) return FCB200_EALIGN;
@@ -818,41 +796,57 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
     // convolution: 528 / 446).  Few row tiles still leave SMs without work; then the gated rows go one by one where that
     // shortens the longest CTA by more than the estimate's error (M = 7 680: 104 -> 87 us, M = 640: 59 -> 36 us).
     const int64_t rows_m = (m + BM - 1) / BM;
-    Groups grp = group_tiles(list, num_tiles, rot_begin, grouping == kFine && !backward ? kFine : kNatural);
-    if (!grp.ok) return FCB200_EINVAL;
+    const Groups natural = group_tiles(list, num_tiles, rot_begin, kNatural);
+    if (!natural.ok) return FCB200_EINVAL;
+    const auto fine = [&] { return Schedule(group_tiles(list, num_tiles, rot_begin, kFine), rows_m); };
+    Schedule run = grouping == kFine && !backward ? fine() : Schedule(natural, rows_m);
+    if (!run.g.ok) return FCB200_EINVAL;
     if (grouping == kAuto && gated) {
-        const Groups fine = group_tiles(list, num_tiles, rot_begin, kFine);
-        if (fine.ok && 10 * makespan(fine, rows_m, sm_count()) < 9 * makespan(grp, rows_m, sm_count())) grp = fine;
+        const Schedule rows = fine();
+        if (rows.g.ok && 10 * rows.span < 9 * run.span) run = rows;
     }
-    // backward: the same, if there is room for the raw rows and the second kernel pays: about 3 us, 300 units of K, and its
-    // reads and the raw rows' writes at the memory's rate, 55 KB a unit.  A row on its own costs 1.6 times its estimate (its
-    // factors are made anew and nothing overlaps its epilogue), one in a group 1.1 times.  Natural against row by row, us:
-    // lmax 2, 960 rows 34 / 19, 3 240 rows 37 / 35, 4 320 rows 38 / 45, 7 680 rows 64 / 67; lmax 4, 960 rows 53 / 41, 3 240
-    // rows 60 / 79, 4 320 rows 105 / 96, 7 680 rows 144 / 165.
+    // On pairs a listed tile costs 0.8 of its K extent where it has a partner, and 230 for the time the tensor core waits for
+    // the accumulators; alone a tile costs its K extent and 192.  So long K goes to pairs, the radial output layer (K = 128)
+    // and small launches do not.  us, alone / on pairs: first convolution, lmax 2, 7 680 rows 98 / 68, 20 580 rows 203 / 182,
+    // 131 072 rows 1122 / 1034; lmax 4, 3 240 rows 117 / 106, 60 000 rows 1930 / 1701; second convolution, lmax 2, 20 580 rows
+    // 74 / 76, 131 072 rows 466 / 430; first convolution's backward, 131 072 rows 1004 / 913; radial output layer, 131 072
+    // rows 260 / 272.  (Seconds of back-to-back launches, at the power cap from some 10 000 rows on.)
+    const bool pairs_only = grouping == kPair;
+    PairGroups two;
+    if (!backward && (pairs_only || (grouping == kAuto && rows_m >= 8))) {  // the fewest rows: no time for the estimate
+        two = pair_tiles(list, natural);
+        two.plan.order.rows = (m + 2 * BM - 1) / (2 * BM);
+        int perm[kMaxPlan];
+        const int64_t span = choose_order(two.plan.order, two.cost, perm, sm_count() / 2);
+        if (!pairs_only && span >= run.span) two.plan.order.groups = 0;
+        else if (two.plan.order.snake) two.plan = reordered(two.plan, perm);
+    }
+    const bool on_pairs = two.plan.order.groups > 0;
+    // backward: rows one by one as above, if there is room for the raw rows and the second kernel pays: about 3 us, 300 units of
+    // K, and its reads and the raw rows' writes at the memory's rate, 55 KB a unit.  A row on its own costs 1.6 times its
+    // estimate (its factors are made anew and nothing overlaps its epilogue), one in a group 1.1 times.
     GateSums sums{};
     bool solo = backward && raw && grouping != kNatural && split_sums(list, num_tiles, sums);
     if (solo && grouping != kFine) {
         const int64_t extra = 300 + m * (sums.begin[sums.degrees] + sums.degrees) * (BN * 8) / 55000;
-        solo = 16 * makespan(group_tiles(list, num_tiles, rot_begin, kFine), rows_m, sm_count()) + 10 * extra < 11 * makespan(grp, rows_m, sm_count());
+        solo = 16 * fine().span + 10 * extra < 11 * run.span;
     }
     if (solo) {
         for (int i = 0; i < num_tiles; ++i)
             if (list[i].mode == kGatedBwd) list[i].flags |= kSolo;
-        grp = group_tiles(list, num_tiles, rot_begin, kFine);
+        run = fine();
     }
-    plan.groups = grp.groups;
-    for (int i = 0; i <= grp.groups; ++i) plan.begin[i] = grp.begin[i];
-    for (int i = 0; i < grp.n; ++i) plan.t[i] = list[grp.tile[i]];
+    run.fill(plan, list);
     CUtensorMap mah, mal, mw[6];
-    int rc = map_half(&mah, a_hi, m, a_cols, lda);
-    if (!rc) rc = map_half(&mal, a_lo, m, a_cols, lda);
+    int rc = on_pairs ? FCB200_OK : map_half(&mah, a_hi, m, a_cols, lda);
+    if (!rc && !on_pairs) rc = map_half(&mal, a_lo, m, a_cols, lda);
     int first = -1;
     for (int i = 0; i < 3 && !rc; ++i) {
         if (!used[i]) continue;
         if (first < 0) first = i;
         if (w_cols[i] % 8 || !aligned16(w_hi[i]) || !aligned16(w_lo[i]) || !(w_scale[i] > 0.f)) return FCB200_EINVAL;
-        rc = map_half(&mw[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i]);
-        if (!rc) rc = map_half(&mw[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i]);
+        if (!on_pairs) rc = map_half(&mw[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i]);
+        if (!rc && !on_pairs) rc = map_half(&mw[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i]);
         prm.w_scale[i] = w_scale[i];
         prm.bias[i] = bias ? bias[i] : nullptr;
         if (prm.bias[i] && (!aligned16(prm.bias[i]) || w_rows[i] % BN)) return FCB200_EALIGN;
@@ -869,11 +863,12 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
     prm.m_total = m, prm.status = status;
     prm.raw = raw, prm.raw_ld = sums.begin[sums.degrees] * BN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t items = rows_m * plan.groups;
+    if (on_pairs) return launch_pair(two.plan, prm, a_hi, a_lo, lda, a_cols, w_hi, w_lo, w_rows, w_cols, used, o_cols, forward, st);
+    const int64_t items = plan.order.rows * plan.order.groups;
     const int grid = (int)(items < sm_count() ? items : sm_count());
     auto launch = [&](auto kernel, bool (&done)[64]) {
         if (const int arc = ensure_dynamic_smem(kernel, kSmemBytes, done)) return arc;
-        launch_pdl(kernel, dim3(grid), dim3(kThreads), kSmemBytes, st, mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm, items);
+        launch_pdl(kernel, dim3(grid), dim3(kThreads), kSmemBytes, st, mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm);
         return launch_status();
     };
     static bool done[3][64] = {};

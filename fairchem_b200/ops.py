@@ -658,7 +658,8 @@ def gemm_f16x2_presplit_(a_hi: Tensor, a_lo: Tensor, w_hi: Tensor, w_lo: Tensor,
 CONV_PLAIN, CONV_SILU, CONV_GATED, CONV_SILU_BWD, CONV_GATED_BWD = 0, 2, 3, 4, 5
 CONV_FIRST, CONV_LAST, CONV_KEEP = 1, 2, 4
 CONV_MAX_TILES = 40
-# How a launch's tile list is cut into work items: 0 the choice of the library, 1 natural groups, 2 fine (csrc/so2_conv_fused.cu)
+# How a launch's tile list is cut into work items: 0 the choice of the library, 1 natural groups, 2 fine, 3 natural
+# groups on pairs of CTAs where that form applies (csrc/so2_conv_fused.cu)
 CONV_GROUPING = 0
 
 

@@ -416,7 +416,8 @@ int fcb200_gemm_f16x2_presplit(const void* a_hi, const void* a_lo, int64_t lda, 
  *   y            [M, y_cols] float32, row stride ldy; o_hi/o_lo [M, o_cols] half planes, row stride ldo, written
  *                times *o_scale (device pointers to powers of two, NULL = 1)
  *   status       as in fcb200_gemm_f16x2_presplit
- *   variant      bits 4..: how the list is cut into work items: 0 the library's choice, 1 natural groups, 2 fine;
+ *   variant      bits 4..: how the list is cut into work items: 0 the library's choice, 1 natural groups, 2 fine, 3 natural
+ *                groups on pairs of CTAs (not the backward gate);
  *                bits 0..3 (0, 1 or 2) are accepted for callers of earlier launch forms and ignored.  Same results.
  *   rot_begin    with gated tiles: the plain tiles before this position are their gate scalars
  * At most 40 tiles; every k a multiple of 32, w_row a multiple of 128.

@@ -83,6 +83,73 @@ def test_fused_convolutions_match_the_separate_kernels(ops, grouping, lmax, e):
     torch.testing.assert_close(gm, gm_ref, rtol=1e-5, atol=1e-5 * float(gm_ref.abs().max()))
 
 
+def _launches(ops, lmax, e, form):
+    """Outputs of every kind of launch that may run on pairs of CTAs, on inputs that depend on (lmax, e) alone."""
+    from fairchem_b200 import backbone as B
+
+    c, nm = 128, ops.SHAPES[lmax].nm
+    torch.manual_seed(e)
+    ew = B.Edgewise(c, c, lmax, 2, [320, 128, 128]).cuda()
+    g = torch.Generator(device="cuda").manual_seed(7 * e + lmax)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda")  # noqa: E731
+    m, gy = _planes(draw(e, nm * 2 * c)), _planes(draw(e, (lmax + nm) * c), 64.0)
+    scale, status = torch.tensor([64.0], device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    # a list with a K tail (96 = 64 + 32), a lone tile and a last tile of 64 columns
+    short, bias = draw(448, 96), draw(512)
+    hi, lo, sc = ops.split_f16(short)
+    tiles = [v for r in (0, 128, 256, 384) for v in (32, 96, 0, r, r, ops.CONV_PLAIN, 0, 0, 0)]
+    with torch.no_grad():
+        ew.so2_conv_1.fc_m0.bias.normal_()
+        ew.so2_conv_2.fc_m0.bias.normal_()
+        ops.CONV_GROUPING = form
+        try:
+            y = torch.full((e, (lmax + nm) * c), float("nan"), device="cuda")
+            a = B._fused_conv1_gate(ew, m, y)
+            ak = B._fused_conv1_gate(ew, m, None)
+            msg = B._fused_conv2(ew, a, torch.full((e, nm * c), float("nan"), device="cuda"))
+            gm = B._fused_conv1_backward(ew, gy, scale)
+            y2 = torch.full((e, 448), float("nan"), device="cuda")
+            ops.so2_conv_fused_.raw(m[0], m[1], [hi], [lo], [sc], None, tiles, 0, y2, None, None, None, None, status)
+            hi, lo, sc = ops.split_f16(torch.cat([short, short[:64]]))
+            y3 = torch.full((e, 512), float("nan"), device="cuda")
+            ops.so2_conv_fused_.raw(m[0], m[1], [hi], [lo], [sc], bias, tiles, 0, y3, None, None, None, None, status)
+        finally:
+            ops.CONV_GROUPING = 0
+    B.check_gemm_status()
+    assert int(status) == 0
+    return [y, a[0], a[1], ak[0], ak[1], msg, gm, y2, y3]
+
+
+# one row, both sides of a warp's, a CTA's and a pair's rows, items group by group (7 680) and row by row
+@pytest.mark.parametrize("lmax,e", [(2, e) for e in (1, 32, 33, 128, 129, 255, 256, 257, 1000, 7680, 21000)] + [(4, 129), (4, 257), (4, 3240)])
+def test_pairs_of_ctas_give_the_same_bits(ops, lmax, e):
+    """Same products in the same order on either form, and every output element written."""
+    alone = _launches(ops, lmax, e, 1)
+    for form in (0, 3):
+        for got, want in zip(_launches(ops, lmax, e, form), alone):
+            assert not bool(torch.isnan(got.float()).any()) and torch.equal(got, want)
+
+
+def test_pairs_of_ctas_report_values_outside_the_half_range(ops):
+    """An infinite input is reported by a plain list and, through the gate, by a forward list."""
+    from fairchem_b200 import backbone as B
+
+    ew = B.Edgewise(128, 128, 2, 2, [320, 128, 128]).cuda()
+    ops.CONV_GROUPING = 3
+    try:
+        for width, launch in ((9 * 256, lambda m: B._fused_conv1_gate(ew, m, None)),
+                              (9 * 128, lambda a: B._fused_conv2(ew, a, torch.empty(300, 9 * 128, device="cuda")))):
+            x = torch.randn(300, width, device="cuda")
+            x[299, 5] = 1e6  # beyond 65 504: its half is infinite
+            with torch.no_grad():
+                launch(_planes(x))
+            with pytest.raises(B.HalfRangeError):
+                B.check_gemm_status()
+            B.check_gemm_status()
+    finally:
+        ops.CONV_GROUPING = 0
+
+
 def test_edge_block_is_the_same_with_and_without_the_fused_launches(ops, grouping):
     """Energy and forces of a small periodic system with the fused convolution launches on and off."""
     from fairchem_b200 import backbone as B
