@@ -228,9 +228,9 @@ struct Run {
         return rc;
     }
 
-    // one launch of tile list c on rows [m] of half planes; raw: see so2_conv_fused
+    // one launch of tile list c on rows [m] of half planes
     int conv(const char* name, const Conv& c, const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, int rot_begin, float* y,
-             int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m, float* raw = nullptr) const {
+             int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m) const {
         const void *hi[3] = {}, *lo[3] = {};
         int64_t rows[3] = {}, cols[3] = {};
         float sc[3] = {1.f, 1.f, 1.f};
@@ -240,7 +240,7 @@ struct Run {
         hook(name, 1, bytes, flops);
         const int rc = so2_conv_fused(a_hi, a_lo, lda, a_cols, hi, lo, rows, cols, sc, c.bias, c.t.data(), c.count(), rot_begin, y,
                                              ldy, y_cols, o ? o->hi : nullptr, o ? o->lo : nullptr, o ? o->ld : 0, o_cols, a_scale,
-                                             o_scale, m, 0, ev.status, stream, raw);
+                                             o_scale, m, 0, ev.status, stream);
         hook(name, 0, bytes, flops);
         return rc;
     }
@@ -540,7 +540,7 @@ int Run::layer_backward(int l) {
         else b1.tile((d.lmax + r) * C, C, 1, (deg - 1) * C, r * C);
     }
     const int64_t fw = (d.lmax + d.nl) * C;
-    FCB_TRY(conv("ffn_out_gate_bwd", b2, L.gp.hi, L.gp.lo, row, row, b2.count(), q.ffn_y, fw, fw, &L.gy2, fw, &s->scale, &s->scale, n, L.gxn));
+    FCB_TRY(conv("ffn_out_gate_bwd", b2, L.gp.hi, L.gp.lo, row, row, b2.count(), q.ffn_y, fw, fw, &L.gy2, fw, &s->scale, &s->scale, n));
     FCB_TRY(conv("ffn_in_bwd", b1, L.gy2.hi, L.gy2.lo, fw, fw, 0, L.gxn, row, row, nullptr, 0, &s->scale, nullptr, n));
     FCB_TRY(op("rms_norm_sh_bwd", n * row * 16, [&] {
         return by_lmax([&](auto lm) {
@@ -588,7 +588,7 @@ int Run::layer_backward(int l) {
                 return 0;
             });
         }));
-        FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, d.yw, d.yw, &L.gy, L.gy.ld, scale, scale, ec, L.gm));
+        FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, d.yw, d.yw, &L.gy, L.gy.ld, scale, scale, ec));
         FCB_TRY(conv("so2_conv_fused_conv1_bwd", c1, L.gy.hi, L.gy.lo, L.gy.ld, L.gy.ld, 0, L.gm, d.nm * 2 * C, d.nm * 2 * C, nullptr, 0, scale, nullptr, ec));
         const int64_t gb = ec * 4LL * (2 * d.nm * C + 2 * 2 * d.nrad * C + d.nw + 12) + (n1 - n0) * row * 4 * 4;
         FCB_TRY(op("gather_rotate_bwd", gb, [&] {

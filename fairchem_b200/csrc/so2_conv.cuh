@@ -17,9 +17,8 @@ enum Mode : int32_t {
     kGatedBwd = 5,  // planes[:, out_col ...] = split(v * sigmoid(gate)); gate gradient summed over consecutive tiles
 };
 // kGateSilu: the gate is sigmoid(silu(g)), the scalar MLP of the node-wise feed-forward, instead of sigmoid(g).
-// kGateSrc (set on the host): a gate tile of the rows that follow.  kSolo (host): a backward gated row on its own; its raw
-// value goes to Params::raw and gate_sum_kernel adds up the rows of a degree.
-enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8, kGateSrc = 16, kSolo = 32 };
+// kGateSrc (set on the host): a gate tile of the rows that follow.
+enum Flags : int32_t { kFirst = 1, kLast = 2, kKeep = 4, kGateSilu = 8, kGateSrc = 16 };
 
 struct Tile {
     int16_t a_col;     // first input column of this tile's K range
@@ -31,7 +30,6 @@ struct Tile {
     int16_t y_col;     // column of y holding this row's raw value (kSilu/kGated keep, kSiluBwd/kGatedBwd read)
     int16_t gate_col;  // column of y (and of the gradient planes) of the gate scalars of this row's degree
     int16_t flags;
-    int16_t raw_col;   // kSolo: column of Params::raw
 };
 constexpr int kMaxTiles = 40;   // tiles a caller may list; lmax 4: 19 rows x 2C = 38 column tiles in the conv-1 backward
 constexpr int kMaxPlan = 80;    // tiles of a plan: a gate tile may be repeated for each of its rows
@@ -64,8 +62,6 @@ struct Params {
     const float* o_scale;  // power of two the output planes are written with (null = 1)
     int64_t m_total;
     int32_t* status;
-    float* raw;        // [m, raw_ld] values of the kSolo tiles
-    int32_t raw_ld;
 };
 
 // Work items are row tiles times groups of tiles; `units` CTAs or pairs take them in turn, either row by row (those that run
@@ -106,6 +102,31 @@ int launch_pair(const PairPlan& plan, const Params& prm, const void* a_hi, const
 // 1 / (1 + e^-v) on the special-function unit (ex2.approx, rcp.approx): relative error ~2^-22, a few instructions
 // instead of the ~20 of expf and an IEEE division -- the epilogue evaluates it for every output element
 __device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+// D[tmem] (+)= A x B^T, issued by one lane of a warp in which every operand is the same in all lanes.
+template <int N, bool kAdd>
+__device__ __forceinline__ void umma_one(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+    if constexpr (kAdd)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "l"(da), "l"(db), "r"(instr_desc(N)) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "l"(da), "l"(db), "r"(instr_desc(N)), "r"(accumulate) : "memory");
+}
+// The warp waits as one, so that everything its loops derive from is the same in all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(kFull, mbar_wait(bar, parity, abort_flag));
+}
+// What a tensor map says, on its way before the first copy needs it.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 
 // Two float32 in a register pair; the packed instructions halve the epilogue's multiply and add count.
 typedef uint64_t f32x2;

@@ -21,19 +21,15 @@
 // and their autograd twins.  Arithmetic and accumulators are those of gemm_f16x2_presplit_kernel.
 //
 // What bounds it, and the layout that follows.  Per 64-deep k-step a 128 x 128 tile takes 768 cycles of MMA and 64 KiB of
-// operands.  Main loop alone (no epilogue), M = 131 072, N = 512, K = 512 / 1024, issued TFLOP/s: two 64 KiB stages
-// 1250 / 1150, three 1527 / 1544, CTA pairs on 256 x 256 tiles with three stages 1555 / 1510; the MMAs alone reach 1516
-// on operands in the 64-byte swizzle and 1736 in the 128-byte one.  So: 128-byte swizzle, 64-deep stages, three of them
-// (192 KiB) -- which leaves 32 KiB for the epilogue, one 4 KiB tile for each of its eight warps.  A warp turns its 32 x 32
-// accumulator block in that tile from a row per lane to whole lines per instruction and does everything else on registers
-// and global memory directly (the forms with TMA-fed input and output tiles needed 64-96 KiB and two or five operand
-// stages of half the depth).
-// us per launch by itself at M = 131 072, lmax 2, four 32-deep or two 64-deep stages with TMA epilogues -> this: conv 1 +
-// gate 1219 -> 985, conv 2 499 -> 377, its backward + gate 780 -> 655, conv 1 backward 1050 -> 890, radial output layer
-// 263 -> 243.  Among the other launches of a 100 000-atom evaluation (129 000 edges each): 1184 -> 1003, 457 -> 395, 642 ->
-// 652 (no gain: its epilogue, not its loop, is what there is to wait for), 1011 -> 891, 220 -> 216.  Still above the main
-// loop's own time: the epilogues' instruction stream (the gate's backward: 1500 per 32 x 32 chunk) and 64-byte plane stores
-// share the SM with it.
+// operands: 128-byte swizzle (the MMAs alone issue 1736 TFLOP/s from it, 1516 from the 64-byte one), 64-deep stages, three of
+// them (192 KiB; two: 1250 against 1527 TFLOP/s), which leaves 32 KiB for the epilogue, one 4 KiB tile for each of its eight
+// warps.  A warp turns its 32 x 32 accumulator block in that tile from a row per lane to whole lines per instruction and does
+// everything else on registers and global memory directly.
+// The products are issued by one lane of a warp that walks the loop as one; from a branch of a single lane each took some 110
+// cycles to issue whatever its shape, and a k-step 1125.  24 k-steps of one row tile (radial output layer's backward), us:
+// 17.8 -> 15.2 with 128 columns an item, 16.2 -> 11.3 with 32.
+// At size a launch runs at the power cap and its energy is what there is to save (see so2_conv_pair.cu); few row tiles are
+// bound by the chain of k-steps of one item, hence items of 64 or 32 columns there.
 #include "so2_conv.cuh"
 
 namespace fcb200 {
@@ -47,16 +43,18 @@ struct Plan {
     Tile t[kMaxPlan];
 };
 
-constexpr int kStages = 3;
-constexpr int kStageBytes = 4 * kPart;               // A_hi | A_lo | W_hi | W_lo
+// NB: columns of a work item, 128, or 64 or 32 where few row tiles would leave SMs without work.
+template <int NB> constexpr int kStages = NB == 128 ? 3 : NB == 64 ? 4 : 5;
+template <int NB> constexpr int kStageBytes = 2 * kPart + 2 * NB * KB * 2;  // A_hi | A_lo | W_hi | W_lo
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 128 + 32 * kEpiWarps;       // warp 0 TMA, warp 1 MMA, 2-3 idle, warps 4-11 epilogue
 // Registers: launched with 168 a thread (12 warps on 4 schedulers); the first warpgroup gives up what the two epilogue
 // warpgroups take, 128 * 40 + 256 * 232 = 384 * 168.
 constexpr int kIdleRegs = 40, kEpiRegs = 232;
 static_assert(128 * kIdleRegs + 32 * kEpiWarps * kEpiRegs <= kThreads * 168, "register split");
-constexpr int kAccCols = 2 * BN, kTmemCols = 2 * kAccCols;
-constexpr int kSmemBytes = kStages * kStageBytes + kEpiWarps * 4096 + 1024 + 256;
+template <int NB> constexpr int kAccCols = 2 * NB;  // main columns [0, NB), corrections [NB, 2 NB); double buffered
+template <int NB> constexpr int kEpiBytes = (NB == 32 ? kEpiWarps / 2 : kEpiWarps) * 4096;
+template <int NB> constexpr int kSmemBytes = kStages<NB> * kStageBytes<NB> + kEpiBytes<NB> + 1024 + 256;
 
 __device__ __forceinline__ void store_split(__half* hi, __half* lo, int off, f32x2 o0, f32x2 o1, bool in, __half2& top) {
     uint2 h, l;
@@ -78,38 +76,41 @@ __device__ __forceinline__ void load_pair(const float* p, f32x2& a, f32x2& b) {
 // [64 h, 64 h + 64) of every tile, h = (w - 4) / 4, in two chunks of 32.  A chunk is turned in the warp's shared tile to
 // "lane = row 4 i + lane / 8, columns 4 (lane % 8)": 128-byte lines per row for every global access, and the same
 // (row, column) in the same thread for every tile, so gates and gate-gradient sums stay in registers.
-template <int KIND>
+// Narrow items have one chunk a warp (NB 64) or for the four warps of the first half alone (NB 32).
+template <int KIND, int NB>
 __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, uint32_t tmem_base, uint32_t tile,
                                          uint32_t tfull0, uint32_t tempty0, volatile int* abort_flag, volatile int* range_flag) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = warp & 3, half = (warp - 4) >> 2;
+    constexpr int kChunks = NB == 128 ? 2 : 1, kSubs = BN / NB;
+    const int base = half * kChunks * 32;  // of this warp's columns in an item
     const int rr = lane >> 3, c4 = (lane & 7) * 4;
     const float a_scale = prm.a_scale ? *prm.a_scale : 1.0f;
     const float o_scale = prm.o_scale ? *prm.o_scale : 1.0f;
     __half2 top = __floats2half2_rn(0.f, 0.f);
     // per chunk and row: forward: o_scale * sigmoid of the gate; backward: gate-gradient sums
-    f32x2 keepv[KIND == kPlainKind ? 1 : 2][16];
+    f32x2 keepv[KIND == kPlainKind ? 1 : kChunks][16];
     // Loads run one chunk ahead where the registers allow it: the second chunk's accumulator columns without a backward
     // input, else the y rows of the next chunk.
     constexpr bool kAhead = KIND != kBackwardKind;
     f32x2 yv[KIND == kBackwardKind ? 16 : 1] = {};
-    f32x2 sg[KIND == kBackwardKind ? 2 : 1][16];  // backward: o_scale * sigmoid of the degree's gate, made at its first row; row 0: the slope
+    f32x2 sg[KIND == kBackwardKind ? kChunks : 1][16];  // backward: o_scale * sigmoid of the degree's gate, made at its first row; row 0: the slope
     auto slot = [&](int i) { return tile + (uint32_t)((rr + 4 * i) * 128 + (((lane & 7) ^ ((rr + 4 * i) & 7)) * 16)); };
     auto put = [](uint32_t at, f32x2 a, f32x2 b) { asm volatile("st.shared.v2.b64 [%0], {%1,%2};" ::"r"(at), "l"(a), "l"(b) : "memory"); };
     auto get = [](uint32_t at, f32x2& a, f32x2& b) { asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "r"(at) : "memory"); };
-    // y lines of a backward tile on their way to L2 one tile early (lane = row; a warp's 64 columns are two lines)
-    auto prefetch = [&](int64_t mt2, int ti2) {
+    // y lines of a backward tile on their way to L2 one tile early (lane = row, a line a chunk)
+    auto prefetch = [&](int64_t mt2, int ti2, int first) {
         if constexpr (KIND == kBackwardKind) {
             const int64_t row = mt2 * BM + q * 32 + lane;
             if (row < prm.m_total) {
                 const Tile& t2 = plan.t[ti2];
-                const float* p = prm.y + row * prm.ldy + t2.y_col + half * 64;
+                const float* p = prm.y + row * prm.ldy + t2.y_col + first;
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
-                if (t2.flags & (kFirst | kSolo)) {
+                if (kChunks == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
+                if (t2.flags & kFirst) {
                     p += t2.gate_col - t2.y_col;
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
+                    if (kChunks == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
                 }
             }
         }
@@ -118,6 +119,8 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
     int64_t tcount = 0, mt;
     int g;
     for (int64_t n = 0; plan.order.item(n, gridDim.x, blockIdx.x, mt, g); ++n) {
+        const int col0 = NB == 128 ? half * 64 : g % kSubs * NB + base;  // of this warp's first chunk in a listed tile
+        if (NB < 128) g /= kSubs;
         const int64_t row0 = mt * BM + q * 32;
         const int live = (int)(prm.m_total - row0 < 32 ? prm.m_total - row0 : 32);  // rows of this warp inside the matrix
         // 32 rows of at most 32 767 columns: offsets inside a warp's block fit 32 bits
@@ -129,7 +132,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     yv[2 * i] = yv[2 * i + 1] = 0;
-                    if (rr + 4 * i < live) load_pair(yrow + 4 * i * prm.ldy + y_col + (half * 2 + c2) * 32, yv[2 * i], yv[2 * i + 1]);
+                    if (rr + 4 * i < live) load_pair(yrow + 4 * i * prm.ldy + y_col + col0 + c2 * 32, yv[2 * i], yv[2 * i + 1]);
                 }
             }
         };
@@ -145,22 +148,21 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
             if constexpr (KIND == kBackwardKind) {
                 int64_t mt2;
                 int g2;
-                if (ti + 1 < plan.begin[g + 1]) prefetch(mt, ti + 1);
-                else if (plan.order.item(n + 1, gridDim.x, blockIdx.x, mt2, g2)) prefetch(mt2, plan.begin[g2]);
+                if (ti + 1 < plan.begin[g + 1]) prefetch(mt, ti + 1, col0);
+                else if (plan.order.item(n + 1, gridDim.x, blockIdx.x, mt2, g2)) prefetch(mt2, plan.begin[g2 / kSubs], NB == 128 ? col0 : g2 % kSubs * NB + base);
             }
             const bool gate_silu = (t.flags & kGateSilu) != 0;
-            const bool solo = (t.flags & kSolo) != 0;
             // What the rows that follow are multiplied by, made while the tensor core works on the tile.  The values pass
             // through the thread's own slots of the shared tile so that the sigmoids are a loop: unrolled for both chunks,
             // and with row 0 and the gate's gradient unrolled too, the code of a tile outgrew the instruction cache and a
             // quarter of the epilogue's stalls were instruction fetches (gated backward launches of an evaluation, 62 118 edges:
             // 1.40 -> 1.26 ms; 775 000: 18.9 -> 17.3).
             if constexpr (KIND == kBackwardKind) {
-                if (mode == kSiluBwd || (t.flags & (kFirst | kSolo))) {
+                if (mode == kSiluBwd || (t.flags & kFirst)) {
                     const bool slope = mode == kSiluBwd;
-                    const float* from = yrow + (slope ? t.y_col : t.gate_col) + half * 64;
+                    const float* from = yrow + (slope ? t.y_col : t.gate_col) + col0;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
+                    for (int i = 0; i < 8 * kChunks; ++i) {
                         f32x2 &a = sg[i >> 3][2 * (i & 7)], &b = sg[i >> 3][2 * (i & 7) + 1];
                         a = b = 0;
                         if (rr + 4 * (i & 7) < live) load_pair(from + 4 * (i & 7) * prm.ldy + (i >> 3) * 32, a, b);
@@ -172,7 +174,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
                         return o_scale * s;
                     };
 #pragma unroll
-                    for (int c2 = 0; c2 < 2; ++c2) {
+                    for (int c2 = 0; c2 < kChunks; ++c2) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) put(slot(i), sg[c2][2 * i], sg[c2][2 * i + 1]);
 #pragma unroll 1
@@ -197,14 +199,14 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
             const float out_scale = 1.0f / (a_scale * prm.w_scale[t.w]);  // a power of two: scaling after the sum is exact
             const f32x2 os2 = pack(out_scale, out_scale);
             const float* bias = prm.bias[t.w];
-            const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols) + ((uint32_t)(q * 32) << 16);  // main columns [0, 128), corrections [128, 256)
+            const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols<NB> + base) + ((uint32_t)(q * 32) << 16);
             if constexpr (kAhead) {
-                FCB_TMEM_LD32(r, acc + (uint32_t)(half * 64));
-                FCB_TMEM_LD32(c, acc + (uint32_t)(BN + half * 64));
+                FCB_TMEM_LD32(r, acc);
+                FCB_TMEM_LD32(c, acc + (uint32_t)NB);
             }
 #pragma unroll
-            for (int c2 = 0; c2 < 2; ++c2) {
-                const int col = (half * 2 + c2) * 32;  // within the tile
+            for (int c2 = 0; c2 < kChunks; ++c2) {
+                const int col = col0 + c2 * 32;  // within the tile
                 // 1. accumulator -> shared tile, row `lane`
                 f32x2 poison = 0;  // becomes NaN if any value is inf or NaN (an overflowed half upstream)
                 auto stage4 = [&](int v4, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3, uint32_t c0, uint32_t c1, uint32_t c2_, uint32_t c3) {
@@ -220,23 +222,23 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
 #pragma unroll
                     for (int v = 0; v < 8; ++v)
                         stage4(v, r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3], c[4 * v], c[4 * v + 1], c[4 * v + 2], c[4 * v + 3]);
-                    if (c2 == 0) {
-                        FCB_TMEM_LD32(r, acc + (uint32_t)(col + 32));
-                        FCB_TMEM_LD32(c, acc + (uint32_t)(BN + col + 32));
+                    if (c2 + 1 < kChunks) {
+                        FCB_TMEM_LD32(r, acc + 32u);
+                        FCB_TMEM_LD32(c, acc + (uint32_t)(NB + 32));
                     }
                 } else {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         uint32_t rh[16], ch[16];
-                        FCB_TMEM_LD16(rh, acc + (uint32_t)(col + 16 * h));
-                        FCB_TMEM_LD16(ch, acc + (uint32_t)(BN + col + 16 * h));
+                        FCB_TMEM_LD16(rh, acc + (uint32_t)(c2 * 32 + 16 * h));
+                        FCB_TMEM_LD16(ch, acc + (uint32_t)(NB + c2 * 32 + 16 * h));
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int v = 0; v < 4; ++v)
                             stage4(4 * h + v, rh[4 * v], rh[4 * v + 1], rh[4 * v + 2], rh[4 * v + 3], ch[4 * v], ch[4 * v + 1], ch[4 * v + 2], ch[4 * v + 3]);
                     }
                 }
-                if (c2 == 1) {  // hand the accumulator back to the MMA thread
+                if (c2 == kChunks - 1) {  // hand the accumulator back to the MMA thread
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     mbar_arrive(tempty0 + 8u * buf);
                 }
@@ -311,12 +313,11 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
                     }
                 } else {
                     rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
-                        if (solo && in) store_pair(prm.raw + (row0 + rr + 4 * i) * prm.raw_ld + t.raw_col + col + c4, x0, x1);
                         keepv[c2][2 * i] = fma2(x0, yv[2 * i], keepv[c2][2 * i]);  // row 0: not used
                         keepv[c2][2 * i + 1] = fma2(x1, yv[2 * i + 1], keepv[c2][2 * i + 1]);
                         store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, sg[c2][2 * i]), mul2(x1, sg[c2][2 * i + 1]), in, top);
                     });
-                    if ((t.flags & kLast) && !solo) {
+                    if (t.flags & kLast) {
                         const float inv = 1.0f / o_scale;
                         auto dsig = [&](float v) { return v * (1.f - v * inv); };  // o_scale * sigmoid'
                         auto dsilu = [&](float v) {
@@ -340,7 +341,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
                         }
                     }
                 }
-                if (c2 == 0) fetch_of(t, 1);
+                if (c2 + 1 < kChunks) fetch_of(t, 1);
                 else if (ti + 1 < plan.begin[g + 1]) fetch_of(plan.t[ti + 1], 0);
                 __syncwarp();  // the shared tile is free again
             }
@@ -349,7 +350,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
     if (!(__half2float(__hmax_nan(__low2half(top), __high2half(top))) <= kHalfMax)) *range_flag = 1;  // inf or NaN
 }
 
-template <int KIND>
+template <int KIND, int NB>
 __global__ void __launch_bounds__(kThreads, 1)
     so2_conv_fused_kernel(const __grid_constant__ CUtensorMap map_ahi, const __grid_constant__ CUtensorMap map_alo,
                           const __grid_constant__ CUtensorMap map_whi0, const __grid_constant__ CUtensorMap map_wlo0,
@@ -358,29 +359,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                           const __grid_constant__ Plan plan, const __grid_constant__ Params prm) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t epi_base = base + kStages * kStageBytes;
-    const uint32_t bar_base = epi_base + kEpiWarps * 4096;
-    // barrier block: full[S] | empty[S] | tmem_full[2] | tmem_empty[2] | tmem slot, abort flag, range flag
+    constexpr int kRing = kStages<NB>, kTmemCols = 2 * kAccCols<NB>;
+    const uint32_t epi_base = base + kRing * kStageBytes<NB>;
+    const uint32_t bar_base = epi_base + kEpiBytes<NB>;
+    // barrier block: full[ring] | empty[ring] | tmem_full[2] | tmem_empty[2] | tmem slot, abort flag, range flag
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
-    auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * kStages + b); };
-    auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * kStages + 2 + b); };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (kRing + s); };
+    auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * kRing + b); };
+    auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * kRing + 2 + b); };
     uint8_t* const bar_generic = smem_raw + (bar_base - smem_u32(smem_raw));
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_generic + 8 * (2 * kStages + 4));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kStages + 4) + 4);
-    volatile int* range_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kStages + 4) + 8);
-    auto part_addr = [&](int s, int which) { return base + s * kStageBytes + which * kPart; };
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_generic + 8 * (2 * kRing + 4));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kRing + 4) + 4);
+    volatile int* range_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kRing + 4) + 8);
+    // A_hi, A_lo, W_hi, W_lo of a stage
+    auto part_addr = [&](int s, int which) { return base + s * kStageBytes<NB> + (which < 2 ? which * kPart : 2 * kPart + (which - 2) * (NB * KB * 2)); };
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kRing; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(tfull_bar(b), 1);
-            mbar_init(tempty_bar(b), 32 * kEpiWarps);
+            mbar_init(tempty_bar(b), NB == 32 ? 128 : 32 * kEpiWarps);
         }
         *abort_flag = 0;
         *range_flag = 0;
@@ -394,6 +397,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (threadIdx.x == 64) {
+        prefetch_map(&map_ahi), prefetch_map(&map_alo);
+        prefetch_map(&map_whi0), prefetch_map(&map_wlo0), prefetch_map(&map_whi1), prefetch_map(&map_wlo1), prefetch_map(&map_whi2), prefetch_map(&map_wlo2);
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -402,11 +409,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (warp >= 4) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
-        epilogue<KIND>(plan, prm, tmem_base, epi_base + (uint32_t)((warp - 4) * 4096), tfull_bar(0), tempty_bar(0), abort_flag, range_flag);
+        if (NB > 32 || warp < 8)
+            epilogue<KIND, NB>(plan, prm, tmem_base, epi_base + (uint32_t)((warp - 4) * 4096), tfull_bar(0), tempty_bar(0), abort_flag, range_flag);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIdleRegs));
         if (warp == 0 && lane == 0) {
-            int64_t it = 0;
+            int s = 0;
+            uint32_t ph = 1;
             bool ok = true;
             // an A tile is fetched again for each of the output tiles of its m-block, the weights by every CTA: keep
             // both in L2 ahead of the streamed outputs
@@ -414,60 +423,77 @@ __global__ void __launch_bounds__(kThreads, 1)
             int64_t mt;
             int g;
             for (int64_t n = 0; ok && plan.order.item(n, gridDim.x, blockIdx.x, mt, g); ++n) {
+                const int row = (int)(mt * BM), sub = NB == 128 ? 0 : g % (BN / NB) * NB;
+                if (NB < 128) g /= BN / NB;
                 for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti) {
                     const Tile& t = plan.t[ti];
                     const CUtensorMap* whi = t.w == 0 ? &map_whi0 : (t.w == 1 ? &map_whi1 : &map_whi2);
                     const CUtensorMap* wlo = t.w == 0 ? &map_wlo0 : (t.w == 1 ? &map_wlo1 : &map_wlo2);
                     const int num_kb = (t.k + KB - 1) / KB;
-                    for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                        const int s = (int)(it % kStages);
-                        const uint32_t ph = (uint32_t)((it / kStages) & 1);
-                        ok = mbar_wait(empty_bar(s), ph ^ 1u, abort_flag);
+                    for (int kb = 0; kb < num_kb; ++kb) {
+                        ok = mbar_wait(empty_bar(s), ph, abort_flag);
                         if (!ok) break;
-                        mbar_expect_tx(full_bar(s), kStageBytes);
-                        tma_load_2d_hint(part_addr(s, 0), &map_ahi, t.a_col + kb * KB, (int)(mt * BM), full_bar(s), keep);
-                        tma_load_2d_hint(part_addr(s, 1), &map_alo, t.a_col + kb * KB, (int)(mt * BM), full_bar(s), keep);
-                        tma_load_2d_hint(part_addr(s, 2), whi, kb * KB, t.w_row, full_bar(s), keep);
-                        tma_load_2d_hint(part_addr(s, 3), wlo, kb * KB, t.w_row, full_bar(s), keep);
+                        mbar_expect_tx(full_bar(s), kStageBytes<NB>);
+                        tma_load_2d_hint(part_addr(s, 0), &map_ahi, t.a_col + kb * KB, row, full_bar(s), keep);
+                        tma_load_2d_hint(part_addr(s, 1), &map_alo, t.a_col + kb * KB, row, full_bar(s), keep);
+                        tma_load_2d_hint(part_addr(s, 2), whi, kb * KB, t.w_row + sub, full_bar(s), keep);
+                        tma_load_2d_hint(part_addr(s, 3), wlo, kb * KB, t.w_row + sub, full_bar(s), keep);
+                        if (++s == kRing) s = 0, ph ^= 1;
                     }
                 }
             }
         }
-        if (warp == 1 && lane == 0) {
-            int64_t it = 0, tcount = 0, mt;
-            int g;
+        // All lanes of the warp walk the loop and one issues: addresses and descriptors are then the same in every lane, which
+        // is where the instruction takes them from.  (Issued from a branch of lane 0 alone, a product cost some 110 cycles
+        // whatever its shape, and a 64-deep step 1125 instead of the 768 its products take.)
+        if (warp == 1) {
+            int s = 0, buf = 0, g;
+            uint32_t ph = 0, free_ph = 1;
+            int64_t mt;
             bool ok = true;
+            const uint64_t desc0 = smem_desc128(base);
             for (int64_t n = 0; ok && plan.order.item(n, gridDim.x, blockIdx.x, mt, g); ++n) {
-                for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti, ++tcount) {
+                if (NB < 128) g /= BN / NB;
+                for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti) {
                     const int k = plan.t[ti].k, num_kb = (k + KB - 1) / KB;
-                    const int buf = (int)(tcount & 1);
-                    const uint32_t use = (uint32_t)((tcount >> 1) & 1);
-                    ok = mbar_wait(tempty_bar(buf), use ^ 1u, abort_flag);  // epilogue has drained this accumulator
+                    ok = mbar_wait_warp(tempty_bar(buf), free_ph, abort_flag);  // epilogue has drained this accumulator
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols);
-                    for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                        const int s = (int)(it % kStages);
-                        const uint32_t ph = (uint32_t)((it / kStages) & 1);
-                        ok = mbar_wait(full_bar(s), ph, abort_flag);
+                    const uint32_t acc = tmem_base + (uint32_t)(buf * kAccCols<NB>);
+                    for (int kb = 0; kb < num_kb; ++kb) {
+                        ok = mbar_wait_warp(full_bar(s), ph, abort_flag);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        // W_hi | W_lo are adjacent: one 256-wide MMA on a_hi gives a_hi*w_hi (main accumulator) and
-                        // a_hi*w_lo (correction accumulator); a 128-wide MMA adds a_lo*w_hi to the correction
-                        const uint64_t da_hi = smem_desc128(part_addr(s, 0)), da_lo = smem_desc128(part_addr(s, 1));
-                        const uint64_t dw = smem_desc128(part_addr(s, 2));
+                        // W_hi | W_lo are adjacent: one MMA of 2 NB columns on a_hi gives a_hi*w_hi (main accumulator) and
+                        // a_hi*w_lo (correction accumulator); one of NB columns adds a_lo*w_hi to the correction
+                        const uint64_t da = desc0 + (uint64_t)(s * (kStageBytes<NB> >> 4));
                         const int steps = (k - kb * KB + 15) / 16;  // columns past k belong to a neighbour: not multiplied
+                        if (elect_one()) {
+                            constexpr uint64_t kLo = kPart >> 4, kW = 2 * kLo;
+                            umma_one<2 * NB, false>(acc, da, da + kW, kb > 0);
+                            umma_one<NB, true>(acc + NB, da + kLo, da + kW, 1u);
+                            if (steps >= KB / 16) {
 #pragma unroll
-                        for (int j = 0; j < KB / 16; ++j) {
-                            if (j >= steps) break;
-                            const uint64_t adv = (uint64_t)(j * 2);
-                            const uint32_t first = (kb > 0 || j > 0) ? 1u : 0u;
-                            umma_f16<2 * BN>(acc, da_hi + adv, dw + adv, first);
-                            umma_f16<BN>(acc + BN, da_lo + adv, dw + adv, 1u);
+                                for (uint64_t j = 2; j < KB / 8; j += 2) {
+                                    umma_one<2 * NB, true>(acc, da + j, da + j + kW, 1u);
+                                    umma_one<NB, true>(acc + NB, da + j + kLo, da + j + kW, 1u);
+                                }
+                            } else {
+                                for (int j = 1; j < steps; ++j) {
+                                    const uint64_t d = da + (uint64_t)(2 * j);
+                                    umma_one<2 * NB, true>(acc, d, d + kW, 1u);
+                                    umma_one<NB, true>(acc + NB, d + kLo, d + kW, 1u);
+                                }
+                            }
+                            umma_commit(empty_bar(s));
                         }
-                        umma_commit(empty_bar(s));
+                        __syncwarp();
+                        if (++s == kRing) s = 0, ph ^= 1;
                     }
-                    if (ok) umma_commit(tfull_bar(buf));
+                    if (ok && elect_one()) umma_commit(tfull_bar(buf));
+                    __syncwarp();
+                    if (buf) free_ph ^= 1;
+                    buf ^= 1;
                 }
             }
         }
@@ -486,53 +512,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-// Gate gradients of a backward launch whose rows ran one by one: per degree sum_r raw_r y_r in row order (the fused
-// multiply-adds of the in-epilogue sum), times the gate's slope, as planes.  One warp per row of the matrix.
-struct GateSums {
-    int32_t degrees, hidden_silu;
-    int16_t gate_col[8], begin[9];
-    int16_t raw_col[kMaxTiles], y_col[kMaxTiles];
-};
-__global__ void __launch_bounds__(256) gate_sum_kernel(const __grid_constant__ GateSums g, const __grid_constant__ Params prm) {
-    pdl_sync();
-    const int lane = threadIdx.x & 31, c = lane * 4;
-    const float o_scale = prm.o_scale ? *prm.o_scale : 1.0f;
-    __half2 top = __floats2half2_rn(0.f, 0.f);
-    for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < prm.m_total; row += (int64_t)gridDim.x * 8) {
-        const float* y = prm.y + row * prm.ldy + c;
-        const float* raw = prm.raw + row * prm.raw_ld + c;
-        for (int d = 0; d < g.degrees; ++d) {
-            f32x2 s0 = 0, s1 = 0, g0, g1;
-            load_pair(y + g.gate_col[d], g0, g1);
-            for (int r = g.begin[d]; r < g.begin[d + 1]; ++r) {
-                f32x2 x0, x1, y0, y1;
-                load_pair(raw + g.raw_col[r], x0, x1);
-                load_pair(y + g.y_col[r], y0, y1);
-                s0 = fma2(x0, y0, s0), s1 = fma2(x1, y1, s1);
-            }
-            auto slope = [&](float v) {
-                float k = 1.f;
-                if (g.hidden_silu) {
-                    const float q = sigmoid_f(v);
-                    k = q * (1.f + v * (1.f - q));
-                    v *= q;
-                }
-                const float q = sigmoid_f(v);
-                return k * q * (1.f - q) * o_scale;
-            };
-            store_split(prm.o_hi + row * prm.ldo + c, prm.o_lo + row * prm.ldo + c, g.gate_col[d], mul2(s0, map2(g0, slope)), mul2(s1, map2(g1, slope)), true, top);
-        }
-    }
-    if (!(__half2float(__hmax_nan(__low2half(top), __high2half(top))) <= kHalfMax) && prm.status) atomicCAS(prm.status, 0, 2);
-}
-
-// 2-D row-major half matrix [rows, cols], row stride ld elements; box = 64 columns x 128 rows, 128-byte swizzle
-static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld) {
+// 2-D row-major half matrix [rows, cols], row stride ld elements; box = 64 columns, 128-byte swizzle
+static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return FCB200_EINVAL;
     cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t gstride[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)KB, (cuuint32_t)BM};
+    cuuint32_t box[2] = {(cuuint32_t)KB, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -544,8 +530,7 @@ static int map_half(CUtensorMap* map, const void* ptr, int64_t rows, int64_t col
 // How a tile list is cut into groups (Plan::groups); a CTA takes (row tile, group) items in turn.
 //   natural  what shares nothing is apart: every plain tile, row 0, and the rows of a degree with their gate tile (forward)
 //            or their gate-gradient sum (backward)
-//   fine     gated rows one by one: forward each after its own copy of the gate tile (the gate is computed again), backward
-//            with the gate-gradient sums left to a second kernel
+//   fine     forward gated rows one by one, each after its own copy of the gate tile (the gate is computed again)
 //   pair     natural groups on CTA pairs, tiles that read the same columns side by side (so2_conv_pair.cu)
 enum Grouping { kAuto = 0, kNatural = 1, kFine = 2, kPair = 3 };
 
@@ -554,13 +539,12 @@ struct Groups {
     int groups = 0;
     int16_t begin[kMaxPlan + 1] = {};
     int16_t tile[kMaxPlan] = {};  // index into the caller's list
-    int cost[kMaxPlan] = {};      // of a group, in units of K
     bool ok = true;
 };
 
-// a tile's fixed share (epilogue, ring start-up) in units of its K extent, from launches of one row tile; of a tile on a pair
-// of CTAs, whose K extent counts 0.8 where it has a partner (see the choice of the form)
-constexpr int kTileCost = 192, kPairTileCost = 230;
+// Units of K: what a tile's K extent counts in items of 128, 64 and 32 columns (percent), a tile's fixed share (epilogue, ring
+// start-up), the same with the gate's backward, and of a tile on a pair of CTAs; from launches of one row tile.
+constexpr int kStepCost[3] = {100, 70, 58}, kTileCost[3] = {192, 150, 130}, kBackwardTileCost[3] = {416, 183, 143}, kPairTileCost = 250;
 
 static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
     Groups g;
@@ -570,7 +554,6 @@ static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
             return;
         }
         g.tile[g.n++] = (int16_t)i;
-        g.cost[g.groups] += t[i].k + kTileCost;
     };
     auto close = [&] { g.begin[++g.groups] = (int16_t)g.n; };
     auto gate_of = [&](int col) {
@@ -602,7 +585,7 @@ static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
             for (int j = i; j < n; ++j) {
                 put(j);
                 done[j] = true;
-                if ((t[j].flags & kLast) || how == kFine) break;
+                if (t[j].flags & kLast) break;
             }
         } else {
             put(i);
@@ -610,24 +593,6 @@ static Groups group_tiles(const Tile* t, int n, int rot_begin, int how) {
         close();
     }
     return g;
-}
-
-// rows of every degree of a backward list and where their raw values go
-static bool split_sums(Tile* t, int n, GateSums& g) {
-    int rows = 0;
-    for (int i = 0; i < n; ++i) {
-        if (t[i].mode != kGatedBwd) continue;
-        if (t[i].flags & kFirst) {
-            if (g.degrees == 8) return false;
-            g.gate_col[g.degrees++] = t[i].gate_col;
-            g.hidden_silu = (t[i].flags & kGateSilu) != 0;
-        }
-        if (!g.degrees || t[i].gate_col != g.gate_col[g.degrees - 1]) return false;
-        t[i].raw_col = (int16_t)(rows * BN);
-        g.raw_col[rows] = t[i].raw_col, g.y_col[rows] = t[i].y_col;
-        g.begin[g.degrees] = (int16_t)++rows;
-    }
-    return g.degrees > 0;
 }
 
 // Natural groups for CTA pairs: tiles of a group two by two where they follow one another and read the same columns; groups
@@ -665,18 +630,27 @@ static PairGroups pair_tiles(const Tile* t, const Groups& g) {
     return out;
 }
 
-// longest of `units` CTAs or pairs, in units of K
-static int64_t makespan(const Order& order, const int* cost, int units) {
+// Longest of `units` CTAs or pairs, in units of K; an item's group is one of `subs` parts of a group of tiles.
+static int64_t makespan(const Order& order, const int* cost, int subs, int units) {
     const int64_t items = order.rows * order.groups;
     int64_t total = 0, most = 0;
-    for (int i = 0; i < order.groups; ++i) total += cost[i], most = cost[i] > most ? cost[i] : most;
-    if (items > 16LL * units * order.groups) return order.rows * total / units + most;
-    int64_t worst = 0, row;
-    int g;
-    for (int c = 0; c < units && c < items; ++c) {
-        int64_t sum = 0;
-        for (int64_t n = 0; order.item(n, units, c, row, g); ++n) sum += cost[g];
-        worst = sum > worst ? sum : worst;
+    for (int i = 0; i < order.groups; ++i) total += cost[i / subs], most = cost[i / subs] > most ? cost[i / subs] : most;
+    if (units > 256 || items > 32LL * units) return order.rows * total / units + most;
+    if (items <= units) return most;
+    int64_t sum[256] = {}, worst = 0;
+    int unit = 0, step = 1, row = 0, group = 0;
+    for (int64_t i = 0; i < items; ++i) {
+        sum[unit] += cost[group / subs];
+        worst = sum[unit] > worst ? sum[unit] : worst;
+        unit += step;
+        if (unit == units || unit < 0) {  // the next round: from the first unit, or back from the last
+            unit = order.snake ? unit - step : 0;
+            step = order.snake ? -step : 1;
+        }
+        if (order.snake ? ++row == order.rows : ++group == order.groups) {
+            group = order.snake ? group + 1 : 0;
+            row = 0;
+        }
     }
     return worst;
 }
@@ -684,22 +658,23 @@ static int64_t makespan(const Order& order, const int* cost, int units) {
 // The order of a launch's items and its makespan.  perm: the groups by falling cost.  Group by group an A tile leaves L2
 // between its groups when there are many rows, so that has to gain more than the extra reads cost (first convolution, lmax 2,
 // us row by row / group by group: 7 680 rows 90 / 68, 20 580 rows 188 / 182, 40 000 rows 332 / 353).
-static int64_t choose_order(Order& order, int* cost, int* perm, int units) {
-    for (int i = 0; i < order.groups; ++i) perm[i] = i;
-    const int64_t by_row = makespan(order, cost, units), items = order.rows * order.groups;
+static int64_t choose_order(Order& order, int* cost, int* perm, int subs, int units) {
+    const int groups = order.groups / subs;
+    for (int i = 0; i < groups; ++i) perm[i] = i;
+    const int64_t by_row = makespan(order, cost, subs, units), items = order.rows * order.groups;
     if (items > 8LL * units || items <= units) return by_row;
     int sorted[kMaxPlan], at[kMaxPlan];
-    for (int i = 0; i < order.groups; ++i) {
+    for (int i = 0; i < groups; ++i) {
         int j = i;
         for (; j > 0 && cost[i] > sorted[j - 1]; --j) sorted[j] = sorted[j - 1], at[j] = at[j - 1];
         sorted[j] = cost[i], at[j] = i;
     }
     Order snake = order;
     snake.snake = 1;
-    const int64_t by_group = makespan(snake, sorted, units);
+    const int64_t by_group = makespan(snake, sorted, subs, units);
     if (100 * by_group >= 96 * by_row) return by_row;
     order = snake;
-    for (int i = 0; i < order.groups; ++i) cost[i] = sorted[i], perm[i] = at[i];
+    for (int i = 0; i < groups; ++i) cost[i] = sorted[i], perm[i] = at[i];
     return by_group;
 }
 static PairPlan reordered(const PairPlan& p, const int* perm) {
@@ -711,17 +686,23 @@ static PairPlan reordered(const PairPlan& p, const int* perm) {
     }
     return q;
 }
-// Groups on single CTAs with the order of their items.
+// Groups on single CTAs, `width` of each tile's 128 columns an item, with the order of their items.
 struct Schedule {
     Groups g;
+    int width, perm[kMaxPlan];
     Order order;
-    int perm[kMaxPlan];
     int64_t span;
-    Schedule(const Groups& groups, int64_t rows) : g(groups), order{rows, groups.groups, 0} { span = choose_order(order, g.cost, perm, sm_count()); }
+    Schedule(const Groups& groups, const Tile* list, int64_t rows, int w) : g(groups), width(w), order{rows, groups.groups * (BN / w), 0} {
+        const int at = w == 128 ? 0 : w == 64 ? 1 : 2;
+        int cost[kMaxPlan] = {};
+        for (int i = 0; i < g.groups; ++i)
+            for (int j = g.begin[i]; j < g.begin[i + 1]; ++j) cost[i] += list[g.tile[j]].k * kStepCost[at] / 100 + (list[g.tile[j]].mode == kGatedBwd ? kBackwardTileCost : kTileCost)[at];
+        span = choose_order(order, cost, perm, BN / w, sm_count());
+    }
     void fill(Plan& plan, const Tile* list) const {
         plan.order = order;
         int n = 0;
-        for (int i = 0; i < order.groups; ++i) {
+        for (int i = 0; i < g.groups; ++i) {
             for (int j = g.begin[perm[i]]; j < g.begin[perm[i] + 1]; ++j) plan.t[n++] = list[g.tile[j]];
             plan.begin[i + 1] = (int16_t)n;
         }
@@ -740,7 +721,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
                                      const float* w_scale, const float* const* bias, const int32_t* tiles, int32_t num_tiles,
                                      int32_t rot_begin, float* y, int64_t ldy, int64_t y_cols, void* o_hi, void* o_lo, int64_t ldo, int64_t o_cols,
                                      const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status,
-                                     void* stream, float* raw) {
+                                     void* stream) {
     using namespace fused;
     if (!a_hi || !a_lo || !w_hi || !w_lo || !w_rows || !w_cols || !w_scale || !tiles || !y || m < 0) return FCB200_EINVAL;
     Plan plan{};
@@ -793,60 +774,59 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         }
     // Row tiles times natural groups are the items: CTAs that run together share an A tile in L2 and the last wave is one
     // group deep, not one list (M = 131 072, second convolution: 417 us row tile by row tile, 377 so; M = 60 000, first
-    // convolution: 528 / 446).  Few row tiles still leave SMs without work; then the gated rows go one by one where that
-    // shortens the longest CTA by more than the estimate's error (M = 7 680: 104 -> 87 us, M = 640: 59 -> 36 us).
+    // convolution: 528 / 446).  Few row tiles leave SMs without work; then the gated rows of a forward list go one by one,
+    // and an item takes a part of its tiles' columns, where that shortens the longest CTA by more than the estimate's error.
+    // us, 128 / 64 / 32 columns: 420 rows of lmax 2, first convolution row by row 20.4 / 16.0 / 15.0, second 8.8 / 7.2 / 6.8, its
+    // gated backward 29.5 / 18.8 / 16.4, radial output layer's backward 15.9 / 12.7 / 11.6; 3 000 rows 34.4 / 37.3 / 56.7, 13.3 / 14.1 /
+    // 20.6, 30.1 / 19.7 / 22.8, 16.0 / 13.1 / 12.2; 7 680 rows, gated backward 36.9 / 38.3 / 53.0.
     const int64_t rows_m = (m + BM - 1) / BM;
     const Groups natural = group_tiles(list, num_tiles, rot_begin, kNatural);
     if (!natural.ok) return FCB200_EINVAL;
-    const auto fine = [&] { return Schedule(group_tiles(list, num_tiles, rot_begin, kFine), rows_m); };
-    Schedule run = grouping == kFine && !backward ? fine() : Schedule(natural, rows_m);
-    if (!run.g.ok) return FCB200_EINVAL;
-    if (grouping == kAuto && gated) {
-        const Schedule rows = fine();
-        if (rows.g.ok && 10 * rows.span < 9 * run.span) run = rows;
+    Schedule run(natural, list, rows_m, BN);
+    if (!backward && grouping == kFine) {
+        run = Schedule(group_tiles(list, num_tiles, rot_begin, kFine), list, rows_m, BN);
+        if (!run.g.ok) return FCB200_EINVAL;
     }
-    // On pairs a listed tile costs 0.8 of its K extent where it has a partner, and 230 for the time the tensor core waits for
+    if (grouping == kAuto) {
+        auto consider = [&](const Groups& g, int width) {
+            if (!g.ok || (width < BN && rows_m * g.groups * (BN / width) > 2 * sm_count())) return;
+            const Schedule other(g, list, rows_m, width);
+            if (10 * other.span < 9 * run.span) run = other;
+        };
+        const Groups fine = gated ? group_tiles(list, num_tiles, rot_begin, kFine) : Groups{};
+        for (int width = BN; width >= 32; width /= 2) {
+            if (width < BN) consider(natural, width);
+            if (gated) consider(fine, width);
+        }
+    }
+    // On pairs a listed tile costs 0.8 of its K extent where it has a partner, and 250 for the time the tensor core waits for
     // the accumulators; alone a tile costs its K extent and 192.  So long K goes to pairs, the radial output layer (K = 128)
-    // and small launches do not.  us, alone / on pairs: first convolution, lmax 2, 7 680 rows 98 / 68, 20 580 rows 203 / 182,
-    // 131 072 rows 1122 / 1034; lmax 4, 3 240 rows 117 / 106, 60 000 rows 1930 / 1701; second convolution, lmax 2, 20 580 rows
-    // 74 / 76, 131 072 rows 466 / 430; first convolution's backward, 131 072 rows 1004 / 913; radial output layer, 131 072
-    // rows 260 / 272.  (Seconds of back-to-back launches, at the power cap from some 10 000 rows on.)
-    const bool pairs_only = grouping == kPair;
+    // and small launches do not.  us, alone / on pairs (seconds of back-to-back launches, at the power cap): first convolution,
+    // lmax 2, 20 580 rows 201 / 179, 131 072 rows 1079 / 1000; lmax 4, 7 000 rows 235 / 217, 60 000 rows 1815 / 1638; second
+    // convolution, lmax 2, 20 580 rows 73 / 76, 131 072 rows 437 / 417; first convolution's backward, 13 000 rows 100 / 99, 131 072
+    // rows 950 / 879; radial output layer, 131 072 rows 260 / 272.
     PairGroups two;
-    if (!backward && (pairs_only || (grouping == kAuto && rows_m >= 8))) {  // the fewest rows: no time for the estimate
+    if (!backward && (grouping == kPair || (grouping == kAuto && rows_m >= 8))) {  // the fewest rows: no time for the estimate
         two = pair_tiles(list, natural);
         two.plan.order.rows = (m + 2 * BM - 1) / (2 * BM);
         int perm[kMaxPlan];
-        const int64_t span = choose_order(two.plan.order, two.cost, perm, sm_count() / 2);
-        if (!pairs_only && span >= run.span) two.plan.order.groups = 0;
+        const int64_t span = choose_order(two.plan.order, two.cost, perm, 1, sm_count() / 2);
+        if (grouping != kPair && span >= run.span) two.plan.order.groups = 0;
         else if (two.plan.order.snake) two.plan = reordered(two.plan, perm);
     }
     const bool on_pairs = two.plan.order.groups > 0;
-    // backward: rows one by one as above, if there is room for the raw rows and the second kernel pays: about 3 us, 300 units of
-    // K, and its reads and the raw rows' writes at the memory's rate, 55 KB a unit.  A row on its own costs 1.6 times its
-    // estimate (its factors are made anew and nothing overlaps its epilogue), one in a group 1.1 times.
-    GateSums sums{};
-    bool solo = backward && raw && grouping != kNatural && split_sums(list, num_tiles, sums);
-    if (solo && grouping != kFine) {
-        const int64_t extra = 300 + m * (sums.begin[sums.degrees] + sums.degrees) * (BN * 8) / 55000;
-        solo = 16 * fine().span + 10 * extra < 11 * run.span;
-    }
-    if (solo) {
-        for (int i = 0; i < num_tiles; ++i)
-            if (list[i].mode == kGatedBwd) list[i].flags |= kSolo;
-        run = fine();
-    }
+    const int width = run.width;
     run.fill(plan, list);
     CUtensorMap mah, mal, mw[6];
-    int rc = on_pairs ? FCB200_OK : map_half(&mah, a_hi, m, a_cols, lda);
-    if (!rc && !on_pairs) rc = map_half(&mal, a_lo, m, a_cols, lda);
+    int rc = on_pairs ? FCB200_OK : map_half(&mah, a_hi, m, a_cols, lda, BM);
+    if (!rc && !on_pairs) rc = map_half(&mal, a_lo, m, a_cols, lda, BM);
     int first = -1;
     for (int i = 0; i < 3 && !rc; ++i) {
         if (!used[i]) continue;
         if (first < 0) first = i;
         if (w_cols[i] % 8 || !aligned16(w_hi[i]) || !aligned16(w_lo[i]) || !(w_scale[i] > 0.f)) return FCB200_EINVAL;
-        if (!on_pairs) rc = map_half(&mw[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i]);
-        if (!rc && !on_pairs) rc = map_half(&mw[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i]);
+        if (!on_pairs) rc = map_half(&mw[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i], width);
+        if (!rc && !on_pairs) rc = map_half(&mw[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i], width);
         prm.w_scale[i] = w_scale[i];
         prm.bias[i] = bias ? bias[i] : nullptr;
         if (prm.bias[i] && (!aligned16(prm.bias[i]) || w_rows[i] % BN)) return FCB200_EALIGN;
@@ -861,25 +841,26 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
     prm.y = y, prm.ldy = (int32_t)ldy, prm.y_cols = (int32_t)y_cols, prm.a_scale = a_scale, prm.o_scale = o_scale;
     prm.o_hi = static_cast<__half*>(o_hi), prm.o_lo = static_cast<__half*>(o_lo), prm.ldo = (int32_t)ldo;
     prm.m_total = m, prm.status = status;
-    prm.raw = raw, prm.raw_ld = sums.begin[sums.degrees] * BN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (on_pairs) return launch_pair(two.plan, prm, a_hi, a_lo, lda, a_cols, w_hi, w_lo, w_rows, w_cols, used, o_cols, forward, st);
     const int64_t items = plan.order.rows * plan.order.groups;
     const int grid = (int)(items < sm_count() ? items : sm_count());
-    auto launch = [&](auto kernel, bool (&done)[64]) {
-        if (const int arc = ensure_dynamic_smem(kernel, kSmemBytes, done)) return arc;
-        launch_pdl(kernel, dim3(grid), dim3(kThreads), kSmemBytes, st, mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm);
+    auto launch = [&](auto kind, auto columns) {
+        constexpr int KIND = decltype(kind)::value, NB = decltype(columns)::value, bytes = kSmemBytes<NB>;
+        static bool done[64] = {};
+        const auto kernel = so2_conv_fused_kernel<KIND, NB>;
+        if (const int arc = ensure_dynamic_smem(kernel, bytes, done)) return arc;
+        launch_pdl(kernel, dim3(grid), dim3(kThreads), bytes, st, mah, mal, mw[0], mw[1], mw[2], mw[3], mw[4], mw[5], plan, prm);
         return launch_status();
     };
-    static bool done[3][64] = {};
-    if (forward) return launch(so2_conv_fused_kernel<kForwardKind>, done[0]);
-    if (backward) {
-        const int brc = launch(so2_conv_fused_kernel<kBackwardKind>, done[1]);
-        if (brc || !solo) return brc;
-        launch_pdl(gate_sum_kernel, dim3(warp_grid(m, 8)), dim3(256), 0, st, sums, prm);
-        return launch_status();
-    }
-    return launch(so2_conv_fused_kernel<kPlainKind>, done[2]);
+    auto by_width = [&](auto kind) {
+        if (width == 32) return launch(kind, std::integral_constant<int, 32>{});
+        if (width == 64) return launch(kind, std::integral_constant<int, 64>{});
+        return launch(kind, std::integral_constant<int, 128>{});
+    };
+    if (forward) return by_width(std::integral_constant<int, kForwardKind>{});
+    if (backward) return by_width(std::integral_constant<int, kBackwardKind>{});
+    return by_width(std::integral_constant<int, kPlainKind>{});
 }
 
 }  // namespace fcb200
@@ -891,5 +872,5 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
                                      const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status,
                                      void* stream) {
     return so2_conv_fused(a_hi, a_lo, lda, a_cols, w_hi, w_lo, w_rows, w_cols, w_scale, bias, tiles, num_tiles, rot_begin, y, ldy, y_cols, o_hi, o_lo, ldo,
-                          o_cols, a_scale, o_scale, m, variant, status, stream, nullptr);
+                          o_cols, a_scale, o_scale, m, variant, status, stream);
 }

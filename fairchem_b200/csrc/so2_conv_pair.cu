@@ -14,9 +14,9 @@
 // through the warp's 4 KiB of shared memory as a TMA store (whole lines, rows past the end are clipped).
 //
 // What bounds it at size is the power cap: back to back launches of either form run at 985 W, so what counts is energy, and
-// half the operand traffic is what this form saves.  us and mJ a launch, alone -> on pairs: first convolution, lmax 2, 131 072
-// rows 1122 / 1120 -> 1034 / 1016, lmax 4, 60 000 rows 1930 / 1908 -> 1701 / 1644; second convolution, lmax 2, 131 072 rows 466 / 451
-// -> 430 / 428; first convolution's backward 1004 / 984 -> 913 / 895.
+// half the operand traffic is what this form saves.  us and mJ a launch, alone / on pairs: first convolution, lmax 2, 131 072
+// rows 1079 / 1075, 1000 / 990; lmax 4, 60 000 rows 1815 / 1794, 1638 / 1616; second convolution, lmax 2, 131 072 rows 437 / 436,
+// 417 / 409; first convolution's backward 950 / 934, 879 / 864.
 #include "so2_conv.cuh"
 
 namespace fcb200 {
@@ -227,25 +227,28 @@ __device__ __forceinline__ void epilogue(const Maps& maps, const PairPlan& plan,
     if (!(__half2float(__hmax_nan(__low2half(top), __high2half(top))) <= kHalfMax)) *range_flag = 1;  // inf or NaN
 }
 
-// All products of one tile.  s, ph: ring stage that comes next and its parity.
+// All products of one tile, issued by one lane of a warp that walks the loop as one (see so2_conv_fused.cu).  s, ph: ring stage that comes next and its parity.
 template <int N>
 __device__ __forceinline__ bool tile_products(uint64_t desc0, uint32_t tmem, int k, uint32_t full0, uint32_t empty0, int& s, uint32_t& ph, volatile int* abort_flag) {
     constexpr uint64_t kLo = kPart >> 4, kW = 2 * (kPart >> 4), kStep = 2;  // in a stage, 16-byte units
     const int num_kb = (k + KB - 1) / KB, tail = (k - (num_kb - 1) * KB + 15) / 16;  // columns past k belong to a neighbour
     for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(full0 + 8u * s, ph, abort_flag)) return false;  // both CTAs' operands have landed
+        if (!mbar_wait_warp(full0 + 8u * s, ph, abort_flag)) return false;  // both CTAs' operands have landed
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t d = desc0 + (uint64_t)(s * (kStageBytes >> 4));
         const int steps = kb + 1 == num_kb ? tail : KB / 16;
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < KB / 16; ++j) {
-            if (j >= steps) break;
-            const uint32_t add = kb > 0 || j > 0;
-            umma_f16_pair<N>(tmem, d + j * kStep, d + kW + j * kStep, add);
-            umma_f16_pair<N>(tmem + kCorr, d + j * kStep, d + kW + kLo + j * kStep, add);
-            umma_f16_pair<N>(tmem + kCorr, d + kLo + j * kStep, d + kW + j * kStep, 1u);
+            for (int j = 0; j < KB / 16; ++j) {
+                if (j >= steps) break;
+                const uint32_t add = kb > 0 || j > 0;
+                umma_f16_pair<N>(tmem, d + j * kStep, d + kW + j * kStep, add);
+                umma_f16_pair<N>(tmem + kCorr, d + j * kStep, d + kW + kLo + j * kStep, add);
+                umma_f16_pair<N>(tmem + kCorr, d + kLo + j * kStep, d + kW + j * kStep, 1u);
+            }
+            umma_commit_pair(empty0 + 8u * s);
         }
-        umma_commit_pair(empty0 + 8u * s);
+        __syncwarp();
         if (++s == kStages) s = 0, ph ^= 1;
     }
     return true;
@@ -269,7 +272,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     volatile int* range_flag = reinterpret_cast<volatile int*>(bar_generic + 8 * (2 * kStages + 2) + 8);
     auto part_addr = [&](int s, int which) { return base + s * kStageBytes + which * kPart; };
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(kFull, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
 
@@ -292,6 +295,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    if (warp == 2 && lane < 11) prefetch_map(lane < 2 ? &maps.a[lane] : lane < 8 ? &maps.w[lane - 2] : lane == 8 ? &maps.y : &maps.o[lane - 9]);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync_all();  // both CTAs' barriers are initialised before either signals the other
@@ -338,7 +342,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
             }
         }
-        if (warp == 1 && lane == 0 && leader) {
+        if (warp == 1 && leader) {
             int s = 0;
             uint32_t ph = 0, acc_free = 1;
             bool ok = true;
@@ -347,13 +351,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             int g;
             for (int64_t n = 0; ok && plan.order.item(n, gridDim.x >> 1, blockIdx.x >> 1, mt, g); ++n) {
                 for (int ti = plan.begin[g]; ti < plan.begin[g + 1] && ok; ++ti, acc_free ^= 1) {
-                    ok = mbar_wait(tempty, acc_free, abort_flag);  // both epilogues have emptied the accumulators
+                    ok = mbar_wait_warp(tempty, acc_free, abort_flag);  // both epilogues have emptied the accumulators
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const int k = plan.t[ti].k;
                     if (plan.t[ti].n > 1) ok = tile_products<2 * BN>(desc0, tmem_base, k, full_bar(0), empty_bar(0), s, ph, abort_flag);
                     else ok = tile_products<BN>(desc0, tmem_base, k, full_bar(0), empty_bar(0), s, ph, abort_flag);
-                    if (ok) umma_commit_pair(tfull);
+                    if (ok && elect_one()) umma_commit_pair(tfull);
+                    __syncwarp();
                 }
             }
         }

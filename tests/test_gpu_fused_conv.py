@@ -84,7 +84,7 @@ def test_fused_convolutions_match_the_separate_kernels(ops, grouping, lmax, e):
 
 
 def _launches(ops, lmax, e, form):
-    """Outputs of every kind of launch that may run on pairs of CTAs, on inputs that depend on (lmax, e) alone."""
+    """Outputs of every kind of launch, on inputs that depend on (lmax, e) alone."""
     from fairchem_b200 import backbone as B
 
     c, nm = 128, ops.SHAPES[lmax].nm
@@ -108,6 +108,8 @@ def _launches(ops, lmax, e, form):
             ak = B._fused_conv1_gate(ew, m, None)
             msg = B._fused_conv2(ew, a, torch.full((e, nm * c), float("nan"), device="cuda"))
             gm = B._fused_conv1_backward(ew, gy, scale)
+            gmsg = _planes(draw(e, nm * c) * 1e-3, 64.0)
+            gc = B._fused_conv2_gate_backward(ew, gmsg, y, scale)
             y2 = torch.full((e, 448), float("nan"), device="cuda")
             ops.so2_conv_fused_.raw(m[0], m[1], [hi], [lo], [sc], None, tiles, 0, y2, None, None, None, None, status)
             hi, lo, sc = ops.split_f16(torch.cat([short, short[:64]]))
@@ -117,13 +119,14 @@ def _launches(ops, lmax, e, form):
             ops.CONV_GROUPING = 0
     B.check_gemm_status()
     assert int(status) == 0
-    return [y, a[0], a[1], ak[0], ak[1], msg, gm, y2, y3]
+    return [y, a[0], a[1], ak[0], ak[1], msg, gm, gc[0], gc[1], y2, y3]
 
 
-# one row, both sides of a warp's, a CTA's and a pair's rows, items group by group (7 680) and row by row
+# one row, both sides of a warp's, a CTA's and a pair's rows; items of 32 and 64 columns (up to 1 000 rows, by the list),
+# group by group (7 680) and row by row
 @pytest.mark.parametrize("lmax,e", [(2, e) for e in (1, 32, 33, 128, 129, 255, 256, 257, 1000, 7680, 21000)] + [(4, 129), (4, 257), (4, 3240)])
-def test_pairs_of_ctas_give_the_same_bits(ops, lmax, e):
-    """Same products in the same order on either form, and every output element written."""
+def test_pairs_of_ctas_and_narrow_items_give_the_same_bits(ops, lmax, e):
+    """Same products in the same order in every form, and every output element written."""
     alone = _launches(ops, lmax, e, 1)
     for form in (0, 3):
         for got, want in zip(_launches(ops, lmax, e, form), alone):
