@@ -345,10 +345,12 @@ static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, co
     // (us of an evaluation, lmax 2: 1 296 nodes 688 -> 656, 1 782 1026 -> 904, 2 000 1198 -> 1002, 2 592 1384 -> 1259, 4 050 2076 ->
     // 1951; where it does not: 1 440 731 -> 771, 3 120 1496 -> 1529, 5 280 2414 -> 2545; lmax 4, 2 048 nodes 9662 -> 7773).
     // More nodes come in several chunks, which hold too few edges of a source to share.
-    const int64_t n = n1 - n0, sms = sm_count(), waves = (n + 12 * sms - 1) / (12 * sms), quarters = (n + 3 * sms - 1) / (3 * sms);
-    if (share_node(n)) {
+    // Fewer nodes: eight warps to a node, one block on an SM, unless four and three blocks take fewer rounds; a round of those
+    // lasts 2.05 times as long (us a launch, 256 nodes 24.5 / 24.5, 686 nodes 56.8 / 50.6; lmax 4, 108 nodes 35 / 73).
+    const int64_t n = n1 - n0, sms = sm_count(), waves = (n + 12 * sms - 1) / (12 * sms), quarters = (n + 3 * sms - 1) / (3 * sms), rounds = (n + sms - 1) / sms;
+    if (share_node(n) && 20 * rounds <= 41 * quarters) {
         FCB_TRY(shared(std::integral_constant<int, 8>{}, done[0]));
-    } else if (waves <= 3 && 11 * quarters < 40 * waves) {
+    } else if (share_node(n) || (waves <= 3 && 11 * quarters < 40 * waves)) {
         FCB_TRY(shared(std::integral_constant<int, 4>{}, done[2]));
     } else {
         FCB_TRY(raise_smem(gather_bwd_kernel<LMAX, HALF, 1, OutSplit>, alone, done[1]));
