@@ -64,17 +64,17 @@ struct Params {
     int32_t* status;
 };
 
-// Work items are row tiles times groups of tiles; `units` CTAs or pairs take them in turn, either row by row (those that run
-// together share an A tile in L2), or, `snake`, group by group with the costly groups first and dealt to and fro, which
-// leaves the last wave short where there are few items.
+// Work items are row tiles times groups of tiles; `units` CTAs or pairs take them in turn, to and fro, either row by row (those
+// that run together share an A tile in L2; to and fro, no unit is left with the costlier of two groups) or, by_group, group by
+// group with the costly groups first, which leaves the last wave short where there are few items.
 struct Order {
     int64_t rows;
-    int32_t groups, snake;
+    int32_t groups, by_group;
     // n-th item of a unit: its row tile and group; false past the last
     __host__ __device__ bool item(int64_t n, int64_t units, int64_t unit, int64_t& row, int& group) const {
-        const int64_t i = n * units + (snake && (n & 1) ? units - 1 - unit : unit);
+        const int64_t i = n * units + (n & 1 ? units - 1 - unit : unit);
         if (i >= rows * groups) return false;
-        if (snake) {
+        if (by_group) {
             group = (int)(i / rows);
             row = i - group * rows;
         } else {
