@@ -289,6 +289,31 @@ def test_layers_that_keep_nothing_per_edge_give_the_same_result(cfg, drop, wants
         assert _rel(got[k], ref[k]) < 1e-6, k
 
 
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+@pytest.mark.parametrize("chunk", [129, 700, 131072])  # items of 32, 64 and 128 columns, rows past the last full tile
+def test_gate_gradients_from_kept_planes_and_from_kept_rows_agree(cfg, chunk, monkeypatch):
+    """With everything kept the gate's backward reads the gated rows as half planes (22 bits: 2.4e-7 of each term), with the
+    radial weights dropped the raw rows in float32."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import step, synthetic
+
+    bb, head = _model(B, cfg, edge_chunk_size=chunk)
+    data = synthetic.merge([synthetic.fcc_cu((3, 3, 4), seed=8), synthetic.molecule_batch(2, 5, 30, seed=9)]).to("cuda")
+    d = data.clone()
+    ref = head(d, bb(d))
+
+    def no_radial(run):
+        run.ev.keep_radial, run.ev.drop_layers = 0, 0
+        step._lib.call("fcb200_model_sizes", step.byref(run.model), step.byref(run.ev), run.sizes)
+        return True
+
+    monkeypatch.setattr(step.BackboneStep, "plan_memory", no_radial)
+    d = data.clone()
+    got = head(d, bb(d))
+    assert torch.equal(got["energy"], ref["energy"])
+    assert _rel(got["forces"], ref["forces"]) < 1e-6
+
+
 @pytest.mark.parametrize("skin", [0.0, 0.5])
 def test_without_the_memory_the_per_op_path_takes_over_the_graph(skin, monkeypatch):
     from fairchem_b200 import backbone as B
