@@ -327,14 +327,22 @@ template <class K> static int raise_smem(K kernel, int bytes, bool (&done)[64]) 
 
 template <int LMAX, int MODE>
 static int launch_rotate_back(const Run& r, const float* msg, int64_t e_base, const float* residual, float* out, int64_t n0, int64_t n1) {
-    constexpr int WPN = LMAX == 2 ? 8 : 4;
     const fcb200_eval& ev = r.ev;
     const float inv = MODE == 1 ? 1.0f / r.md.rescale : 1.0f;
-    if (share_node(n1 - n0)) {
-        constexpr int bytes = WPN * Shape<LMAX>::kL * C * 4;
+    auto shared = [&](auto tag) {
+        constexpr int WPN = decltype(tag)::value, bytes = WPN * Shape<LMAX>::kL * C * 4;
         static bool done[64] = {};
         FCB_TRY(raise_smem(rotate_back_kernel<LMAX, MODE, WPN>, bytes, done));
         launch_pdl((rotate_back_kernel<LMAX, MODE, WPN>), dim3((int)(n1 - n0)), dim3(WPN * 32), bytes, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
+        return (int)FCB200_OK;
+    };
+    // Eight warps to a node.  At lmax 4 one such block fills an SM's registers and lasts 0.63 times as long as one of four warps, of
+    // which two fit: whichever takes less in all (us a launch: 108 nodes, 8 / 4 / 2 warps 12.3 / 19.5 / 29.3; lmax 2, 256 nodes 9.1 /
+    // 13.2 / 22.9, 686 nodes 32.5 / 36.6 / 38.2).
+    const int64_t n = n1 - n0, sms = sm_count(), rounds = (n + sms - 1) / sms, halves = (n + 2 * sms - 1) / (2 * sms);
+    if (share_node(n)) {
+        if (LMAX == 2 || 63 * rounds < 100 * halves) FCB_TRY(shared(std::integral_constant<int, 8>{}));
+        else FCB_TRY(shared(std::integral_constant<int, 4>{}));
     } else {
         launch_pdl((rotate_back_kernel<LMAX, MODE, 1>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
     }
