@@ -29,9 +29,8 @@ def _unplane(p, scale=1.0):
 
 @pytest.fixture(params=[0, 1, 2], ids=["per_launch_choice", "natural_groups", "row_by_row"])
 def grouping(request, ops):
-    """How the tile list of a launch is cut into work items (forward; row by row, the gate is computed again for each).  A
-    backward launch cuts its rows one by one only with the scratch block that the whole-model evaluation gives it:
-    tests/test_gpu_step.py has systems on both sides of that rule."""
+    """How the tile list of a launch is cut into work items.  Row by row, the gate is computed again for each row of a forward
+    list; the other lists then keep their natural groups."""
     ops.CONV_GROUPING = request.param
     yield request.param
     ops.CONV_GROUPING = 0
