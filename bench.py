@@ -38,10 +38,10 @@ from fairchem_b200 import synthetic, weights  # noqa: E402
 ACC = 9.648533e-3  # (eV/A)/amu -> A/fs^2
 MASS = {1: 1.008, 6: 12.011, 7: 14.007, 8: 15.999, 24: 51.996, 25: 54.938, 26: 55.845, 27: 58.933, 28: 58.693, 29: 63.546}
 CPU_SAMPLE_ATOMS = 1500
-# DRAM bytes (read + write) per edge of one launch of so2_conv_fused_kernel, mean over its four convolution plans, from the
-# ncu capture of 62 118-edge launches:
-# (886 + 587) + (288 + 235) + (770 + 314) + (355 + 517) MB over 4 launches; traffic grows in proportion to the edges
-FUSED_TRAFFIC_PER_EDGE_LAUNCH = (1473e6 + 523e6 + 1084e6 + 872e6) / 4 / 62118
+# DRAM bytes (read + write) per edge of one convolution launch, mean over the four convolution plans, from an ncu capture of
+# 155 200-edge launches that keep the rows of the first convolution in float32, as the default workload does:
+# (1701 + 1619) + (718 + 659) + (1794 + 834) + (884 + 1372) MB over 4 launches; traffic grows in proportion to the edges
+FUSED_TRAFFIC_PER_EDGE_LAUNCH = (3320e6 + 1377e6 + 2628e6 + 2256e6) / 4 / 155200
 
 
 def load_peaks():
