@@ -474,3 +474,38 @@ def test_evaluation_inside_inference_mode(forces, mode):
     assert set(out) == set(ref)
     for k in ref:
         assert _rel(out[k], ref[k]) < 1e-6
+
+
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+@pytest.mark.parametrize("chunk", [129, 700, 131072])
+@pytest.mark.parametrize("gates", ["half_open", "closed"])
+def test_free_memory_does_not_change_a_bit(cfg, chunk, gates, monkeypatch):
+    """What is kept for the backward pass follows from the free memory and decides only what is computed again.  Gates
+    closed to sigmoid = 6e-6 as well: their gradients are made from values far below the normal range of a half.
+    Forces are sums in a fixed order; energy and stress end in float64 atomics, which are not."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import step, synthetic
+
+    bb, head = _model(B, cfg, edge_chunk_size=chunk)
+    if gates == "closed":
+        for block in bb.blocks:
+            conv = block.edge_wise.so2_conv_1
+            with torch.no_grad():
+                conv.fc_m0.bias[: bb.lmax * 128] = -12.0
+    data = synthetic.merge([synthetic.fcc_cu((3, 3, 4), seed=8), synthetic.bcc_alloy((2, 2, 3), seed=9)]).to("cuda")
+    runs = []
+
+    def forced(run):
+        run.ev.keep_radial, run.ev.drop_layers = kept
+        step._lib.call("fcb200_model_sizes", step.byref(run.model), step.byref(run.ev), run.sizes)
+        runs.append((int(run.ev.keep_radial), int(run.ev.drop_layers)))
+        return True
+
+    monkeypatch.setattr(step.BackboneStep, "plan_memory", forced)
+    sets, out = [(1, 0), (0, 0), (0, 1), (0, len(bb.blocks))], []
+    for kept in sets:
+        d = data.clone()
+        out.append(head(d, bb(d)))
+    assert runs == sets
+    for got in out[1:]:
+        assert torch.equal(got["forces"], out[0]["forces"])
