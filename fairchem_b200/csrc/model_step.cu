@@ -327,13 +327,16 @@ static int launch_rotate_back(const Run& r, const float* msg, int64_t e_base, co
         launch_pdl((rotate_back_kernel<LMAX, MODE, WPN>), dim3((int)(n1 - n0)), dim3(WPN * 32), bytes, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
         return (int)FCB200_OK;
     };
-    // Eight warps to a node.  At lmax 4 one such block fills an SM's registers and lasts 0.63 times as long as one of four warps, of
-    // which two fit: whichever takes less in all (us a launch: 108 nodes, 8 / 4 / 2 warps 12.3 / 19.5 / 29.3; lmax 2, 256 nodes 9.1 /
-    // 13.2 / 22.9, 686 nodes 32.5 / 36.6 / 38.2).
-    const int64_t n = n1 - n0, sms = sm_count(), rounds = (n + sms - 1) / sms, halves = (n + 2 * sms - 1) / (2 * sms);
+    // Eight warps to a node, or four where those take less in all at lmax 4: a round of blocks of eight (one fills an SM) lasts 0.59
+    // times as long as one of blocks of four, of which two fit an SM's registers, three with the m = 0 rows alone.  us a launch, 8 / 4
+    // warps, by nodes: 144 16.8 / 20.9, 256 28.7 / 26.6, 400 42.8 / 47.0, 576 58.8 / 53.4, 720 69.9 / 71.7, 864 80.1 / 75.3, 1 176 109 / 99;
+    // m = 0 rows 144 11.2 / 14.3, 256 16.6 / 14.6, 400 23.6 / 16.9, 720 38.7 / 27.8.  lmax 2: 256 12.6 / 14.7, 400 18.7 / 16.7, 720 31.1 / 31.5.
+    constexpr int kFours = MODE == 0 ? 2 : 3;
+    const int64_t n = n1 - n0, sms = sm_count(), rounds = (n + sms - 1) / sms, fours = (n + kFours * sms - 1) / (kFours * sms);
     if (share_node(n)) {
-        if (LMAX == 2 || 63 * rounds < 100 * halves) FCB_TRY(shared(std::integral_constant<int, 8>{}));
-        else FCB_TRY(shared(std::integral_constant<int, 4>{}));
+        if constexpr (LMAX == 4)
+            if (59 * rounds >= 100 * fours) return shared(std::integral_constant<int, 4>{});
+        return shared(std::integral_constant<int, 8>{});
     } else {
         launch_pdl((rotate_back_kernel<LMAX, MODE, 1>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
     }

@@ -509,3 +509,27 @@ def test_free_memory_does_not_change_a_bit(cfg, chunk, gates, monkeypatch):
     assert runs == sets
     for got in out[1:]:
         assert torch.equal(got["forces"], out[0]["forces"])
+
+
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+@pytest.mark.parametrize("cells", [(3, 3, 4), (3, 4, 4), (4, 5, 5), (5, 5, 5), (5, 5, 6)])  # one to five rounds of 148 nodes
+def test_every_way_of_sharing_a_nodes_edges_among_warps(cfg, cells):
+    """Eight or four warps to a node, by node count, lmax and kernel, against the per-op path's one warp."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, cfg)
+    data = synthetic.fcc_cu(cells, seed=11).to("cuda")
+    out = {}
+    for native in (True, False):
+        B._GemmState.native = native
+        try:
+            d = data.clone()
+            emb = bb(d)
+            assert ("step" in emb) == native
+            out[native] = head(d, emb)
+        finally:
+            B._GemmState.native = True
+    e, ref = out[True]["energy"], out[False]["energy"]
+    assert bool(((e - ref).abs() < 5e-6 * ref.abs().clamp_min(0.1 * len(data.pos))).all())
+    assert _rel(out[True]["forces"], out[False]["forces"]) < 2e-5
