@@ -414,12 +414,15 @@ int launch_pair(const PairPlan& plan, const Params& prm, const void* a_hi, const
         rc = map_half(&maps.w[2 * i], w_hi[i], w_rows[i], w_cols[i], w_cols[i], 64);
         if (!rc) rc = map_half(&maps.w[2 * i + 1], w_lo[i], w_rows[i], w_cols[i], w_cols[i], 64);
     }
-    if (!rc) rc = map_2d(&maps.y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, prm.y, m, prm.y_cols, prm.ldy, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B);
-    maps.o[0] = maps.o[1] = maps.y;
-    if (!rc && prm.o_hi) {
+    // a list without float32 tiles need not have a column of y, one without split tiles no planes: those have no map
+    const bool stores_y = prm.y_cols > 0;
+    if (!rc && stores_y) rc = map_2d(&maps.y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, prm.y, m, prm.y_cols, prm.ldy, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc && forward) {
         rc = map_2d(&maps.o[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, prm.o_hi, m, o_cols, prm.ldo, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
         if (!rc) rc = map_2d(&maps.o[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, prm.o_lo, m, o_cols, prm.ldo, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
     }
+    if (!stores_y) maps.y = maps.o[0];
+    if (!forward) maps.o[0] = maps.o[1] = maps.y;
     if (rc) return rc;
     for (int i = 0; i < 3; ++i)
         if (!used[i]) maps.w[2 * i] = maps.w[2 * first], maps.w[2 * i + 1] = maps.w[2 * first + 1];

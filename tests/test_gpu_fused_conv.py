@@ -198,3 +198,36 @@ def test_edge_block_is_the_same_with_per_node_and_per_edge_source_gradients(ops)
     (e0, f0), (e1, f1) = results
     assert abs(float(e1[0] - e0[0])) <= 1e-9 * abs(float(e0[0]))  # the forward pass is the same code
     assert float((f1 - f0).abs().max()) <= 2e-6
+
+
+def _silu_list(ops, y_cols, planes, variant):
+    """Status code and output planes of a list of one row-0 tile, which stores nothing to y, straight at the C entry."""
+    from ctypes import c_float, c_int32, c_int64, c_void_p
+
+    from fairchem_b200 import _lib
+
+    m, k = 2048, 128
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a = _planes(torch.randn(m, k, generator=g, device="cuda"))
+    hi, lo, sc = ops.split_f16(torch.randn(128, k, generator=g, device="cuda"))
+    y = torch.zeros(m, 128, device="cuda")
+    out = [torch.zeros(m, 128, dtype=torch.float16, device="cuda") for _ in range(2)]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tiles = [0, k, 0, 0, 0, ops.CONV_SILU if planes else ops.CONV_PLAIN, 0, 0, 0]
+    rc = _lib.load().fcb200_so2_conv_fused(
+        a[0].data_ptr(), a[1].data_ptr(), k, k, (c_void_p * 3)(hi.data_ptr()), (c_void_p * 3)(lo.data_ptr()), (c_int64 * 3)(128), (c_int64 * 3)(k),
+        (c_float * 3)(sc, 1.0, 1.0), (c_void_p * 3)(), (c_int32 * 9)(*tiles), 1, 0, y.data_ptr(), y_cols, y_cols, out[0].data_ptr(),
+        out[1].data_ptr(), 128 if planes else 0, 128 if planes else 0, None, None, m, 16 * variant, status.data_ptr(),
+        torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    return rc, [y, *out]
+
+
+@pytest.mark.parametrize("planes", [True, False])  # no column of y; planes that are passed but have no column
+def test_pairs_of_ctas_take_lists_that_use_one_output(ops, planes):
+    y_cols = 0 if planes else 128
+    want = _silu_list(ops, y_cols, planes, 1)
+    got = _silu_list(ops, y_cols, planes, 3)
+    assert want[0] == got[0] == 0
+    assert all(torch.equal(a, b) for a, b in zip(want[1], got[1])) and bool(got[1][1 if planes else 0].any())
