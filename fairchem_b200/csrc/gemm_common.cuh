@@ -49,6 +49,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return true;
 }
 
+// Before a CTA leaves: after an expired wait, copies and products that are still under way may reach its memory; let them end.
+__device__ __forceinline__ void settle(volatile int* abort_flag) {
+    if (*abort_flag) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < (1LL << 21)) {}
+    }
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"

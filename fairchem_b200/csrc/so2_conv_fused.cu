@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     }
 
+    settle(abort_flag);
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

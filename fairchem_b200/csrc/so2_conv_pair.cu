@@ -364,10 +364,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
     }
 
-    if (*abort_flag) {  // copies and products that are still under way may reach this CTA: let them end
-        const long long t0 = clock64();
-        while (clock64() - t0 < (1LL << 21)) {}
-    }
+    settle(abort_flag);
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // all stores of this warp have landed
     }
 
+    settle(abort_flag);
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

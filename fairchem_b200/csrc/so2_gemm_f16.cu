@@ -285,6 +285,7 @@ __device__ __forceinline__ void gemm_f16x2_body(const CUtensorMap& map_a, const 
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // all stores of this warp have landed
     }
 
+    settle(abort_flag);
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
