@@ -231,3 +231,14 @@ def test_pairs_of_ctas_take_lists_that_use_one_output(ops, planes):
     got = _silu_list(ops, y_cols, planes, 3)
     assert want[0] == got[0] == 0
     assert all(torch.equal(a, b) for a, b in zip(want[1], got[1])) and bool(got[1][1 if planes else 0].any())
+
+
+# 7 680 rows: the first convolution's input alone is past the 64 MiB from which row 0 may join the group of degree 1; 21 000: the gate's
+# backward too.  257: on neither.
+@pytest.mark.parametrize("lmax,e", [(2, 257), (2, 7680), (2, 21000), (4, 3900), (4, 9000)])
+def test_row_0_in_the_group_of_degree_1_gives_the_same_bits(ops, lmax, e):
+    """Row by row (2) never joins groups, and a backward list then keeps its natural ones; the other forms may join them."""
+    apart = _launches(ops, lmax, e, 2)
+    for form in (0, 1, 3):
+        for got, want in zip(_launches(ops, lmax, e, form), apart):
+            assert torch.equal(got, want)
