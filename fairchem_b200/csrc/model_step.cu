@@ -360,11 +360,9 @@ static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, co
     // 1951; where it does not: 1 440 731 -> 771, 3 120 1496 -> 1529, 5 280 2414 -> 2545; lmax 4, 2 048 nodes 9662 -> 7773).
     // More nodes come in several chunks, which hold too few edges of a source to share.
     // Fewer nodes: eight warps to a node, one block on an SM, unless four and three blocks take fewer rounds; a round of those
-    // lasts 1.9 times as long, at lmax 4 2.05 times (us a launch, mean of by source and by target, 8 / 4 warps, by nodes: 144 15.5 / 19.7,
-    // 256 27.2 / 26.2, 432 39.6 / 32.8, 500 46.9 / 45.2, 720 60.5 / 53.6, 1 176 94 / 81; lmax 4, 144 41 / 55, 256 61 / 65, 432 94 / 84,
-    // 500 117 / 129, 720 161 / 148, 1 176 270 / 230).
+    // lasts 2.05 times as long (us a launch, 256 nodes 24.5 / 24.5, 686 nodes 56.8 / 50.6; lmax 4, 108 nodes 35 / 73).
     const int64_t n = n1 - n0, sms = sm_count(), waves = (n + 12 * sms - 1) / (12 * sms), quarters = (n + 3 * sms - 1) / (3 * sms), rounds = (n + sms - 1) / sms;
-    if (share_node(n) && 20 * rounds <= (LMAX == 2 ? 38 : 41) * quarters) {
+    if (share_node(n) && 20 * rounds <= 41 * quarters) {
         FCB_TRY(shared(std::integral_constant<int, 8>{}, done[0]));
     } else if (share_node(n) || (waves <= 3 && 11 * quarters < 40 * waves)) {
         FCB_TRY(shared(std::integral_constant<int, 4>{}, done[2]));
