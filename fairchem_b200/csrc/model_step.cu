@@ -327,15 +327,15 @@ static int launch_rotate_back(const Run& r, const float* msg, int64_t e_base, co
         launch_pdl((rotate_back_kernel<LMAX, MODE, WPN>), dim3((int)(n1 - n0)), dim3(WPN * 32), bytes, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
         return (int)FCB200_OK;
     };
-    // Eight warps to a node, or four where those take less in all at lmax 4: a round of blocks of eight (one fills an SM) lasts 0.59
-    // times as long as one of blocks of four, of which two fit an SM's registers, three with the m = 0 rows alone.  us a launch, 8 / 4
-    // warps, by nodes: 144 16.8 / 20.9, 256 28.7 / 26.6, 400 42.8 / 47.0, 576 58.8 / 53.4, 720 69.9 / 71.7, 864 80.1 / 75.3, 1 176 109 / 99;
-    // m = 0 rows 144 11.2 / 14.3, 256 16.6 / 14.6, 400 23.6 / 16.9, 720 38.7 / 27.8.  lmax 2: 256 12.6 / 14.7, 400 18.7 / 16.7, 720 31.1 / 31.5.
-    constexpr int kFours = MODE == 0 ? 2 : 3;
-    const int64_t n = n1 - n0, sms = sm_count(), rounds = (n + sms - 1) / sms, fours = (n + kFours * sms - 1) / (kFours * sms);
+    // Eight warps to a node, or four where those take less in all at lmax 4: one block of eight fills an SM's registers and lasts 0.63
+    // times as long as one of four, of which two fit.  us a launch, 8 / 4 warps, by nodes: 108 14.8 / 18.8, 256 28.7 / 26.6, 400 42.8 / 47.0,
+    // 576 58.8 / 53.4, 864 80.1 / 75.3, 1 176 109 / 99; lmax 2, 256 12.6 / 14.7, 720 31.1 / 31.5.  Off by little, and left so because the number of
+    // warps is the order of a node's sum: lmax 4, 720 nodes 69.9 / 71.7; the m = 0 rows alone (three blocks of four fit), 400 nodes
+    // 23.6 / 16.9 once an evaluation of 15.6 ms; lmax 2, 400 nodes 18.7 / 16.7.
+    const int64_t n = n1 - n0, sms = sm_count(), rounds = (n + sms - 1) / sms, halves = (n + 2 * sms - 1) / (2 * sms);
     if (share_node(n)) {
         if constexpr (LMAX == 4)
-            if (59 * rounds >= 100 * fours) return shared(std::integral_constant<int, 4>{});
+            if (63 * rounds >= 100 * halves) return shared(std::integral_constant<int, 4>{});
         return shared(std::integral_constant<int, 8>{});
     } else {
         launch_pdl((rotate_back_kernel<LMAX, MODE, 1>), dim3(warp_grid(n1 - n0, 4)), dim3(128), 0, r.st, msg, r.L.wig, r.L.env, ev.row_ptr, e_base, residual, r.md.element_emb, ev.z, r.L.sys, ev.batch, out, inv, n0, n1);
@@ -360,7 +360,9 @@ static int launch_gather_bwd(const Run& r, const float* x, const int32_t* lo, co
     // 1951; where it does not: 1 440 731 -> 771, 3 120 1496 -> 1529, 5 280 2414 -> 2545; lmax 4, 2 048 nodes 9662 -> 7773).
     // More nodes come in several chunks, which hold too few edges of a source to share.
     // Fewer nodes: eight warps to a node, one block on an SM, unless four and three blocks take fewer rounds; a round of those
-    // lasts 2.05 times as long (us a launch, 256 nodes 24.5 / 24.5, 686 nodes 56.8 / 50.6; lmax 4, 108 nodes 35 / 73).
+    // lasts 2.05 times as long (us a launch, mean of by source and by target, 8 / 4 warps, by nodes: 144 15.5 / 19.7, 432 39.6 / 32.8,
+    // 720 60.5 / 53.6, 1 176 94 / 81; lmax 4, 144 41 / 55, 256 61 / 65, 432 94 / 84, 500 117 / 129, 720 161 / 148, 1 176 270 / 230).  At lmax 2 the ratio is
+    // just below 2 (256 nodes 27.2 / 26.2, 500 nodes 46.9 / 45.2); left so because the number of warps is the order of a node's sum.
     const int64_t n = n1 - n0, sms = sm_count(), waves = (n + 12 * sms - 1) / (12 * sms), quarters = (n + 3 * sms - 1) / (3 * sms), rounds = (n + sms - 1) / sms;
     if (share_node(n) && 20 * rounds <= 41 * quarters) {
         FCB_TRY(shared(std::integral_constant<int, 8>{}, done[0]));
