@@ -37,21 +37,28 @@ struct Planes {
     __half *hi = nullptr, *lo = nullptr;
     int64_t ld = 0;  // elements per row
     OutSplit out() const { return OutSplit{hi, lo, 1.0f}; }
+    Planes from(int64_t row) const {
+        Planes p = *this;
+        p.hi += row * ld, p.lo += row * ld;
+        return p;
+    }
 };
 
 // sizes that follow from lmax
 struct Dims {
-    int lmax, nl, nm, nw, nrad, gates, yw;
+    int lmax, nl, nm, nw, nrad, gates, yw, kw;  // yw: conv 1's columns, kw: of those, gates and row 0
     explicit Dims(int l) : lmax(l), nl((l + 1) * (l + 1)), nm((l + 1) + 2 * l + 2 * (l - 1)), nw(l == 2 ? Shape<2>::kW : Shape<4>::kW),
-                           nrad(3 * l), gates(l * C), yw((l + nm) * C) {}
+                           nrad(3 * l), gates(l * C), yw((l + nm) * C), kw((l + 1) * C) {}
 };
 
 struct Layer {
     float *x0, *xn1, *st1, *x1, *st2, *ffn_y;  // inputs of the two norms, first norm's output, feed-forward pre-activation
     float *y, *msg, *rad;                      // conv-1 output, messages, radial weights (per edge); null: not kept
-    // The conv-1 output stays float32: the gate's backward made from the gated rows as conv 2 read them (y sigmoid(g) in half
-    // planes, 4 of 23 KB an edge not written; 25 000 atoms of water 120.5 -> 118.8 ms) has 22 bits of a term, fewer for gates that are
-    // nearly closed, and forces that change with what fits the free memory.
+    // Where everything fits, the gated rows are kept for the backward pass as conv 2 read them, and of the conv-1 output only
+    // the gates and row 0: one row more to keep, but eight (lmax 4: 18) of 4 bytes fewer to write.  Forces then differ by some 2e-7 from
+    // those of the smaller kept sets, whose gate gradients are made from float32 rows and which agree bit for bit among themselves.
+    Planes a;
+    int64_t yw = 0;                            // columns of y
 };
 
 struct Layout {
@@ -128,7 +135,9 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         q.st2 = k.take<float>(n * 2);
         q.ffn_y = k.take<float>(n * (md.lmax + d.nl) * C);
         const bool edges = keep && l >= ev.drop_layers;
-        q.y = edges ? k.take<float>(er * d.yw) : nullptr;
+        q.yw = ev.keep_radial ? d.kw : d.yw;
+        q.y = edges ? k.take<float>(er * q.yw) : nullptr;
+        q.a = edges && ev.keep_radial ? planes(k, er, d.nm * C) : Planes{};
         q.msg = edges ? k.take<float>(er * d.nm * C) : nullptr;
         q.rad = edges && ev.keep_radial ? k.take<float>(er * d.nrad * 2 * C) : nullptr;
     }
@@ -141,8 +150,8 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         L.r3 = b.take<float>(ec * (md.lmax + 1) * C);
         L.radial = b.take<float>(ec * d.nrad * 2 * C);
         L.m = planes(b, ec, d.nm * 2 * C);
-        L.a = planes(b, ec, d.nm * C);
         const bool all = keep && ev.drop_layers <= 0;
+        if (!all || !ev.keep_radial) L.a = planes(b, ec, d.nm * C);
         L.y_c = all ? nullptr : b.take<float>(ec * d.gates);
         L.msg_c = all ? nullptr : b.take<float>(ec * d.nm * C);
         L.xn2 = planes(b, n, d.nl * C);
@@ -233,7 +242,7 @@ struct Run {
 
     // one launch of tile list c on rows [m] of half planes
     int conv(const char* name, const Conv& c, const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, int rot_begin, float* y,
-             int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m) const {
+             int64_t ldy, int64_t y_cols, const Planes* o, int64_t o_cols, const float* a_scale, const float* o_scale, int64_t m, const Planes* gated = nullptr) const {
         const void *hi[3] = {}, *lo[3] = {};
         int64_t rows[3] = {}, cols[3] = {};
         float sc[3] = {1.f, 1.f, 1.f};
@@ -243,7 +252,7 @@ struct Run {
         hook(name, 1, bytes, flops);
         const int rc = so2_conv_fused(a_hi, a_lo, lda, a_cols, hi, lo, rows, cols, sc, c.bias, c.t.data(), c.count(), rot_begin, y,
                                              ldy, y_cols, o ? o->hi : nullptr, o ? o->lo : nullptr, o ? o->ld : 0, o_cols, a_scale,
-                                             o_scale, m, 0, ev.status, stream);
+                                             o_scale, m, 0, ev.status, stream, gated ? gated->hi : nullptr, gated ? gated->lo : nullptr, gated ? gated->ld : 0);
         hook(name, 0, bytes, flops);
         return rc;
     }
@@ -275,7 +284,8 @@ struct Run {
         if (r < 2 * d.lmax) return r % d.lmax + 1;
         return (r - 2 * d.lmax) % (d.lmax - 1) + 2;
     }
-    Conv conv1_gate(int l, bool keep) const;
+    enum Keep { kNothing, kRow0, kRows };  // which of conv 1's raw rows go to y
+    Conv conv1_gate(int l, Keep keep) const;
     int messages(int l, const Conv& c1, int64_t e0, int64_t ec, float* y, int64_t yw, float* msg) const;
     int forward();
     int energy();
@@ -405,8 +415,8 @@ int Run::radial_hidden_forward() {
     });
 }
 
-// conv 1 with the gate in its epilogue: gate tiles first, then the rows; keep: the rows' raw values too
-Conv Run::conv1_gate(int l, bool keep) const {
+// conv 1 with the gate in its epilogue: gate tiles first, then the rows
+Conv Run::conv1_gate(int l, Keep keep) const {
     Conv c = blocks(md.layers[l].conv1);
     c.bias[0] = md.layers[l].conv1_bias;
     for (int i = d.lmax; i < c.count(); ++i) {
@@ -416,7 +426,7 @@ Conv Run::conv1_gate(int l, bool keep) const {
         t[5] = r == 0 ? kSilu : kGated;
         t[6] = (d.lmax + r) * C;
         t[7] = r == 0 ? 0 : (degree_of_row(r) - 1) * C;
-        t[8] = keep ? kKeep : 0;
+        t[8] = keep == kRows || (keep == kRow0 && r == 0) ? kKeep : 0;
     }
     return c;
 }
@@ -433,10 +443,11 @@ int Run::messages(int l, const Conv& c1, int64_t e0, int64_t ec, float* y, int64
             return 0;
         });
     }));
-    FCB_TRY(conv("so2_conv_fused_conv1_gate", c1, L.m.hi, L.m.lo, L.m.ld, L.m.ld, d.lmax, y, yw, yw, &L.a, L.a.ld, nullptr, nullptr, ec));
+    const Planes a = q.a.hi ? q.a.from(e0) : L.a;
+    FCB_TRY(conv("so2_conv_fused_conv1_gate", c1, L.m.hi, L.m.lo, L.m.ld, L.m.ld, d.lmax, y, yw, yw, &a, a.ld, nullptr, nullptr, ec));
     Conv c2 = blocks(md.layers[l].conv2);
     c2.bias[0] = md.layers[l].conv2_bias;
-    return conv("so2_conv_fused_conv2", c2, L.a.hi, L.a.lo, L.a.ld, L.a.ld, 0, msg, d.nm * C, d.nm * C, nullptr, 0, nullptr, nullptr, ec);
+    return conv("so2_conv_fused_conv2", c2, a.hi, a.lo, a.ld, a.ld, 0, msg, d.nm * C, d.nm * C, nullptr, 0, nullptr, nullptr, ec);
 }
 
 int Run::layer_forward(int l, const float* ffn_prev) {
@@ -451,10 +462,10 @@ int Run::layer_forward(int l, const float* ffn_prev) {
             return 0;
         });
     }));
-    const Conv c1 = conv1_gate(l, q.y != nullptr);
+    const Conv c1 = conv1_gate(l, q.a.hi ? kRow0 : q.y ? kRows : kNothing);
     return chunks([&](int, int64_t e0, int64_t ec, int64_t n0, int64_t n1) {
         float* msg = q.msg ? q.msg + e0 * d.nm * C : L.msg_c;
-        FCB_TRY(messages(l, c1, e0, ec, q.y ? q.y + e0 * d.yw : L.y_c, q.y ? d.yw : d.gates, msg));
+        FCB_TRY(messages(l, c1, e0, ec, q.y ? q.y + e0 * q.yw : L.y_c, q.y ? q.yw : d.gates, msg));
         return op("rotate_back_reduce_fwd", ec * 4 * (d.nm * C + d.nw) + (n1 - n0) * row * 8,
                   [&] { return by_lmax([&](auto lm) { return launch_rotate_back<decltype(lm)::value, 0>(*this, msg, e0, q.x0, q.x1, n0, n1); }); });
     });
@@ -575,7 +586,7 @@ int Run::layer_backward(int l) {
         auto add = [&](int r, int flags) {
             const int32_t* t = &p.t[9 * r];
             const int deg = degree_of_row(r);
-            c2.tile(t[0], t[1], t[2], t[3], d.gates + r * C, r == 0 ? kSiluBwd : kGatedBwd, d.gates + r * C, r == 0 ? 0 : (deg - 1) * C, flags);
+            c2.tile(t[0], t[1], t[2], t[3], d.gates + r * C, r == 0 ? kSiluBwd : kGatedBwd, (r > 0 && q.a.hi ? 0 : d.gates) + r * C, r == 0 ? 0 : (deg - 1) * C, flags);
         };
         add(0, 0);
         for (int deg = 1; deg <= d.lmax; ++deg) {
@@ -590,9 +601,9 @@ int Run::layer_backward(int l) {
         }
     }
     const bool first_layer = l == md.num_layers - 1;
-    const Conv again = q.y ? Conv{} : conv1_gate(l, true);
+    const Conv again = q.y ? Conv{} : conv1_gate(l, kRows);
     FCB_TRY(chunks([&](int c, int64_t e0, int64_t ec, int64_t n0, int64_t n1) {
-        float* y = q.y ? q.y + e0 * d.yw : L.y_c;
+        float* y = q.y ? q.y + e0 * q.yw : L.y_c;
         float* msg = q.msg ? q.msg + e0 * d.nm * C : L.msg_c;
         if (!q.y) {
             FCB_TRY(messages(l, again, e0, ec, y, d.yw, msg));
@@ -606,7 +617,9 @@ int Run::layer_backward(int l) {
                 return 0;
             });
         }));
-        FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, d.yw, d.yw, &L.gy, L.gy.ld, scale, scale, ec));
+        const Planes gated = q.a.hi ? q.a.from(e0) : Planes{};
+        const int64_t yw = q.y ? q.yw : d.yw;
+        FCB_TRY(conv("so2_conv_fused_conv2_gate_bwd", c2, L.gmsg.hi, L.gmsg.lo, L.gmsg.ld, L.gmsg.ld, c2.count(), y, yw, yw, &L.gy, L.gy.ld, scale, scale, ec, q.a.hi ? &gated : nullptr));
         FCB_TRY(conv("so2_conv_fused_conv1_bwd", c1, L.gy.hi, L.gy.lo, L.gy.ld, L.gy.ld, 0, L.gm, d.nm * 2 * C, d.nm * 2 * C, nullptr, 0, scale, nullptr, ec));
         const int64_t gb = ec * 4LL * (2 * d.nm * C + 2 * 2 * d.nrad * C + d.nw + 12) + (n1 - n0) * row * 4 * 4;
         FCB_TRY(op("gather_rotate_bwd", gb, [&] {

@@ -35,7 +35,8 @@ constexpr int kMaxTiles = 40;   // tiles a caller may list; lmax 4: 19 rows x 2C
 constexpr int kMaxPlan = 80;    // tiles of a plan: a gate tile may be repeated for each of its rows
 
 // What the epilogue of a launch has to be able to do; fixes how many registers it keeps between tiles.
-enum Kind { kPlainKind = 0, kForwardKind = 1, kBackwardKind = 2 };
+// kPlanesKind: the gate's backward from the gated rows' own planes (see Params::rows_hi).
+enum Kind { kPlainKind = 0, kForwardKind = 1, kBackwardKind = 2, kPlanesKind = 3 };
 
 constexpr int KB = 64;               // k extent of a ring stage: 128-byte rows, 128-byte swizzle
 constexpr int kPart = BM * KB * 2;   // 128 rows of one half plane of a stage, 16 KiB
@@ -60,6 +61,11 @@ struct Params {
     int32_t ldo;
     const float* a_scale;  // power of two the A planes were written with (null = 1)
     const float* o_scale;  // power of two the output planes are written with (null = 1)
+    // kPlanesKind: a gated row's gate gradient is made from what the forward pass gave the second convolution, a = y sigmoid(g),
+    // instead of y: sum x y sigmoid'(g) = (1 - sigmoid(g)) sum x a.  Tile::y_col is a column of these planes.  a has 22 bits, below
+    // 6e-5 (high half subnormal) an absolute error of 1.5e-11: a nearly closed gate's gradient is exact to that times sum |x|, no closer.
+    const __half *rows_hi, *rows_lo;
+    int32_t ld_rows;
     int64_t m_total;
     int32_t* status;
 };
@@ -164,6 +170,17 @@ __device__ __forceinline__ void split2(f32x2 v, uint32_t& hi, uint32_t& lo, __ha
     top = __hmax2_nan(top, __habs2(h));
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// hi and lo halves of four values -> the values
+__device__ __forceinline__ void join2(uint64_t hi, uint64_t lo, f32x2& a, f32x2& b) {
+    const uint32_t h[2] = {(uint32_t)hi, (uint32_t)(hi >> 32)}, l[2] = {(uint32_t)lo, (uint32_t)(lo >> 32)};
+    const f32x2 s = pack(1.0f / kLoScale, 1.0f / kLoScale);
+    auto wide = [](uint32_t v) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+        return pack(f.x, f.y);
+    };
+    a = fma2(wide(l[0]), s, wide(h[0])), b = fma2(wide(l[1]), s, wide(h[1]));
 }
 
 #define FCB_TMEM_LD16(r, taddr)                                                                                           \

@@ -13,7 +13,12 @@
 //   conv 2 backward: A = message gradient planes -> tiles = rows of the gate output's gradient; the epilogue
 //                    reads the kept y, writes the gradient of the conv-1 output as (hi, lo) planes and sums the
 //                    gate-scalar gradients over the rows of a degree in registers (the tiles of a degree are
-//                    consecutive: the first resets the sums, the last writes them into the planes)
+//                    consecutive: the first resets the sums, the last writes them into the planes); where the gated rows
+//                    were kept as planes it reads those instead of the rows of y, which are then not written at all
+//                    (4 of 23 KB an edge that conv 1 moves at lmax 2; 2 000 atoms of alloy 10.35 -> 10.15 ms, 25 000 of water 124.4 -> 121.5).
+//                    Planes hold 22 bits of y sigmoid(g), below 6e-5 1.5e-11 absolute, what conv 2 itself has read.  Forces against
+//                    float64 of 105 evaluations (lmax 2 and 4; gates half open, closed to 2e-9, spread over both): in none of ten
+//                    groups is the mean error more than 1.002 times that of float32 rows; it is the larger one in 53.
 //   conv 1 backward: plain float32 output (gradient of the rotated rows)
 //
 // Replaces SO2_Convolution.forward + GateActivation.forward of the reference
@@ -89,26 +94,33 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
     const float o_scale = prm.o_scale ? *prm.o_scale : 1.0f;
     __half2 top = __floats2half2_rn(0.f, 0.f);
     // per chunk and row: forward: o_scale * sigmoid of the gate; backward: gate-gradient sums
+    constexpr bool kBackward = KIND >= kBackwardKind, kFromPlanes = KIND == kPlanesKind;
     f32x2 keepv[KIND == kPlainKind ? 1 : kChunks][16];
     // Loads run one chunk ahead where the registers allow it: the second chunk's accumulator columns without a backward
     // input, else the y rows of the next chunk.
-    constexpr bool kAhead = KIND != kBackwardKind;
-    f32x2 yv[KIND == kBackwardKind ? 16 : 1] = {};
-    f32x2 sg[KIND == kBackwardKind ? kChunks : 1][16];  // backward: o_scale * sigmoid of the degree's gate, made at its first row; row 0: the slope
+    constexpr bool kAhead = !kBackward;
+    f32x2 yv[kBackward ? 16 : 1] = {};  // from planes: hi and lo of four columns
+    f32x2 sg[kBackward ? kChunks : 1][16];  // backward: o_scale * sigmoid of the degree's gate, made at its first row; row 0: the slope
     auto slot = [&](int i) { return tile + (uint32_t)((rr + 4 * i) * 128 + (((lane & 7) ^ ((rr + 4 * i) & 7)) * 16)); };
     auto put = [](uint32_t at, f32x2 a, f32x2 b) { asm volatile("st.shared.v2.b64 [%0], {%1,%2};" ::"r"(at), "l"(a), "l"(b) : "memory"); };
     auto get = [](uint32_t at, f32x2& a, f32x2& b) { asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "r"(at) : "memory"); };
     // y lines of a backward tile on their way to L2 one tile early (lane = row, a line a chunk)
     auto prefetch = [&](int64_t mt2, int ti2, int first) {
-        if constexpr (KIND == kBackwardKind) {
+        if constexpr (kBackward) {
             const int64_t row = mt2 * BM + q * 32 + lane;
             if (row < prm.m_total) {
                 const Tile& t2 = plan.t[ti2];
-                const float* p = prm.y + row * prm.ldy + t2.y_col + first;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-                if (kChunks == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
+                const float* p = prm.y + row * prm.ldy + first;
+                if (kFromPlanes && t2.mode == kGatedBwd) {
+                    const int64_t at = row * prm.ld_rows + t2.y_col + first;
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(prm.rows_hi + at));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(prm.rows_lo + at));
+                } else {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + t2.y_col));
+                    if (kChunks == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + t2.y_col + 32));
+                }
                 if (t2.flags & kFirst) {
-                    p += t2.gate_col - t2.y_col;
+                    p += t2.gate_col;
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
                     if (kChunks == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 32));
                 }
@@ -128,7 +140,17 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
         __half* const ohi = prm.o_hi + (row0 + rr) * prm.ldo + c4;
         __half* const olo = prm.o_lo + (row0 + rr) * prm.ldo + c4;
         auto fetch = [&](int y_col, int c2) {
-            if constexpr (KIND == kBackwardKind) {
+            if constexpr (kFromPlanes) {
+                const int64_t at = (row0 + rr) * prm.ld_rows + y_col + col0 + c2 * 32 + c4;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    yv[2 * i] = yv[2 * i + 1] = 0;
+                    if (rr + 4 * i < live) {
+                        yv[2 * i] = *reinterpret_cast<const uint64_t*>(prm.rows_hi + at + 4 * i * prm.ld_rows);
+                        yv[2 * i + 1] = *reinterpret_cast<const uint64_t*>(prm.rows_lo + at + 4 * i * prm.ld_rows);
+                    }
+                }
+            } else if constexpr (kBackward) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     yv[2 * i] = yv[2 * i + 1] = 0;
@@ -145,7 +167,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
             const int mode = t.mode;
             const int buf = (int)(tcount & 1);
             const uint32_t use = (uint32_t)((tcount >> 1) & 1);
-            if constexpr (KIND == kBackwardKind) {
+            if constexpr (kBackward) {
                 int64_t mt2;
                 int g2;
                 if (ti + 1 < plan.begin[g + 1]) prefetch(mt, ti + 1, col0);
@@ -157,7 +179,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
             // and with row 0 and the gate's gradient unrolled too, the code of a tile outgrew the instruction cache and a
             // quarter of the epilogue's stalls were instruction fetches (gated backward launches of an evaluation, 62 118 edges:
             // 1.40 -> 1.26 ms; 775 000: 18.9 -> 17.3).
-            if constexpr (KIND == kBackwardKind) {
+            if constexpr (kBackward) {
                 if (mode == kSiluBwd || (t.flags & kFirst)) {
                     const bool slope = mode == kSiluBwd;
                     const float* from = yrow + (slope ? t.y_col : t.gate_col) + col0;
@@ -254,7 +276,7 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
                 const f32x2 b01 = pack(b.x, b.y), b23 = pack(b.z, b.w);
                 // body(i, x01, x23, in): row rr + 4 i of the chunk, four columns
                 auto row_of = [&](int i, f32x2 x0, f32x2 x1, auto&& body) {
-                    if constexpr (KIND == kBackwardKind) body(i, mul2(x0, os2), mul2(x1, os2), rr + 4 * i < live);
+                    if constexpr (kBackward) body(i, mul2(x0, os2), mul2(x1, os2), rr + 4 * i < live);
                     else body(i, fma2(x0, os2, b01), fma2(x1, os2, b23), rr + 4 * i < live);
                 };
                 // Shared reads of four rows first: a read keeps its place behind another row's stores, and so behind its
@@ -313,13 +335,15 @@ __device__ __forceinline__ void epilogue(const Plan& plan, const Params& prm, ui
                     }
                 } else {
                     rows([&](int i, f32x2 x0, f32x2 x1, bool in) {
-                        keepv[c2][2 * i] = fma2(x0, yv[2 * i], keepv[c2][2 * i]);  // row 0: not used
-                        keepv[c2][2 * i + 1] = fma2(x1, yv[2 * i + 1], keepv[c2][2 * i + 1]);
+                        f32x2 y0 = yv[2 * i], y1 = yv[2 * i + 1];
+                        if constexpr (kFromPlanes) join2(yv[2 * i], yv[2 * i + 1], y0, y1);
+                        keepv[c2][2 * i] = fma2(x0, y0, keepv[c2][2 * i]);  // row 0: not used
+                        keepv[c2][2 * i + 1] = fma2(x1, y1, keepv[c2][2 * i + 1]);
                         store_split(ph, pl, 4 * i * prm.ldo, mul2(x0, sg[c2][2 * i]), mul2(x1, sg[c2][2 * i + 1]), in, top);
                     });
                     if (t.flags & kLast) {
                         const float inv = 1.0f / o_scale;
-                        auto dsig = [&](float v) { return v * (1.f - v * inv); };  // o_scale * sigmoid'
+                        auto dsig = [&](float v) { return kFromPlanes ? o_scale - v : v * (1.f - v * inv); };  // o_scale * sigmoid', or that over sigmoid
                         auto dsilu = [&](float v) {
                             const float q = sigmoid_f(v);
                             return q * (1.f + v * (1.f - q));
@@ -739,7 +763,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
                                      const float* w_scale, const float* const* bias, const int32_t* tiles, int32_t num_tiles,
                                      int32_t rot_begin, float* y, int64_t ldy, int64_t y_cols, void* o_hi, void* o_lo, int64_t ldo, int64_t o_cols,
                                      const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status,
-                                     void* stream) {
+                                     void* stream, const __half* rows_hi, const __half* rows_lo, int64_t ld_rows) {
     using namespace fused;
     if (!a_hi || !a_lo || !w_hi || !w_lo || !w_rows || !w_cols || !w_scale || !tiles || !y || m < 0) return FCB200_EINVAL;
     Plan plan{};
@@ -775,7 +799,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         const bool reads_gate = t.mode == kGated || t.mode == kGatedBwd;
         if (reads_gate && (t.gate_col % 4 || t.gate_col + BN > y_cols)) return FCB200_EINVAL;
         const bool uses_y = t.mode == kSiluBwd || t.mode == kGatedBwd || ((t.mode == kSilu || t.mode == kGated) && (t.flags & kKeep));
-        if (uses_y && (t.y_col % 4 || t.y_col + BN > y_cols)) return FCB200_EINVAL;
+        if (uses_y && (t.y_col % 4 || t.y_col + BN > (rows_hi && t.mode == kGatedBwd ? ld_rows : y_cols))) return FCB200_EINVAL;
         if (t.mode == kGatedBwd && t.gate_col + BN > o_cols) return FCB200_EINVAL;
         used[t.w] = true;
         gated = gated || t.mode == kGated;
@@ -783,6 +807,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         backward = backward || t.mode == kSiluBwd || t.mode == kGatedBwd;
     }
     if (forward && backward) return FCB200_EINVAL;
+    if (rows_hi && (!rows_lo || ld_rows % 4 || ld_rows > 32767 || !aligned16(rows_hi) || !aligned16(rows_lo))) return FCB200_EINVAL;
     if (m == 0) return FCB200_OK;
     for (int i = 0; i < rot_begin && gated; ++i)
         if (list[i].mode == kPlain) {
@@ -874,6 +899,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
     if (ldy > 32767 || ldo > 32767) return FCB200_ERANGE;
     prm.y = y, prm.ldy = (int32_t)ldy, prm.y_cols = (int32_t)y_cols, prm.a_scale = a_scale, prm.o_scale = o_scale;
     prm.o_hi = static_cast<__half*>(o_hi), prm.o_lo = static_cast<__half*>(o_lo), prm.ldo = (int32_t)ldo;
+    prm.rows_hi = rows_hi, prm.rows_lo = rows_lo, prm.ld_rows = (int32_t)ld_rows;
     prm.m_total = m, prm.status = status;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (on_pairs) return launch_pair(two.plan, prm, a_hi, a_lo, lda, a_cols, w_hi, w_lo, w_rows, w_cols, used, o_cols, forward, st);
@@ -893,6 +919,7 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
         return launch(kind, std::integral_constant<int, 128>{});
     };
     if (forward) return by_width(std::integral_constant<int, kForwardKind>{});
+    if (backward && rows_hi) return by_width(std::integral_constant<int, kPlanesKind>{});
     if (backward) return by_width(std::integral_constant<int, kBackwardKind>{});
     return by_width(std::integral_constant<int, kPlainKind>{});
 }
@@ -906,5 +933,5 @@ extern "C" int fcb200_so2_conv_fused(const void* a_hi, const void* a_lo, int64_t
                                      const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status,
                                      void* stream) {
     return so2_conv_fused(a_hi, a_lo, lda, a_cols, w_hi, w_lo, w_rows, w_cols, w_scale, bias, tiles, num_tiles, rot_begin, y, ldy, y_cols, o_hi, o_lo, ldo,
-                          o_cols, a_scale, o_scale, m, variant, status, stream);
+                          o_cols, a_scale, o_scale, m, variant, status, stream, nullptr, nullptr, 0);
 }

@@ -8,11 +8,12 @@
 
 namespace fcb200 {
 
-// fcb200_so2_conv_fused for callers in C++
+// fcb200_so2_conv_fused for callers in C++; rows_hi, rows_lo: a backward gated list reads the gated rows' planes at its y
+// columns in place of y (null: y)
 int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_cols, const void* const* w_hi, const void* const* w_lo,
                    const int64_t* w_rows, const int64_t* w_cols, const float* w_scale, const float* const* bias, const int32_t* tiles,
                    int32_t num_tiles, int32_t rot_begin, float* y, int64_t ldy, int64_t y_cols, void* o_hi, void* o_lo, int64_t ldo, int64_t o_cols,
-                   const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status, void* stream);
+                   const float* a_scale, const float* o_scale, int64_t m, int32_t variant, int32_t* status, void* stream, const __half* rows_hi, const __half* rows_lo, int64_t ld_rows);
 
 namespace step {
 

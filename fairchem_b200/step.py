@@ -368,7 +368,11 @@ class BackboneStep:
 
     def plan_memory(self) -> bool:
         """Decide what is kept for the backward pass: everything, all but the radial weights, or, layer by layer, no conv-1
-        output and messages either.  False when not even the smallest set fits the free memory."""
+        output and messages either.  False when not even the smallest set fits the free memory.
+
+        The sets that fit less give the same bits; with everything kept the gate's gradient is made from half planes, and
+        forces differ by some 2e-7 of their norm from those.  So near the limit of the first set two calls on one system
+        agree to that, not bit for bit, when other allocations come or go between them."""
         e, sizes, layers = self.ev, self.sizes, self.model.num_layers
         for keep_radial, drop in chain(((1, 0),), ((0, n) for n in range(layers + 1))) if e.want_grad else ((0, 0),):
             e.keep_radial, e.drop_layers = keep_radial, drop

@@ -476,39 +476,78 @@ def test_evaluation_inside_inference_mode(forces, mode):
         assert _rel(out[k], ref[k]) < 1e-6
 
 
-@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
-@pytest.mark.parametrize("chunk", [129, 700, 131072])
-@pytest.mark.parametrize("gates", ["half_open", "closed"])
-def test_free_memory_does_not_change_a_bit(cfg, chunk, gates, monkeypatch):
-    """What is kept for the backward pass follows from the free memory and decides only what is computed again.  Gates
-    closed to sigmoid = 6e-6 as well: their gradients are made from values far below the normal range of a half.
-    Forces are sums in a fixed order; energy and stress end in float64 atomics, which are not."""
-    from fairchem_b200 import backbone as B
-    from fairchem_b200 import step, synthetic
+def _close_gates(bb, value):
+    """The gates of every edge block near sigmoid(value)."""
+    for block in bb.blocks:
+        with torch.no_grad():
+            block.edge_wise.so2_conv_1.fc_m0.bias[: bb.lmax * 128] = value
 
-    bb, head = _model(B, cfg, edge_chunk_size=chunk)
-    if gates == "closed":
-        for block in bb.blocks:
-            conv = block.edge_wise.so2_conv_1
-            with torch.no_grad():
-                conv.fc_m0.bias[: bb.lmax * 128] = -12.0
-    data = synthetic.merge([synthetic.fcc_cu((3, 3, 4), seed=8), synthetic.bcc_alloy((2, 2, 3), seed=9)]).to("cuda")
+
+def _force_kept_set(monkeypatch, kept):
+    """Evaluations keep (radial weights, layers without per-edge tensors) = kept[-1]; returns what they were planned with."""
+    from fairchem_b200 import step
+
     runs = []
 
     def forced(run):
-        run.ev.keep_radial, run.ev.drop_layers = kept
+        run.ev.keep_radial, run.ev.drop_layers = kept[-1]
         step._lib.call("fcb200_model_sizes", step.byref(run.model), step.byref(run.ev), run.sizes)
         runs.append((int(run.ev.keep_radial), int(run.ev.drop_layers)))
         return True
 
     monkeypatch.setattr(step.BackboneStep, "plan_memory", forced)
-    sets, out = [(1, 0), (0, 0), (0, 1), (0, len(bb.blocks))], []
-    for kept in sets:
+    return runs
+
+
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+@pytest.mark.parametrize("chunk", [129, 700, 131072])
+@pytest.mark.parametrize("gates", [0.0, -12.0])
+def test_what_the_free_memory_decides(cfg, chunk, gates, monkeypatch):
+    """Kept sets without the radial weights differ in what is computed again, by the same kernels on the same inputs: the same
+    bits.  With them the gate's gradient is made from half planes (2.4e-7 of a term): forces to 1e-6 of the norm."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic
+
+    bb, head = _model(B, cfg, edge_chunk_size=chunk)
+    if gates:
+        _close_gates(bb, gates)
+    data = synthetic.merge([synthetic.fcc_cu((3, 3, 4), seed=8), synthetic.bcc_alloy((2, 2, 3), seed=9)]).to("cuda")
+    kept, forces = [], []
+    runs = _force_kept_set(monkeypatch, kept)
+    for k in [(1, 0), (0, 0), (0, 1), (0, len(bb.blocks))]:
+        kept.append(k)
         d = data.clone()
-        out.append(head(d, bb(d)))
-    assert runs == sets
-    for got in out[1:]:
-        assert torch.equal(got["forces"], out[0]["forces"])
+        forces.append(head(d, bb(d))["forces"])
+    assert runs == kept
+    assert all(torch.equal(f, forces[1]) for f in forces[2:])
+    assert _rel(forces[0], forces[1]) < 1e-6
+
+
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+@pytest.mark.parametrize("gates", [-6.0, -12.0, -20.0])
+@pytest.mark.parametrize("kept", [(1, 0), (0, 0)])
+def test_closed_gates_against_float64(cfg, gates, kept, monkeypatch):
+    """Gates closed to sigmoid = 2.5e-3, 6e-6 and 2e-9: the planes of the gated rows hold 1.5e-11 absolute, not 22 bits, there,
+    and what such gates carry is as small."""
+    from fairchem_b200 import backbone as B
+    from fairchem_b200 import synthetic, weights
+    from oracle import escn_md_oracle as O
+
+    bb, head = _model(B, cfg)
+    _close_gates(bb, gates)
+    data = synthetic.fcc_cu((2, 3, 3), seed=12)
+    runs = _force_kept_set(monkeypatch, [kept])
+    d = data.to("cuda")
+    forces = head(d, bb(d))["forces"].cpu()
+    assert runs == [kept]
+    shape = dict(getattr(weights, cfg), num_layers=len(bb.blocks))
+    sd = weights.random_init_state_dict(shape, 0)
+    for i in range(len(bb.blocks)):
+        sd[f"blocks.{i}.edge_wise.so2_conv_1.fc_m0.bias"][: bb.lmax * 128] = gates
+    sd = {k: v.double() if v.is_floating_point() else v for k, v in sd.items()}
+    graph = bb.last_graph
+    _, ref = O.energy_and_forces(sd, shape, data, graph["edge_index"].cpu(), graph["cell_offsets"].cpu())
+    assert _rel(forces, ref) < 2e-5
 
 
 @pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
