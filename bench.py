@@ -267,7 +267,7 @@ def run_b200(args):
     if rank != 0:
         return
     peaks = load_peaks()
-    # the fused convolution kernel is one kernel launched with four tile plans: one roofline entry for it
+    # the convolutions are four tile plans of two kernels that share their tiles and epilogues: one roofline entry for them
     by_kernel = {}
     for k, v in summary.items():
         # (the radial MLP's output layer runs on the same kernel but is bound by storing its wide output: own entry)
@@ -280,22 +280,24 @@ def run_b200(args):
     if name in ("gemm_f16x2", "gemm_f16x2_presplit", "so2_conv_fused", "so2_conv_fused_radial_out"):
         peak = peaks["bf16_tflops"]
         ach = rec["flops"] / (rec["ms"] * 1e-3) / 1e12 if rec["ms"] else 0.0
-        traffic = None
+        traffic, captured = None, ""
         if name == "gemm_f16x2_presplit" and rec["launches"]:
             # ncu on a 62 119-edge chunk: 203.6 MB of DRAM traffic per launch, equal to the algorithmic bytes
             # (A_hi + A_lo + C once); per-launch traffic grows with the edges per launch
             n_chunks = max(1, -(-edges // args.chunk)) if world == 1 else None
             if n_chunks:
-                traffic = 203.6e6 * (edges / n_chunks) / 62119.0
+                traffic, captured = 203.6e6 * (edges / n_chunks) / 62119.0, "a 62 119-edge launch"
         if name == "so2_conv_fused" and rec["launches"] and FUSED_TRAFFIC_PER_EDGE_LAUNCH:
             per_rank = edges / world  # every rank launches over its own targets' edges
-            traffic = FUSED_TRAFFIC_PER_EDGE_LAUNCH * per_rank / max(1, -(-int(per_rank) // args.chunk))
-        roof = {"kernel": name + "_kernel", "bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
+            traffic, captured = FUSED_TRAFFIC_PER_EDGE_LAUNCH * per_rank / max(1, -(-int(per_rank) // args.chunk)), "155 200-edge launches"
+        # on pairs of CTAs where a launch has the rows for it: conv 1, its backward and conv 2, not the gate's backward
+        kernels = "so2_conv_pair_kernel, so2_conv_fused_kernel" if name == "so2_conv_fused" else name.replace("_radial_out", "") + "_kernel"
+        roof = {"kernel": kernels, "bound": "tensor", "achieved": ach, "peak": peak, "unit": "TFLOP/s",
                 "frac": ach / peak, "traffic": traffic, "launches": rec["launches"], "issued": ach * 3, "frac_issued": ach * 3 / peak,
                 "peak_source": f"{peaks['source']} bf16 sustained (kind::f16 issues at the bf16 rate)",
                 "note": "achieved counts algorithmic float32 FLOPs; float32-accurate mode issues 3 half-precision MMAs per "
-                        "product, so `issued` = 3 x achieved is what the tensor pipe executes; traffic is scaled from an ncu "
-                        "capture of a 62 119-edge launch by the edges per launch"}
+                        "product, so `issued` = 3 x achieved is what the tensor pipe executes"
+                        + (f"; traffic is scaled from an ncu capture of {captured} by the edges per launch" if captured else "")}
     elif name == "gemm_tf32":
         peak = peaks["bf16_tflops"] / 2.0
         ach = rec["flops"] / (rec["ms"] * 1e-3) / 1e12 if rec["ms"] else 0.0
