@@ -698,8 +698,9 @@ static int64_t makespan(const Order& order, const int* cost, int subs, int units
 }
 
 // The order of a launch's items and its makespan.  perm: the groups by falling cost.  Group by group an A tile leaves L2
-// between its groups when there are many rows, so that has to gain more than the extra reads cost (first convolution, lmax 2,
-// us row by row / group by group: 7 680 rows 90 / 68, 20 580 rows 188 / 182, 40 000 rows 332 / 353).
+// between its groups when there are many rows, so that has to gain more than the extra reads cost (us row by row / group by group,
+// lmax 2: first convolution, 7 200 rows 75.7 / 54.9, 14 000 rows 110 / 101, 40 000 rows 271 / 301; second convolution's backward, 7 200 rows 62.7 /
+// 35.8, 14 000 rows 99 / 67; second convolution, 5 000 rows 19.0 / 16.9, 14 000 rows 47.1 / 48.6).
 static int64_t choose_order(Order& order, int* cost, int* perm, int subs, int units) {
     const int groups = order.groups / subs;
     for (int i = 0; i < groups; ++i) perm[i] = i;
@@ -816,18 +817,18 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
                 if (list[j].mode == kGated && list[j].gate_col == list[i].out_col) list[i].flags |= list[j].flags & kGateSilu;
         }
     // Row tiles times natural groups are the items: CTAs that run together share an A tile in L2 and the last wave is one
-    // group deep, not one list (M = 131 072, second convolution: 417 us row tile by row tile, 377 so; M = 60 000, first
-    // convolution: 528 / 446).  Few row tiles leave SMs without work; then the gated rows of a forward list go one by one,
-    // and an item takes a part of its tiles' columns, where that shortens the longest CTA by more than the estimate's error.
-    // us, 128 / 64 / 32 columns: 420 rows of lmax 2, first convolution row by row 20.4 / 16.0 / 15.0, second 8.8 / 7.2 / 6.8, its
-    // gated backward 29.5 / 18.8 / 16.4, radial output layer's backward 15.9 / 12.7 / 11.6; 3 000 rows 34.4 / 37.3 / 56.7, 13.3 / 14.1 /
-    // 20.6, 30.1 / 19.7 / 22.8, 16.0 / 13.1 / 12.2; 7 680 rows, gated backward 36.9 / 38.3 / 53.0.
+    // group deep, not one list (whole lists, row tile by row tile, took 11 % longer in the second convolution at 131 072 rows, 18 % in
+    // the first at 60 000).  Few row tiles leave SMs without work; then the gated rows of a forward list go one by one, and an item
+    // takes a part of its tiles' columns, where that shortens the longest CTA by more than the estimate's error.
+    // us, replayed from a graph, 128 / 64 / 32 columns: 420 rows of lmax 2, first convolution row by row 19.8 / 15.7 / 14.6, second
+    // 8.8 / 7.3 / 6.8, its gated backward from float32 rows 29.0 / 20.1 / 17.5, radial output layer's backward 15.7 / 12.5 / 11.5; 3 000
+    // rows 32.4 / 35.8 / 56.3, 13.1 / 13.5 / 20.1, 29.8 / 20.8 / 23.7, 15.9 / 12.8 / 11.8; 7 680 rows, gated backward 36.7 / 42.1 / 54.9.
     const int64_t rows_m = (m + BM - 1) / BM;
     const Groups natural = group_tiles(list, num_tiles, rot_begin, kNatural);
     if (!natural.ok) return FCB200_EINVAL;
     // Where the input does not stay in L2, groups of one row tile that run apart read it from memory again: at 131 072 rows
     // of lmax 2 the first convolution read 1.43 times its input, the second's backward with its y rows 1.25 times; 1.18 and
-    // 1.13 times with row 0 in the group of degree 1 (972 -> 945 us, 630 -> 613; 25 000 atoms of water 117.2 -> 116.7 ms).
+    // 1.13 times with row 0 in the group of degree 1 (1019 -> 970 us on pairs, 670 -> 627; 25 000 atoms of water 117.2 -> 116.7 ms).
     const Groups joined = with_row0(list, natural);
     const bool spill = m * a_cols * 4 > (64LL << 20) && joined.ok;
     Schedule run(natural, list, rows_m, BN);
@@ -854,9 +855,9 @@ int so2_conv_fused(const void* a_hi, const void* a_lo, int64_t lda, int64_t a_co
     // On pairs a listed tile costs 0.8 of its K extent where it has a partner, and 250 for the time the tensor core waits for
     // the accumulators; alone a tile costs its K extent and 192.  So long K goes to pairs, the radial output layer (K = 128)
     // and small launches do not.  us, alone / on pairs (seconds of back-to-back launches, at the power cap): first convolution,
-    // lmax 2, 20 580 rows 201 / 179, 131 072 rows 1079 / 1000; lmax 4, 7 000 rows 235 / 217, 60 000 rows 1815 / 1638; second
-    // convolution, lmax 2, 20 580 rows 73 / 76, 131 072 rows 437 / 417; first convolution's backward, 13 000 rows 100 / 99, 131 072
-    // rows 950 / 879; radial output layer, 131 072 rows 260 / 272.
+    // lmax 2, 20 580 rows 196 / 176, 131 072 rows 1040 / 980; lmax 4, 7 000 rows 229 / 209, 60 000 rows 1796 / 1594; second
+    // convolution, lmax 2, 20 580 rows 71 / 74, 131 072 rows 435 / 410; first convolution's backward, 13 000 rows 98 / 96, 131 072
+    // rows 940 / 872; radial output layer, 131 072 rows 246 / 259.
     PairGroups two;
     if (!backward && (grouping == kPair || (grouping == kAuto && rows_m >= 8))) {  // the fewest rows: no time for the estimate
         int64_t best = grouping == kPair ? INT64_MAX / 100 : run.span;

@@ -13,10 +13,10 @@
 // Epilogue: lane = row, 32 columns at a time, for every tile of the list, so gates stay in registers; a 32 x 32 block leaves
 // through the warp's 4 KiB of shared memory as a TMA store (whole lines, rows past the end are clipped).
 //
-// What bounds it at size is the power cap: back to back launches of either form run at 985 W, so what counts is energy, and
-// half the operand traffic is what this form saves.  us and mJ a launch, alone / on pairs: first convolution, lmax 2, 131 072
-// rows 1079 / 1075, 1000 / 990; lmax 4, 60 000 rows 1815 / 1794, 1638 / 1616; second convolution, lmax 2, 131 072 rows 437 / 436,
-// 417 / 409; first convolution's backward 950 / 934, 879 / 864.
+// What bounds it at size is the power cap: back to back launches of either form run at 985 W (a us is a mJ), so what counts is
+// energy, and half the operand traffic is what this form saves.  us a launch, alone / on pairs, one board: first convolution, lmax 2,
+// 131 072 rows 1040 / 980; lmax 4, 60 000 rows 1796 / 1594; second convolution, lmax 2, 131 072 rows 435 / 410; first convolution's
+// backward 940 / 872.  (The forward kind spills 128 bytes a thread, the plain one 40.)
 #include "so2_conv.cuh"
 
 namespace fcb200 {
