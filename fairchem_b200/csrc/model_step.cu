@@ -99,7 +99,7 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
     const int64_t ec = L.ec;
     L.nets = md.num_layers + 1;
     L.rw = (int64_t)L.nets * C;
-    const bool keep = ev.want_grad != 0;
+    const bool keep = ev.want_grad != 0, planes_kept = ev.keep_radial == 1;
     // per-edge tensors that only the backward pass reads shrink to one chunk when there is none; row counts of the large
     // ones are rounded up so that a slowly changing edge count (molecular dynamics) asks for the same block every step
     int64_t unit = 1024;  // 1/64 to 1/32 of the edges
@@ -135,9 +135,9 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         q.st2 = k.take<float>(n * 2);
         q.ffn_y = k.take<float>(n * (md.lmax + d.nl) * C);
         const bool edges = keep && l >= ev.drop_layers;
-        q.yw = ev.keep_radial ? d.kw : d.yw;
+        q.yw = planes_kept ? d.kw : d.yw;
         q.y = edges ? k.take<float>(er * q.yw) : nullptr;
-        q.a = edges && ev.keep_radial ? planes(k, er, d.nm * C) : Planes{};
+        q.a = edges && planes_kept ? planes(k, er, d.nm * C) : Planes{};
         q.msg = edges ? k.take<float>(er * d.nm * C) : nullptr;
         q.rad = edges && ev.keep_radial ? k.take<float>(er * d.nrad * 2 * C) : nullptr;
     }
@@ -151,7 +151,7 @@ static void lay_out(const fcb200_model& md, const fcb200_eval& ev, bool backward
         L.radial = b.take<float>(ec * d.nrad * 2 * C);
         L.m = planes(b, ec, d.nm * 2 * C);
         const bool all = keep && ev.drop_layers <= 0;
-        if (!all || !ev.keep_radial) L.a = planes(b, ec, d.nm * C);
+        if (!all || !planes_kept) L.a = planes(b, ec, d.nm * C);
         L.y_c = all ? nullptr : b.take<float>(ec * d.gates);
         L.msg_c = all ? nullptr : b.take<float>(ec * d.nm * C);
         L.xn2 = planes(b, n, d.nl * C);

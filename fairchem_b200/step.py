@@ -367,14 +367,14 @@ class BackboneStep:
         e.chunk_node, e.chunk_edge = ctypes.addressof(graph.chunk_node), ctypes.addressof(graph.chunk_edge)
 
     def plan_memory(self) -> bool:
-        """Decide what is kept for the backward pass: everything, all but the radial weights, or, layer by layer, no conv-1
-        output and messages either.  False when not even the smallest set fits the free memory.
+        """Decide what is kept for the backward pass: everything with the gated rows as half planes (1), everything with them
+        in float32 (2), all but the radial weights (0), or, layer by layer, no conv-1 output and messages either.  False when not even the smallest set fits the free memory.
 
-        The sets that fit less give the same bits; with everything kept the gate's gradient is made from half planes, and
-        forces differ by some 2e-7 of their norm from those.  So near the limit of the first set two calls on one system
+        All but the first give the same bits; in the first the gate's gradient is made from half planes, and forces differ by
+        some 2e-7 of their norm from those.  So near the limit of the first set two calls on one system
         agree to that, not bit for bit, when other allocations come or go between them."""
         e, sizes, layers = self.ev, self.sizes, self.model.num_layers
-        for keep_radial, drop in chain(((1, 0),), ((0, n) for n in range(layers + 1))) if e.want_grad else ((0, 0),):
+        for keep_radial, drop in chain(((1, 0), (2, 0)), ((0, n) for n in range(layers + 1))) if e.want_grad else ((0, 0),):
             e.keep_radial, e.drop_layers = keep_radial, drop
             _lib.call("fcb200_model_sizes", byref(self.model), byref(e), sizes)
             need = sizes[0] + max(sizes[1], sizes[2] if e.want_grad else 0)
@@ -383,7 +383,7 @@ class BackboneStep:
             if not hasattr(self, "avail"):
                 free, self.total = torch.cuda.mem_get_info(self.device)
                 self.avail = free + self._cached()
-            # the largest kept set only with room to spare
+            # the radial weights only with room to spare
             if need * (1.15 if keep_radial else 1.0) + 0.03 * self.total < self.avail:
                 return True
         return False

@@ -594,7 +594,8 @@ typedef struct {
     int64_t num_nodes, num_edges;
     int32_t num_systems, num_chunks;
     int32_t want_grad;   /* keep what the backward pass needs */
-    int32_t keep_radial; /* also keep the radial weights (else recomputed per chunk) */
+    int32_t keep_radial; /* 0: radial weights recomputed per chunk, 2: kept, 1: kept, and the gated rows as half planes beside
+                            the gates and row 0 in place of the float32 rows (512 bytes an edge and layer more) */
     int32_t drop_layers; /* the first layers, as many, keep no conv-1 output, messages and radial weights either: the
                             backward pass computes them again per chunk */
     const float *pos, *shift, *gamma; /* [N,3]; [E,3] or null; [E] or null */

@@ -484,7 +484,7 @@ def _close_gates(bb, value):
 
 
 def _force_kept_set(monkeypatch, kept):
-    """Evaluations keep (radial weights, layers without per-edge tensors) = kept[-1]; returns what they were planned with."""
+    """Evaluations are planned with (keep_radial, drop_layers) = kept[-1]; returns what they were planned with."""
     from fairchem_b200 import step
 
     runs = []
@@ -503,8 +503,8 @@ def _force_kept_set(monkeypatch, kept):
 @pytest.mark.parametrize("chunk", [129, 700, 131072])
 @pytest.mark.parametrize("gates", [0.0, -12.0])
 def test_what_the_free_memory_decides(cfg, chunk, gates, monkeypatch):
-    """Kept sets without the radial weights differ in what is computed again, by the same kernels on the same inputs: the same
-    bits.  With them the gate's gradient is made from half planes (2.4e-7 of a term): forces to 1e-6 of the norm."""
+    """Kept sets differ in what is computed again, by the same kernels on the same inputs: the same bits, but for the first,
+    where the gate's gradient is made from half planes (2.4e-7 of a term): forces to 1e-6 of the norm."""
     from fairchem_b200 import backbone as B
     from fairchem_b200 import synthetic
 
@@ -514,7 +514,7 @@ def test_what_the_free_memory_decides(cfg, chunk, gates, monkeypatch):
     data = synthetic.merge([synthetic.fcc_cu((3, 3, 4), seed=8), synthetic.bcc_alloy((2, 2, 3), seed=9)]).to("cuda")
     kept, forces = [], []
     runs = _force_kept_set(monkeypatch, kept)
-    for k in [(1, 0), (0, 0), (0, 1), (0, len(bb.blocks))]:
+    for k in [(1, 0), (2, 0), (0, 0), (0, 1), (0, len(bb.blocks))]:
         kept.append(k)
         d = data.clone()
         forces.append(head(d, bb(d))["forces"])

@@ -194,6 +194,40 @@ def test_what_is_kept_follows_the_free_memory_layer_by_layer(cfg, monkeypatch):
     assert kept(10 ** 12)[:2] == (0, 0)
 
 
+@pytest.mark.parametrize("cfg", ["UMA_S", "ESCN_MD_L4"])
+def test_radial_weights_stay_where_only_the_planes_do_not_fit(cfg, monkeypatch):
+    """Planes cost 512 bytes an edge and layer more than float32 rows; where that is too much the rows go, not the radial weights."""
+    cfg = getattr(weights, cfg)
+    run = object.__new__(step.BackboneStep)
+    layers = (step.LayerStruct * cfg["num_layers"])()
+    run.model = m = step.ModelStruct()
+    m.lmax, m.num_layers, m.num_basis, m.layers = cfg["lmax"], cfg["num_layers"], cfg["num_distance_basis"], layers
+    run.ev = e = step.EvalStruct()
+    nodes, edges, chunks = 60_000, 1_860_000, 15
+    node, edge = ((ctypes.c_int64 * (chunks + 1))(*(n * i // chunks for i in range(chunks + 1))) for n in (nodes, edges))
+    e.num_nodes, e.num_edges, e.num_systems, e.num_chunks, e.want_grad = nodes, edges, 1, chunks, 1
+    e.chunk_node, e.chunk_edge = ctypes.addressof(node), ctypes.addressof(edge)
+    run.sizes, run.device = (ctypes.c_int64 * 3)(), torch.device("cuda", 0)
+    total = 10 ** 12
+    monkeypatch.setattr(step.BackboneStep, "_cached", lambda self: 0)
+
+    def kept(avail):
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (int(avail), total))
+        run.__dict__.pop("avail", None)
+        assert run.plan_memory()
+        return e.keep_radial, e.drop_layers, run.sizes[0] + max(run.sizes[1], run.sizes[2])
+
+    planes = kept(10 ** 13)
+    assert planes[:2] == (1, 0)
+    rows = kept(1.15 * planes[2] + 0.03 * total)  # not enough, by a byte
+    assert rows[:2] == (2, 0)
+    extra = edges * cfg["num_layers"] * 512
+    rounding = 33 / 32
+    assert 0 < planes[2] - rows[2] <= extra * rounding
+    assert kept(1.15 * rows[2] + 0.03 * total + 1)[:2] == (2, 0)
+    assert kept(1.15 * rows[2] + 0.03 * total)[:2] == (0, 0)
+
+
 class _Stream:
     def __init__(self, handle, log):
         self.cuda_stream, self.log = handle, log
